@@ -32,7 +32,9 @@
 #include <utility>
 
 #include "../../include/gint_b200.h"
+#include "gint_dispatch.h"
 #include "gint_fused.h"
+#include "gint_hot_handlers.h"
 #include "gint_opcodes.h"
 #include "gint_types.h"
 
@@ -44,12 +46,13 @@
 #else
 #define GINT_GUARD_TRIPPED
 #endif
+#define GINT_GUARD_LEAVE asm volatile("bra.uni GLEAVE; // %0" ::"n"(0) : "memory")
 #ifdef GINT_GUARD
 #define GINT_GUARD_STEP                                                                                               \
     {                                                                                                                 \
         uint32_t left;                                                                                                \
         asm volatile("sub.u32 %%gbudget, %%gbudget, 1; mov.u32 %0, %%gbudget;" : "=r"(left));                         \
-        if ((int)left < 0) { GINT_GUARD_TRIPPED; return; }                                                            \
+        if ((int)left < 0) { GINT_GUARD_TRIPPED; GINT_GUARD_LEAVE; }                                                  \
     }
 #else
 #define GINT_GUARD_STEP
@@ -532,6 +535,8 @@ template <int K, int A, int B, int KI> __device__ __forceinline__ void slot_swap
 /* ------------------------------------------------------------------------------------------------ */
 /* one instruction at one stack depth, for one of the warp's K tiles                                 */
 
+/* What handlers use besides the pool. Every handler takes its own copy from named registers right after its label
+ * (handler_context), so that nothing it computes with stems from code in front of the label. */
 struct Ctx {
     TileInfo *tiles;   // this warp's K tile descriptors (shared memory)
     int lane;
@@ -539,43 +544,45 @@ struct Ctx {
     uint32_t ring_mask; // bytes of the warp's ring of early-issued loads (4 or 8 slots of K x 512 bytes) minus 1
     uint32_t rows;     // shared-memory address of this warp's staged row blocks (tile 0); tile k is rows_stride bytes further
     uint32_t rows_stride;
-    const LaunchArgs *args;   // the launch parameters (direct mode), for the kernels that derive the four values above on demand
 };
 
 /* The widest kernels (12 slots x 2 tiles = 96 pool registers) have about a dozen registers left for everything else, and the
  * handlers with the most temporaries (runtime lane selects) spilled. They do not keep hidden / ring_mask / rows / rows_stride
- * in registers between handlers: the few handlers that need them recompute them from the launch parameters (constant bank)
+ * in registers between handlers: the few handlers that need them derive them from the block's scalars in shared memory
  * and the warp index. */
 template <int P, int K> __host__ __device__ constexpr bool lean_ctx() { return P * K >= 24; }
 
-/* shared-memory address of the first byte after the block's tile descriptors (see geval_direct_body for the layout) */
-template <int K> __device__ __forceinline__ uint32_t cx_after_tiles(const Ctx &cx, uint32_t warp)
+/* per-block scalars of the shared-memory layout (see geval_direct_body): bytes of a warp's ring, bytes per tile of the staged
+ * rows, shared-memory addresses of the rings, of the staged row blocks and of the exchange area behind them */
+enum { BS_RING_BYTES = 0, BS_ROW_BYTES, BS_RINGS, BS_ROWS, BS_AUX, BS_COUNT };
+static __shared__ uint32_t g_block[BS_COUNT];
+__device__ __forceinline__ uint32_t block_scalar(int i) { return *reinterpret_cast<volatile uint32_t *>(g_block + i); }
+__device__ __forceinline__ uint32_t warp_here()
 {
-    return (uint32_t)__cvta_generic_to_shared(cx.tiles) + ((uint32_t)kWarpsPerBlock - warp) * (uint32_t)(K * sizeof(TileInfo));
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t >> 5;
 }
+
 template <int P, int K> __device__ __forceinline__ uint32_t cx_ring_mask(const Ctx &cx)
 {
-    if constexpr (lean_ctx<P, K>()) return (uint32_t)K * cx.args->ring_bytes - 1u;
+    if constexpr (lean_ctx<P, K>()) return block_scalar(BS_RING_BYTES) - 1u;
     else return cx.ring_mask;
 }
 template <int P, int K> __device__ __forceinline__ uint32_t cx_rows_stride(const Ctx &cx)
 {
-    if constexpr (lean_ctx<P, K>()) return cx.args->row_area_bytes;
+    if constexpr (lean_ctx<P, K>()) return block_scalar(BS_ROW_BYTES);
     else return cx.rows_stride;
 }
 template <int P, int K> __device__ __forceinline__ uint32_t cx_hidden(const Ctx &cx)
 {
-    if constexpr (lean_ctx<P, K>()) {
-        const uint32_t warp = threadIdx.x >> 5;
-        return cx_after_tiles<K>(cx, warp) + warp * (uint32_t)K * cx.args->ring_bytes + (uint32_t)cx.lane * 4u;
-    } else return cx.hidden;
+    if constexpr (lean_ctx<P, K>()) return block_scalar(BS_RINGS) + warp_here() * block_scalar(BS_RING_BYTES) + (uint32_t)cx.lane * 4u;
+    else return cx.hidden;
 }
 template <int P, int K> __device__ __forceinline__ uint32_t cx_rows(const Ctx &cx)
 {
-    if constexpr (lean_ctx<P, K>()) {
-        const uint32_t warp = threadIdx.x >> 5;
-        return cx_after_tiles<K>(cx, warp) + (uint32_t)(kWarpsPerBlock * K) * cx.args->ring_bytes + warp * (uint32_t)K * cx.args->row_area_bytes;
-    } else return cx.rows;
+    if constexpr (lean_ctx<P, K>()) return block_scalar(BS_ROWS) + warp_here() * (uint32_t)K * block_scalar(BS_ROW_BYTES);
+    else return cx.rows;
 }
 
 template <int OP> struct OpInfo;
@@ -820,13 +827,12 @@ template <int K, int SLOT, int KI> __device__ __forceinline__ void take_rows(uin
     asm volatile("ld.shared.v2.b64 {%%gs%0, %%gs%1}, [%2];" ::"n"(gs<K>(SLOT, KI, 0)), "n"(gs<K>(SLOT, KI, 1)), "r"(at) : "memory");
 }
 
-/* %grf as a value (kernels built with GINT_RF). Not volatile: the register is written once, before the first handler runs, so
- * the compiler may merge the reads of the K tiles and of the members of a fused sequence. */
+/* %grf as a value (kernels built with GINT_RF) */
 __device__ __forceinline__ uint32_t rf_base()
 {
     uint32_t v = 0;
 #ifdef GINT_RF
-    asm("mov.b32 %0, %%grf;" : "=r"(v));
+    asm volatile("mov.b32 %0, %%grf;" : "=r"(v));
 #endif
     return v;
 }
@@ -964,7 +970,7 @@ __device__ __forceinline__ void exec_tile(const uint32_t operand, const Ctx &cx)
         if constexpr (OP == OP_RLoadP) {
             o0 = (operand >> 9) & 0x180u; o1 = (operand >> 11) & 0x180u; o2 = (operand >> 13) & 0x180u; o3 = (operand >> 15) & 0x180u;
         }
-        const uint32_t at = rf_base() + (operand & 0xFFFFu) * (uint32_t)K;   // (not volatile: computed once for all K tiles)
+        const uint32_t at = rf_base() + (operand & 0xFFFFu) * (uint32_t)K;
         asm volatile("{\n\t.reg .b32 t<4>;\n\t"
                      "ld.shared.b32 t0, [%2+%6];\n\tld.shared.b32 t1, [%3+%6];\n\tld.shared.b32 t2, [%4+%6];\n\tld.shared.b32 t3, [%5+%6];\n\t"
                      "mov.b64 %%gs%0, {t0, t1};\n\tmov.b64 %%gs%1, {t2, t3};\n\t}"
@@ -1089,9 +1095,7 @@ __device__ __forceinline__ void exec_all(const uint32_t operand, const Ctx &cx, 
     } else if constexpr (OP == OP_RemapVN) {
         /* top of the stack from the vector layout (lane l: elements 4l..4l+3 of the tile) to the natural one (lane l: elements
          * l, l+32, l+64, l+96): through the warp's 512-byte-per-tile exchange area (aux_bytes; after the staged row blocks) */
-        const uint32_t warp = threadIdx.x >> 5;
-        const uint32_t area = cx_after_tiles<K>(cx, warp) + (uint32_t)(kWarpsPerBlock * K) * (cx.args->ring_bytes + cx.args->row_area_bytes) +
-                              warp * (uint32_t)(K * 512);
+        const uint32_t area = block_scalar(BS_AUX) + warp_here() * (uint32_t)(K * 512);
         constexpr int T = SP - 1;
         (put_vector<K, T, KI>(area + (uint32_t)(KI * 512 + cx.lane * 16)), ...);
         __syncwarp();
@@ -1203,31 +1207,45 @@ template <int N> __device__ __forceinline__ void pool_clear()
 
 /*
  * Interpreter state that is carried from one handler to the next lives, like the pool, in named PTX registers:
- *   %gc          address of the next stream entry to fetch (shared-memory address, or a global pointer in indirect mode)
+ *   %gc          address of the next stream entry to fetch (shared-memory address)
  *   %ge0, %ge1   the current stream entry {operand of this instruction, opcode of the next one}
- *   %gkey        dispatch key for the C++ fallback switch (dead once the jump tables are in place)
+ *   %gkey        dispatch key: the first opcode; in kernels that are not threaded the key of every dispatch
  *   %gbudget     instructions left before the interpreter gives up (only with GINT_GUARD, a debugging aid)
  *   %gring       byte offset of the current slot in the warp's ring of early-issued loads
  *   %gzero       64 bits of zero that reach the kernel as a launch parameter (see fma_barrier)
  *   %grf         shared-memory address of the warp's virtual registers plus 4 * lane (kernels built with GINT_RF)
- * so no C++ value is live from handler to handler and a handler's basic block can be entered from any other handler.
+ *   %gx0 .. 5    the fields of Ctx (tiles as an offset into the dynamic shared memory)
+ * so no C++ value is live from handler to handler and a handler can be entered from any other handler.
  */
-template <bool SMEM> __device__ __forceinline__ void state_declare()
+__device__ __forceinline__ void state_declare()
 {
-#ifdef GINT_RF
-    asm volatile(".reg .b32 %%grf; // %0" ::"n"(0));
-#endif
     // (the unused "n" operand makes nvcc treat the string as a template, so that %% means %)
-    if constexpr (SMEM) asm volatile(".reg .b32 %%gc; .reg .b32 %%ge<2>; .reg .b32 %%gkey; .reg .b32 %%gbudget; .reg .b32 %%gring; .reg .b64 %%gzero; // %0" ::"n"(0));
-    else asm volatile(".reg .b64 %%gc; .reg .b32 %%ge<2>; .reg .b32 %%gkey; .reg .b32 %%gbudget; .reg .b32 %%gring; .reg .b64 %%gzero; // %0" ::"n"(0));
+    asm volatile(".reg .b32 %%gc; .reg .b32 %%ge<2>; .reg .b32 %%gkey; .reg .b32 %%gbudget; .reg .b32 %%gring; .reg .b64 %%gzero; "
+                 ".reg .b32 %%grf; .reg .b32 %%gx<6>; // %0" ::"n"(0));
+}
+
+extern __shared__ __align__(16) unsigned char g_smem[];
+
+__device__ __forceinline__ void context_set(const Ctx &cx)
+{
+    asm volatile("mov.b32 %%gx0, %0; mov.b32 %%gx1, %1; mov.b32 %%gx2, %2; mov.b32 %%gx3, %3; mov.b32 %%gx4, %4; mov.b32 %%gx5, %5;"
+                 ::"r"((uint32_t)(reinterpret_cast<unsigned char *>(cx.tiles) - g_smem)), "r"(cx.lane), "r"(cx.hidden), "r"(cx.ring_mask), "r"(cx.rows), "r"(cx.rows_stride));
+}
+__device__ __forceinline__ Ctx handler_context()
+{
+    Ctx cx;
+    uint32_t tiles;
+    asm volatile("mov.b32 %0, %%gx0; mov.b32 %1, %%gx1; mov.b32 %2, %%gx2; mov.b32 %3, %%gx3; mov.b32 %4, %%gx4; mov.b32 %5, %%gx5;"
+                 : "=r"(tiles), "=r"(cx.lane), "=r"(cx.hidden), "=r"(cx.ring_mask), "=r"(cx.rows), "=r"(cx.rows_stride));
+    cx.tiles = reinterpret_cast<TileInfo *>(g_smem + tiles);
+    return cx;
 }
 
 /* read the current entry, then start loading the following one */
-template <bool SMEM> __device__ __forceinline__ void state_advance(uint32_t &operand, uint32_t &next_opcode)
+__device__ __forceinline__ void state_advance(uint32_t &operand, uint32_t &next_opcode)
 {
     asm volatile("mov.b32 %0, %%ge0; mov.b32 %1, %%ge1;" : "=r"(operand), "=r"(next_opcode));
-    if constexpr (SMEM) asm volatile("ld.shared.v2.u32 {%%ge0, %%ge1}, [%%gc]; add.u32 %%gc, %%gc, 8; // %0" ::"n"(0) : "memory");
-    else asm volatile("ld.global.nc.v2.u32 {%%ge0, %%ge1}, [%%gc]; add.u64 %%gc, %%gc, 8; // %0" ::"n"(0) : "memory");
+    asm volatile("ld.shared.v2.u32 {%%ge0, %%ge1}, [%%gc]; add.u32 %%gc, %%gc, 8; // %0" ::"n"(0) : "memory");
 }
 
 /*
@@ -1238,13 +1256,19 @@ template <bool SMEM> __device__ __forceinline__ void state_advance(uint32_t &ope
  * dispatch, so there is one indirect branch per interpreted instruction and the jump-table lookup for the next handler can
  * be issued before the current handler's payload.
  *
- * The marker comments survive into the PTX. nvcc lowers a C++ switch to a compare tree (about ten dependent branches for
- * this many cases) and never emits an indirect branch; the build step gint_b200/ptx_dispatch.py ends every handler with
- * one `brx.idx` jump-table branch, indexed by the opcode into the table of that handler's next stack depth and targeting
- * the blocks that carry TARGET markers. Without that step the code below is still a correct (slower) interpreter: every
- * handler loops back to the switch. With THREADED = false only the loop-top dispatch becomes a jump table (over all
- * (depth, opcode) keys) and handlers branch back to it: one more branch per instruction, but a control-flow graph that
- * ptxas digests in seconds whatever surrounds the interpreter.
+ * nvcc lowers a dense C++ switch to a compare tree (about ten dependent branches for this many cases). The dispatch is
+ * therefore written in PTX: a handler starts with its own label GL<depth>_<opcode> and ends with one `brx.idx`, indexed by
+ * the next opcode into the table of the handler's next stack depth (GT<depth>, gint_dispatch.h). The C++ switch around the
+ * handlers is only what makes all of them reachable for the compiler; control never comes back to it. What makes that sound:
+ *   - the state that handlers share lives in named registers that only inline assembly touches, so the compiler has no value
+ *     to carry from one handler to another;
+ *   - behind its label a handler computes with operands, descriptors and context that it read from those registers there
+ *     (volatile, hence after the label); what it writes to memory is written before its brx (memory clobber);
+ *   - an asm statement that the compiler duplicated would define a label twice, which the assembler refuses.
+ * A (depth, opcode) pair without a handler has its label in the default block, which ends the program.
+ * Threaded dispatch gives each handler a branch of its own. Kernels that are not THREADED branch back to one dispatch over
+ * all (depth, opcode) keys: one more branch per instruction, but a control-flow graph that ptxas digests in seconds whatever
+ * surrounds the interpreter.
  */
 /* A fused handler covers n consecutive instructions but only m = S::entries() stream entries (see SeqFetch). On entry %ge
  * holds the first of them, {operand of the first member, opcode after the sequence if m == 1}, and %gc points at the
@@ -1256,7 +1280,7 @@ __device__ __forceinline__ void run_fused(const Ctx &cx, uint32_t &next_opcode)
     constexpr int m = S::entries();
     uint32_t ops[GINT_MAX_FUSED_LEN];
     if constexpr (m == 1) {
-        state_advance<true>(ops[0], next_opcode);
+        state_advance(ops[0], next_opcode);
     } else {
         uint32_t base;
         asm volatile("mov.b32 %0, %%ge0; mov.b32 %1, %%gc;" : "=r"(ops[0]), "=r"(base));
@@ -1267,71 +1291,139 @@ __device__ __forceinline__ void run_fused(const Ctx &cx, uint32_t &next_opcode)
     {
         uint32_t left;
         asm volatile("sub.u32 %%gbudget, %%gbudget, %1; mov.u32 %0, %%gbudget;" : "=r"(left) : "n"(S::n));
-        if ((int)left < 0) { GINT_GUARD_TRIPPED; return; }
+        if ((int)left < 0) { GINT_GUARD_TRIPPED; GINT_GUARD_LEAVE; }
     }
 #endif
     SeqRun<S, SP, P, K, 0>::run(cx, ops);
 }
 
-template <int P, int K, bool SMEM_CODE, bool THREADED>
-__device__ __forceinline__ void interpret(const uint2 *code, uint32_t n_entries, const Ctx &cx)
+/* Order of the handlers in the code. A kernel holds one handler per (opcode, depth), 2 to 6 MB of machine code, of which any
+ * one program runs a few dozen; in plain key order the few-instruction handlers that a program jumps between lie scattered
+ * between tile accesses and inlined math routines of kilobytes each. The handlers that recorded programs run come first
+ * (gint_hot_handlers.h, written by the build from hot_handlers.json), then the other short ones, then the long ones. */
+#if defined(GINT_RF)
+#define GINT_HOT_LIST GINT_HOT_RF
+#elif defined(GINT_VEC)
+#define GINT_HOT_LIST GINT_HOT_VEC
+#else
+#define GINT_HOT_LIST GINT_HOT_PLAIN
+#endif
+struct HotTable {
+    bool hot[(GINT_MAX_STACK + 1) * GINT_N_TABLE];
+    constexpr HotTable() : hot()
+    {
+#define GINT_X_HOT(num, sp) hot[(sp) * GINT_N_TABLE + (num)] = true;
+        GINT_HOT_LIST(GINT_X_HOT)
+#undef GINT_X_HOT
+    }
+};
+template <int OP> __host__ __device__ constexpr bool long_handler()
+{
+    if constexpr (GINT_IS_FUSED(OP)) return true;
+    else return MemOp<OP>::is || is_scalar_binary<OP>() || is_scalar_unary<OP>() || (OP >= OP_WarpAllReduceSum && OP <= OP_WarpAllReduceProd) ||
+                OP == OP_LoadGlobal1DF32Indirect || OP == OP_StoreGlobal1DF32Indirect || OP == OP_PfIssue1D || OP == OP_PfTakeIssue1D || OP == OP_StageRows;
+}
+enum { RANK_HOT = 0, RANK_SHORT, RANK_LONG };
+template <int OP, int SP> __host__ __device__ constexpr int handler_rank()
+{
+    constexpr HotTable t;
+    if constexpr (t.hot[SP * GINT_N_TABLE + OP]) return RANK_HOT;
+    else return long_handler<OP>() ? RANK_LONG : RANK_SHORT;
+}
+
+template <int NUM, int SP, int P, int K, bool THREADED> __device__ __forceinline__ void handler()
+{
+    constexpr int next_depth = SP + OpInfo<NUM>::net_effect;
+    uint32_t operand, opc;
+    const Ctx cx = handler_context();
+    if constexpr (GINT_IS_FUSED(NUM)) {
+        run_fused<NUM, SP, P, K>(cx, opc);
+    } else {
+        state_advance(operand, opc);
+        GINT_GUARD_STEP
+        exec_all<NUM, SP, P, K>(operand, cx, std::make_integer_sequence<int, K>());
+    }
+    if constexpr (THREADED) asm volatile("brx.idx.uni %0, GT%1; // %2 %3" ::"r"(opc), "n"(next_depth), "n"(SP), "n"(NUM) : "memory");
+    else asm volatile("add.u32 %%gkey, %0, %1;\n\tbra.uni GTOP; // %2 %3" ::"r"(opc), "n"(next_depth * GINT_N_TABLE), "n"(SP), "n"(NUM) : "memory");
+}
+
+/* labels of the (depth, opcode) pairs that have no handler in this kernel */
+template <int P, int K, int KEY> __device__ __forceinline__ void missing_label()
+{
+    constexpr int sp = KEY / GINT_N_TABLE, num = KEY % GINT_N_TABLE;
+    constexpr bool known = num < GINT_FUSED_FIRST + GINT_N_FUSED
+#ifdef GINT_RF
+                           || (num >= GINT_N_DISPATCH_PLAIN && num < GINT_N_DISPATCH_RF)
+#elif defined(GINT_VEC)
+                           || num == OP_RemapVN
+#endif
+        ;
+    if constexpr (!known) asm volatile("GL%0_%1:" ::"n"(sp), "n"(num) : "memory");
+    else if constexpr (!op_valid<num, sp, P, K>()) asm volatile("GL%0_%1:" ::"n"(sp), "n"(num) : "memory");
+}
+template <int P, int K, int... KEY> __device__ __forceinline__ void missing_labels(std::integer_sequence<int, KEY...>)
+{
+    (missing_label<P, K, KEY>(), ...);
+}
+
+template <int P, int K, bool THREADED>
+__device__ __forceinline__ void interpret(const uint2 *code, uint32_t n_entries)
 {
     pool_clear<2 * P * K>();
-    if constexpr (SMEM_CODE) {
-        const uint32_t a = (uint32_t)__cvta_generic_to_shared(code);
-        asm volatile("ld.shared.u32 %%gkey, [%0+4]; ld.shared.v2.u32 {%%ge0, %%ge1}, [%0+8]; add.u32 %%gc, %0, 16; mov.u32 %%gbudget, %1; mov.u32 %%gring, 0;"
-                     ::"r"(a), "r"(n_entries) : "memory");
-    } else {
-        asm volatile("ld.global.nc.u32 %%gkey, [%0+4]; ld.global.nc.v2.u32 {%%ge0, %%ge1}, [%0+8]; add.u64 %%gc, %0, 16; mov.u32 %%gbudget, %1; mov.u32 %%gring, 0;"
-                     ::"l"(code), "r"(n_entries) : "memory");
-    }
+    asm volatile("ld.shared.u32 %%gkey, [%0+4]; ld.shared.v2.u32 {%%ge0, %%ge1}, [%0+8]; add.u32 %%gc, %0, 16; mov.u32 %%gbudget, %1; mov.u32 %%gring, 0;"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(code)), "r"(n_entries) : "memory");
+    if constexpr (THREADED) asm volatile(GINT_BRANCH_TABLES "// %0" ::"n"(0));
+    else asm volatile(GINT_BRANCH_TABLE_ALL "// %0" ::"n"(0));
     for (;;) {
         uint32_t key;
-        asm volatile("mov.b32 %0, %%gkey;" : "=r"(key));
-        if constexpr (THREADED) asm volatile("// GINT_DISPATCH %0 site entry depth 0;" ::"r"(key));
-        else asm volatile("// GINT_DISPATCH %0 site entry depth all;" ::"r"(key));
+        if constexpr (THREADED) asm volatile("mov.b32 %0, %%gkey;\n\tbrx.idx.uni %%gkey, GT0;" : "=r"(key) :: "memory");
+        else asm volatile("GTOP:\n\tmov.b32 %0, %%gkey;\n\tbrx.idx.uni %%gkey, GTALL;" : "=r"(key) :: "memory");
         switch (key) {
-#define GINT_CASE_SP(num, spv)                                                                          \
-    case (spv) * GINT_N_DISPATCH + (num):                                                                \
-        if constexpr (op_valid<num, spv, P, K>()) {                                                     \
-            asm volatile("// GINT_TARGET %0;" ::"n"((spv) * GINT_N_DISPATCH + (num)));                   \
+#define GINT_CASE(num, spv, rank)                                                                       \
+    case (rank) * GINT_N_KEYS + (spv) * GINT_N_TABLE + (num):                                            \
+        if constexpr (op_valid<num, spv, P, K>() && handler_rank<num, spv>() == (rank)) {                \
+            asm volatile("GL%0_%1:" ::"n"(spv), "n"(num) : "memory");                                    \
             if constexpr ((num) == OP_Halt) return;                                                     \
-            else {                                                                                      \
-                constexpr int next_depth = (spv) + OpInfo<num>::net_effect;                             \
-                uint32_t operand, opc;                                                                  \
-                if constexpr (GINT_IS_FUSED(num)) {                                                     \
-                    run_fused<num, spv, P, K>(cx, opc);                                                 \
-                } else {                                                                                \
-                    state_advance<SMEM_CODE>(operand, opc);                                             \
-                    GINT_GUARD_STEP                                                                     \
-                    exec_all<num, spv, P, K>(operand, cx, std::make_integer_sequence<int, K>());        \
-                }                                                                                       \
-                asm volatile("add.u32 %%gkey, %0, %1;" ::"r"(opc), "n"(next_depth * GINT_N_DISPATCH));   \
-                if constexpr (THREADED)                                                                 \
-                    asm volatile("// GINT_DISPATCH %0 site %1 depth %2;" ::"r"(opc),                     \
-                                 "n"((spv) * GINT_N_DISPATCH + (num)), "n"(next_depth));                 \
-            }                                                                                           \
+            else handler<num, spv, P, K, THREADED>();                                                   \
         }                                                                                               \
         continue;
-#define GINT_X_CASES(name, num, md, net)                                                                           \
-    GINT_CASE_SP(num, 0) GINT_CASE_SP(num, 1) GINT_CASE_SP(num, 2) GINT_CASE_SP(num, 3) GINT_CASE_SP(num, 4)       \
-    GINT_CASE_SP(num, 5) GINT_CASE_SP(num, 6) GINT_CASE_SP(num, 7) GINT_CASE_SP(num, 8)
-            GINT_OPCODE_LIST(GINT_X_CASES)
-            GINT_INTERNAL_OPCODE_LIST(GINT_X_CASES)
-#define GINT_X_FCASES(num, len, ...) GINT_X_CASES(fused, num, 0, 0)
-            GINT_FUSED_LIST(GINT_X_FCASES)
+#define GINT_CASES(num, rank)                                                                                          \
+    GINT_CASE(num, 0, rank) GINT_CASE(num, 1, rank) GINT_CASE(num, 2, rank) GINT_CASE(num, 3, rank) GINT_CASE(num, 4, rank) \
+    GINT_CASE(num, 5, rank) GINT_CASE(num, 6, rank) GINT_CASE(num, 7, rank) GINT_CASE(num, 8, rank)
+#define GINT_X_HOT(num, sp) GINT_CASE(num, sp, RANK_HOT)
+            GINT_HOT_LIST(GINT_X_HOT)
+#undef GINT_X_HOT
+#define GINT_X_SHORT(name, num, md, net) GINT_CASES(num, RANK_SHORT)
+#define GINT_X_LONG(name, num, md, net) GINT_CASES(num, RANK_LONG)
+#define GINT_X_FUSED(num, len, ...) GINT_CASES(num, RANK_LONG)
 #ifdef GINT_RF
-            GINT_RF_OPCODE_LIST(GINT_X_CASES)
-            GINT_RF_FUSED_LIST(GINT_X_FCASES)
+#define GINT_X_OWN(X) GINT_RF_OPCODE_LIST(X)
+            GINT_RF_FUSED_LIST(GINT_X_FUSED)
+#elif defined(GINT_VEC)
+#define GINT_X_OWN(X) GINT_VEC_OPCODE_LIST(X)
+#else
+#define GINT_X_OWN(X)
 #endif
-#ifdef GINT_VEC
-            GINT_VEC_OPCODE_LIST(GINT_X_CASES)
+            GINT_OPCODE_LIST(GINT_X_SHORT)
+            GINT_INTERNAL_OPCODE_LIST(GINT_X_SHORT)
+            GINT_X_OWN(GINT_X_SHORT)
+            GINT_FUSED_LIST(GINT_X_FUSED)
+            GINT_OPCODE_LIST(GINT_X_LONG)
+            GINT_INTERNAL_OPCODE_LIST(GINT_X_LONG)
+            GINT_X_OWN(GINT_X_LONG)
+#undef GINT_X_OWN
+#undef GINT_X_FUSED
+#undef GINT_X_LONG
+#undef GINT_X_SHORT
+#undef GINT_CASES
+#undef GINT_CASE
+#ifdef GINT_GUARD
+        case 3 * GINT_N_KEYS:
+            asm volatile("GLEAVE: // %0" ::"n"(0) : "memory");
+            return;
 #endif
-#undef GINT_X_FCASES
-#undef GINT_X_CASES
-#undef GINT_CASE_SP
         default:
-            asm volatile("// GINT_TARGET default;");
+            missing_labels<P, K>(std::make_integer_sequence<int, GINT_N_KEYS>());
 #ifdef GINT_CHECKED
             chk_record(GINT_DEVICE_BAD_DISPATCH, -1, (u64)key);
 #endif
@@ -1395,9 +1487,9 @@ static __device__ __noinline__ void stage_for_warp(uint2 *code_s, const uint2 *c
 template <int P, int K, bool THREADED = true>
 __device__ __forceinline__ void geval_direct_body(const LaunchArgs &a)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char *const smem = g_smem;
     pool_declare<P, K>();
-    state_declare<true>();
+    state_declare();
     asm volatile("mov.b64 %%gzero, %0;" ::"l"((u64)a.zero));
     uint2 *code_s = reinterpret_cast<uint2 *>(smem);
     gint_tensor_info *ti_s = reinterpret_cast<gint_tensor_info *>(smem + a.code_smem_bytes);
@@ -1415,6 +1507,17 @@ __device__ __forceinline__ void geval_direct_body(const LaunchArgs &a)
         int *dst = reinterpret_cast<int *>(ti_s);
         for (uint32_t i = threadIdx.x; i < sizeof(gint_tensor_info) / 4; i += kThreadsPerBlock) dst[i] = src[i];
     }
+#ifndef GINT_VEC
+    if constexpr (lean_ctx<P, K>())
+#endif
+    if (threadIdx.x == 0) {
+        const uint32_t rings = (uint32_t)__cvta_generic_to_shared(tiles_s + kWarpsPerBlock * K);
+        g_block[BS_RING_BYTES] = (uint32_t)K * a.ring_bytes;
+        g_block[BS_ROW_BYTES] = a.row_area_bytes;
+        g_block[BS_RINGS] = rings;
+        g_block[BS_ROWS] = rings + (uint32_t)(kWarpsPerBlock * K) * a.ring_bytes;
+        g_block[BS_AUX] = rings + (uint32_t)(kWarpsPerBlock * K) * (a.ring_bytes + a.row_area_bytes);
+    }
 #ifdef GINT_CHECKED
     if (threadIdx.x < GINT_MAX_TENSORS) {
         g_chk.lo[threadIdx.x] = a.chk_lo[threadIdx.x];
@@ -1431,8 +1534,7 @@ __device__ __forceinline__ void geval_direct_body(const LaunchArgs &a)
     Ctx cx;
     cx.tiles = tiles_s + warp * K;
     cx.lane = lane;
-    cx.args = &a;
-    if constexpr (!lean_ctx<P, K>()) {   // after the tile descriptors: the ring of early-issued loads (ring_bytes per tile), then the staged row blocks
+    {   // after the tile descriptors: the ring of early-issued loads (ring_bytes per tile), then the staged row blocks
         unsigned char *after = reinterpret_cast<unsigned char *>(tiles_s + kWarpsPerBlock * K);
 #ifdef GINT_VEC
         cx.hidden = (uint32_t)__cvta_generic_to_shared(after + (size_t)(warp * K) * a.ring_bytes + lane * 16);   // lane l owns elements 4l..4l+3
@@ -1443,6 +1545,7 @@ __device__ __forceinline__ void geval_direct_body(const LaunchArgs &a)
         cx.rows_stride = a.row_area_bytes;
         cx.ring_mask = (uint32_t)K * a.ring_bytes - 1u;
     }
+    context_set(cx);
 #ifdef GINT_RF
     {   /* after the staged row blocks: the virtual registers, rf_bytes (512 per register) per tile */
         unsigned char *after = reinterpret_cast<unsigned char *>(tiles_s + kWarpsPerBlock * K);
@@ -1461,12 +1564,8 @@ __device__ __forceinline__ void geval_direct_body(const LaunchArgs &a)
         if (lane == 0) g_chk.logical[warp] = a.first + g * (uint32_t)K;
         __syncwarp();
 #endif
-#ifdef GINT_CHECKED
-        /* the instruction budget: a stream entry stands for at most GINT_MAX_FUSED_LEN instructions (a fused handler) */
-        interpret<P, K, true, THREADED>(code_s, a.n_slots * (uint32_t)GINT_MAX_FUSED_LEN, cx);
-#else
-        interpret<P, K, true, THREADED>(code_s, a.n_slots, cx);
-#endif
+        /* (the instruction budget of GINT_GUARD: a stream entry stands for at most GINT_MAX_FUSED_LEN instructions) */
+        interpret<P, K, THREADED>(code_s, a.n_slots * (uint32_t)GINT_MAX_FUSED_LEN);
     }
 }
 
@@ -1476,9 +1575,9 @@ __device__ __forceinline__ void geval_direct_body(const LaunchArgs &a)
 template <int P>
 __device__ __forceinline__ void geval_indirect_body(const IndirectArgs &a)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char *const smem = g_smem;
     pool_declare<P, 1>();
-    state_declare<true>();
+    state_declare();
     asm volatile("mov.b64 %%gzero, %0;" ::"l"((u64)a.reserved));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char *mine = smem + (size_t)warp * (sizeof(TileInfo) + kTensorInfoSmemBytes + a.code_smem_bytes);
@@ -1491,7 +1590,7 @@ __device__ __forceinline__ void geval_indirect_body(const IndirectArgs &a)
     cx.rows = 0;
     cx.rows_stride = 0;
     cx.ring_mask = 0;
-    cx.args = nullptr;
+    context_set(cx);
     for (uint32_t g = blockIdx.x * kWarpsPerBlock + warp; g < a.grid_dim; g += gridDim.x * kWarpsPerBlock) {
         const IndirectEntry e = a.table[g];
         __syncwarp();  // every lane is done with the previous program's code and descriptors
@@ -1502,7 +1601,7 @@ __device__ __forceinline__ void geval_indirect_body(const IndirectArgs &a)
             __syncwarp();
         }
         decode_tiles<1>(ti_s, (int)a.n_tensors, g, a.grid_dim, cx.tiles, lane);
-        interpret<P, 1, true, false>(code_s, e.n_slots, cx);
+        interpret<P, 1, false>(code_s, e.n_slots);
     }
 }
 

@@ -16,7 +16,6 @@ typedef unsigned long long u64;
 constexpr int kWarpsPerBlock = 4;
 constexpr int kThreadsPerBlock = kWarpsPerBlock * 32;
 constexpr int kTensorInfoSmemBytes = 640;  // 608-byte descriptor block, padded to a 128-byte multiple
-constexpr int kNumKeys = (GINT_MAX_STACK + 1) * GINT_N_DISPATCH;
 
 /* Slots of the ring of early-issued loads: how many tile loads per logical program are in flight ahead of their use. The
  * host chooses per program: 8 for programs that stream long rows (many loads, mostly memory instructions), 4 otherwise. */

@@ -1,9 +1,8 @@
 /*
  * gint_variants.h -- the interpreter kernels shipped inside libgint_b200.so.
  *
- * Each (pool size P, tiles per warp K) pair is compiled separately (gint_b200/csrc/kernels/), its dispatch switch is
- * turned into a jump table at the PTX level (gint_b200/ptx_dispatch.py), and the resulting sm_100a cubin is embedded in
- * the library as a byte array. The host loads the arrays with cudaLibraryLoadData and looks the kernels up by name.
+ * Each (pool size P, tiles per warp K) pair is compiled separately (gint_b200/csrc/kernels/) and the resulting sm_100a cubin
+ * is embedded in the library as a byte array. The host loads the arrays with cudaLibraryLoadData and looks the kernels up by name.
  */
 #ifndef GINT_VARIANTS_H
 #define GINT_VARIANTS_H

@@ -5,7 +5,7 @@
 The interpreter kernels hold one handler per (opcode, stack depth): well over a thousand blocks of code, of which any one
 program runs a few dozen. Which ones are run is far from uniform -- frontend- and conductor-generated programs live at small
 stack depths and use a few dozen opcodes -- and the instruction cache works best when the handlers a program jumps between lie
-close together. The build step (``gint_b200/ptx_dispatch.py``) therefore emits the handlers listed here first, next to each
+close together. The kernels' dispatch switch (``csrc/gint_interp.cuh``) therefore has the handlers listed here first, next to each
 other, before all others: a profile-guided layout, with the recorded programs of ``gint_b200/data/programs.json`` (streams
 recorded from the reference's frontend, small-matrix helpers and torch.compile backend at many sizes) as the profile.
 
