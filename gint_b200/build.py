@@ -31,7 +31,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libgint_b200.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-lineinfo", "-O3", "-std=c++17",
-          "-fmad=false"]   # the bytecode's FMul/FAdd must stay separate roundings; FMA is its own opcode
+          "-fmad=false", "--diag-suppress", "20013"]   # the bytecode's FMul/FAdd must stay separate roundings; FMA is its own opcode
 
 
 def _nvcc() -> str:

@@ -631,8 +631,8 @@ bool vec_is_commutative(int op) { return op == OP_FAdd || op == OP_FMul || op ==
 
 /* `prog`: the early-issue stream after the fast-access pass, before lowering and fusion. On success `out` is the stream for the
  * vector-layout kernels (RemapVN inserted) and the counts say how much it is worth. */
-bool vec_transform(const std::vector<Insn> &prog, std::vector<Insn> *out, int *n_vector_accesses, int *n_remaps)
-{
+bool vec_transform(const std::vector<Insn> &prog, std::vector<Insn> *out, int *n_vector_accesses, int *n_remaps, bool widths_stay = false)
+{   // widths_stay: the layouts differ in which lane has an element, not in its width value (2DT tiles): a lane-uniform value mixes with both
     SymbolTable st;
     std::vector<LaneValue> stack;
     LaneValue regs[8];
@@ -641,11 +641,11 @@ bool vec_transform(const std::vector<Insn> &prog, std::vector<Insn> *out, int *n
     out->clear();
     *n_vector_accesses = 0;
     *n_remaps = 0;
-    auto join = [](const LaneValue &a, const LaneValue &b, LaneValue::Kind *k) {   // layout of an element-wise result; false: they clash
+    auto join = [widths_stay](const LaneValue &a, const LaneValue &b, LaneValue::Kind *k) {   // layout of an element-wise result; false: they clash
         if (a.kind == LaneValue::W && b.kind == LaneValue::W) { *k = LaneValue::W; return true; }
         const LaneValue &data = a.kind != LaneValue::W ? a : b, &other = a.kind != LaneValue::W ? b : a;
         if (other.kind == LaneValue::W) {
-            if (data.kind == LaneValue::V && !other.uniform()) return false;   // width w means other elements in the two layouts
+            if (data.kind == LaneValue::V && !widths_stay && !other.uniform()) return false;   // width w means other elements in the two layouts
             *k = data.kind;
             return true;
         }
@@ -836,6 +836,12 @@ uint64_t tensor_extent_bytes(const gint_tensor_info &ti, int t)
     return (uint64_t)elems * (uint64_t)(ti.elm_size[t] > 4 ? ti.elm_size[t] : 4);
 }
 
+}  // namespace
+
+#include "gint_wide_host.h"
+
+namespace {
+
 struct Variant {
     int P, K;
     const void *fn;   // cudaKernel_t of the loaded cubin, usable wherever the runtime takes a kernel function
@@ -844,6 +850,7 @@ struct Variant {
     int resident_warps;   // warps of this kernel the whole device holds when a block needs only its minimum of shared memory
     bool rf = false;      // virtual registers in shared memory (pool = operand stack only)
     bool vec = false;     // 1-D tiles in the vector layout
+    int wide = 0;         // streaming kernel (K tiles of a loop body at a time): 1 natural, 2 vector layout
 };
 
 /* The embedded cubins are loaded once per process (a cudaLibrary_t is not tied to a device or context). */
@@ -857,6 +864,7 @@ struct KernelImage {
     bool loaded;
     bool rf;
     bool vec = false;
+    int wide = 0;
 };
 
 KernelImage g_images[] = {
@@ -868,6 +876,12 @@ KernelImage g_images[] = {
 #undef GINT_X_IMG
 #define GINT_X_IMG(P, K) {gint_cubin_vec_##P##_##K, gint_cubin_vec_##P##_##K##_end, "gint_geval_vec_" #P "_" #K, P, K, nullptr, nullptr, false, false, true},
     GINT_VEC_VARIANTS(GINT_X_IMG)
+#undef GINT_X_IMG
+#define GINT_X_IMG(P, K) {gint_cubin_wide_##P##_##K, gint_cubin_wide_##P##_##K##_end, "gint_geval_wide_" #P "_" #K, P, K, nullptr, nullptr, false, false, false, 1},
+    GINT_WIDE_VARIANTS(GINT_X_IMG)
+#undef GINT_X_IMG
+#define GINT_X_IMG(P, K) {gint_cubin_widev_##P##_##K, gint_cubin_widev_##P##_##K##_end, "gint_geval_widev_" #P "_" #K, P, K, nullptr, nullptr, false, false, false, 2},
+    GINT_WIDEV_VARIANTS(GINT_X_IMG)
 #undef GINT_X_IMG
 #define GINT_X_IMG(P) {gint_cubin_indirect_##P, gint_cubin_indirect_##P##_end, "gint_geval_indirect_" #P, P, 0, nullptr, nullptr, false, false},
     GINT_INDIRECT_VARIANTS(GINT_X_IMG)
@@ -905,6 +919,7 @@ struct Geometry {
     uint32_t code_smem;
     int blocks_per_sm;
     uint32_t grid;
+    uint32_t threads;
 };
 
 struct PlanMemo { bool valid; uint32_t count; int opt_k, opt_blocks; Geometry g; };
@@ -947,7 +962,22 @@ struct Program {
     uint32_t vec_slots = 0;
     int vec_remaps = 0;
     uint2 vec_inline[gint::kInlineCodeSlots];
-    PlanMemo memo[4] = {};      // last launch plan of the plain stream [0], the early-issue stream [1], the RF stream [2], the vector-layout stream [3]
+    /* the stream for the streaming kernels (wide_slots == 0: none), see gint_wide_host.h */
+    uint2 *wide_dev = nullptr;
+    uint32_t wide_slots = 0;
+    int wide_depth = 0, wide_tiles = 0;
+    uint32_t flat_tiles = 0, flat_grid = 0;
+    uint8_t wide_alias[GINT_MAX_TENSORS] = {};
+    uint64_t wide_extent[GINT_MAX_TENSORS] = {};
+    uint32_t wide_align[GINT_MAX_TENSORS] = {};   // alignment of the base pointers that the vector-layout kernels need (minus 1); all 0: never
+    bool wide_vector = false;
+    /* Rows of f32 in the 1-D layout: where they are aligned the tile kernels' 16-byte early-issued copies are as fast or faster (RMSNorm
+     * 16384 x 4096: 125 us there, 121 us here; row sums of 65536 x 1024: 50 against 75), so only unaligned rows come here
+     * (10007 x 2029: 77 us there, 55 here). */
+    bool wide_rows_f32 = false;
+    uint32_t wide_rows = 0;     // slots of which every logical program has its own part
+    uint2 wide_inline[gint::kInlineCodeSlots];
+    PlanMemo memo[6] = {};      // last launch plan of the plain stream [0], the early-issue stream [1], the RF stream [2], the vector-layout stream [3], the streaming kernels in the natural [4] and the vector layout [5]
     std::mutex memo_mu;
 };
 
@@ -1006,6 +1036,7 @@ struct gint_ctx {
     int opt_lower = 1;          // DupBroadcastW -> Bcast_k (lower_lane_moves); applies to programs created afterwards
     int opt_rf = 1;             // launches use a program's RF stream (virtual registers in shared memory) when it has one
     int opt_rf_create = 1;      // programs created from now on get an RF stream when they qualify
+    int opt_wide = 1;           // launches use a program's stream with loops (streaming kernels) when it has one
     int opt_vec = 0;            // vector-layout stream and kernels for the programs that qualify (creation and launch). Off unless asked
                                 // for: measured on the conductor graph, the fused program alone gains 2-3 % (175 -> 169 us) but the whole
                                 // graph through the benchmark's plan loses 1-2 % (340 -> 345 us)
@@ -1055,7 +1086,7 @@ Program *lookup(gint_ctx *ctx, uint64_t handle)
 Variant *find_variant(gint_ctx *ctx, int P, int K, bool rf = false, bool vec = false)
 {
     for (auto &v : ctx->direct)
-        if (v.P == P && v.K == K && v.rf == rf && v.vec == vec && v.ok) return &v;
+        if (v.P == P && v.K == K && v.rf == rf && v.vec == vec && !v.wide && v.ok) return &v;
     return nullptr;
 }
 
@@ -1173,6 +1204,40 @@ int plan_direct(gint_ctx *ctx, const Program *p, const StreamView &sv, uint32_t 
     return GINT_OK;
 }
 
+constexpr uint64_t kFlatMinTiles = 16384;
+
+/* A launch runs on the streaming kernels if the program has a stream for them and the caller has not asked for a particular
+ * configuration of the tile kernels. */
+bool use_wide(const gint_ctx *ctx, const Program *p)
+{
+    return p->wide_slots != 0 && ctx->opt_wide && ctx->opt_early_issue && ctx->opt_tiles_per_warp == 0 && !ctx->opt_prefetch && !(ctx->opt_vec && p->vec_dev);
+}
+
+int plan_wide(gint_ctx *ctx, const Program *p, bool vector, uint32_t count, Geometry *g)
+{
+    /* the kernel with the most tiles at a time whose slots hold the program and whose tiles the loops fill */
+    Variant *v = nullptr;
+    for (auto &c : ctx->direct)
+        if (c.wide == (vector ? 2 : 1) && c.ok && c.P >= p->wide_depth && (!v || (p->flat_tiles || p->wide_tiles >= 8 ? c.K > v->K : c.K < v->K))) v = &c;
+    if (!v) return fail(ctx, GINT_ERR_TOO_LARGE, "no streaming kernel fits this program");
+    const uint64_t groups = p->flat_tiles ? ((uint64_t)count * p->flat_tiles + (uint64_t)v->K - 1) / (uint64_t)v->K : count;
+    /* few groups: blocks of one warp, so that every group has an SM's memory path to itself */
+    const uint32_t warps = groups <= 4ull * (uint64_t)ctx->num_sms ? 1u : (uint32_t)gint::kWarpsPerBlock;
+    g->v = v;
+    g->threads = warps * 32u;
+    g->code_smem = (p->wide_slots * 8u + 127u) & ~127u;
+    g->smem = g->code_smem + gint::kTensorInfoSmemBytes + warps * ((uint32_t)sizeof(gint::TileInfo) + (vector ? 512u : 0u));
+    int bps = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, v->fn, (int)g->threads, g->smem);
+    if (e != cudaSuccess || bps < 1) { cudaGetLastError(); return fail(ctx, GINT_ERR_CUDA, "occupancy query (streaming kernel)", e); }
+    g->blocks_per_sm = bps;
+    uint64_t resident = (uint64_t)bps * (uint64_t)ctx->num_sms;
+    if (ctx->opt_max_blocks > 0 && (uint64_t)ctx->opt_max_blocks < resident) resident = (uint64_t)ctx->opt_max_blocks;
+    const uint64_t blocks = (groups + warps - 1) / warps;
+    g->grid = (uint32_t)(blocks < resident ? blocks : resident);
+    return GINT_OK;
+}
+
 struct GatherArgs {
     uint32_t mask;            // tensor slots whose innermost batch index goes through the row index
     const long long *index;   // device pointer
@@ -1192,17 +1257,60 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
     DeviceGuard guard(ctx->device);
     /* The early-issue stream is used unless a tensor whose loads were moved across stores overlaps, at this launch's
      * addresses, one of the tensors those stores write. */
-    bool early = ctx->opt_early_issue && p->early_dev != nullptr;
-    for (int t = 0; early && t < n_tensors; t++) {
-        if (!p->alias_slots[t]) continue;
-        for (int b = 0; early && b < n_tensors; b++) {
-            if (!((p->alias_slots[t] >> b) & 1u)) continue;
-            const bool ga = gather && ((gather->mask >> t) & 1u), gb = gather && ((gather->mask >> b) & 1u);
-            const uint64_t a0 = base_ptrs[t], a1 = a0 + (ga ? gather->extent_bytes : p->extent[t]);
-            const uint64_t b0 = base_ptrs[b], b1 = b0 + (gb ? gather->extent_bytes : p->extent[b]);
-            if (a0 < b1 && b0 < a1) early = false;
+    auto disjoint = [&](const uint8_t *alias_slots, const uint64_t *extent) {
+        for (int t = 0; t < n_tensors; t++) {
+            if (!alias_slots[t]) continue;
+            for (int b = 0; b < n_tensors; b++) {
+                if (!((alias_slots[t] >> b) & 1u)) continue;
+                const bool ga = gather && ((gather->mask >> t) & 1u), gb = gather && ((gather->mask >> b) & 1u);
+                const uint64_t a0 = base_ptrs[t], a1 = a0 + (ga ? gather->extent_bytes : extent[t]);
+                const uint64_t b0 = base_ptrs[b], b1 = b0 + (gb ? gather->extent_bytes : extent[b]);
+                if (a0 < b1 && b0 < a1) return false;
+            }
         }
+        return true;
+    };
+    /* A flat launch of at most 2^21 elements is a few microseconds of latency either way; the tile kernels spread it over more
+     * blocks (a + b over 2^20 elements: 9.4 us per pass, 9.9 on the streaming kernel). */
+    bool vector = p->wide_vector;   // the vector layout, given aligned base pointers
+    for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
+    if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid || (uint64_t)count * p->flat_tiles <= kFlatMinTiles)) &&
+        !(p->wide_rows_f32 && vector) && disjoint(p->wide_alias, p->wide_extent)) {
+        Geometry g;
+        {
+            std::lock_guard<std::mutex> lk(p->memo_mu);
+            PlanMemo *m = &p->memo[vector ? 5 : 4];
+            if (m->valid && m->count == count && m->opt_blocks == ctx->opt_max_blocks) g = m->g;
+            else {
+                int rc = plan_wide(ctx, p, vector, count, &g);
+                if (rc != GINT_OK) return rc;
+                *m = PlanMemo{true, count, 0, ctx->opt_max_blocks, g};
+            }
+        }
+        LaunchArgs a;
+        const bool inline_code = p->wide_slots <= (uint32_t)gint::kInlineCodeSlots;
+        a.code = inline_code ? nullptr : p->wide_dev;
+        a.n_slots = p->wide_slots;
+        a.n_tensors = (uint32_t)p->n_tensors;
+        a.first = first;
+        a.end = first + count;
+        a.code_smem_bytes = g.code_smem;
+        a.flat_tiles = p->flat_tiles;
+        a.prefetch_mask = p->flat_tiles ? 0u : p->prefetch_mask & p->wide_rows;
+        if (a.prefetch_mask)
+            for (int t = 0; t < GINT_MAX_TENSORS; t++) a.fp[t] = p->fp[t];
+        a.gather_mask = gather ? gather->mask : 0u;
+        a.gather_index = gather ? gather->index : nullptr;
+        a.gather_rows = gather ? gather->rows : 0u;
+        a.ti = p->ti;
+        for (int i = 0; i < n_tensors; i++) a.ti.base_ptr[i] = (int64_t)base_ptrs[i];
+        if (inline_code) memcpy(a.inline_code, p->wide_inline, sizeof(a.inline_code));
+        void *args[1] = {&a};
+        cudaError_t e = cudaLaunchKernel(g.v->fn, dim3(g.grid), dim3(g.threads), args, g.smem, (cudaStream_t)stream);
+        if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaLaunchKernel", e);
+        return GINT_OK;
     }
+    bool early = ctx->opt_early_issue && p->early_dev != nullptr && disjoint(p->alias_slots, p->extent);
     for (int t = 0; early && t < n_tensors; t++)
         if (((p->fast_slots >> t) & 1u) && (base_ptrs[t] & 15u) != 0) early = false;   // fast accesses need aligned bases
     /* the stream with the virtual registers in shared memory, when the stream it was made from is the one this launch may use */
@@ -1388,7 +1496,7 @@ int gint_create(int device, gint_ctx **out)
         if (!im.loaded) continue;
         if (im.K == 0) ctx->indirect.fn = (const void *)im.kernel;
         else if (im.K < 0) ctx->checked.fn = (const void *)im.kernel;
-        else ctx->direct.push_back(Variant{im.P, im.K, (const void *)im.kernel, 0, false, 0, im.rf, im.vec});
+        else ctx->direct.push_back(Variant{im.P, im.K, (const void *)im.kernel, 0, false, 0, im.rf, im.vec, im.wide});
     }
     int usable = 0;
     for (auto &v : ctx->direct) {
@@ -1433,6 +1541,7 @@ void gint_destroy(gint_ctx *ctx)
                 if (p->early_dev) cudaFree(p->early_dev);
                 if (p->rf_dev) cudaFree(p->rf_dev);
                 if (p->vec_dev) cudaFree(p->vec_dev);
+                if (p->wide_dev) cudaFree(p->wide_dev);
                 delete p;
             }
         }
@@ -1475,7 +1584,49 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
     if (ti) p->ti = *ti;
     for (int t = 0; t < GINT_MAX_TENSORS; t++) p->ti.base_ptr[t] = 0;
     compute_footprints(code, p->st.num_instructions, p->ti, n_tensors, p);
-    std::vector<uint2> early, rfs, vecs;
+    std::vector<uint2> early, rfs, vecs, wides;
+    for (int t = 0; t < n_tensors; t++) p->extent[t] = tensor_extent_bytes(p->ti, t);
+    {
+        std::vector<Insn> prog;
+        normalise(code, n_words, n_tensors, &prog);
+        WideStream ws;
+        bool fits = false;
+        if (wide_transform(prog, p->ti, n_tensors, &ws))
+            for (auto &v : ctx->direct) fits = fits || (v.wide == 1 && v.ok && v.P >= ws.max_depth);
+        if (fits) {
+            std::vector<Insn> numbered = ws.prog;
+            if (ctx->opt_fuse) wide_fuse_loops(&numbered);
+            bool inside = false;
+            for (Insn &x : numbered) {
+                const int op = x.op;
+                if (inside) x.op -= GINT_WIDE_TABLE_FIRST;
+                if (op == WOP_LoopBegin) inside = true;
+                if (op == WOP_LoopEnd) inside = false;
+            }
+            emit_stream(numbered, &wides);
+            p->wide_depth = ws.max_depth;
+            p->wide_tiles = ws.max_tiles;
+            p->flat_tiles = ws.flat_tiles;
+            p->flat_grid = ws.flat_grid;
+            p->wide_rows_f32 = ws.flat_tiles == 0;
+            for (const Insn &x : ws.prog)
+                if (x.op >= GINT_WIDE_FIRST && GINT_WIDE_TILE_OP(x.op - GINT_WIDE_FIRST) && x.op != GINT_WIDE_FIRST + OP_LoadGlobal1DF32 && x.op != GINT_WIDE_FIRST + OP_StoreGlobal1DF32)
+                    p->wide_rows_f32 = false;
+            memcpy(p->wide_alias, ws.alias_slots, sizeof(p->wide_alias));
+            bool have_vector = false;
+            for (auto &v : ctx->direct) have_vector = have_vector || (v.wide == 2 && v.ok && v.P >= ws.max_depth);
+            p->wide_vector = ws.vector && have_vector;
+            for (int t = 0; t < n_tensors; t++) {
+                const uint32_t elem = (uint32_t)p->ti.elm_size[t] > ws.access_bytes[t] ? (uint32_t)p->ti.elm_size[t] : ws.access_bytes[t];
+                p->wide_extent[t] = tensor_extent_bytes(p->ti, t) / (uint64_t)(p->ti.elm_size[t] > 4 ? p->ti.elm_size[t] : 4) * elem;
+                for (int j = 0; j < 4; j++)
+                    if (p->ti.batch_shape[t][j] > 1 && p->ti.batch_strides[t][j] != 0) p->wide_rows |= 1u << t;
+                if (ws.access_bytes[t]) p->wide_align[t] = 4 * ws.access_bytes[t] - 1;
+            }
+            /* the streaming kernels hold the program and the descriptors in the default 48 KB of shared memory */
+            if (wides.size() * 8 + gint::kTensorInfoSmemBytes + gint::kWarpsPerBlock * (sizeof(gint::TileInfo) + 512) + 128 > 48u * 1024u) wides.clear();
+        }
+    }
     {
         std::vector<Insn> prog;
         normalise(code, n_words, n_tensors, &prog);
@@ -1573,10 +1724,12 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
     p->early_slots = (uint32_t)early.size();
     p->rf_slots = (uint32_t)rfs.size();
     p->vec_slots = (uint32_t)vecs.size();
+    p->wide_slots = (uint32_t)wides.size();
     for (int i = 0; i < gint::kInlineCodeSlots; i++) {
         p->code_inline[i] = (size_t)i < pre.size() ? pre[(size_t)i] : make_uint2(0u, OP_Halt);
         p->early_inline[i] = (size_t)i < early.size() ? early[(size_t)i] : make_uint2(0u, OP_Halt);
         p->rf_inline[i] = (size_t)i < rfs.size() ? rfs[(size_t)i] : make_uint2(0u, OP_Halt);
+        p->wide_inline[i] = (size_t)i < wides.size() ? wides[(size_t)i] : make_uint2(0u, OP_Halt);
         p->vec_inline[i] = (size_t)i < vecs.size() ? vecs[(size_t)i] : make_uint2(0u, OP_Halt);
     }
     {
@@ -1606,11 +1759,24 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
                 return fail(ctx, GINT_ERR_OUT_OF_MEMORY, "cudaMalloc/cudaMemcpy(register-file program)", e);
             }
         }
+        if (wides.size() > (size_t)gint::kInlineCodeSlots) {   // (shorter ones travel in the launch parameters)
+            e = cudaMalloc(&p->wide_dev, wides.size() * sizeof(uint2));
+            if (e == cudaSuccess) e = cudaMemcpy(p->wide_dev, wides.data(), wides.size() * sizeof(uint2), cudaMemcpyHostToDevice);
+            if (e != cudaSuccess) {
+                if (p->wide_dev) cudaFree(p->wide_dev);
+                if (p->rf_dev) cudaFree(p->rf_dev);
+                if (p->early_dev) cudaFree(p->early_dev);
+                cudaFree(p->code_dev);
+                delete p;
+                return fail(ctx, GINT_ERR_OUT_OF_MEMORY, "cudaMalloc/cudaMemcpy(program with loops)", e);
+            }
+        }
         if (!vecs.empty()) {
             e = cudaMalloc(&p->vec_dev, vecs.size() * sizeof(uint2));
             if (e == cudaSuccess) e = cudaMemcpy(p->vec_dev, vecs.data(), vecs.size() * sizeof(uint2), cudaMemcpyHostToDevice);
             if (e != cudaSuccess) {
                 if (p->vec_dev) cudaFree(p->vec_dev);
+                if (p->wide_dev) cudaFree(p->wide_dev);
                 if (p->rf_dev) cudaFree(p->rf_dev);
                 if (p->early_dev) cudaFree(p->early_dev);
                 cudaFree(p->code_dev);
@@ -1642,6 +1808,7 @@ int gint_program_destroy(gint_ctx *ctx, uint64_t handle)
     if (p->early_dev) cudaFree(p->early_dev);
     if (p->rf_dev) cudaFree(p->rf_dev);
     if (p->vec_dev) cudaFree(p->vec_dev);
+    if (p->wide_dev) cudaFree(p->wide_dev);
     delete p;
     return GINT_OK;
 }
@@ -2076,6 +2243,13 @@ int gint_debug_transform(const int32_t *code, int n_words, const gint_tensor_inf
     std::vector<Insn> prog;
     int rc = normalise(code, n_words, n_tensors, &prog);
     if (rc != GINT_OK) return rc;
+    if (early_issue & 8) {   // the stream with loops for the streaming kernels, if the program qualifies; a flat one starts with LoopBegin 0
+        WideStream ws;
+        if (!ti || !wide_transform(prog, *ti, n_tensors, &ws)) return 0;
+        if ((int)ws.prog.size() > max_insns) return GINT_ERR_INVALID_ARGUMENT;
+        for (size_t i = 0; i < ws.prog.size(); i++) { out_ops[i] = ws.prog[i].op; out_operands[i] = ws.prog[i].operand; }
+        return (int)ws.prog.size();
+    }
     if (early_issue & 1) {
         gint_bytecode_stats st;
         analyze(code, n_words, &st);
@@ -2164,6 +2338,10 @@ int gint_set_option(gint_ctx *ctx, const char *name, int value)
     }
     if (strcmp(name, "register_file") == 0) {   // virtual registers in shared memory: programs created and launches made from now on
         ctx->opt_rf = ctx->opt_rf_create = value != 0;
+        return GINT_OK;
+    }
+    if (strcmp(name, "streaming") == 0) {   // launches made from now on
+        ctx->opt_wide = value != 0;
         return GINT_OK;
     }
     if (strcmp(name, "vector_layout") == 0) {   // programs created and launches made from now on

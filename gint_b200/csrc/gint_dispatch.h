@@ -38,4 +38,17 @@
     "GTALL: .branchtargets\n\t" GINT_LABELS(0) ",\n\t" GINT_LABELS(1) ",\n\t" GINT_LABELS(2) ",\n\t" GINT_LABELS(3) ",\n\t"  \
     GINT_LABELS(4) ",\n\t" GINT_LABELS(5) ",\n\t" GINT_LABELS(6) ",\n\t" GINT_LABELS(7) ",\n\t" GINT_LABELS(8) ";\n\t"
 
+/* The streaming kernels have two tables per depth (0 .. 4), outside of loops GTN<depth> (opcodes 0 .. 129) and inside GTW<depth>
+ * (from GINT_WIDE_TABLE_FIRST = 100 on): half the edges in the control-flow graph. */
+#define GINT_LABELS_NARROW(d)                                                                                            \
+    GINT_L10(d, ) ",\n\t" GINT_L10(d, 1) ",\n\t" GINT_L10(d, 2) ",\n\t" GINT_L10(d, 3) ",\n\t" GINT_L10(d, 4) ",\n\t"       \
+    GINT_L10(d, 5) ",\n\t" GINT_L10(d, 6) ",\n\t" GINT_L10(d, 7) ",\n\t" GINT_L10(d, 8) ",\n\t" GINT_L10(d, 9) ",\n\t" GINT_L10(d, 10) ",\n\t"     \
+    GINT_L10(d, 11) ",\n\t" GINT_L10(d, 12)
+#define GINT_LABELS_WIDE(d)                                                                                              \
+    GINT_L10(d, 10) ",\n\t" GINT_L10(d, 11) ",\n\t" GINT_L10(d, 12) ",\n\t" GINT_L10(d, 13) ",\n\t" GINT_L10(d, 14) ",\n\t"  \
+    GINT_L10(d, 15) ",\n\t" GINT_L10(d, 16) ",\n\t" GINT_L10(d, 17) ",\n\t" GINT_L10(d, 18) ",\n\t" GINT_L10(d, 19) ",\n\t"  \
+    GINT_L10(d, 20) ",\n\t" GINT_L10(d, 21) ",\n\t" GINT_L10(d, 22) ",\n\t" GINT_L10(d, 23)
+#define GINT_TABLE_PAIR(d) "GTN" #d ": .branchtargets\n\t" GINT_LABELS_NARROW(d) ";\n\tGTW" #d ": .branchtargets\n\t" GINT_LABELS_WIDE(d) ";\n\t"
+#define GINT_WIDE_BRANCH_TABLES GINT_TABLE_PAIR(0) GINT_TABLE_PAIR(1) GINT_TABLE_PAIR(2) GINT_TABLE_PAIR(3) GINT_TABLE_PAIR(4)
+
 #endif /* GINT_DISPATCH_H */

@@ -182,6 +182,49 @@
  * and the host puts this in front of it (gint_capi.cu: vec_transform):
  *   RemapVN   rearrange the top of the stack from the vector layout into the natural one (through shared memory) */
 #define GINT_VEC_OPCODE_LIST(X) X(RemapVN, 180, 1, 0)
+/*
+ * The streaming kernels (GINT_WIDE, gint_wide.cuh) have a dispatch space of their own: the format's opcodes on one tile, the
+ * opcodes below, and GINT_WIDE_FIRST + op for instruction `op` of a loop body, which works on all U tiles:
+ *   LoopBegin n      the instructions up to LoopEnd run for n tiles, U at a time (0: the launch has set the range); what is on the
+ *                    stack is copied from tile 0 to the slots' other tiles
+ *   LoopEnd
+ *   Remap            the top value from the vector layout to the natural one (kernels in the natural layout: nothing)
+ *   AccAdd           FAdd / AccFMA  FMA into a running value in tile 0, tile after tile; AccFMASquare  Dup, AccFMA
+ *   Square           Dup, FMul
+ *   MulKeep          [s, x] -> [s, s * x]   (Dup, <load x>, Swap, FMul with the load moved in front)
+ *   Silu c           Dup, FNeg, FExp, FAddImm c, FRDiv
+ */
+#define GINT_WIDE_OWN_LIST(X) \
+    X(LoopBegin, 106) X(Remap, 107) X(AccAdd, 110) X(AccFMA, 111) X(AccFMASquare, 112) X(Square, 113) \
+    X(MulKeep, 114) X(Silu, 115) X(LoopEnd, 116)
+#define GINT_WIDE_FIRST 128
+/*
+ * Whole loops as one instruction: the bodies that frontend and torch.compile lowerings are made of (row reductions, scale-and-store
+ * passes). Their handlers run all iterations with the body's values in local
+ * registers; any other body is interpreted. X(name, opcode, expression, layout, element type, stack depth, length, body ...); opcodes
+ * 117 .. 121. In the stream: the instruction with the number of tiles, then
+ * one entry per operand of the body.
+ */
+#define GINT_W(op) (GINT_WIDE_FIRST + OP_##op)
+#define GINT_WIDE_LOOP_LIST(X)                                                                                                            \
+    X(SumSquares, 117, LX_SUMSQ, LAY_1D, DT_F32, 1, 3, GINT_W(LoadGlobal1DF32), WOP_Square, WOP_AccAdd)                                     \
+    X(Sum, 118, LX_SUM, LAY_1D, DT_F32, 1, 2, GINT_W(LoadGlobal1DF32), WOP_AccAdd)                                                          \
+    X(Scale, 119, LX_SCALE, LAY_1D, DT_F32, 1, 5, GINT_W(LoadGlobal1DF32), WOP_MulKeep, GINT_W(LoadGlobal1DF32), GINT_W(FMul), GINT_W(StoreGlobal1DF32)) \
+    X(SumSquares2DT, 120, LX_FMASQ, LAY_2DT, DT_BF16, 1, 2, GINT_W(LoadGlobal2DTBF16), WOP_AccFMASquare)                                    \
+    X(Scale2DT, 121, LX_SCALE, LAY_2DT, DT_BF16, 1, 5, GINT_W(LoadGlobal2DTBF16), WOP_MulKeep, GINT_W(LoadGlobal2DTBF16), GINT_W(FMul), GINT_W(StoreGlobal2DTBF16))
+enum { LX_SUMSQ = 0, LX_SUM, LX_FMASQ, LX_SCALE };
+#define GINT_WIDE_TABLE_FIRST 100   /* the stream numbers what is dispatched inside a loop (up to LoopEnd) from here */
+/* instructions that run outside of the format's own math library calls: the element-wise ones that a streaming kernel has */
+#define GINT_WIDE_ELEMENTWISE(op)                                                                                               \
+    (((op) >= OP_Nop && (op) <= OP_FRDiv) || ((op) >= OP_LoadImm && (op) <= OP_FMAImm) || ((op) >= OP_Pop && (op) <= OP_Select) || \
+     (op) == OP_FSqrt || (op) == OP_FSin || (op) == OP_FCos || (op) == OP_FExp || (op) == OP_FExp2 || (op) == OP_FRSqrt ||         \
+     ((op) >= OP_Swap && (op) <= OP_ISub) || ((op) >= OP_IShl && (op) <= OP_IXor) || (op) == OP_LoadImm4F || (op) == OP_LoadImm4I || (op) == OP_FRcp)
+#define GINT_WIDE_TILE_OP(op) (((op) >= OP_LoadGlobal1DF32 && (op) <= OP_LoadGlobal1DU8) || ((op) >= OP_LoadGlobal2DTF32 && (op) <= OP_LoadGlobal2DTU8))
+#define GINT_WIDE_OP(op) (GINT_WIDE_ELEMENTWISE(op) || GINT_WIDE_TILE_OP(op))
+#define GINT_WIDE_NARROW_OP(op)                                                                                                 \
+    (GINT_WIDE_OP(op) || ((op) >= OP_WarpAllReduceSum && (op) <= OP_WarpAllReduceProd) || ((op) >= OP_LoadGlobal2DWF32 && (op) <= OP_LoadGlobal2DWU8) || \
+     (op) == OP_DupBroadcastW || (op) == OP_FPermW || (op) == OP_FShuf2)
+#define GINT_N_DISPATCH_WIDE 234   /* GINT_WIDE_FIRST + GINT_N_OPCODES */
 #define GINT_N_DISPATCH_PLAIN 150
 #define GINT_N_DISPATCH_RF 176
 #define GINT_N_DISPATCH_VEC 181
@@ -189,6 +232,8 @@
 #define GINT_N_DISPATCH GINT_N_DISPATCH_RF
 #elif defined(GINT_VEC)
 #define GINT_N_DISPATCH GINT_N_DISPATCH_VEC
+#elif defined(GINT_WIDE)
+#define GINT_N_DISPATCH GINT_N_DISPATCH_WIDE
 #else
 #define GINT_N_DISPATCH GINT_N_DISPATCH_PLAIN
 #endif
@@ -200,6 +245,9 @@ enum gint_opcode {
     GINT_RF_OPCODE_LIST(GINT_X_ENUM)
     GINT_VEC_OPCODE_LIST(GINT_X_ENUM)
 #undef GINT_X_ENUM
+#define GINT_X_WENUM(name, num) WOP_##name = num,
+    GINT_WIDE_OWN_LIST(GINT_X_WENUM)
+#undef GINT_X_WENUM
 };
 
 #endif /* GINT_OPCODES_H */

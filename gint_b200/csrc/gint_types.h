@@ -63,6 +63,7 @@ struct LaunchArgs {
     uint32_t zero;            // always 0; a zero the assembler cannot see (fma_barrier in gint_interp.cuh)
     uint32_t row_area_bytes;  // shared-memory bytes per tile for staged row blocks (StageRows), 0 if the program has none
     uint32_t ring_bytes;      // shared-memory bytes per tile for the ring of early-issued loads, 0 if the stream has none
+    uint32_t flat_tiles;      // streaming kernels: tiles per logical program if the launch is one flat loop, else 0
     uint32_t rf_bytes;        // shared-memory bytes per tile for virtual registers (kernels built with GINT_RF; 512 per register), else 0
     Footprint fp[GINT_MAX_TENSORS];
     gint_tensor_info ti;      // descriptor block, base pointers patched per call: travels as a kernel parameter

@@ -1,0 +1,5 @@
+// Streaming interpreter kernel (gint_wide.cuh), vector layout: 3 pool slots of 8 tiles.
+#define GINT_WIDE 1
+#define GINT_WIDE_V 1
+#include "../gint_wide.cuh"
+GINT_DEFINE_WIDE_KERNEL(3, 8, 4)

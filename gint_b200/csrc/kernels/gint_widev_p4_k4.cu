@@ -1,0 +1,5 @@
+// Streaming interpreter kernel (gint_wide.cuh), vector layout: 4 pool slots of 4 tiles.
+#define GINT_WIDE 1
+#define GINT_WIDE_V 1
+#include "../gint_wide.cuh"
+GINT_DEFINE_WIDE_KERNEL(4, 4, 5)

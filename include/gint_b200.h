@@ -127,7 +127,8 @@ int gint_predecode(const int32_t *code, int n_words, uint32_t *out_keys, int max
  * "fast" forms (provably full, aligned tiles). early_issue is a bit set: 1 = the early-issue pass, 2 = the stream for the
  * kernels that keep the virtual registers in shared memory (FLoadRegN / FStoreRegN become RLoad / RStore with the register in
  * the operand; returns 0 if the program does not qualify for them), 4 = the stream for the vector-layout kernels (with 1; RemapVN
- * inserted where a value must be in the natural layout; 0 if the program does not qualify). Returns the number of instructions
+ * inserted where a value must be in the natural layout; 0 if the program does not qualify), 8 = the stream with loops for the
+ * streaming kernels (alone; 0 if the program does not qualify). Returns the number of instructions
  * (including the Halt) or < 0. */
 int gint_debug_transform(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, int early_issue, int fuse,
                          int32_t *out_ops, uint32_t *out_operands, int max_insns);
@@ -157,6 +158,8 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
 int gint_program_destroy(gint_ctx *ctx, uint64_t handle);
 
 /* Geometry the library would use to launch `handle` over grid_dim logical programs. */
+/* The geometry of the tile kernels for this program. A launch that qualifies for the streaming kernels (option "streaming")
+ * has a geometry of its own, which is not reported. */
 int gint_program_launch_info(gint_ctx *ctx, uint64_t handle, uint32_t grid_dim, gint_launch_info *out);
 
 /* ---- launches ----------------------------------------------------------------------------------- */
@@ -278,7 +281,8 @@ int gint_execute_indirect_static(gint_ctx *ctx, const uint64_t *handles, int n_p
  * virtual registers keep those in shared memory and run on a kernel whose pool is the operand stack alone, default),
  * "vector_layout" (1 = programs created from now on whose full 1-D tiles can live in the pool as four consecutive elements
  * per lane run on the kernels that access them with one 16-byte access per lane; default 0: no measurable gain on the
- * benchmark programs). */
+ * benchmark programs), "streaming" (1 = launches use the streaming kernels for programs whose tile loops were found again,
+ * default; results are the same bits, but for sums of 2-byte 2DT tiles, whose terms are added in another order). */
 int gint_set_option(gint_ctx *ctx, const char *name, int value);
 
 #ifdef __cplusplus
