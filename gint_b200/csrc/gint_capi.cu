@@ -1014,6 +1014,7 @@ void compute_footprints(const int32_t *code, int n_insns, const gint_tensor_info
         p->prefetch_mask |= 1u << t;
     }
 }
+    uint32_t wide_loop_slots = 0;   // slots that a loop accesses
 
 }  // namespace
 
@@ -1275,7 +1276,7 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
     bool vector = p->wide_vector;   // the vector layout, given aligned base pointers
     for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
     if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid || (uint64_t)count * p->flat_tiles <= kFlatMinTiles)) &&
-        !(p->wide_rows_f32 && vector) && disjoint(p->wide_alias, p->wide_extent)) {
+        !(p->wide_rows_f32 && fast_rows) && disjoint(p->wide_alias, p->wide_extent)) {
         Geometry g;
         {
             std::lock_guard<std::mutex> lk(p->memo_mu);
@@ -1311,6 +1312,8 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
         return GINT_OK;
     }
     bool early = ctx->opt_early_issue && p->early_dev != nullptr && disjoint(p->alias_slots, p->extent);
+    bool fast_rows = p->early_dev != nullptr && (p->wide_loop_slots & ~p->fast_slots) == 0;   // every loop access is a fast one of the tile kernels
+    for (int t = 0; fast_rows && t < n_tensors; t++) fast_rows = !((p->fast_slots >> t) & 1u) || (base_ptrs[t] & 15u) == 0;
     for (int t = 0; early && t < n_tensors; t++)
         if (((p->fast_slots >> t) & 1u) && (base_ptrs[t] & 15u) != 0) early = false;   // fast accesses need aligned bases
     /* the stream with the virtual registers in shared memory, when the stream it was made from is the one this launch may use */
@@ -1609,9 +1612,12 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
             p->flat_tiles = ws.flat_tiles;
             p->flat_grid = ws.flat_grid;
             p->wide_rows_f32 = ws.flat_tiles == 0;
-            for (const Insn &x : ws.prog)
-                if (x.op >= GINT_WIDE_FIRST && GINT_WIDE_TILE_OP(x.op - GINT_WIDE_FIRST) && x.op != GINT_WIDE_FIRST + OP_LoadGlobal1DF32 && x.op != GINT_WIDE_FIRST + OP_StoreGlobal1DF32)
-                    p->wide_rows_f32 = false;
+            for (const Insn &x : ws.prog) {
+                const int op = x.op - GINT_WIDE_FIRST;
+                if (op < 0 || !GINT_WIDE_TILE_OP(op)) continue;
+                p->wide_loop_slots |= 1u << (x.operand & 15u);
+                if (op != OP_LoadGlobal1DF32 && op != OP_StoreGlobal1DF32) p->wide_rows_f32 = false;
+            }
             memcpy(p->wide_alias, ws.alias_slots, sizeof(p->wide_alias));
             bool have_vector = false;
             for (auto &v : ctx->direct) have_vector = have_vector || (v.wide == 2 && v.ok && v.P >= ws.max_depth);
