@@ -208,6 +208,45 @@ int predecode(const int32_t *code, int n_words, int n_tensors, std::vector<uint2
     return GINT_OK;
 }
 
+/* predecode() for batches of candidate programs: the same checks, in the same order, and the same stream in one pass over the
+ * words, written where it is uploaded from (the generic form walks a program four times through two vectors: 270 ns per candidate
+ * of 26 instructions). `out` has room for n_words / 2 + 4 entries. */
+int predecode_into(const int32_t *code, int n_words, int n_tensors, uint2 *out, uint32_t *n_out)
+{
+    int depth = 0, slot_error = GINT_OK;
+    uint32_t n = 1, operand_before = 0;      // entry n - 1 awaits the opcode of the instruction at hand
+    for (int i = 0; i + 1 < n_words; i += 2) {
+        const int op = code[i];
+        uint32_t operand = (uint32_t)code[i + 1];
+        if (op == OP_Halt) {
+            if (slot_error != GINT_OK) return slot_error;
+            out[n - 1] = make_uint2(operand_before, OP_Halt);
+            out[n++] = make_uint2(0u, OP_Halt);
+            out[n++] = make_uint2(0u, OP_Halt);
+            if (n & 1) out[n++] = make_uint2(0u, OP_Halt);
+            *n_out = n;
+            return GINT_OK;
+        }
+        if (op < 0 || op >= GINT_N_OPCODES) return GINT_ERR_UNKNOWN_OPCODE;
+        if (depth < kEffects[op].min_depth) return GINT_ERR_STACK_UNDERFLOW;
+        const int post = depth + kEffects[op].net;
+        if ((post > depth ? post : depth) > GINT_MAX_STACK) return GINT_ERR_STACK_OVERFLOW;
+        depth = post;
+        if (is_tensor_op(op)) {
+            if ((int)(operand & 15u) >= n_tensors) slot_error = GINT_ERR_INVALID_ARGUMENT;
+        } else if (op == OP_DupBroadcastW) {
+            const int32_t s = (int32_t)operand;
+            operand = s < 0 ? 0u : s > 3 ? 3u : (uint32_t)s;
+        } else if (op == OP_FPermW || op == OP_FShuf2) {
+            operand = clamp_lane_bytes(operand);
+        }
+        out[n - 1] = make_uint2(operand_before, (uint32_t)op);
+        n++;
+        operand_before = operand;
+    }
+    return GINT_ERR_NO_HALT;
+}
+
 bool writes_tensor(int op)
 {
     return op == OP_StoreGlobal1DF32 || op == OP_StoreGlobal1DF16 || op == OP_StoreGlobal1DBF16 || op == OP_StoreGlobal1DF32Indirect ||
@@ -975,6 +1014,7 @@ struct Program {
      * 16384 x 4096: 125 us there, 121 us here; row sums of 65536 x 1024: 50 against 75), so only unaligned rows come here
      * (10007 x 2029: 77 us there, 55 here). */
     bool wide_rows_f32 = false;
+    uint32_t wide_loop_slots = 0;   // slots that a loop accesses
     uint32_t wide_rows = 0;     // slots of which every logical program has its own part
     uint2 wide_inline[gint::kInlineCodeSlots];
     PlanMemo memo[6] = {};      // last launch plan of the plain stream [0], the early-issue stream [1], the RF stream [2], the vector-layout stream [3], the streaming kernels in the natural [4] and the vector layout [5]
@@ -1014,7 +1054,6 @@ void compute_footprints(const int32_t *code, int n_insns, const gint_tensor_info
         p->prefetch_mask |= 1u << t;
     }
 }
-    uint32_t wide_loop_slots = 0;   // slots that a loop accesses
 
 }  // namespace
 
@@ -1273,6 +1312,8 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
     };
     /* A flat launch of at most 2^21 elements is a few microseconds of latency either way; the tile kernels spread it over more
      * blocks (a + b over 2^20 elements: 9.4 us per pass, 9.9 on the streaming kernel). */
+    bool fast_rows = p->early_dev != nullptr && (p->wide_loop_slots & ~p->fast_slots) == 0;   // every loop access is a fast one of the tile kernels
+    for (int t = 0; fast_rows && t < n_tensors; t++) fast_rows = !((p->fast_slots >> t) & 1u) || (base_ptrs[t] & 15u) == 0;
     bool vector = p->wide_vector;   // the vector layout, given aligned base pointers
     for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
     if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid || (uint64_t)count * p->flat_tiles <= kFlatMinTiles)) &&
@@ -1312,8 +1353,6 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
         return GINT_OK;
     }
     bool early = ctx->opt_early_issue && p->early_dev != nullptr && disjoint(p->alias_slots, p->extent);
-    bool fast_rows = p->early_dev != nullptr && (p->wide_loop_slots & ~p->fast_slots) == 0;   // every loop access is a fast one of the tile kernels
-    for (int t = 0; fast_rows && t < n_tensors; t++) fast_rows = !((p->fast_slots >> t) & 1u) || (base_ptrs[t] & 15u) == 0;
     for (int t = 0; early && t < n_tensors; t++)
         if (((p->fast_slots >> t) & 1u) && (base_ptrs[t] & 15u) != 0) early = false;   // fast accesses need aligned bases
     /* the stream with the virtual registers in shared memory, when the stream it was made from is the one this launch may use */
@@ -1473,6 +1512,19 @@ int gint_predecode(const int32_t *code, int n_words, uint32_t *out_keys, int max
         for (int i = 0; i < n; i++) out_keys[i] = (uint32_t)depths[(size_t)i] * GINT_N_OPCODES + pre[(size_t)i].y;
     }
     return n;
+}
+
+int gint_debug_predecode_batch(const int32_t *code, int n_words, int n_tensors, uint32_t *out_words, int max_words)
+{
+    std::vector<uint2> whole;
+    std::vector<uint2> once((size_t)(n_words / 2 + 4));
+    uint32_t n = 0;
+    const int rc = predecode(code, n_words, n_tensors, &whole), rc1 = predecode_into(code, n_words, n_tensors, once.data(), &n);
+    if (rc != rc1) return INT32_MIN;
+    if (rc != GINT_OK) return rc;
+    if (n != whole.size() || memcmp(whole.data(), once.data(), n * sizeof(uint2)) != 0) return INT32_MIN;
+    if (out_words) memcpy(out_words, once.data(), (n * 2 < (uint32_t)max_words ? n * 2 : (uint32_t)max_words) * sizeof(uint32_t));
+    return (int)n;
 }
 
 int gint_create(int device, gint_ctx **out)
@@ -2115,7 +2167,6 @@ int gint_execute_batch(gint_ctx *ctx, const int32_t *codes, int n_programs, int 
     const char *d_base = (const char *)ctx->ind_dev;
     *h_ti = *ti;
     for (int t = 0; t < n_tensors; t++) h_ti->base_ptr[t] = (int64_t)base_ptrs[t];
-    std::vector<uint2> pre;
     int n_valid = 0;
     for (int i = 0; i < n_programs; i++) {
         IndirectEntry &en = h_tab[i];
@@ -2123,15 +2174,10 @@ int gint_execute_batch(gint_ctx *ctx, const int32_t *codes, int n_programs, int 
         en.ti = (const gint_tensor_info *)d_base;
         en.patch_slot = (uint32_t)out_slot + 1u;
         en.patch_ptr = base_ptrs[out_slot] + (uint64_t)i * out_stride_bytes;
-        const int rc = predecode(codes + (size_t)i * (size_t)n_words, n_words, n_tensors, &pre);
+        en.n_slots = 0;                     // of an invalid candidate: the warp skips it, its output row is left as it is
+        const int rc = predecode_into(codes + (size_t)i * (size_t)n_words, n_words, n_tensors, h_code + (size_t)i * stride, &en.n_slots);
         if (status_out) status_out[i] = rc;
-        if (rc != GINT_OK || pre.size() > stride) {
-            if (status_out && rc == GINT_OK) status_out[i] = GINT_ERR_TOO_LARGE;
-            en.n_slots = 0;                 // the warp skips this candidate; its output row is left as it is
-            continue;
-        }
-        en.n_slots = (uint32_t)pre.size();
-        memcpy(h_code + (size_t)i * stride, pre.data(), pre.size() * sizeof(uint2));
+        if (rc != GINT_OK) continue;
         n_valid++;
     }
     cudaError_t e = cudaMemcpyAsync(ctx->ind_dev, ctx->ind_host, need, cudaMemcpyHostToDevice, stream);

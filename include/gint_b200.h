@@ -121,6 +121,10 @@ int gint_analyze(const int32_t *code, int n_words, gint_bytecode_stats *out);
  * instruction i (stack depth * number of opcodes + opcode). Returns the instruction count incl. Halt, or < 0. */
 int gint_predecode(const int32_t *code, int n_words, uint32_t *out_keys, int max_keys);
 
+/* The stream gint_execute_batch makes of one candidate (for tests): the number of entries (two words each, copied to out_words as
+ * far as they fit), the candidate's status, or INT32_MIN if it differs from what programs created one by one run. */
+int gint_debug_predecode_batch(const int32_t *code, int n_words, int n_tensors, uint32_t *out_words, int max_words);
+
 /* The instruction list the kernels actually run for a program, after the optional early-issue and fusion passes (for
  * tests; no GPU needed): out_ops[i] is a format opcode, an internal opcode (>= 106) or -1 for an instruction absorbed into
  * the fused handler before it. With early_issue != 0 the descriptors in `ti` also decide which 1-D accesses become their
