@@ -1250,7 +1250,7 @@ constexpr uint64_t kFlatMinTiles = 16384;
  * configuration of the tile kernels. */
 bool use_wide(const gint_ctx *ctx, const Program *p)
 {
-    return p->wide_slots != 0 && ctx->opt_wide && ctx->opt_early_issue && ctx->opt_tiles_per_warp == 0 && !ctx->opt_prefetch && !(ctx->opt_vec && p->vec_dev);
+    return p->wide_slots != 0 && ctx->opt_wide && ctx->opt_early_issue && ctx->opt_tiles_per_warp == 0 && !ctx->opt_prefetch && !(ctx->opt_vec && p->vec_slots);
 }
 
 int plan_wide(gint_ctx *ctx, const Program *p, bool vector, uint32_t count, Geometry *g)
@@ -1285,18 +1285,20 @@ struct GatherArgs {
     uint32_t rows;            // rows of the gathered table
 };
 
-int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int n_tensors, uint32_t first, uint32_t count,
-                  void *stream, const GatherArgs *gather = nullptr)
+/* Which of a program's streams a launch runs, and on which kernels. */
+struct Route {
+    int wide = 0;         // streaming kernels: 1 natural, 2 vector layout; 0: the tile kernels, with
+    bool early = false;   // ... the early-issue stream
+    bool rf = false;      // ... the stream with the virtual registers in shared memory
+    bool vec = false;     // ... the vector-layout stream
+};
+
+Route choose_route(const gint_ctx *ctx, const Program *p, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather)
 {
-    if (!ctx || (!base_ptrs && n_tensors > 0)) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "null argument");
-    Program *p = lookup(ctx, handle);
-    if (!p) return fail(ctx, GINT_ERR_BAD_HANDLE, "unknown program handle");
-    if (n_tensors != p->n_tensors) return fail(ctx, GINT_ERR_ARG_COUNT, "number of arguments does not match the program");
-    if (count == 0) return GINT_OK;
-    if ((uint64_t)first + (uint64_t)count > 0xFFFFFFFFull) return fail(ctx, GINT_ERR_TOO_LARGE, "logical program range overflows 32 bits");
-    DeviceGuard guard(ctx->device);
-    /* The early-issue stream is used unless a tensor whose loads were moved across stores overlaps, at this launch's
-     * addresses, one of the tensors those stores write. */
+    const int n_tensors = p->n_tensors;
+    Route r;
+    /* A stream in which accesses moved is used unless a tensor whose accesses moved overlaps, at this launch's addresses, one of
+     * the tensors they were moved across. */
     auto disjoint = [&](const uint8_t *alias_slots, const uint64_t *extent) {
         for (int t = 0; t < n_tensors; t++) {
             if (!alias_slots[t]) continue;
@@ -1310,14 +1312,41 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
         }
         return true;
     };
+    bool fast_ok = true;   // fast accesses need aligned bases
+    for (int t = 0; t < n_tensors; t++) fast_ok = fast_ok && !(((p->fast_slots >> t) & 1u) && (base_ptrs[t] & 15u) != 0);
     /* A flat launch of at most 2^21 elements is a few microseconds of latency either way; the tile kernels spread it over more
      * blocks (a + b over 2^20 elements: 9.4 us per pass, 9.9 on the streaming kernel). */
-    bool fast_rows = p->early_dev != nullptr && (p->wide_loop_slots & ~p->fast_slots) == 0;   // every loop access is a fast one of the tile kernels
-    for (int t = 0; fast_rows && t < n_tensors; t++) fast_rows = !((p->fast_slots >> t) & 1u) || (base_ptrs[t] & 15u) == 0;
-    bool vector = p->wide_vector;   // the vector layout, given aligned base pointers
-    for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
-    if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid || (uint64_t)count * p->flat_tiles <= kFlatMinTiles)) &&
-        !(p->wide_rows_f32 && fast_rows) && disjoint(p->wide_alias, p->wide_extent)) {
+    if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid || (uint64_t)count * p->flat_tiles <= kFlatMinTiles))) {
+        const bool fast_rows = p->early_slots != 0 && fast_ok && (p->wide_loop_slots & ~p->fast_slots) == 0;   // every loop access is a fast one of the tile kernels
+        if (!(p->wide_rows_f32 && fast_rows) && disjoint(p->wide_alias, p->wide_extent)) {
+            bool vector = p->wide_vector;   // the vector layout, given aligned base pointers
+            for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
+            r.wide = vector ? 2 : 1;
+            return r;
+        }
+    }
+    r.early = ctx->opt_early_issue && p->early_slots != 0 && fast_ok && disjoint(p->alias_slots, p->extent);
+    /* the stream with the virtual registers in shared memory, when the stream it was made from is the one this launch may use */
+    r.rf = ctx->opt_rf && p->rf_slots != 0 && p->rf_from_early == r.early;
+    /* the vector-layout stream, for programs that run more than one tile per warp (measured: the conductor graph's fused program
+     * 174 -> 164 us at two tiles per warp; RMSNorm at one tile per warp 110 -> 112 us, so it stays on the ordinary kernel) */
+    r.vec = ctx->opt_vec && p->vec_slots != 0 && r.early && !r.rf && !p->prefer_narrow && ctx->opt_tiles_per_warp != 1;
+    return r;
+}
+
+int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int n_tensors, uint32_t first, uint32_t count,
+                  void *stream, const GatherArgs *gather = nullptr)
+{
+    if (!ctx || (!base_ptrs && n_tensors > 0)) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "null argument");
+    Program *p = lookup(ctx, handle);
+    if (!p) return fail(ctx, GINT_ERR_BAD_HANDLE, "unknown program handle");
+    if (n_tensors != p->n_tensors) return fail(ctx, GINT_ERR_ARG_COUNT, "number of arguments does not match the program");
+    if (count == 0) return GINT_OK;
+    if ((uint64_t)first + (uint64_t)count > 0xFFFFFFFFull) return fail(ctx, GINT_ERR_TOO_LARGE, "logical program range overflows 32 bits");
+    DeviceGuard guard(ctx->device);
+    const Route route = choose_route(ctx, p, base_ptrs, first, count, gather);
+    if (route.wide) {
+        const bool vector = route.wide == 2;
         Geometry g;
         {
             std::lock_guard<std::mutex> lk(p->memo_mu);
@@ -1352,14 +1381,8 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
         if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaLaunchKernel", e);
         return GINT_OK;
     }
-    bool early = ctx->opt_early_issue && p->early_dev != nullptr && disjoint(p->alias_slots, p->extent);
-    for (int t = 0; early && t < n_tensors; t++)
-        if (((p->fast_slots >> t) & 1u) && (base_ptrs[t] & 15u) != 0) early = false;   // fast accesses need aligned bases
-    /* the stream with the virtual registers in shared memory, when the stream it was made from is the one this launch may use */
-    bool rf = ctx->opt_rf && p->rf_dev != nullptr && p->rf_from_early == early;
-    /* the vector-layout stream, for programs that run more than one tile per warp (measured: the conductor graph's fused program
-     * 174 -> 164 us at two tiles per warp; RMSNorm at one tile per warp 110 -> 112 us, so it stays on the ordinary kernel) */
-    bool vec = ctx->opt_vec && p->vec_dev != nullptr && early && !rf && !p->prefer_narrow && ctx->opt_tiles_per_warp != 1;
+    const bool early = route.early;
+    bool rf = route.rf, vec = route.vec;
     StreamView sv = stream_view(p, early, rf, vec);   // geometry depends on the stream
     Geometry g;
     {
@@ -1411,212 +1434,15 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
     return GINT_OK;
 }
 
-}  // namespace
-
-/* ------------------------------------------------------------------------------------------------ */
-/* Allocation-free indirect launches: the per-launch tables live in a fixed device array instead of context-owned
- * scratch that is grown with cudaMalloc.                                                                          */
-
-#define GINT_STATIC_MAX_PROGRAMS 64
-#define GINT_STATIC_MAX_GRID 4096
-
-struct StaticScratch {
-    gint_tensor_info ti[GINT_STATIC_MAX_PROGRAMS];        // per-program descriptor blocks, base pointers filled in
-    gint::IndirectEntry table[GINT_STATIC_MAX_GRID];       // per-logical-program {code, descriptors, length}
+/* What a program's creation decides on the host: the streams (pre-decoded instructions, to be copied to the device) and, in the
+ * Program, what a launch has to know about them. */
+struct ProgramStreams {
+    std::vector<uint2> pre, early, rf, vec, wide;
 };
 
-/* 166 KiB that every GPU which loads this library holds until the process exits. In host code this name is only a
- * stand-in for the device object: it must never be handed to a kernel; the device address comes from
- * cudaGetSymbolAddress (static_scratch_for_device below). */
-static __device__ __align__(256) unsigned char g_static_scratch[sizeof(StaticScratch)];
-
-namespace {
-
-constexpr int kMaxDevices = 64;
-void *g_static_scratch_dev[kMaxDevices];          // device address of g_static_scratch, per device; nullptr = not set up
-unsigned char g_static_host[sizeof(StaticScratch)];  // host image of the tables for the call in progress
-std::mutex g_static_mu;                            // one allocation-free launch at a time: set-up, table upload and kernel launch
-
-/* Once per device, with that device current: resolve the device address of the scratch array. The caller holds g_static_mu,
- * so two threads making their first call at the same time do the set-up once and neither sees a half-made entry. Nothing has
- * to be cleared: every call writes each table entry that its kernel reads before that kernel is queued. */
-int static_scratch_for_device(gint_ctx *ctx, void **out)
+int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, Program **out, ProgramStreams *streams)
 {
-    if (ctx->device < 0 || ctx->device >= kMaxDevices) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "device ordinal out of range");
-    if (!g_static_scratch_dev[ctx->device]) {
-        void *ptr = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&ptr, g_static_scratch);
-        if (e != cudaSuccess || !ptr) return fail(ctx, GINT_ERR_CUDA, "cudaGetSymbolAddress(static scratch)", e);
-        g_static_scratch_dev[ctx->device] = ptr;
-    }
-    *out = g_static_scratch_dev[ctx->device];
-    return GINT_OK;
-}
-
-/* The indirect entry points upload their tables from a host image that the next call overwrites; a captured copy would read
- * that image again at every replay. They therefore refuse a stream that is being captured. */
-int refuse_capture(gint_ctx *ctx, cudaStream_t stream, const char *who)
-{
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaError_t e = cudaStreamIsCapturing(stream, &st);
-    if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, GINT_ERR_CUDA, "cudaStreamIsCapturing", e); }
-    if (st != cudaStreamCaptureStatusNone) {
-        std::string msg = std::string(who) + ": the stream is being captured; indirect launches cannot be part of a CUDA graph";
-        return fail(ctx, GINT_ERR_INVALID_ARGUMENT, msg.c_str());
-    }
-    return GINT_OK;
-}
-
-}  // namespace
-
-/* ================================================================================================ */
-
-extern "C" {
-
-int gint_version(void) { return 100; }
-
-const char *gint_status_string(int status)
-{
-    switch (status) {
-    case GINT_OK: return "ok";
-    case GINT_ERR_INVALID_ARGUMENT: return "invalid argument";
-    case GINT_ERR_UNKNOWN_OPCODE: return "unknown opcode";
-    case GINT_ERR_STACK_UNDERFLOW: return "stack underflow";
-    case GINT_ERR_STACK_OVERFLOW: return "stack overflow";
-    case GINT_ERR_NO_HALT: return "program is not terminated by Halt";
-    case GINT_ERR_BAD_HANDLE: return "bad program handle";
-    case GINT_ERR_ARG_COUNT: return "number of arguments does not match the program";
-    case GINT_ERR_CUDA: return "CUDA error";
-    case GINT_ERR_NO_DEVICE: return "no usable device or kernel image";
-    case GINT_ERR_TOO_LARGE: return "program or batch too large";
-    case GINT_ERR_OUT_OF_MEMORY: return "out of memory";
-    }
-    return "unknown status";
-}
-
-int gint_sizeof_tensor_info(void) { return (int)sizeof(gint_tensor_info); }
-
-int gint_analyze(const int32_t *code, int n_words, gint_bytecode_stats *out) { return analyze(code, n_words, out); }
-
-int gint_predecode(const int32_t *code, int n_words, uint32_t *out_keys, int max_keys)
-{
-    std::vector<uint2> pre;
-    std::vector<int> depths;
-    int rc = predecode(code, n_words, GINT_MAX_TENSORS, &pre, &depths);
-    if (rc != GINT_OK) return rc;
-    gint_bytecode_stats st;
-    analyze(code, n_words, &st);
-    const int n = st.num_instructions + 1;
-    if (out_keys) {
-        if (max_keys < n) return GINT_ERR_INVALID_ARGUMENT;
-        for (int i = 0; i < n; i++) out_keys[i] = (uint32_t)depths[(size_t)i] * GINT_N_OPCODES + pre[(size_t)i].y;
-    }
-    return n;
-}
-
-int gint_debug_predecode_batch(const int32_t *code, int n_words, int n_tensors, uint32_t *out_words, int max_words)
-{
-    std::vector<uint2> whole;
-    std::vector<uint2> once((size_t)(n_words / 2 + 4));
-    uint32_t n = 0;
-    const int rc = predecode(code, n_words, n_tensors, &whole), rc1 = predecode_into(code, n_words, n_tensors, once.data(), &n);
-    if (rc != rc1) return INT32_MIN;
-    if (rc != GINT_OK) return rc;
-    if (n != whole.size() || memcmp(whole.data(), once.data(), n * sizeof(uint2)) != 0) return INT32_MIN;
-    if (out_words) memcpy(out_words, once.data(), (n * 2 < (uint32_t)max_words ? n * 2 : (uint32_t)max_words) * sizeof(uint32_t));
-    return (int)n;
-}
-
-int gint_create(int device, gint_ctx **out)
-{
-    if (!out) return GINT_ERR_INVALID_ARGUMENT;
-    *out = nullptr;
-    int count = 0;
-    if (cudaGetDeviceCount(&count) != cudaSuccess || device < 0 || device >= count) {
-        cudaGetLastError();
-        return GINT_ERR_NO_DEVICE;
-    }
-    DeviceGuard guard(device);
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) { cudaGetLastError(); return GINT_ERR_NO_DEVICE; }
-    gint_ctx *ctx = new gint_ctx();
-    ctx->device = device;
-    ctx->num_sms = prop.multiProcessorCount;
-    ctx->max_smem_optin = (int)prop.sharedMemPerBlockOptin;
-    if (load_images() == 0) {  // the library carries sm_100a code only
-        delete ctx;
-        return GINT_ERR_NO_DEVICE;
-    }
-    for (auto &im : g_images) {
-        if (!im.loaded) continue;
-        if (im.K == 0) ctx->indirect.fn = (const void *)im.kernel;
-        else if (im.K < 0) ctx->checked.fn = (const void *)im.kernel;
-        else ctx->direct.push_back(Variant{im.P, im.K, (const void *)im.kernel, 0, false, 0, im.rf, im.vec, im.wide});
-    }
-    int usable = 0;
-    for (auto &v : ctx->direct) {
-        cudaFuncAttributes attr;
-        cudaError_t e = cudaFuncGetAttributes(&attr, v.fn);
-        if (e == cudaSuccess) {
-            v.regs = attr.numRegs;
-            v.ok = true;
-            usable++;
-            int bps = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, v.fn, gint::kThreadsPerBlock, 2048) == cudaSuccess)
-                v.resident_warps = bps * ctx->num_sms * gint::kWarpsPerBlock;
-            else cudaGetLastError();
-        } else cudaGetLastError();
-    }
-    if (ctx->indirect.fn) {
-        cudaFuncAttributes attr;
-        if (cudaFuncGetAttributes(&attr, ctx->indirect.fn) == cudaSuccess) { ctx->indirect.regs = attr.numRegs; ctx->indirect.ok = true; }
-        else cudaGetLastError();
-    }
-    if (ctx->checked.fn) {
-        cudaFuncAttributes attr;
-        if (cudaFuncGetAttributes(&attr, ctx->checked.fn) == cudaSuccess) { ctx->checked.regs = attr.numRegs; ctx->checked.ok = true; }
-        else cudaGetLastError();
-    }
-    if (usable == 0) {
-        delete ctx;
-        return GINT_ERR_NO_DEVICE;
-    }
-    *out = ctx;
-    return GINT_OK;
-}
-
-void gint_destroy(gint_ctx *ctx)
-{
-    if (!ctx) return;
-    {
-        DeviceGuard guard(ctx->device);
-        for (Program *p : ctx->programs) {
-            if (p) {
-                if (p->code_dev) cudaFree(p->code_dev);
-                if (p->early_dev) cudaFree(p->early_dev);
-                if (p->rf_dev) cudaFree(p->rf_dev);
-                if (p->vec_dev) cudaFree(p->vec_dev);
-                if (p->wide_dev) cudaFree(p->wide_dev);
-                delete p;
-            }
-        }
-        if (ctx->status_dev) cudaFree(ctx->status_dev);
-        if (ctx->ind_dev) cudaFree(ctx->ind_dev);
-        if (ctx->ind_host) cudaFreeHost(ctx->ind_host);
-        if (ctx->ind_event) cudaEventDestroy(ctx->ind_event);
-        if (ctx->ind_kernel_event) cudaEventDestroy(ctx->ind_kernel_event);
-    }
-    delete ctx;
-}
-
-const char *gint_last_error(gint_ctx *ctx) { return ctx ? ctx->last_error.c_str() : "no context"; }
-
-int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors,
-                        uint64_t *out_handle)
-{
-    if (!ctx || !code || !out_handle || (!ti && n_tensors > 0)) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "null argument");
-    if (n_tensors < 0 || n_tensors > GINT_MAX_TENSORS) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "at most 8 tensors");
-    std::vector<uint2> pre;
+    std::vector<uint2> &pre = streams->pre, &early = streams->early, &rfs = streams->rf, &vecs = streams->vec, &wides = streams->wide;
     {
         std::vector<Insn> plain;
         int rc = normalise(code, n_words, n_tensors, &plain);
@@ -1639,7 +1465,6 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
     if (ti) p->ti = *ti;
     for (int t = 0; t < GINT_MAX_TENSORS; t++) p->ti.base_ptr[t] = 0;
     compute_footprints(code, p->st.num_instructions, p->ti, n_tensors, p);
-    std::vector<uint2> early, rfs, vecs, wides;
     for (int t = 0; t < n_tensors; t++) p->extent[t] = tensor_extent_bytes(p->ti, t);
     {
         std::vector<Insn> prog;
@@ -1783,6 +1608,243 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
     p->rf_slots = (uint32_t)rfs.size();
     p->vec_slots = (uint32_t)vecs.size();
     p->wide_slots = (uint32_t)wides.size();
+    *out = p;
+    return GINT_OK;
+}
+
+}  // namespace
+
+/* ------------------------------------------------------------------------------------------------ */
+/* Allocation-free indirect launches: the per-launch tables live in a fixed device array instead of context-owned
+ * scratch that is grown with cudaMalloc.                                                                          */
+
+#define GINT_STATIC_MAX_PROGRAMS 64
+#define GINT_STATIC_MAX_GRID 4096
+
+struct StaticScratch {
+    gint_tensor_info ti[GINT_STATIC_MAX_PROGRAMS];        // per-program descriptor blocks, base pointers filled in
+    gint::IndirectEntry table[GINT_STATIC_MAX_GRID];       // per-logical-program {code, descriptors, length}
+};
+
+/* 166 KiB that every GPU which loads this library holds until the process exits. In host code this name is only a
+ * stand-in for the device object: it must never be handed to a kernel; the device address comes from
+ * cudaGetSymbolAddress (static_scratch_for_device below). */
+static __device__ __align__(256) unsigned char g_static_scratch[sizeof(StaticScratch)];
+
+namespace {
+
+constexpr int kMaxDevices = 64;
+void *g_static_scratch_dev[kMaxDevices];          // device address of g_static_scratch, per device; nullptr = not set up
+unsigned char g_static_host[sizeof(StaticScratch)];  // host image of the tables for the call in progress
+std::mutex g_static_mu;                            // one allocation-free launch at a time: set-up, table upload and kernel launch
+
+/* Once per device, with that device current: resolve the device address of the scratch array. The caller holds g_static_mu,
+ * so two threads making their first call at the same time do the set-up once and neither sees a half-made entry. Nothing has
+ * to be cleared: every call writes each table entry that its kernel reads before that kernel is queued. */
+int static_scratch_for_device(gint_ctx *ctx, void **out)
+{
+    if (ctx->device < 0 || ctx->device >= kMaxDevices) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "device ordinal out of range");
+    if (!g_static_scratch_dev[ctx->device]) {
+        void *ptr = nullptr;
+        cudaError_t e = cudaGetSymbolAddress(&ptr, g_static_scratch);
+        if (e != cudaSuccess || !ptr) return fail(ctx, GINT_ERR_CUDA, "cudaGetSymbolAddress(static scratch)", e);
+        g_static_scratch_dev[ctx->device] = ptr;
+    }
+    *out = g_static_scratch_dev[ctx->device];
+    return GINT_OK;
+}
+
+/* The indirect entry points upload their tables from a host image that the next call overwrites; a captured copy would read
+ * that image again at every replay. They therefore refuse a stream that is being captured. */
+int refuse_capture(gint_ctx *ctx, cudaStream_t stream, const char *who)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(stream, &st);
+    if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, GINT_ERR_CUDA, "cudaStreamIsCapturing", e); }
+    if (st != cudaStreamCaptureStatusNone) {
+        std::string msg = std::string(who) + ": the stream is being captured; indirect launches cannot be part of a CUDA graph";
+        return fail(ctx, GINT_ERR_INVALID_ARGUMENT, msg.c_str());
+    }
+    return GINT_OK;
+}
+
+}  // namespace
+
+/* ================================================================================================ */
+
+extern "C" {
+
+int gint_version(void) { return 100; }
+
+const char *gint_status_string(int status)
+{
+    switch (status) {
+    case GINT_OK: return "ok";
+    case GINT_ERR_INVALID_ARGUMENT: return "invalid argument";
+    case GINT_ERR_UNKNOWN_OPCODE: return "unknown opcode";
+    case GINT_ERR_STACK_UNDERFLOW: return "stack underflow";
+    case GINT_ERR_STACK_OVERFLOW: return "stack overflow";
+    case GINT_ERR_NO_HALT: return "program is not terminated by Halt";
+    case GINT_ERR_BAD_HANDLE: return "bad program handle";
+    case GINT_ERR_ARG_COUNT: return "number of arguments does not match the program";
+    case GINT_ERR_CUDA: return "CUDA error";
+    case GINT_ERR_NO_DEVICE: return "no usable device or kernel image";
+    case GINT_ERR_TOO_LARGE: return "program or batch too large";
+    case GINT_ERR_OUT_OF_MEMORY: return "out of memory";
+    }
+    return "unknown status";
+}
+
+int gint_sizeof_tensor_info(void) { return (int)sizeof(gint_tensor_info); }
+
+int gint_analyze(const int32_t *code, int n_words, gint_bytecode_stats *out) { return analyze(code, n_words, out); }
+
+int gint_predecode(const int32_t *code, int n_words, uint32_t *out_keys, int max_keys)
+{
+    std::vector<uint2> pre;
+    std::vector<int> depths;
+    int rc = predecode(code, n_words, GINT_MAX_TENSORS, &pre, &depths);
+    if (rc != GINT_OK) return rc;
+    gint_bytecode_stats st;
+    analyze(code, n_words, &st);
+    const int n = st.num_instructions + 1;
+    if (out_keys) {
+        if (max_keys < n) return GINT_ERR_INVALID_ARGUMENT;
+        for (int i = 0; i < n; i++) out_keys[i] = (uint32_t)depths[(size_t)i] * GINT_N_OPCODES + pre[(size_t)i].y;
+    }
+    return n;
+}
+
+int gint_debug_predecode_batch(const int32_t *code, int n_words, int n_tensors, uint32_t *out_words, int max_words)
+{
+    std::vector<uint2> whole;
+    std::vector<uint2> once((size_t)(n_words / 2 + 4));
+    uint32_t n = 0;
+    const int rc = predecode(code, n_words, n_tensors, &whole), rc1 = predecode_into(code, n_words, n_tensors, once.data(), &n);
+    if (rc != rc1) return INT32_MIN;
+    if (rc != GINT_OK) return rc;
+    if (n != whole.size() || memcmp(whole.data(), once.data(), n * sizeof(uint2)) != 0) return INT32_MIN;
+    if (out_words) memcpy(out_words, once.data(), (n * 2 < (uint32_t)max_words ? n * 2 : (uint32_t)max_words) * sizeof(uint32_t));
+    return (int)n;
+}
+
+int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs, uint32_t first,
+                     uint32_t count, uint32_t gather_mask, uint64_t gather_extent_bytes)
+{
+    if (!code || (!(ti && base_ptrs) && n_tensors > 0) || n_tensors < 0 || n_tensors > GINT_MAX_TENSORS) return GINT_ERR_INVALID_ARGUMENT;
+    gint_ctx ctx;   // (the default options; no device)
+    for (const auto &im : g_images)
+        if (im.K > 0) {
+            ctx.direct.push_back(Variant{im.P, im.K, nullptr, 0, false, 0, im.rf, im.vec, im.wide});
+            ctx.direct.back().ok = true;
+        }
+    Program *p = nullptr;
+    ProgramStreams streams;
+    const int rc = build_program(&ctx, code, n_words, ti, n_tensors, &p, &streams);
+    if (rc != GINT_OK) return rc;
+    const GatherArgs ga{gather_mask, nullptr, gather_extent_bytes, 1u};
+    const Route r = choose_route(&ctx, p, base_ptrs, first, count, gather_mask ? &ga : nullptr);
+    const bool flat = p->flat_tiles != 0;
+    delete p;
+    return r.wide ? (r.wide << 4) | (flat ? 1 << 6 : 0) : (r.early ? 1 : 0) | (r.rf ? 2 : 0) | (r.vec ? 4 : 0);
+}
+
+int gint_create(int device, gint_ctx **out)
+{
+    if (!out) return GINT_ERR_INVALID_ARGUMENT;
+    *out = nullptr;
+    int count = 0;
+    if (cudaGetDeviceCount(&count) != cudaSuccess || device < 0 || device >= count) {
+        cudaGetLastError();
+        return GINT_ERR_NO_DEVICE;
+    }
+    DeviceGuard guard(device);
+    cudaDeviceProp prop;
+    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) { cudaGetLastError(); return GINT_ERR_NO_DEVICE; }
+    gint_ctx *ctx = new gint_ctx();
+    ctx->device = device;
+    ctx->num_sms = prop.multiProcessorCount;
+    ctx->max_smem_optin = (int)prop.sharedMemPerBlockOptin;
+    if (load_images() == 0) {  // the library carries sm_100a code only
+        delete ctx;
+        return GINT_ERR_NO_DEVICE;
+    }
+    for (auto &im : g_images) {
+        if (!im.loaded) continue;
+        if (im.K == 0) ctx->indirect.fn = (const void *)im.kernel;
+        else if (im.K < 0) ctx->checked.fn = (const void *)im.kernel;
+        else ctx->direct.push_back(Variant{im.P, im.K, (const void *)im.kernel, 0, false, 0, im.rf, im.vec, im.wide});
+    }
+    int usable = 0;
+    for (auto &v : ctx->direct) {
+        cudaFuncAttributes attr;
+        cudaError_t e = cudaFuncGetAttributes(&attr, v.fn);
+        if (e == cudaSuccess) {
+            v.regs = attr.numRegs;
+            v.ok = true;
+            usable++;
+            int bps = 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, v.fn, gint::kThreadsPerBlock, 2048) == cudaSuccess)
+                v.resident_warps = bps * ctx->num_sms * gint::kWarpsPerBlock;
+            else cudaGetLastError();
+        } else cudaGetLastError();
+    }
+    if (ctx->indirect.fn) {
+        cudaFuncAttributes attr;
+        if (cudaFuncGetAttributes(&attr, ctx->indirect.fn) == cudaSuccess) { ctx->indirect.regs = attr.numRegs; ctx->indirect.ok = true; }
+        else cudaGetLastError();
+    }
+    if (ctx->checked.fn) {
+        cudaFuncAttributes attr;
+        if (cudaFuncGetAttributes(&attr, ctx->checked.fn) == cudaSuccess) { ctx->checked.regs = attr.numRegs; ctx->checked.ok = true; }
+        else cudaGetLastError();
+    }
+    if (usable == 0) {
+        delete ctx;
+        return GINT_ERR_NO_DEVICE;
+    }
+    *out = ctx;
+    return GINT_OK;
+}
+
+void gint_destroy(gint_ctx *ctx)
+{
+    if (!ctx) return;
+    {
+        DeviceGuard guard(ctx->device);
+        for (Program *p : ctx->programs) {
+            if (p) {
+                if (p->code_dev) cudaFree(p->code_dev);
+                if (p->early_dev) cudaFree(p->early_dev);
+                if (p->rf_dev) cudaFree(p->rf_dev);
+                if (p->vec_dev) cudaFree(p->vec_dev);
+                if (p->wide_dev) cudaFree(p->wide_dev);
+                delete p;
+            }
+        }
+        if (ctx->status_dev) cudaFree(ctx->status_dev);
+        if (ctx->ind_dev) cudaFree(ctx->ind_dev);
+        if (ctx->ind_host) cudaFreeHost(ctx->ind_host);
+        if (ctx->ind_event) cudaEventDestroy(ctx->ind_event);
+        if (ctx->ind_kernel_event) cudaEventDestroy(ctx->ind_kernel_event);
+    }
+    delete ctx;
+}
+
+const char *gint_last_error(gint_ctx *ctx) { return ctx ? ctx->last_error.c_str() : "no context"; }
+
+int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors,
+                        uint64_t *out_handle)
+{
+    if (!ctx || !code || !out_handle || (!ti && n_tensors > 0)) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "null argument");
+    if (n_tensors < 0 || n_tensors > GINT_MAX_TENSORS) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "at most 8 tensors");
+    Program *p = nullptr;
+    ProgramStreams streams;
+    {
+        const int rc = build_program(ctx, code, n_words, ti, n_tensors, &p, &streams);
+        if (rc != GINT_OK) return rc;
+    }
+    const std::vector<uint2> &pre = streams.pre, &early = streams.early, &rfs = streams.rf, &vecs = streams.vec, &wides = streams.wide;
     for (int i = 0; i < gint::kInlineCodeSlots; i++) {
         p->code_inline[i] = (size_t)i < pre.size() ? pre[(size_t)i] : make_uint2(0u, OP_Halt);
         p->early_inline[i] = (size_t)i < early.size() ? early[(size_t)i] : make_uint2(0u, OP_Halt);
@@ -1878,9 +1940,9 @@ int gint_program_launch_info(gint_ctx *ctx, uint64_t handle, uint32_t grid_dim, 
     if (!p) return fail(ctx, GINT_ERR_BAD_HANDLE, "unknown program handle");
     DeviceGuard guard(ctx->device);
     Geometry g;
-    const bool early = ctx->opt_early_issue && p->early_dev != nullptr;
-    const bool rf = ctx->opt_rf && p->rf_dev != nullptr && p->rf_from_early == early;
-    const bool vec = ctx->opt_vec && p->vec_dev != nullptr && early && !rf && !p->prefer_narrow && ctx->opt_tiles_per_warp != 1;
+    const bool early = ctx->opt_early_issue && p->early_slots != 0;
+    const bool rf = ctx->opt_rf && p->rf_slots != 0 && p->rf_from_early == early;
+    const bool vec = ctx->opt_vec && p->vec_slots != 0 && early && !rf && !p->prefer_narrow && ctx->opt_tiles_per_warp != 1;
     StreamView sv = stream_view(p, early, rf, vec);
     int rc = plan_direct(ctx, p, sv, grid_dim ? grid_dim : 1, &g);
     if (rc != GINT_OK && (rf || vec)) {

@@ -125,6 +125,12 @@ int gint_predecode(const int32_t *code, int n_words, uint32_t *out_keys, int max
  * far as they fit), the candidate's status, or INT32_MIN if it differs from what programs created one by one run. */
 int gint_debug_predecode_batch(const int32_t *code, int n_words, int n_tensors, uint32_t *out_words, int max_words);
 
+/* Which kernels a launch of this program with these arguments would run on (default options; needs no device): bits 4-5 the
+ * streaming kernels (1 natural, 2 vector layout; bit 6: as one flat loop), else bit 0 the early-issue stream, bit 1 virtual
+ * registers in shared memory, bit 2 the vector-layout stream, 0 the stream as written. Negative: the status of a refused program. */
+int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs,
+                     uint32_t first, uint32_t count, uint32_t gather_mask, uint64_t gather_extent_bytes);
+
 /* The instruction list the kernels actually run for a program, after the optional early-issue and fusion passes (for
  * tests; no GPU needed): out_ops[i] is a format opcode, an internal opcode (>= 106) or -1 for an instruction absorbed into
  * the fused handler before it. With early_issue != 0 the descriptors in `ti` also decide which 1-D accesses become their
