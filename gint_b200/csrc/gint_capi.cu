@@ -1312,14 +1312,19 @@ Route choose_route(const gint_ctx *ctx, const Program *p, const uint64_t *base_p
         }
         return true;
     };
-    bool fast_ok = true;   // fast accesses need aligned bases
+    /* Slots whose rows this launch finds through the row index while their stride is no whole number of 4-element groups: the index
+     * is multiplied with the stride also where the batch has one row, which program creation takes for "never moves". */
+    uint32_t ragged_rows = 0;
+    for (int t = 0; gather && t < n_tensors; t++)
+        if (((gather->mask >> t) & 1u) && p->ti.batch_strides[t][0] % 4 != 0) ragged_rows |= 1u << t;
+    bool fast_ok = (p->fast_slots & ragged_rows) == 0;   // fast accesses need aligned bases
     for (int t = 0; t < n_tensors; t++) fast_ok = fast_ok && !(((p->fast_slots >> t) & 1u) && (base_ptrs[t] & 15u) != 0);
     /* A flat launch of at most 2^21 elements is a few microseconds of latency either way; the tile kernels spread it over more
      * blocks (a + b over 2^20 elements: 9.4 us per pass, 9.9 on the streaming kernel). */
     if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid || (uint64_t)count * p->flat_tiles <= kFlatMinTiles))) {
         const bool fast_rows = p->early_slots != 0 && fast_ok && (p->wide_loop_slots & ~p->fast_slots) == 0;   // every loop access is a fast one of the tile kernels
         if (!(p->wide_rows_f32 && fast_rows) && disjoint(p->wide_alias, p->wide_extent)) {
-            bool vector = p->wide_vector;   // the vector layout, given aligned base pointers
+            bool vector = p->wide_vector && ragged_rows == 0;   // the vector layout, given aligned base pointers
             for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
             r.wide = vector ? 2 : 1;
             return r;

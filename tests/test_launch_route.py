@@ -1,0 +1,95 @@
+"""Which kernels a launch runs on, asked of the library without a device (gint_debug_route): every condition that a fast or a
+reordered stream rests on has to hold for the launch's own addresses and options."""
+import ctypes
+import os
+import sys
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+if ROOT not in sys.path:
+    sys.path.insert(0, ROOT)
+
+from gint_b200 import opcodes as O  # noqa: E402
+from gint_b200.host import capi  # noqa: E402
+
+EARLY, WIDE, WIDE_VECTOR, FLAT = 1, 1 << 4, 2 << 4, 1 << 6
+
+
+def slot(shape1, stride1=1, elm=4, batch=(1, 0), grid1=1, step1=0, shape2=1, stride2=0):
+    """One tensor slot: (shape1, stride1, elm_size, (batch shape, stride), grid dim 1, grid step 1, shape2, stride2)."""
+    return shape1, stride1, elm, batch, grid1, step1, shape2, stride2
+
+
+def descriptors(slots):
+    ti = capi.HTensorInfo()
+    for t, (shape1, stride1, elm, batch, grid1, step1, shape2, stride2) in enumerate(slots):
+        ti.elm_size[t] = elm
+        for j in range(4):
+            ti.batch_shape[t][j], ti.batch_strides[t][j] = (batch if j == 0 else (1, 0))
+        ti.block_shape_stride_1[t][0], ti.block_shape_stride_1[t][1] = shape1, stride1
+        ti.block_shape_stride_2[t][0], ti.block_shape_stride_2[t][1] = shape2, stride2
+        ti.block_grid_dims[t][0], ti.block_grid_dims[t][1] = grid1, 1
+        ti.block_grid_steps[t][0], ti.block_grid_steps[t][1] = step1, 0
+    return ti
+
+
+def words(prog):
+    return np.array([[op, operand & 0xFFFFFFFF] for op, operand in prog], dtype=np.uint32).view(np.int32).reshape(-1)
+
+
+def route(prog, slots, bases=None, first=0, count=64, gather_mask=0, gather_extent=1 << 30):
+    code, ti, n = words(prog), descriptors(slots), len(slots)
+    addr = (ctypes.c_uint64 * 8)(*(bases or [(t + 1) << 36 for t in range(n)]))
+    r = capi.load_library().gint_debug_route(code.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), code.size, ctypes.byref(ti), n, addr, first, count,
+                                             gather_mask, gather_extent)
+    assert r >= 0, r
+    return r
+
+
+def at(op, off, t):
+    return op, (off << 4) | t
+
+
+HALF = (O.LoadGlobal1DF16, O.StoreGlobal1DF16)
+SINGLE = (O.LoadGlobal1DF32, O.StoreGlobal1DF32)
+
+
+def scaled_rows(load, store, n, tiles):
+    """out = 2 * x, one row per logical program."""
+    p = []
+    for k in range(tiles):
+        p += [at(load, 128 * k, 0), (O.FMulImm, 0x40000000), at(store, 128 * k, 1)]
+    return p + [(O.Halt, 0)]
+
+
+def test_a_gathered_row_is_aligned_for_every_index():
+    """A gathered launch multiplies the row index with the batch stride also where the batch has one row, so 4-element accesses need
+    a stride of whole groups of 4 elements there too (an odd row of an odd stride starts at any byte)."""
+    for rows in (1, 2):
+        for n, aligned in ((1024, True), (1029, False), (1026, False), (1028, True)):
+            slots = [slot(n, elm=2, batch=(rows, n)), slot(n, elm=2, batch=(rows, 1032))]
+            r = route(scaled_rows(*HALF, n, 8), slots, count=rows, gather_mask=1)
+            assert r == (WIDE_VECTOR if aligned else WIDE), (rows, n, r)
+    # without the gather a batch of one row never uses its stride
+    assert route(scaled_rows(*HALF, 1029, 8), [slot(1029, elm=2, batch=(1, 1029)), slot(1029, elm=2, batch=(1, 1032))], count=1) == WIDE_VECTOR
+
+
+def test_a_gathered_f32_row_is_aligned_for_every_index():
+    """The 16-byte accesses of the tile kernels rest on the same rule."""
+    for rows in (1, 2):
+        for stride, aligned in ((1024, True), (1029, False), (1026, False)):
+            slots = [slot(1024, batch=(rows, stride)), slot(1024, batch=(rows, 1024))]
+            r = route(scaled_rows(*SINGLE, 1024, 8), slots, count=rows, gather_mask=1)
+            assert (r == EARLY) == aligned and r != WIDE_VECTOR, (rows, stride, r)
+
+
+def test_gathered_matrix_rows_are_aligned_for_every_index():
+    """... and so do 2DW rows and staged row blocks."""
+    prog = [at(O.LoadGlobal2DWF32, 0, 0), at(O.StoreGlobal2DWF32, 0, 1), (O.Halt, 0)]
+    for rows in (1, 2):
+        for stride, aligned in ((128, True), (129, False)):
+            slots = [slot(32, 4, batch=(rows, stride), shape2=4, stride2=1), slot(32, 4, batch=(rows, 128), shape2=4, stride2=1)]
+            r = route(prog, slots, count=rows, gather_mask=1)
+            assert (r == EARLY) == aligned, (rows, stride, r)
