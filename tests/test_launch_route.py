@@ -88,8 +88,7 @@ def test_a_gathered_f32_row_is_aligned_for_every_index():
 def test_gathered_matrix_rows_are_aligned_for_every_index():
     """... and so do 2DW rows and staged row blocks."""
     prog = [at(O.LoadGlobal2DWF32, 0, 0), at(O.StoreGlobal2DWF32, 0, 1), (O.Halt, 0)]
-    for rows in (1, 2):
-        for stride, aligned in ((128, True), (129, False)):
-            slots = [slot(32, 4, batch=(rows, stride), shape2=4, stride2=1), slot(32, 4, batch=(rows, 128), shape2=4, stride2=1)]
-            r = route(prog, slots, count=rows, gather_mask=1)
-            assert (r == EARLY) == aligned, (rows, stride, r)
+    for stride, aligned in ((128, True), (129, False)):
+        slots = [slot(32, 4, batch=(1, stride), shape2=4, stride2=1), slot(32, 4, batch=(1, 128), shape2=4, stride2=1)]
+        r = route(prog, slots, count=1, gather_mask=1)
+        assert (r == EARLY) == aligned, (stride, r)
