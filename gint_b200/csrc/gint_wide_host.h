@@ -38,7 +38,7 @@ bool wide_repeats(const Insn &a, const Insn &b, int tiles)
 
 /* One loop body, checked and rewritten: `body` holds format instructions, executed at stack depth d0. Fails if an instruction
  * has no wide form or touches what lies below the body's own stack other than by reading it or by adding to it. */
-bool wide_body(const std::vector<Insn> &body, int d0, std::vector<Insn> *out, int *max_depth, bool *accumulates)
+bool wide_body(const std::vector<Insn> &body, int d0, std::vector<Insn> *out, int *max_depth, int *accumulations)
 {
     std::vector<Insn> b;
     for (size_t i = 0; i < body.size();) {       // sequences with a form of their own
@@ -56,7 +56,7 @@ bool wide_body(const std::vector<Insn> &body, int d0, std::vector<Insn> *out, in
         } else b.push_back(body[i++]);
     }
     out->clear();
-    *accumulates = false;
+    *accumulations = 0;
     int d = d0, acc_reads = 0;
     auto reads_below = [&](int pos) { if (pos == d0 - 1) acc_reads = 1; return pos >= 0; };
     for (size_t i = 0; i < b.size(); i++) {
@@ -71,18 +71,18 @@ bool wide_body(const std::vector<Insn> &body, int d0, std::vector<Insn> *out, in
             return false;
         } else if (in.op == OP_Dup && i + 1 < b.size() && b[i + 1].op == OP_FMA && d - 2 == d0 - 1 && d0 >= 1) {   // acc, x: acc + x * x
             out->push_back(Insn{WOP_AccFMASquare, 0u});
-            *accumulates = true;
+            ++*accumulations;
             i++;
             d -= 1;
             continue;
         } else if (in.op == OP_FAdd && d - 2 == d0 - 1 && d0 >= 1) {
             out->push_back(Insn{WOP_AccAdd, 0u});
-            *accumulates = true;
+            ++*accumulations;
             d -= 1;
             continue;
         } else if (in.op == OP_FMA && d - 3 == d0 - 1 && d0 >= 1) {
             out->push_back(Insn{WOP_AccFMA, 0u});
-            *accumulates = true;
+            ++*accumulations;
             d -= 2;
             continue;
         } else {
@@ -97,7 +97,7 @@ bool wide_body(const std::vector<Insn> &body, int d0, std::vector<Insn> *out, in
         if (d < d0) return false;
     }
     if (d != d0) return false;
-    if (*accumulates && acc_reads) return false;   // the running value itself is also read
+    if (*accumulations && acc_reads) return false;   // the running value itself is also read
     return true;
 }
 
@@ -236,10 +236,10 @@ bool wide_transform(const std::vector<Insn> &in, const gint_tensor_info &ti, int
         }
         std::vector<Insn> body, wide;
         int body_depth = depth;
-        bool accumulates = false;
+        int accumulations = 0;
         if (len) {
             body.assign(prog.begin() + (long)i, prog.begin() + (long)(i + len));
-            if (!wide_body(body, depth, &wide, &body_depth, &accumulates) || !wide_hazards(body, ti, out->alias_slots)) len = 0;
+            if (!wide_body(body, depth, &wide, &body_depth, &accumulations) || !wide_hazards(body, ti, out->alias_slots)) len = 0;
         }
         if (!len) {
             const int post = depth + kEffects[prog[i].op].net;
@@ -250,16 +250,19 @@ bool wide_transform(const std::vector<Insn> &in, const gint_tensor_info &ti, int
             continue;
         }
         i += len * (size_t)count;
-        if (accumulates && body.back().op == OP_FAdd && p.size() - narrow_from >= len - 1) {
+        /* (the body's one sum is its last instruction: what stands before it in the first tile's instructions touches nothing below) */
+        if (accumulations == 1 && wide.back().op == WOP_AccAdd && p.size() - narrow_from >= len - 1) {
             const size_t first = p.size() - (len - 1);
+            std::vector<Insn> from_first = body, from_first_wide;
             bool same = true;
             for (size_t j = 0; same && j + 1 < len; j++) same = wide_repeats(p[first + j], body[j], 1);
-            if (same) {
-                for (size_t j = 0; j + 1 < len; j++) body[j].operand = p[first + j].operand;
+            for (size_t j = 0; same && j + 1 < len; j++) from_first[j].operand = p[first + j].operand;
+            if (same && wide_body(from_first, depth, &from_first_wide, &body_depth, &accumulations)) {
+                body = from_first;
+                wide = from_first_wide;
                 p.resize(first);
                 p.push_back(Insn{OP_LoadImm, 0x80000000u});
                 count++;
-                wide_body(body, depth, &wide, &body_depth, &accumulates);
             }
         }
         p.push_back(Insn{WOP_LoopBegin, (uint32_t)count});
@@ -273,8 +276,8 @@ bool wide_transform(const std::vector<Insn> &in, const gint_tensor_info &ti, int
     if (out->max_tiles == 0) {
         std::vector<Insn> body(prog.begin(), prog.begin() + (long)n), wide;
         int body_depth = 0;
-        bool accumulates = false;
-        if (!wide_body(body, 0, &wide, &body_depth, &accumulates) || !wide_hazards(body, ti, out->alias_slots)) return false;
+        int accumulations = 0;
+        if (!wide_body(body, 0, &wide, &body_depth, &accumulations) || !wide_hazards(body, ti, out->alias_slots)) return false;
         p.clear();
         p.push_back(Insn{WOP_LoopBegin, 1u});
         p.insert(p.end(), wide.begin(), wide.end());
