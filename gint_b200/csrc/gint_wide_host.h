@@ -98,6 +98,7 @@ bool wide_body(const std::vector<Insn> &body, int d0, std::vector<Insn> *out, in
     }
     if (d != d0) return false;
     if (*accumulations && acc_reads) return false;   // the running value itself is also read
+    if (*accumulations > 1) return false;            // U terms of one kind, then U of the other: not the program's order
     return true;
 }
 

@@ -195,3 +195,9 @@ def test_a_second_sum_below_the_running_one():
     body = [(op, arg + (128 << 4) if op in STEP else arg) for op, arg in [X, (O.FAdd, 0), Y, (O.FAdd, 0)]]
     prog = [(O.LoadImm, 0x40A00000)] + first + loop(body, 7) + [(O.FMul, 0), STORE, (O.Halt, 0)]
     check(prog, rows(3), 8)
+
+
+def test_a_sum_with_two_terms_per_tile():
+    """acc + x0 + y0 + x1 + y1 + ...: the terms keep their order."""
+    prog = [(O.LoadImm, 0)] + loop([X, (O.FAdd, 0), Y, (O.FAdd, 0)], 8) + [STORE, (O.Halt, 0)]
+    check(prog, rows(3), 8)
