@@ -114,7 +114,8 @@ bool wide_strides_disjoint(const gint_tensor_info &ti, int t, bool two_d)
 /* Accesses whose order the loop changes: tiles of one iteration group are all loaded before the first of them is stored, and
  * stores to two slots no longer alternate. Slots that a loop stores to must therefore not overlap any other slot it uses
  * (recorded, checked against the launch's address ranges); a slot that is stored to and accessed a second time must be accessed
- * at the same place, so that every tile stays with itself. */
+ * at the same place with elements of the same width, so that every tile stays with itself (tile k in f16 covers the second half of
+ * tile k / 2 in f32). */
 bool wide_hazards(const std::vector<Insn> &body, const gint_tensor_info &ti, uint8_t *alias_slots)
 {
     for (const Insn &s : body) {
@@ -125,7 +126,7 @@ bool wide_hazards(const std::vector<Insn> &body, const gint_tensor_info &ti, uin
             if (!GINT_WIDE_TILE_OP(x.op) || &x == &s) continue;
             const int u = (int)(x.operand & 15u);
             if (u != t) alias_slots[u] |= (uint8_t)(1u << t);
-            else if (x.operand != s.operand || wide_is_2dt(x.op) || wide_is_2dt(s.op)) return false;
+            else if (x.operand != s.operand || wide_element_bytes(x.op) != wide_element_bytes(s.op) || wide_is_2dt(x.op) || wide_is_2dt(s.op)) return false;
         }
     }
     return true;

@@ -201,3 +201,10 @@ def test_a_sum_with_two_terms_per_tile():
     """acc + x0 + y0 + x1 + y1 + ...: the terms keep their order."""
     prog = [(O.LoadImm, 0)] + loop([X, (O.FAdd, 0), Y, (O.FAdd, 0)], 8) + [STORE, (O.Halt, 0)]
     check(prog, rows(3), 8)
+
+
+@pytest.mark.parametrize("load,store", [(O.LoadGlobal1DF16, O.StoreGlobal1DF32), (O.LoadGlobal1DF32, O.StoreGlobal1DF16)])
+def test_a_slot_stored_to_with_another_width(load, store):
+    """Tile k of one width covers other elements than tile k of the other: the tiles' loads and stores keep their order."""
+    prog = loop([at(load, 0, 0), (O.FAddImm, 0x3F800000), at(store, 0, 0)], 8) + [(O.Halt, 0)]
+    check(prog, rows(1), 8)
