@@ -32,8 +32,8 @@ bool wide_repeats(const Insn &a, const Insn &b, int tiles)
 {
     if (a.op != b.op) return false;
     if (!GINT_WIDE_TILE_OP(a.op)) return a.operand == b.operand || !GINT_OP_USES_OPERAND(a.op);
-    const uint32_t step = wide_is_2dt(a.op) ? 32u : 128u;
-    return b.operand == a.operand + (uint32_t)tiles * (step << 4);
+    const uint64_t step = wide_is_2dt(a.op) ? 32u : 128u;
+    return b.operand == a.operand + (uint64_t)tiles * (step << 4);   // (no wrap: an offset has 28 bits, the one behind the last is 0)
 }
 
 /* One loop body, checked and rewritten: `body` holds format instructions, executed at stack depth d0. Fails if an instruction

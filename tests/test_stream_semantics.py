@@ -208,3 +208,12 @@ def test_a_slot_stored_to_with_another_width(load, store):
     """Tile k of one width covers other elements than tile k of the other: the tiles' loads and stores keep their order."""
     prog = loop([at(load, 0, 0), (O.FAddImm, 0x3F800000), at(store, 0, 0)], 8) + [(O.Halt, 0)]
     check(prog, rows(1), 8)
+
+
+def test_offsets_that_wrap():
+    """The offset of an access has 28 bits: after 2^28 - 128 comes 0, which is no further tile of a loop."""
+    def body(k):
+        off = ((1 << 28) + 128 * (k - 2)) % (1 << 28)
+        return [at(O.LoadGlobal1DF32, off, 0), at(O.StoreGlobal1DF32, off, 1)]
+    prog = [x for k in range(4) for x in body(k)] + [(O.Halt, 0)]
+    check(prog, rows(2), 4)
