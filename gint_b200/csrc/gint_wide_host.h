@@ -297,11 +297,14 @@ bool wide_transform(const std::vector<Insn> &in, const gint_tensor_info &ti, int
     for (size_t i = 1; i + 2 < p.size(); i++)
         flat = flat && p[i].op >= WOP_LoopBegin && p[i].op != WOP_LoopBegin && p[i].op != WOP_LoopEnd && !wide_is_2dt(p[i].op - GINT_WIDE_FIRST);
     uint32_t grid = 0;
+    int64_t last_offset = 0;   // of the program as written; a flat loop adds up to the whole grid's elements to it
+    for (size_t i = 0; i < n; i++)
+        if (is_tensor_op(prog[i].op) && (int64_t)(prog[i].operand >> 4) > last_offset) last_offset = (int64_t)(prog[i].operand >> 4);
     for (int t = 0; flat && t < n_tensors; t++) {
         if (!((used >> t) & 1u)) continue;
         const int64_t gd1 = (uint32_t)ti.block_grid_dims[t][0];
         flat = (uint32_t)ti.block_grid_dims[t][1] == 1u && ti.block_grid_steps[t][0] == out->max_tiles * 128 && gd1 >= 1 &&
-               gd1 * ti.block_grid_steps[t][0] < (1ll << 31) - 8192 && (grid == 0 || grid == (uint32_t)gd1);
+               gd1 * ti.block_grid_steps[t][0] + last_offset < (1ll << 31) - 8192 && (grid == 0 || grid == (uint32_t)gd1);
         for (int j = 0; j < 4; j++) flat = flat && ti.batch_shape[t][j] == 1;
         grid = (uint32_t)gd1;
     }

@@ -92,3 +92,14 @@ def test_gathered_matrix_rows_are_aligned_for_every_index():
         slots = [slot(32, 4, batch=(1, stride), shape2=4, stride2=1), slot(32, 4, batch=(1, 128), shape2=4, stride2=1)]
         r = route(prog, slots, count=1, gather_mask=1)
         assert (r == EARLY) == aligned, (stride, r)
+
+
+def test_a_flat_loop_stays_below_31_bits():
+    """A flat launch counts elements through the whole grid, and the offset written in the program comes on top: the sum has to fit an
+    int, or a masked access far behind the tensor becomes an unmasked one in front of it."""
+    n_programs = 15_000_000
+    for off in (0, 128, (1 << 28) - 128):
+        prog = [at(O.LoadGlobal1DF32, off, 0), at(O.StoreGlobal1DF32, off, 1), (O.Halt, 0)]
+        slots = [slot(100000, grid1=n_programs, step1=128)] * 2
+        r = route(prog, slots, count=n_programs)
+        assert bool(r & FLAT) == (n_programs * 128 + off < (1 << 31) - 8192), (off, r)
