@@ -217,3 +217,66 @@ def test_offsets_that_wrap():
         return [at(O.LoadGlobal1DF32, off, 0), at(O.StoreGlobal1DF32, off, 1)]
     prog = [x for k in range(4) for x in body(k)] + [(O.Halt, 0)]
     check(prog, rows(2), 4)
+
+
+def random_body(rng, depth):
+    """Instructions with no net effect on the stack that read a few values below it."""
+    out, d = [], depth
+    for _ in range(rng.randrange(2, 9)):
+        choice = [[X], [Y], [at(O.LoadGlobal1DF32, 128, 0)], [(O.LoadImm, rng.randrange(4))]] if d < 4 else []
+        if d >= 1:
+            choice += [[(O.Dup, 0)], [(O.FMulImm, rng.randrange(4))], [(O.FNeg, 0)], [STORE], [(O.Pop, 0)]]
+        if d >= 2:
+            choice += [[(op, 0)] for op in (O.FAdd, O.FMul, O.FSub, O.Swap, O.DupX1, O.Dup2, O.FGt)] + [[(O.FAdd, 0)]] * 3
+            choice += [[(O.Dup, 0), (O.FMul, 0)], [(O.Dup, 0), X, (O.FMul, 0)], [(O.Dup, 0), Y, (O.Swap, 0), (O.FMul, 0)]]
+        if d >= 3:
+            choice += [[(op, 0)] for op in (O.FMA, O.Select, O.DupX2)] + [[(O.Dup, 0), (O.FMA, 0)]]
+        if d >= 1:
+            choice += [[(O.Dup, 0), (O.FNeg, 0), (O.FExp, 0), (O.FAddImm, 0x3F800000), (O.FRDiv, 0)]]
+        for ins in rng.choice(choice):
+            out.append(ins)
+            d += EFFECT[ins[0]]
+    while d > depth:
+        out.append((rng.choice((O.FAdd, O.Pop)), 0) if d >= 2 else (O.Pop, 0))
+        d -= 1
+    while d < depth:
+        out.append(X)
+        d += 1
+    return out
+
+
+EFFECT = {O.LoadGlobal1DF32: 1, O.StoreGlobal1DF32: -1, O.LoadImm: 1, O.Dup: 1, O.FMulImm: 0, O.FNeg: 0, O.Pop: -1, O.FAdd: -1, O.FMul: -1, O.FSub: -1,
+          O.Swap: 0, O.DupX1: 1, O.Dup2: 2, O.FGt: -1, O.FMA: -2, O.Select: -2, O.DupX2: 1, O.FExp: 0, O.FAddImm: 0, O.FRDiv: -1}
+
+
+@pytest.mark.parametrize("seed", range(60))
+def test_random_loops(seed):
+    """Bodies repeated over tiles, some behind a first tile whose last instructions are missing, at several stack depths."""
+    rng, streams = random.Random(seed), 0
+    for _ in range(120):
+        depth, tiles = rng.randrange(4), rng.randrange(2, 12)
+        prog = [(O.LoadImm, 100 + k) for k in range(depth)]
+        for _ in range(rng.randrange(1, 3)):
+            body = random_body(rng, depth)
+            whole = loop(body, tiles)
+            cut = rng.choice((0, 0, 1, 2))
+            lost = body[len(body) - cut:]
+            if cut and body[-1][0] == O.FAdd and depth + 1 <= 4 and sum(EFFECT[op] for op, _ in lost) < 0:
+                d0 = depth - sum(EFFECT[op] for op, _ in body[:len(body) - cut])
+                if d0 < 0 or d0 > depth:
+                    continue
+                whole = whole[:len(body) - cut] + whole[len(body):]
+                prog += whole + [(O.Pop, 0)] * (-sum(EFFECT[op] for op, _ in lost))
+            else:
+                prog += whole
+        prog.append((O.Halt, 0))
+        d, ok = 0, True
+        for op, _ in prog[:-1]:
+            need = {O.FMA: 3, O.Select: 3, O.DupX2: 3}.get(op, 2 if op in (O.FAdd, O.FMul, O.FSub, O.Swap, O.DupX1, O.Dup2, O.FGt, O.FRDiv) else
+                                                           0 if op in (O.LoadGlobal1DF32, O.LoadImm) else 1)
+            ok = ok and d >= need
+            d += EFFECT[op]
+            ok = ok and d <= 8
+        if ok:
+            streams += check(prog, rows(3), tiles)
+    assert streams >= 5
