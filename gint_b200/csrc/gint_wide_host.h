@@ -164,9 +164,10 @@ bool wide_vector(WideStream *ws, const gint_tensor_info &ti, int n_tensors)
         } else switch (x.op) {
         case WOP_LoopBegin: if (x.operand % 4u != 0) in_fours = false; break;
         case WOP_LoopEnd: break;
-        case WOP_AccAdd: accumulates = true; emit(OP_FAdd, 0u, i); break;
-        case WOP_AccFMA: accumulates = true; emit(OP_FMA, 0u, i); break;
-        case WOP_AccFMASquare: accumulates = true; emit(OP_Dup, 0u, i); emit(OP_FMA, 0u, i); break;
+        /* (the addition that follows a sum stands for "after this loop's tiles": equal sums of two loops are two values) */
+        case WOP_AccAdd: accumulates = true; emit(OP_FAdd, 0u, i); emit(OP_FAddImm, (uint32_t)i, i); break;
+        case WOP_AccFMA: accumulates = true; emit(OP_FMA, 0u, i); emit(OP_FAddImm, (uint32_t)i, i); break;
+        case WOP_AccFMASquare: accumulates = true; emit(OP_Dup, 0u, i); emit(OP_FMA, 0u, i); emit(OP_FAddImm, (uint32_t)i, i); break;
         case WOP_Square: emit(OP_Dup, 0u, i); emit(OP_FMul, 0u, i); break;
         case WOP_MulKeep: emit(OP_Swap, 0u, i); emit(OP_DupX1, 0u, i); emit(OP_FMul, 0u, i); break;   // [s, x] -> [x, s] -> [s, x, s] -> [s, s x]
         case WOP_Silu: emit(OP_Dup, 0u, i); emit(OP_FNeg, 0u, i); emit(OP_FExp, 0u, i); emit(OP_FAddImm, x.operand, i); emit(OP_FRDiv, 0u, i); break;

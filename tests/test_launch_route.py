@@ -103,3 +103,22 @@ def test_a_flat_loop_stays_below_31_bits():
         slots = [slot(100000, grid1=n_programs, step1=128)] * 2
         r = route(prog, slots, count=n_programs)
         assert bool(r & FLAT) == (n_programs * 128 + off < (1 << 31) - 8192), (off, r)
+
+
+def counted(tiles):
+    """A running value that counts the tiles of a copy loop."""
+    return [(O.LoadImm, 0)] + [i for k in range(tiles) for i in (at(HALF[0], 128 * k, 0), at(HALF[1], 128 * k, 1), (O.LoadImm, 0x3F800000), (O.FAdd, 0))]
+
+
+@pytest.mark.parametrize("second", [4, 8])
+def test_equal_running_values_of_two_loops_are_not_one_value(second):
+    """A value that is the same in all four width positions may multiply data in the vector layout. Two loops that add the same terms
+    to the same start give the same value only if they run equally often, so a shuffle of both is not such a value."""
+    prog = counted(4) + counted(second) + [(O.FShuf2, 0)]      # two positions of each
+    for k in range(8):
+        prog += [(O.Dup, 0), at(HALF[0], 128 * k, 0), (O.FMul, 0), at(HALF[1], 128 * k, 1)]
+    prog += [(O.Pop, 0), (O.Halt, 0)]
+    rows = [slot(1024, elm=2, batch=(64, 1024))] * 2
+    assert route(prog, rows) == WIDE
+    one = counted(4) + [i for k in range(8) for i in ((O.Dup, 0), at(HALF[0], 128 * k, 0), (O.FMul, 0), at(HALF[1], 128 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
+    assert route(one, rows) == WIDE_VECTOR
