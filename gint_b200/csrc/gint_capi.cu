@@ -1006,7 +1006,7 @@ struct Program {
     uint32_t wide_slots = 0;
     int wide_depth = 0, wide_tiles = 0;
     uint32_t flat_tiles = 0, flat_grid = 0;
-    uint8_t wide_alias[GINT_MAX_TENSORS] = {};
+    uint8_t wide_alias[GINT_MAX_TENSORS] = {}, wide_vector_alias[GINT_MAX_TENSORS] = {};
     uint64_t wide_extent[GINT_MAX_TENSORS] = {};
     uint32_t wide_align[GINT_MAX_TENSORS] = {};   // alignment of the base pointers that the vector-layout kernels need (minus 1); all 0: never
     bool wide_vector = false;
@@ -1326,6 +1326,7 @@ Route choose_route(const gint_ctx *ctx, const Program *p, const uint64_t *base_p
         if (!(p->wide_rows_f32 && fast_rows) && disjoint(p->wide_alias, p->wide_extent)) {
             bool vector = p->wide_vector && ragged_rows == 0;   // the vector layout, given aligned base pointers
             for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
+            vector = vector && disjoint(p->wide_vector_alias, p->wide_extent);
             r.wide = vector ? 2 : 1;
             return r;
         }
@@ -1501,6 +1502,7 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
                 if (op != OP_LoadGlobal1DF32 && op != OP_StoreGlobal1DF32) p->wide_rows_f32 = false;
             }
             memcpy(p->wide_alias, ws.alias_slots, sizeof(p->wide_alias));
+            memcpy(p->wide_vector_alias, ws.vector_alias, sizeof(p->wide_vector_alias));
             bool have_vector = false;
             for (auto &v : ctx->direct) have_vector = have_vector || (v.wide == 2 && v.ok && v.P >= ws.max_depth);
             p->wide_vector = ws.vector && have_vector;

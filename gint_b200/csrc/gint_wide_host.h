@@ -14,6 +14,7 @@ struct WideStream {
     uint32_t flat_tiles = 0;                       // tiles per logical program if the program is one flat loop, else 0
     uint32_t flat_grid = 0;                        // logical programs the flat form covers
     uint32_t access_bytes[GINT_MAX_TENSORS] = {};  // widest element with which the program accesses a slot
+    uint8_t vector_alias[GINT_MAX_TENSORS] = {};   // ... of accesses in different loops, which the vector layout makes with other lanes
     bool vector = false;                           // the kernels in the vector layout may run it (base pointers aligned to 4 elements)
 };
 
@@ -142,6 +143,23 @@ bool wide_hazards(const std::vector<Insn> &body, const gint_tensor_info &ti, uin
  */
 bool wide_vector(WideStream *ws, const gint_tensor_info &ti, int n_tensors)
 {
+    /* What a loop stores a later one may access with another lane than in the natural layout: two slots that meet in memory, or one
+     * slot at offsets that are not whole groups of 128 elements apart. Within a loop an accessed tile stays with itself. */
+    struct Access { int loop; bool store; uint32_t operand; };
+    std::vector<Access> accesses;
+    int loop = 0;
+    for (const Insn &x : ws->prog) {
+        if (x.op == WOP_LoopBegin) loop++;
+        const int op = x.op - GINT_WIDE_FIRST;
+        if (op >= 0 && GINT_WIDE_TILE_OP(op)) accesses.push_back(Access{loop, writes_tensor(op), x.operand});
+    }
+    for (const Access &s : accesses)
+        for (const Access &x : accesses) {
+            if (!s.store || x.loop == s.loop) continue;
+            const uint32_t t = s.operand & 15u, u = x.operand & 15u;
+            if (u != t) ws->vector_alias[u] |= (uint8_t)(1u << t);
+            else if (((x.operand >> 4) - (s.operand >> 4)) % 128u != 0) return false;
+        }
     std::vector<Insn> rep, marked;
     std::vector<size_t> origin;
     bool any_2dt = false, any_1d = false, accumulates = false, in_fours = true;

@@ -122,3 +122,19 @@ def test_equal_running_values_of_two_loops_are_not_one_value(second):
     assert route(prog, rows) == WIDE
     one = counted(4) + [i for k in range(8) for i in ((O.Dup, 0), at(HALF[0], 128 * k, 0), (O.FMul, 0), at(HALF[1], 128 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
     assert route(one, rows) == WIDE_VECTOR
+
+
+@pytest.mark.parametrize("shift,bases,want", [(0, None, WIDE_VECTOR), (128, None, WIDE_VECTOR), (32, None, WIDE), (64, None, WIDE),
+                                              (None, 0, WIDE), (None, 64, WIDE), (None, 1 << 20, WIDE_VECTOR)])
+def test_what_one_loop_stores_the_same_lanes_load_in_the_next(shift, bases, want):
+    """Nothing but a lane's own program order stands between a store of one loop and a load of the next. In the natural layout
+    accesses 32 elements apart meet in the same lane, in the vector layout only those 128 apart: by one slot (`shift`) or by two
+    slots over one buffer (`bases`: bytes between them)."""
+    n_slot, off = (1, shift) if shift is not None else (3, 0)
+    prog = [i for k in range(8) for i in (at(HALF[0], 128 * k, 0), at(HALF[1], 128 * k, 1))]
+    prog += [i for k in range(4) for i in (at(HALF[0], 128 * k + off, n_slot), (O.FNeg, 0), at(HALF[1], 128 * k, 2))] + [(O.Halt, 0)]
+    rows = [slot(1024, elm=2, batch=(64, 1024))] * 4
+    addr = [t << 36 for t in range(1, 5)]
+    if bases is not None:
+        addr[3] = addr[1] + bases
+    assert route(prog, rows, bases=addr) == want
