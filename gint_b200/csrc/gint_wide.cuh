@@ -14,7 +14,8 @@
  * all U tiles of its slots (its opcode is GINT_WIDE_FIRST + op); outside of loops on tile 0 alone, with the ordinary handlers.
  * LoopBegin copies what is on the stack to all U tiles. A running
  * sum is kept in tile 0 and takes the U tiles in order (AccAdd, AccFMA), so every sum has the terms and the order of the
- * program as written: results are bit-identical.
+ * program as written: results are bit-identical. The one exception are sums of 2-byte 2DT tiles in the vector layout, whose terms
+ * are added in another order (wide_vector in gint_wide_host.h).
  *
  * One warp runs one logical program. Programs that are nothing but one loop over 1-D tiles, whose logical programs follow one
  * another in memory, run "flat": the whole launch is one loop, cut among all warps.

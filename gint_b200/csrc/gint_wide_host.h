@@ -139,7 +139,8 @@ bool wide_hazards(const std::vector<Insn> &body, const gint_tensor_info &ti, uin
  * elements. And nothing may tell the layouts apart: decided by vec_transform on the stream with each loop body written once
  * (what holds after one pass of a body holds after any number). Where it asks for a rearrangement outside of loops the stream
  * gets a Remap. 2DT tiles are only taken in fours (a loop of 4 n tiles), and the one thing that may look across their lanes is a
- * sum over the warp: a lane then adds the squares of other elements than in the natural layout, and the same elements are summed.
+ * sum over the warp: a lane then adds the terms of other elements than in the natural layout, and the same elements are summed. The
+ * order of the additions is another one, so it is done for elements of 2 bytes alone; sums of f32 and u8 elements keep theirs.
  */
 bool wide_vector(WideStream *ws, const gint_tensor_info &ti, int n_tensors)
 {
@@ -162,7 +163,7 @@ bool wide_vector(WideStream *ws, const gint_tensor_info &ti, int n_tensors)
         }
     std::vector<Insn> rep, marked;
     std::vector<size_t> origin;
-    bool any_2dt = false, any_1d = false, accumulates = false, in_fours = true;
+    bool any_2dt = false, any_1d = false, accumulates = false, in_fours = true, two_bytes = true;
     auto emit = [&](int op, uint32_t operand, size_t from) { rep.push_back(Insn{op, operand}); origin.push_back(from); };
     for (size_t i = 0; i < ws->prog.size(); i++) {
         const Insn &x = ws->prog[i];
@@ -171,6 +172,7 @@ bool wide_vector(WideStream *ws, const gint_tensor_info &ti, int n_tensors)
             if (!GINT_WIDE_TILE_OP(op)) { emit(op, x.operand, i); continue; }
             const bool two = wide_is_2dt(op);
             (two ? any_2dt : any_1d) = true;
+            if (wide_element_bytes(op) != 2 && !writes_tensor(op)) two_bytes = false;
             bool ok = t < n_tensors && ti.block_shape_stride_1[t][1] == 1 && ti.elm_size[t] == wide_element_bytes(op) && ((x.operand >> 4) & 3u) == 0;
             if (ok && ti.block_grid_dims[t][0] != 1 && ti.block_grid_steps[t][0] % 4 != 0) ok = false;
             if (ok && two && ti.block_shape_stride_2[t][1] % 4 != 0) ok = false;
@@ -192,7 +194,7 @@ bool wide_vector(WideStream *ws, const gint_tensor_info &ti, int n_tensors)
         default: emit(x.op, x.operand, i);
         }
     }
-    if (any_1d == any_2dt || (any_2dt && accumulates && !in_fours)) return false;
+    if (any_1d == any_2dt || (any_2dt && accumulates && !(in_fours && two_bytes))) return false;
     int n_vector = 0, n_remaps = 0;
     if (!vec_transform(rep, &marked, &n_vector, &n_remaps, any_2dt)) return false;
     std::vector<size_t> remap_before;

@@ -292,7 +292,8 @@ int gint_execute_indirect_static(gint_ctx *ctx, const uint64_t *handles, int n_p
  * "vector_layout" (1 = programs created from now on whose full 1-D tiles can live in the pool as four consecutive elements
  * per lane run on the kernels that access them with one 16-byte access per lane; default 0: no measurable gain on the
  * benchmark programs), "streaming" (1 = launches use the streaming kernels for programs whose tile loops were found again,
- * default; results are the same bits, but for sums of 2-byte 2DT tiles, whose terms are added in another order). */
+ * default; results are the same bits, but for sums of f16 and bf16 2DT tiles whose rows and base pointers are aligned to 4
+ * elements: their terms are added in another order). */
 int gint_set_option(gint_ctx *ctx, const char *name, int value);
 
 #ifdef __cplusplus

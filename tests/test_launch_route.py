@@ -138,3 +138,15 @@ def test_what_one_loop_stores_the_same_lanes_load_in_the_next(shift, bases, want
     if bases is not None:
         addr[3] = addr[1] + bases
     assert route(prog, rows, bases=addr) == want
+
+
+@pytest.mark.parametrize("load,elm,want", [(O.LoadGlobal2DTF16, 2, WIDE_VECTOR), (O.LoadGlobal2DTBF16, 2, WIDE_VECTOR), (O.LoadGlobal2DTF32, 4, WIDE),
+                                           (O.LoadGlobal2DTU8, 1, WIDE)])
+def test_only_sums_of_two_byte_2dt_tiles_change_their_order(load, elm, want):
+    """The vector layout adds the elements of 2DT tiles in another order. That is taken for 2-byte elements alone, whose values carry far
+    fewer bits than the sum; f32 and u8 sums keep the program's order, as every other sum does."""
+    prog = [(O.LoadImm, 0)] + [i for k in range(4) for i in ((load, (32 * k << 4)), (O.Dup, 0), (O.FMul, 0), (O.FAdd, 0))]
+    prog += [(O.WarpAllReduceSum, 0)]
+    prog += [i for k in range(4) for i in ((O.Dup, 0), (load, (32 * k << 4)), (O.FMul, 0), at(O.StoreGlobal2DTBF16, 32 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
+    rows = [slot(128, elm=elm, batch=(64, 512), shape2=4, stride2=128), slot(128, elm=2, batch=(64, 512), shape2=4, stride2=128)]
+    assert route(prog, rows) == want
