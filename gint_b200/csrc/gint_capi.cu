@@ -1614,6 +1614,8 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
     p->early_slots = (uint32_t)early.size();
     p->rf_slots = (uint32_t)rfs.size();
     p->vec_slots = (uint32_t)vecs.size();
+    uint32_t code_smem;
+    if ((int)direct_smem(stream_view(p, !early.empty()), 1, &code_smem) > ctx->max_smem_optin) wides.clear();   // the tile kernels refuse it
     p->wide_slots = (uint32_t)wides.size();
     *out = p;
     return GINT_OK;
@@ -1740,6 +1742,7 @@ int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *t
 {
     if (!code || (!(ti && base_ptrs) && n_tensors > 0) || n_tensors < 0 || n_tensors > GINT_MAX_TENSORS) return GINT_ERR_INVALID_ARGUMENT;
     gint_ctx ctx;   // (the default options; no device)
+    ctx.max_smem_optin = 227 * 1024;
     for (const auto &im : g_images)
         if (im.K > 0) {
             ctx.direct.push_back(Variant{im.P, im.K, nullptr, 0, false, 0, im.rf, im.vec, im.wide});

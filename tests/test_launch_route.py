@@ -150,3 +150,11 @@ def test_only_sums_of_two_byte_2dt_tiles_change_their_order(load, elm, want):
     prog += [i for k in range(4) for i in ((O.Dup, 0), (load, (32 * k << 4)), (O.FMul, 0), at(O.StoreGlobal2DTBF16, 32 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
     rows = [slot(128, elm=elm, batch=(64, 512), shape2=4, stride2=128), slot(128, elm=2, batch=(64, 512), shape2=4, stride2=128)]
     assert route(prog, rows) == want
+
+
+@pytest.mark.parametrize("tiles,want", [(4000, WIDE_VECTOR), (12000, 0)])
+def test_a_program_too_long_for_the_tile_kernels_has_no_other_route(tiles, want):
+    """The tile kernels keep the whole program in shared memory and refuse one that does not fit; whether a launch is refused must not
+    depend on addresses, so such a program has no stream with loops either."""
+    rows = [slot(128 * tiles, elm=2, batch=(64, 128 * tiles))] * 2
+    assert route(scaled_rows(*HALF, 128 * tiles, tiles), rows) == want
