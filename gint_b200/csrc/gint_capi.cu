@@ -1950,28 +1950,32 @@ int gint_program_launch_info(gint_ctx *ctx, uint64_t handle, uint32_t grid_dim, 
     if (!p) return fail(ctx, GINT_ERR_BAD_HANDLE, "unknown program handle");
     DeviceGuard guard(ctx->device);
     Geometry g;
-    const bool early = ctx->opt_early_issue && p->early_slots != 0;
-    const bool rf = ctx->opt_rf && p->rf_slots != 0 && p->rf_from_early == early;
-    const bool vec = ctx->opt_vec && p->vec_slots != 0 && early && !rf && !p->prefer_narrow && ctx->opt_tiles_per_warp != 1;
-    StreamView sv = stream_view(p, early, rf, vec);
-    int rc = plan_direct(ctx, p, sv, grid_dim ? grid_dim : 1, &g);
-    if (rc != GINT_OK && (rf || vec)) {
-        sv = stream_view(p, early, false);
-        rc = plan_direct(ctx, p, sv, grid_dim ? grid_dim : 1, &g);
+    uint64_t base_ptrs[GINT_MAX_TENSORS];   // aligned and far from one another
+    for (int t = 0; t < GINT_MAX_TENSORS; t++) base_ptrs[t] = (uint64_t)(t + 1) << 44;
+    const uint32_t count = grid_dim ? grid_dim : 1;
+    const Route route = choose_route(ctx, p, base_ptrs, 0u, count, nullptr);
+    int rc;
+    if (route.wide) {
+        rc = plan_wide(ctx, p, route.wide == 2, count, &g);
+    } else {
+        rc = plan_direct(ctx, p, stream_view(p, route.early, route.rf, route.vec), count, &g);
+        if (rc != GINT_OK && (route.rf || route.vec)) rc = plan_direct(ctx, p, stream_view(p, route.early, false), count, &g);
+        g.threads = gint::kThreadsPerBlock;
     }
     if (rc != GINT_OK) return rc;
     memset(out, 0, sizeof(*out));
     out->pool_size = g.v->P;
     out->tiles_per_warp = g.v->K;
-    out->warps_per_block = gint::kWarpsPerBlock;
+    out->warps_per_block = (int32_t)g.threads / 32;
     out->grid_blocks = (int32_t)g.grid;
     out->smem_bytes = (int32_t)g.smem;
     out->regs_per_thread = g.v->regs;
     out->blocks_per_sm = g.blocks_per_sm;
     out->num_sms = ctx->num_sms;
-    out->early_loads = p->n_early;
+    out->early_loads = route.wide ? 0 : p->n_early;
     out->registers_in_smem = g.v->rf ? p->st.max_reg_idx + 1 : 0;
-    out->vector_layout = g.v->vec ? 1 : 0;
+    out->vector_layout = g.v->vec || g.v->wide == 2 ? 1 : 0;
+    out->streaming = g.v->wide ? 1 : 0;
     return GINT_OK;
 }
 

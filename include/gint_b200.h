@@ -65,10 +65,11 @@ typedef struct gint_bytecode_stats {
     int32_t reserved;
 } gint_bytecode_stats;
 
-/* How a program will be / was launched; for tests and benchmarks. */
+/* How a program will be / was launched with base pointers that are 16-byte aligned and tensors that do not overlap; for tests and
+ * benchmarks. */
 typedef struct gint_launch_info {
-    int32_t pool_size;        /* 4, 7, 12 */
-    int32_t tiles_per_warp;   /* logical programs interpreted together by one warp: 1, 2 or 4 */
+    int32_t pool_size;        /* 4, 7, 12; streaming kernels: 3, 4 */
+    int32_t tiles_per_warp;   /* logical programs interpreted together by one warp: 1, 2 or 4; streaming kernels: tiles per instruction, 8 or 4 */
     int32_t warps_per_block;
     int32_t grid_blocks;
     int32_t smem_bytes;
@@ -78,7 +79,8 @@ typedef struct gint_launch_info {
     int32_t early_loads;      /* tile loads per logical program that are started ahead of their use (early issue) */
     int32_t registers_in_smem; /* virtual registers kept in shared memory (the pool then holds the operand stack alone); 0: in the pool */
     int32_t vector_layout;    /* 1: full 1-D tiles live in the pool with lane l holding elements 4l..4l+3 (16-byte accesses) */
-    int32_t reserved[5];
+    int32_t streaming;        /* 1: a streaming kernel (tile loops found again) */
+    int32_t reserved[4];
 } gint_launch_info;
 
 /* What a checked launch (gint_execute_checked) found; all zero = nothing. The FIRST event is described, `count` counts all. */
@@ -167,9 +169,7 @@ int gint_program_create(gint_ctx *ctx, const int32_t *code, int n_words, const g
                         int n_tensors, uint64_t *out_handle);
 int gint_program_destroy(gint_ctx *ctx, uint64_t handle);
 
-/* Geometry the library would use to launch `handle` over grid_dim logical programs. */
-/* The geometry of the tile kernels for this program. A launch that qualifies for the streaming kernels (option "streaming")
- * has a geometry of its own, which is not reported. */
+/* Kernel and geometry with which the library would launch `handle` over grid_dim logical programs. */
 int gint_program_launch_info(gint_ctx *ctx, uint64_t handle, uint32_t grid_dim, gint_launch_info *out);
 
 /* ---- launches ----------------------------------------------------------------------------------- */

@@ -29,14 +29,24 @@ def test_recorded_programs():
 def test_random_words(seed):
     """Mostly invalid programs: every error in its place, opcodes beyond the table, negative ones, slots out of range, no Halt."""
     rng = np.random.default_rng(seed)
-    valid = 0
+    effects = {O.LoadGlobal1DF32: (0, 1), O.LoadImm: (0, 1), O.FAdd: (2, -1), O.Dup: (1, 1), O.Pop: (1, -1), O.FPermW: (1, 0), O.DupBroadcastW: (1, 1),
+               O.Swap: (2, 0), O.StoreGlobal1DF32: (1, -1)}
+    valid = broken = 0
     for _ in range(300):
-        n = int(rng.integers(1, 30))
-        code = np.stack([rng.choice([O.LoadGlobal1DF32, O.LoadImm, O.FAdd, O.Dup, O.Pop, O.FPermW, O.DupBroadcastW, O.Swap, O.StoreGlobal1DF32], n),
-                         rng.integers(-5, 40, n)], 1).astype(np.int32)
-        bad = rng.random(n) < 0.02
-        code[bad, 0] = rng.integers(-3, 140, bad.sum())
+        ops, depth = [], 0
+        for _ in range(int(rng.integers(1, 30))):     # correct as far as the stack goes, slots out of range now and then
+            op = rng.choice([op for op, (need, net) in effects.items() if depth >= need and depth + net <= 8])
+            ops.append(op)
+            depth += effects[op][1]
+        slots = rng.integers(0, 8 if rng.random() < 0.1 else 4, len(ops))
+        code = np.stack([ops, np.where([op in (O.LoadGlobal1DF32, O.StoreGlobal1DF32) for op in ops], (rng.integers(0, 40, len(ops)) << 4) | slots,
+                                       rng.integers(-5, 40, len(ops)))], 1).astype(np.int32)
+        if rng.random() < 0.5:                        # then spoilt
+            bad = rng.random(len(ops)) < 0.05
+            code[bad, 0] = rng.choice([*effects, -3, 106, 139], bad.sum())
         if rng.random() < 0.9:
-            code[-1] = O.Halt, 0
-        valid += check(code, int(rng.integers(1, 9))) > 0
-    assert check(np.zeros((0, 2)), 1) < 0 and valid >= 0
+            code = np.concatenate([code, [[O.Halt, 0]]]).astype(np.int32)
+        r = check(code, 4)
+        valid, broken = valid + (r > 0), broken + (r < 0)
+    assert valid > 50 and broken > 20
+    assert check(np.zeros((0, 2)), 1) < 0

@@ -19,6 +19,7 @@ from gint_b200 import opcodes as O  # noqa: E402
 from gint_b200.host import capi, frontend as F  # noqa: E402
 from gint_b200.host.utils import fill_tensor_info  # noqa: E402
 from gint_b200.programs import load_records, recorded  # noqa: E402
+from test_launch_route import EARLY, FLAT, WIDE, WIDE_VECTOR  # noqa: E402
 from test_predecode_transforms import fold_repeated_loads, normalised  # noqa: E402
 
 LOOP_BEGIN, REMAP, _, _, ACC_ADD, ACC_FMA, ACC_FMA_SQUARE, SQUARE, MUL_KEEP, SILU, LOOP_END = range(106, 117)
@@ -143,6 +144,38 @@ def test_what_is_no_loop_has_no_stream(kw):
 
 # ---------------------------------------------------------------------------------------------- on the GPU
 
+def route_of(program, tensors, first, count, gathered=(), **kw):
+    """The kernels that a launch of `program` on these tensors runs on (gint_debug_route)."""
+    args = C.to_interfaces(tensors)
+    pd = program.get_program(*args, **kw)
+    code = np.ascontiguousarray(np.asarray(pd.program, dtype=np.int32).reshape(-1))
+    ti = capi.HTensorInfo()
+    fill_tensor_info(ti, pd.input_infos)
+    order = list(getattr(pd, "input_indices", None) or range(len(pd.input_infos)))
+    bases = (ctypes.c_uint64 * 8)(*[tensors[i].data_ptr() for i in order])
+    mask = sum(1 << k for k, i in enumerate(order) if i in gathered)
+    extent = max([tensors[i].numel() * tensors[i].element_size() for i in gathered], default=0)
+    return capi.load_library().gint_debug_route(code.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), code.size, ctypes.byref(ti), len(order), bases,
+                                                first, count, mask, extent)
+
+
+def both(launch):
+    """What `launch` returns on the kernels of its route and on the tile kernels."""
+    ex, got = get_executor(), []
+    for on in (1, 0):
+        ex.set_option("streaming", on)
+        try:
+            got.append([t.cpu() for t in launch()])
+        finally:
+            ex.set_option("streaming", 1)
+    return got
+
+
+def same_bits(launch):
+    for a, b in zip(*both(launch)):
+        assert bits_equal(a, b), mismatch_report(a, b)
+
+
 def _perf_cases():
     import importlib.util
     spec = importlib.util.spec_from_file_location("timed_cases", os.path.join(ROOT, "perf", "cases.py"))
@@ -161,20 +194,20 @@ EDGES = ([{"kind": "add", "n": n} for n in (1, 127, 128, 1024, 1025, 4096, 40003
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", EDGES, ids=lambda c: "-".join(str(v) for v in c.values()))
 def test_streaming_kernels_give_the_bits_of_the_tile_kernels(case):
-    m, ex = _perf_cases(), get_executor()
-    got = []
-    for on in (1, 0):
-        ex.set_option("streaming", on)
-        try:
-            r = m.run(m.prepare(dict(case, name="edge"), 7))
-            got.append([t.cpu() for t in (r if isinstance(r, tuple) else (r,))])
-        finally:
-            ex.set_option("streaming", 1)
-    for a, b in zip(*got):
-        if case["kind"] == "head_rmsnorm":   # rows of 128: the squares are added in another order, a last-place difference before one bf16 rounding
-            torch.testing.assert_close(a.float(), b.float(), rtol=2.0 ** -7, atol=0.0)
-        else:
-            assert bits_equal(a, b), mismatch_report(a, b)
+    """(Flat programs of these sizes, and aligned rows of whole tiles, have the tile kernels as their route.)"""
+    m = _perf_cases()
+
+    def launch():
+        r = m.run(m.prepare(dict(case, name="edge"), 7))
+        return r if isinstance(r, tuple) else (r,)
+    if case["kind"] == "head_rmsnorm" and case["dim"] == 128:   # the squares are added in another order; one bf16 rounding after it
+        t = m.inputs(dict(case, name="edge"), 7)
+        x = t["x"].double()
+        want = (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-5) * t["w"].double()).cpu()
+        for (y,) in both(launch):
+            torch.testing.assert_close(y.double(), want, rtol=2.0 ** -8 + 2.0 ** -18, atol=0.0)
+    else:
+        same_bits(launch)
 
 
 @bytecode
@@ -233,8 +266,8 @@ def test_rows_of_half_precision(rows, n, shift):
 @pytest.mark.gpu
 @pytest.mark.parametrize("first,count", [(0, 3), (5, 1), (2, 9)])
 def test_streaming_range_and_in_place(first, count):
-    """A range of the logical programs touches exactly its tiles (flat and row programs), and an output that overlaps an input gives
-    the bits of the program as written."""
+    """A range of the logical programs touches exactly its tiles (row programs on the streaming kernels, a flat program too small for
+    them), and an output that overlaps an input, which keeps the tile kernels, gives the bits of the program as written."""
     from gint_b200.host.executor import _convert_arg
     m, ex = _perf_cases(), get_executor()
     g = torch.Generator(device="cuda").manual_seed(3)
@@ -254,3 +287,123 @@ def test_streaming_range_and_in_place(first, count):
             ex.set_option("streaming", 1)
     for p, q in zip(*got):
         assert bits_equal(p, q), mismatch_report(p, q)
+
+
+N_FLAT = 2 ** 21 + 128 * 3000      # above the 2^21 elements from which flat programs run on the streaming kernels
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,dtype", [("add", "f32"), ("gated_silu", "f32"), ("gated_silu", "f16"), ("gated_silu", "bf16")])
+@pytest.mark.parametrize("rest,shift", [(0, 0), (1, 0), (77, 0), (1024 + 640 + 3, 0), (77, 1), (130, (0, 1, 0))])
+def test_flat_streaming(kind, dtype, rest, shift):
+    """Flat launches: lengths that fill no last group of tiles, base pointers off by one element (the natural layout), and ranges that
+    start and end inside the grid, which touch exactly their own elements. The bits of the tile kernels, guard bands included."""
+    m, ex = _perf_cases(), get_executor()
+    dt = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}[dtype]
+    n, shifts = N_FLAT + rest, shift if isinstance(shift, tuple) else (shift,) * 3
+    g = torch.Generator(device="cuda").manual_seed(rest)
+    a, b = [torch.randn(n + 64, device="cuda", generator=g).to(dt)[s:s + n] for s in shifts[1:]]
+    program, kw, per = (m.add, {}, 128) if kind == "add" else (m.gated_silu, {"dtype": dtype}, 512)
+    total = -(-n // per)
+    aligned = not any(shifts)
+    for first, count in ((0, total), (0, total - 3), (total - -(-16385 * 128 // per), -(-16385 * 128 // per)), (5, total - 9)):
+        def launch():
+            buffer = torch.full((n + 128,), 9.0, dtype=dt, device="cuda")
+            out = buffer[64 + shifts[0]:64 + shifts[0] + n]
+            assert route_of(program, [out, a, b], first, count, **kw) == (WIDE_VECTOR if aligned else WIDE) | FLAT
+            ex.execute_range(program, C.to_interfaces([out, a, b]), first, count, cuda_stream=torch.cuda.current_stream().cuda_stream, **kw)
+            return [buffer]
+        same_bits(launch)
+
+
+@bytecode
+def rows_2dt(x, y, w, REGW, WARP, load="fldg_2dt", weight="fldg_2dt", store="fstg_2dt"):
+    """rmsnorm of (rows, dim), four rows per logical program, one per width value."""
+    T, H = x.shape
+    xb, yb = [F.make_block_2d(t, [H, T], [1, t.strides[0]], [1, -(-T // REGW)], [0, REGW]) for t in (x, y)]
+    wb = F.make_block_2d(w, [H, T], [1, 0], [1, -(-T // REGW)], [0, REGW])
+    F.fpush(0.0)
+    for c in range(0, H, WARP):
+        getattr(F, load)(c, xb)
+        F.dup()
+        F.fma()
+    F.warp_allreduce_fsum()
+    F.fmaimm(1 / H, 1e-5)
+    F.frsqrt()
+    for c in range(0, H, WARP):
+        F.dup()
+        getattr(F, load)(c, xb)
+        F.fmul()
+        getattr(F, weight)(c, wb)
+        F.fmul()
+        getattr(F, store)(c, yb)
+    F.halt()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 37, 4000])
+@pytest.mark.parametrize("dim", [64, 80, 128, 132, 384])
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16", "u8"])
+def test_streaming_2dt_rows(rows, dim, dtype):
+    """Every element type of 2DT tiles. f32 and u8 sums, and sums over a number of tiles that is no multiple of four, have the bits of the
+    tile kernels; the others, whose terms are added in another order, are held to a 64-bit reference within one rounding of the result's type."""
+    dt = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16, "u8": torch.uint8}[dtype]
+    suffix = {"f32": "", "u8": "_u8"}.get(dtype, "_" + dtype)
+    g = torch.Generator(device="cuda").manual_seed(rows + dim)
+    x = torch.randint(0, 256, (rows, dim), device="cuda", generator=g).to(dt) if dtype == "u8" else torch.randn(rows, dim, device="cuda", generator=g).to(dt)
+    out_type = torch.float32 if dtype == "u8" else dt
+    w = torch.rand(dim, device="cuda", generator=g).to(out_type)
+    kw = {"load": "fldg_2dt" + suffix, "weight": "fldg_2dt" + ("" if dtype == "u8" else suffix), "store": "fstg_2dt" + ("" if dtype == "u8" else suffix)}
+
+    def launch():
+        y = torch.full((rows, dim), 9.0, dtype=out_type, device="cuda")
+        r = route_of(rows_2dt, [x, y, w], 0, -(-rows // 4), **kw)
+        assert r in (WIDE, WIDE_VECTOR) and (r == WIDE or dtype in ("f16", "bf16"))
+        rows_2dt(x, y, w, grid_dim=-(-rows // 4), **kw)
+        return [y]
+    if dtype in ("f32", "u8") or -(-dim // 32) % 4 != 0:
+        same_bits(launch)
+        return
+    xd = x.double()
+    want = (xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()).cpu()
+    half_ulp = 2.0 ** (-8 if dtype == "bf16" else -11)      # relative; the f32 steps before it (sums of at most 384 terms, rsqrt) add below 2^-18
+    for y, in both(launch):
+        torch.testing.assert_close(y.double(), want, rtol=half_ulp + 2.0 ** -18, atol=2.0 ** -25 if dtype == "f16" else 0.0)   # (half of f16's smallest subnormal)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,rows,n,want", [("f16", 40, 1028, WIDE_VECTOR), ("f16", 40, 1029, WIDE), ("f16", 1, 1029, WIDE), ("f32", 33, 2029, WIDE), ("f32", 40, 1024, EARLY)])
+def test_streaming_gathered_rows(dtype, rows, n, want):
+    """Rows read through an index, on the kernels that their alignment allows: the bits of the rows gathered first."""
+    m, ex = _perf_cases(), get_executor()
+    dt, program = (torch.float16, rmsnorm_f16) if dtype == "f16" else (torch.float32, m.rmsnorm)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    table, w = torch.randn(rows, n, device="cuda", generator=g).to(dt), torch.rand(n, device="cuda", generator=g).to(dt)
+    idx = torch.randint(0, rows, (rows,), device="cuda", generator=g)
+    copy = table[idx].contiguous()
+
+    def launch(gather):
+        out = torch.full((rows, n), 9.0, dtype=dt, device="cuda")
+        if gather:
+            assert route_of(program, [table, w, out], 0, rows, gathered=(0,)) == want
+            ex.execute_gathered(program, C.to_interfaces([table, w, out]), rows, (0,), idx, cuda_stream=torch.cuda.current_stream().cuda_stream)
+        else:
+            program(copy, w, out, grid_dim=rows)
+        return [out]
+    same_bits(lambda: launch(True))
+    (got,), (tile,) = both(lambda: launch(True))[0], both(lambda: launch(False))[1]
+    assert bits_equal(got, tile), mismatch_report(got, tile)
+
+
+@pytest.mark.gpu
+def test_launch_info_reports_the_streaming_kernel():
+    m, ex = _perf_cases(), get_executor()
+    x, w, out = torch.zeros(100, 2029, device="cuda"), torch.zeros(2029, device="cuda"), torch.zeros(100, 2029, device="cuda")
+    info = ex.launch_info(m.rmsnorm, [x, w, out], 100)
+    assert (info["streaming"], info["pool_size"], info["tiles_per_warp"], info["warps_per_block"]) == (1, 3, 8, 1), info
+    ex.set_option("streaming", 0)
+    try:
+        info = ex.launch_info(m.rmsnorm, [x, w, out], 100)
+        assert info["streaming"] == 0 and info["pool_size"] == 4 and info["warps_per_block"] == 4, info
+    finally:
+        ex.set_option("streaming", 1)
