@@ -1214,7 +1214,8 @@ template <int N> __device__ __forceinline__ void pool_clear()
  *   %gring       byte offset of the current slot in the warp's ring of early-issued loads
  *   %gzero       64 bits of zero that reach the kernel as a launch parameter (see fma_barrier)
  *   %grf         shared-memory address of the warp's virtual registers plus 4 * lane (kernels built with GINT_RF)
- *   %gx0 .. 5    the fields of Ctx (tiles as an offset into the dynamic shared memory)
+ *   %gx0 .. 5    the fields of Ctx (tiles as a shared-memory address: an offset from the block's shared array makes every handler
+ *                work that array's address out again; RMSNorm 16384 x 4096 120.1 -> 117.5 us, bf16 heads 153 -> 146)
  * so no C++ value is live from handler to handler and a handler can be entered from any other handler.
  */
 __device__ __forceinline__ void state_declare()
@@ -1229,7 +1230,7 @@ extern __shared__ __align__(16) unsigned char g_smem[];
 __device__ __forceinline__ void context_set(const Ctx &cx)
 {
     asm volatile("mov.b32 %%gx0, %0; mov.b32 %%gx1, %1; mov.b32 %%gx2, %2; mov.b32 %%gx3, %3; mov.b32 %%gx4, %4; mov.b32 %%gx5, %5;"
-                 ::"r"((uint32_t)(reinterpret_cast<unsigned char *>(cx.tiles) - g_smem)), "r"(cx.lane), "r"(cx.hidden), "r"(cx.ring_mask), "r"(cx.rows), "r"(cx.rows_stride));
+                 ::"r"((uint32_t)__cvta_generic_to_shared(cx.tiles)), "r"(cx.lane), "r"(cx.hidden), "r"(cx.ring_mask), "r"(cx.rows), "r"(cx.rows_stride));
 }
 __device__ __forceinline__ Ctx handler_context()
 {
@@ -1237,7 +1238,8 @@ __device__ __forceinline__ Ctx handler_context()
     uint32_t tiles;
     asm volatile("mov.b32 %0, %%gx0; mov.b32 %1, %%gx1; mov.b32 %2, %%gx2; mov.b32 %3, %%gx3; mov.b32 %4, %%gx4; mov.b32 %5, %%gx5;"
                  : "=r"(tiles), "=r"(cx.lane), "=r"(cx.hidden), "=r"(cx.ring_mask), "=r"(cx.rows), "=r"(cx.rows_stride));
-    cx.tiles = reinterpret_cast<TileInfo *>(g_smem + tiles);
+    cx.tiles = reinterpret_cast<TileInfo *>(__cvta_shared_to_generic(tiles));
+    __builtin_assume(__isShared(cx.tiles));   // its accesses are shared-memory instructions on that address
     return cx;
 }
 
