@@ -540,6 +540,7 @@ template <int K, int A, int B, int KI> __device__ __forceinline__ void slot_swap
 struct Ctx {
     TileInfo *tiles;   // this warp's K tile descriptors (shared memory)
     int lane;
+    u64 lane4;         // 4 * lane, the lane's byte offset in a row of 32 floats
     uint32_t hidden;   // shared-memory address of slot 0, tile 0 of the warp's load staging area, plus 4 * lane
     uint32_t ring_mask; // bytes of the warp's ring of early-issued loads (4 or 8 slots of K x 512 bytes) minus 1
     uint32_t rows;     // shared-memory address of this warp's staged row blocks (tile 0); tile k is rows_stride bytes further
@@ -783,11 +784,11 @@ __device__ __forceinline__ char *fast_tile_address(const TileInfo *ti, uint32_t 
 template <int K, int KI>
 __device__ __forceinline__ void tile_issue_fast(const TileInfo *ti, uint32_t operand, const Ctx &cx, uint32_t slot)
 {
-    const char *p = fast_tile_address(ti, operand) + cx.lane * 16;
+    const char *p = fast_tile_address(ti, operand) + cx.lane4 * 4u;
 #ifdef GINT_VEC
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + (uint32_t)(KI * 512)), "l"(p) : "memory");
 #else
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + (uint32_t)(KI * 512 + cx.lane * 12)), "l"(p) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + (uint32_t)(KI * 512) + (uint32_t)cx.lane4 * 3u), "l"(p) : "memory");
 #endif
 }
 template <int K, int SLOT, int KI> __device__ __forceinline__ void take_hidden(uint32_t slot)
@@ -1015,7 +1016,7 @@ __device__ __forceinline__ void exec_tile(const uint32_t operand, const Ctx &cx)
             return;
         }
 #endif
-        const char *p = fast_tile_address(cx.tiles + KI, operand) + cx.lane * 4;
+        const char *p = fast_tile_address(cx.tiles + KI, operand) + cx.lane4;
         asm volatile("{\n\t.reg .b32 t<4>;\n\t"
                      "ld.global.b32 t0, [%2];\n\tld.global.b32 t1, [%2+128];\n\tld.global.b32 t2, [%2+256];\n\tld.global.b32 t3, [%2+384];\n\t"
                      "mov.b64 %%gs%0, {t0, t1};\n\tmov.b64 %%gs%1, {t2, t3};\n\t}" ::"n"(LO(SP)), "n"(HI(SP)), "l"(p) : "memory");
@@ -1027,7 +1028,7 @@ __device__ __forceinline__ void exec_tile(const uint32_t operand, const Ctx &cx)
             return;
         }
 #endif
-        char *p = fast_tile_address(cx.tiles + KI, operand) + cx.lane * 4;
+        char *p = fast_tile_address(cx.tiles + KI, operand) + cx.lane4;
         asm volatile("{\n\t.reg .b32 t<4>;\n\t"
                      "mov.b64 {t0, t1}, %%gs%0;\n\tmov.b64 {t2, t3}, %%gs%1;\n\t"
                      "st.global.b32 [%2], t0;\n\tst.global.b32 [%2+128], t1;\n\tst.global.b32 [%2+256], t2;\n\tst.global.b32 [%2+384], t3;\n\t}"
@@ -1216,26 +1217,31 @@ template <int N> __device__ __forceinline__ void pool_clear()
  *   %grf         shared-memory address of the warp's virtual registers plus 4 * lane (kernels built with GINT_RF)
  *   %gx0 .. 5    the fields of Ctx (tiles as a shared-memory address: an offset from the block's shared array makes every handler
  *                work that array's address out again; RMSNorm 16384 x 4096 120.1 -> 117.5 us, bf16 heads 153 -> 146)
+ *   %gl4         4 * lane (kept, because every fast access adds it to an address: RMSNorm 16384 x 4096 115.9 -> 113.7 us, bmm4x4
+ *                162.8 -> 160.3)
  * so no C++ value is live from handler to handler and a handler can be entered from any other handler.
  */
 __device__ __forceinline__ void state_declare()
 {
     // (the unused "n" operand makes nvcc treat the string as a template, so that %% means %)
     asm volatile(".reg .b32 %%gc; .reg .b32 %%ge<2>; .reg .b32 %%gkey; .reg .b32 %%gbudget; .reg .b32 %%gring; .reg .b64 %%gzero; "
-                 ".reg .b32 %%grf; .reg .b32 %%gx<6>; // %0" ::"n"(0));
+                 ".reg .b32 %%grf; .reg .b32 %%gl4; .reg .b32 %%gx<6>; // %0" ::"n"(0));
 }
 
 extern __shared__ __align__(16) unsigned char g_smem[];
 
 __device__ __forceinline__ void context_set(const Ctx &cx)
 {
+    asm volatile("mov.b32 %%gl4, %0;" ::"r"(cx.lane * 4));
     asm volatile("mov.b32 %%gx0, %0; mov.b32 %%gx1, %1; mov.b32 %%gx2, %2; mov.b32 %%gx3, %3; mov.b32 %%gx4, %4; mov.b32 %%gx5, %5;"
                  ::"r"((uint32_t)__cvta_generic_to_shared(cx.tiles)), "r"(cx.lane), "r"(cx.hidden), "r"(cx.ring_mask), "r"(cx.rows), "r"(cx.rows_stride));
 }
 __device__ __forceinline__ Ctx handler_context()
 {
     Ctx cx;
-    uint32_t tiles;
+    uint32_t tiles, lane4;
+    asm volatile("mov.b32 %0, %%gl4;" : "=r"(lane4));
+    cx.lane4 = lane4;
     asm volatile("mov.b32 %0, %%gx0; mov.b32 %1, %%gx1; mov.b32 %2, %%gx2; mov.b32 %3, %%gx3; mov.b32 %4, %%gx4; mov.b32 %5, %%gx5;"
                  : "=r"(tiles), "=r"(cx.lane), "=r"(cx.hidden), "=r"(cx.ring_mask), "=r"(cx.rows), "=r"(cx.rows_stride));
     cx.tiles = reinterpret_cast<TileInfo *>(__cvta_shared_to_generic(tiles));
