@@ -1307,8 +1307,14 @@ __device__ __forceinline__ void run_fused(const Ctx &cx, uint32_t &next_opcode)
 
 /* Order of the handlers in the code. A kernel holds one handler per (opcode, depth), 2 to 6 MB of machine code, of which any
  * one program runs a few dozen; in plain key order the few-instruction handlers that a program jumps between lie scattered
- * between tile accesses and inlined math routines of kilobytes each. The handlers that recorded programs run come first
- * (gint_hot_handlers.h, written by the build from hot_handlers.json), then the other short ones, then the long ones. */
+ * between tile accesses and inlined math routines of kilobytes each. They stand in four groups: those that recorded programs run
+ * (gint_hot_handlers.h, written by the build from hot_handlers.json), short ones before long ones, then the other short ones, then
+ * the other long ones. The compiler places code by how likely it takes it to be, not by source order, so each group has a switch of
+ * its own, in front of the next one's by a condition that it is told to expect. Measured, one order without groups -> groups:
+ * misses of the instruction cache in the 4x4 inverse 1.07 M -> 0.41 M per 1 M matrices and 327 -> 299 us at full size, the gathered
+ * graph 250 -> 247. The hot long ones are a group only where that is the faster half: registers in shared memory (308 without it),
+ * one tile per warp (RMSNorm of 8192 rows 73 -> 68 us under ncu); with two or four tiles in the pool they are among the other long
+ * ones (gathered graph 247, 251 as a group). */
 #if defined(GINT_RF)
 #define GINT_HOT_LIST GINT_HOT_RF
 #elif defined(GINT_VEC)
@@ -1325,17 +1331,27 @@ struct HotTable {
 #undef GINT_X_HOT
     }
 };
+/* tile accesses, out-of-line and inlined math, reductions, anything with branches of its own; a fused handler with such a member */
+template <int OP> __host__ __device__ constexpr bool long_handler();
+template <int... OPS> __host__ __device__ constexpr bool long_members(Seq<OPS...>) { return (long_handler<OPS>() || ...); }
 template <int OP> __host__ __device__ constexpr bool long_handler()
 {
-    if constexpr (GINT_IS_FUSED(OP)) return true;
+    if constexpr (GINT_IS_FUSED(OP)) return long_members(typename FusedSeq<OP>::type{});
     else return MemOp<OP>::is || is_scalar_binary<OP>() || is_scalar_unary<OP>() || (OP >= OP_WarpAllReduceSum && OP <= OP_WarpAllReduceProd) ||
-                OP == OP_LoadGlobal1DF32Indirect || OP == OP_StoreGlobal1DF32Indirect || OP == OP_PfIssue1D || OP == OP_PfTakeIssue1D || OP == OP_StageRows;
+                OP == OP_LoadGlobal1DF32Indirect || OP == OP_StoreGlobal1DF32Indirect || OP == OP_PfIssue1D || OP == OP_PfTakeIssue1D ||
+                OP == OP_PfTakeIssue1DFast || OP == OP_StageRows;
 }
-enum { RANK_HOT = 0, RANK_SHORT, RANK_LONG };
-template <int OP, int SP> __host__ __device__ constexpr int handler_rank()
+enum { RANK_HOT = 0, RANK_HOT_LONG, RANK_SHORT, RANK_LONG };
+template <int OP, int SP, int K> __host__ __device__ constexpr int handler_rank()
 {
     constexpr HotTable t;
-    if constexpr (t.hot[SP * GINT_N_TABLE + OP]) return RANK_HOT;
+#ifdef GINT_RF
+    constexpr bool hot_long = true;
+#else
+    constexpr bool hot_long = K == 1;
+#endif
+    if constexpr (t.hot[SP * GINT_N_TABLE + OP] && !long_handler<OP>()) return RANK_HOT;
+    else if constexpr (t.hot[SP * GINT_N_TABLE + OP] && hot_long) return RANK_HOT_LONG;
     else return long_handler<OP>() ? RANK_LONG : RANK_SHORT;
 }
 
@@ -1374,6 +1390,14 @@ template <int P, int K, int... KEY> __device__ __forceinline__ void missing_labe
     (missing_label<P, K, KEY>(), ...);
 }
 
+/* A condition that the compiler takes for likely and cannot know; never evaluated (control does not come back to the switches). */
+__device__ __forceinline__ bool this_group_first()
+{
+    uint32_t x;
+    asm volatile("mov.b32 %0, %%gkey;" : "=r"(x));
+    return __builtin_expect(x != 0u, 1);
+}
+
 template <int P, int K, bool THREADED>
 __device__ __forceinline__ void interpret(const uint2 *code, uint32_t n_entries)
 {
@@ -1386,10 +1410,9 @@ __device__ __forceinline__ void interpret(const uint2 *code, uint32_t n_entries)
         uint32_t key;
         if constexpr (THREADED) asm volatile("mov.b32 %0, %%gkey;\n\tbrx.idx.uni %%gkey, GT0;" : "=r"(key) :: "memory");
         else asm volatile("GTOP:\n\tmov.b32 %0, %%gkey;\n\tbrx.idx.uni %%gkey, GTALL;" : "=r"(key) :: "memory");
-        switch (key) {
 #define GINT_CASE(num, spv, rank)                                                                       \
     case (rank) * GINT_N_KEYS + (spv) * GINT_N_TABLE + (num):                                            \
-        if constexpr (op_valid<num, spv, P, K>() && handler_rank<num, spv>() == (rank)) {                \
+        if constexpr (op_valid<num, spv, P, K>() && handler_rank<num, spv, K>() == (rank)) {             \
             asm volatile("GL%0_%1:" ::"n"(spv), "n"(num) : "memory");                                    \
             if constexpr ((num) == OP_Halt) return;                                                     \
             else handler<num, spv, P, K, THREADED>();                                                   \
@@ -1399,34 +1422,58 @@ __device__ __forceinline__ void interpret(const uint2 *code, uint32_t n_entries)
     GINT_CASE(num, 0, rank) GINT_CASE(num, 1, rank) GINT_CASE(num, 2, rank) GINT_CASE(num, 3, rank) GINT_CASE(num, 4, rank) \
     GINT_CASE(num, 5, rank) GINT_CASE(num, 6, rank) GINT_CASE(num, 7, rank) GINT_CASE(num, 8, rank)
 #define GINT_X_HOT(num, sp) GINT_CASE(num, sp, RANK_HOT)
-            GINT_HOT_LIST(GINT_X_HOT)
-#undef GINT_X_HOT
+#define GINT_X_HOT_LONG(num, sp) GINT_CASE(num, sp, RANK_HOT_LONG)
 #define GINT_X_SHORT(name, num, md, net) GINT_CASES(num, RANK_SHORT)
 #define GINT_X_LONG(name, num, md, net) GINT_CASES(num, RANK_LONG)
-#define GINT_X_FUSED(num, len, ...) GINT_CASES(num, RANK_LONG)
-#ifdef GINT_RF
+#define GINT_X_FUSED_SHORT(num, len, ...) GINT_CASES(num, RANK_SHORT)
+#define GINT_X_FUSED_LONG(num, len, ...) GINT_CASES(num, RANK_LONG)
+#if defined(GINT_RF)
 #define GINT_X_OWN(X) GINT_RF_OPCODE_LIST(X)
-            GINT_RF_FUSED_LIST(GINT_X_FUSED)
+#define GINT_X_OWN_FUSED(X) GINT_RF_FUSED_LIST(X)
 #elif defined(GINT_VEC)
 #define GINT_X_OWN(X) GINT_VEC_OPCODE_LIST(X)
+#define GINT_X_OWN_FUSED(X)
 #else
 #define GINT_X_OWN(X)
+#define GINT_X_OWN_FUSED(X)
 #endif
-            GINT_OPCODE_LIST(GINT_X_SHORT)
-            GINT_INTERNAL_OPCODE_LIST(GINT_X_SHORT)
-            GINT_X_OWN(GINT_X_SHORT)
-            GINT_FUSED_LIST(GINT_X_FUSED)
+        if (this_group_first()) {
+            switch (key) { GINT_HOT_LIST(GINT_X_HOT) default: break; }
+            continue;
+        }
+        if (this_group_first()) {
+            switch (key) { GINT_HOT_LIST(GINT_X_HOT_LONG) default: break; }
+            continue;
+        }
+        if (this_group_first()) {
+            switch (key) {
+                GINT_OPCODE_LIST(GINT_X_SHORT)
+                GINT_INTERNAL_OPCODE_LIST(GINT_X_SHORT)
+                GINT_X_OWN(GINT_X_SHORT)
+                GINT_FUSED_LIST(GINT_X_FUSED_SHORT)
+                GINT_X_OWN_FUSED(GINT_X_FUSED_SHORT)
+            default: break;
+            }
+            continue;
+        }
+        switch (key) {
+            GINT_X_OWN_FUSED(GINT_X_FUSED_LONG)
+            GINT_FUSED_LIST(GINT_X_FUSED_LONG)
             GINT_OPCODE_LIST(GINT_X_LONG)
             GINT_INTERNAL_OPCODE_LIST(GINT_X_LONG)
             GINT_X_OWN(GINT_X_LONG)
+#undef GINT_X_OWN_FUSED
 #undef GINT_X_OWN
-#undef GINT_X_FUSED
+#undef GINT_X_FUSED_LONG
+#undef GINT_X_FUSED_SHORT
 #undef GINT_X_LONG
 #undef GINT_X_SHORT
+#undef GINT_X_HOT_LONG
+#undef GINT_X_HOT
 #undef GINT_CASES
 #undef GINT_CASE
 #ifdef GINT_GUARD
-        case 3 * GINT_N_KEYS:
+        case 4 * GINT_N_KEYS:
             asm volatile("GLEAVE: // %0" ::"n"(0) : "memory");
             return;
 #endif
