@@ -19,7 +19,7 @@ from gint_b200 import opcodes as O  # noqa: E402
 from gint_b200.host import capi, frontend as F  # noqa: E402
 from gint_b200.host.utils import fill_tensor_info  # noqa: E402
 from gint_b200.programs import load_records, recorded  # noqa: E402
-from test_launch_route import EARLY, FLAT, WIDE, WIDE_VECTOR  # noqa: E402
+from test_launch_route import EARLY, FLAT, WIDE as STREAMING, WIDE_VECTOR as STREAMING_VECTOR  # noqa: E402
 from test_predecode_transforms import fold_repeated_loads, normalised  # noqa: E402
 
 LOOP_BEGIN, REMAP, _, _, ACC_ADD, ACC_FMA, ACC_FMA_SQUARE, SQUARE, MUL_KEEP, SILU, LOOP_END = range(106, 117)
@@ -310,7 +310,7 @@ def test_flat_streaming(kind, dtype, rest, shift):
         def launch():
             buffer = torch.full((n + 128,), 9.0, dtype=dt, device="cuda")
             out = buffer[64 + shifts[0]:64 + shifts[0] + n]
-            assert route_of(program, [out, a, b], first, count, **kw) == (WIDE_VECTOR if aligned else WIDE) | FLAT
+            assert route_of(program, [out, a, b], first, count, **kw) == (STREAMING_VECTOR if aligned else STREAMING) | FLAT
             ex.execute_range(program, C.to_interfaces([out, a, b]), first, count, cuda_stream=torch.cuda.current_stream().cuda_stream, **kw)
             return [buffer]
         same_bits(launch)
@@ -328,7 +328,8 @@ def rows_2dt(x, y, w, REGW, WARP, load="fldg_2dt", weight="fldg_2dt", store="fst
         F.dup()
         F.fma()
     F.warp_allreduce_fsum()
-    F.fmaimm(1 / H, 1e-5)
+    F.fmulimm(1 / H)      # (one f32 each: the two immediates of FMAImm share a word)
+    F.faddimm(1e-5)
     F.frsqrt()
     for c in range(0, H, WARP):
         F.dup()
@@ -358,7 +359,7 @@ def test_streaming_2dt_rows(rows, dim, dtype):
     def launch():
         y = torch.full((rows, dim), 9.0, dtype=out_type, device="cuda")
         r = route_of(rows_2dt, [x, y, w], 0, -(-rows // 4), **kw)
-        assert r in (WIDE, WIDE_VECTOR) and (r == WIDE or dtype in ("f16", "bf16"))
+        assert r in (STREAMING, STREAMING_VECTOR) and (r == STREAMING or dtype in ("f16", "bf16"))
         rows_2dt(x, y, w, grid_dim=-(-rows // 4), **kw)
         return [y]
     if dtype in ("f32", "u8") or -(-dim // 32) % 4 != 0:
@@ -372,7 +373,7 @@ def test_streaming_2dt_rows(rows, dim, dtype):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dtype,rows,n,want", [("f16", 40, 1028, WIDE_VECTOR), ("f16", 40, 1029, WIDE), ("f16", 1, 1029, WIDE), ("f32", 33, 2029, WIDE), ("f32", 40, 1024, EARLY)])
+@pytest.mark.parametrize("dtype,rows,n,want", [("f16", 40, 1028, STREAMING_VECTOR), ("f16", 40, 1029, STREAMING), ("f16", 1, 1029, STREAMING), ("f32", 33, 2029, STREAMING), ("f32", 40, 1024, EARLY)])
 def test_streaming_gathered_rows(dtype, rows, n, want):
     """Rows read through an index, on the kernels that their alignment allows: the bits of the rows gathered first."""
     m, ex = _perf_cases(), get_executor()
