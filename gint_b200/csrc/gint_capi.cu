@@ -1010,11 +1010,10 @@ struct Program {
     uint64_t wide_extent[GINT_MAX_TENSORS] = {};
     uint32_t wide_align[GINT_MAX_TENSORS] = {};   // alignment of the base pointers that the vector-layout kernels need (minus 1); all 0: never
     bool wide_vector = false;
-    /* Rows of f32 in the 1-D layout: where they are aligned the tile kernels' 16-byte early-issued copies are as fast or faster (RMSNorm
-     * 16384 x 4096: 125 us there, 121 us here; row sums of 65536 x 1024: 50 against 75), so only unaligned rows come here
-     * (10007 x 2029: 77 us there, 55 here). */
-    bool wide_rows_f32 = false;
     uint32_t wide_loop_slots = 0;   // slots that a loop accesses
+    /* what wide_pays looks at: element types and layout of the loops' accesses, whether a loop has out-of-line math, whether two
+     * loops load the same tiles */
+    bool wide_f32 = false, wide_f16 = false, wide_bf16 = false, wide_u8 = false, wide_2dt = false, wide_math = false, wide_rereads = false;
     uint32_t wide_rows = 0;     // slots of which every logical program has its own part
     uint2 wide_inline[gint::kInlineCodeSlots];
     PlanMemo memo[6] = {};      // last launch plan of the plain stream [0], the early-issue stream [1], the RF stream [2], the vector-layout stream [3], the streaming kernels in the natural [4] and the vector layout [5]
@@ -1244,7 +1243,53 @@ int plan_direct(gint_ctx *ctx, const Program *p, const StreamView &sv, uint32_t 
     return GINT_OK;
 }
 
-constexpr uint64_t kFlatMinTiles = 16384;
+constexpr uint64_t kFlatMinTiles = 16384;   // 2^21 elements
+
+/*
+ * Is the streaming kernel the faster one for this launch? `fast`: every access of its loops is a fast one of the tile kernels
+ * (f32, whole aligned tiles). The lines are drawn where the time per launch on the device crosses (one B200, cold buffers, both
+ * kernels in turn; ratio = tile kernel / streaming kernel); tiles = tiles of the longest loop, rows = logical programs.
+ *
+ * Flat programs. Without an f32 access 1.0 to 2.5 from 2^21 elements on (gated SiLU f16 2.1 M: 1.00, 2.5 M: 1.18, 24 M: 1.4; a + b f16
+ * 1.6 to 2.5), narrow loads with f32 stores 1.3 to 2.3. f32 alone: a + b of ragged length 0.94 to 0.98 at 2.5 and 3 M elements, 1.10 to 1.18 from 4 M on;
+ * of whole tiles 0.95 to 1.02 at 4 M, 1.00 to 1.05 from 8 M on (the tile kernels' 16-byte copies); with division, square root or SiLU 0.77 to 1.0, with u8 loads
+ * and square root 0.94 at 2.5 M, 1.1 to 1.4 from 4 M on; bodies that need a fourth slot 0.85 to 1.0.
+ *
+ * f32 rows that are not fast. RMSNorm, which loads its row twice: 2 tiles 1.15 at 1000 rows, 0.99 at 2400, 0.60 at 200 000; 3 tiles 1.36 at
+ * 1000, 1.04 at 10 000, 0.87 at 60 000; 4 tiles 1.25 at 10 000, 1.07 at 60 000, 0.96 at 200 000; 5 and more 1.06 to 2.8. Rows loaded once
+ * (sums, scaling): 3 to 9 tiles 0.7 to 1.05, 16 and 32 tiles 1.0 to 1.5 up to 1000 rows, 0.84 to 1.07 above. Fast rows: RMSNorm
+ * 16384 x 4096 114 us there, 121 here; sums of 65536 x 1024 50 against 75.
+ *
+ * Rows of narrow elements, vector layout: 4 tiles 1.05 to 1.2, 5 tiles 0.8 to 1.1 (a group of four and one of one), 8 tiles 1.3 to 1.8,
+ * 10 tiles 1.25 to 1.4 up to 1000 rows, 0.94 at 20 000; 11 tiles 1.02 to 1.6, 15 and more 1.2 to 3.2. Natural layout: 2 to 9 tiles 0.5 to 1.2,
+ * 11 and 13 tiles 1.07 to 1.4 up to 1000 rows where the row is loaded twice, 0.8 to 1.05 above, 16 and more 1.1 to 2.6.
+ *
+ * 2DT rows. Vector layout, 4 tiles and more: 1.07 to 2.9. Natural layout: 2 and 3 tiles 0.47 to 1.02; bf16 5 tiles 1.01 to 1.09, more 1.08 to 2.1;
+ * f32 5 tiles 0.94 to 0.98, 6 and more 1.06 to 3.0; f16 5 and 6 tiles 0.88 to 0.95, 9 tiles 0.93 to 0.98, 10 and more 1.03 to 1.8 (u8: as f16).
+ */
+bool wide_pays(const gint_ctx *ctx, const Program *p, bool vector, bool fast, uint32_t count)
+{
+    const int tiles = p->wide_tiles;
+    const uint64_t sms = (uint64_t)ctx->num_sms;
+    const bool few_rows = count <= 8 * sms;
+    const bool f32_only = p->wide_f32 && !p->wide_f16 && !p->wide_bf16 && !p->wide_u8;
+    if (p->flat_tiles) {
+        const uint64_t n = (uint64_t)count * p->flat_tiles;
+        if (f32_only) return !p->wide_math && p->wide_depth <= 3 && n > (fast ? 4 : 2) * kFlatMinTiles;
+        return n > (p->wide_f32 && p->wide_math ? 2 : 1) * kFlatMinTiles;
+    }
+    if (p->wide_2dt) {
+        if (vector) return tiles >= 4;
+        return tiles >= (p->wide_f16 || p->wide_u8 ? 10 : f32_only ? 6 : 5);
+    }
+    if (f32_only) {
+        if (fast) return false;
+        if (p->wide_rereads) return tiles >= 5 || count <= (tiles == 4 ? 400 : tiles == 3 ? 64 : 8) * sms;
+        return tiles >= 16 && few_rows;
+    }
+    if (vector) return tiles == 4 || tiles == 8 || tiles >= 11 || (tiles >= 9 && few_rows);
+    return tiles >= 16 || (p->wide_rereads && tiles >= 11 && few_rows);
+}
 
 /* A launch runs on the streaming kernels if the program has a stream for them and the caller has not asked for a particular
  * configuration of the tile kernels. */
@@ -1319,14 +1364,12 @@ Route choose_route(const gint_ctx *ctx, const Program *p, const uint64_t *base_p
         if (((gather->mask >> t) & 1u) && p->ti.batch_strides[t][0] % 4 != 0) ragged_rows |= 1u << t;
     bool fast_ok = (p->fast_slots & ragged_rows) == 0;   // fast accesses need aligned bases
     for (int t = 0; t < n_tensors; t++) fast_ok = fast_ok && !(((p->fast_slots >> t) & 1u) && (base_ptrs[t] & 15u) != 0);
-    /* A flat launch of at most 2^21 elements is a few microseconds of latency either way; the tile kernels spread it over more
-     * blocks (a + b over 2^20 elements: 9.4 us per pass, 9.9 on the streaming kernel). */
-    if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid || (uint64_t)count * p->flat_tiles <= kFlatMinTiles))) {
-        const bool fast_rows = p->early_slots != 0 && fast_ok && (p->wide_loop_slots & ~p->fast_slots) == 0;   // every loop access is a fast one of the tile kernels
-        if (!(p->wide_rows_f32 && fast_rows) && disjoint(p->wide_alias, p->wide_extent)) {
-            bool vector = p->wide_vector && ragged_rows == 0;   // the vector layout, given aligned base pointers
-            for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
-            vector = vector && disjoint(p->wide_vector_alias, p->wide_extent);
+    if (use_wide(ctx, p) && !(p->flat_tiles && (gather || (uint64_t)first + count > p->flat_grid))) {
+        bool vector = p->wide_vector && ragged_rows == 0;   // the vector layout, given aligned base pointers
+        for (int t = 0; vector && t < n_tensors; t++) vector = (base_ptrs[t] & p->wide_align[t]) == 0;
+        vector = vector && disjoint(p->wide_vector_alias, p->wide_extent);
+        const bool fast = p->early_slots != 0 && fast_ok && (p->wide_loop_slots & ~p->fast_slots) == 0;
+        if (wide_pays(ctx, p, vector, fast, count) && disjoint(p->wide_alias, p->wide_extent)) {
             r.wide = vector ? 2 : 1;
             return r;
         }
@@ -1494,12 +1537,23 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
             p->wide_tiles = ws.max_tiles;
             p->flat_tiles = ws.flat_tiles;
             p->flat_grid = ws.flat_grid;
-            p->wide_rows_f32 = ws.flat_tiles == 0;
+            std::vector<uint32_t> loaded;   // operands of the loops so far
+            size_t loaded_before = 0;       // ... of the loops before this one
             for (const Insn &x : ws.prog) {
                 const int op = x.op - GINT_WIDE_FIRST;
+                if (x.op == WOP_LoopBegin) loaded_before = loaded.size();
+                if (x.op == WOP_Silu || wide_out_of_line(op)) p->wide_math = true;
                 if (op < 0 || !GINT_WIDE_TILE_OP(op)) continue;
                 p->wide_loop_slots |= 1u << (x.operand & 15u);
-                if (op != OP_LoadGlobal1DF32 && op != OP_StoreGlobal1DF32) p->wide_rows_f32 = false;
+                if (wide_is_2dt(op)) p->wide_2dt = true;
+                const int bytes = wide_element_bytes(op);
+                if (bytes == 4) p->wide_f32 = true;
+                else if (bytes == 1) p->wide_u8 = true;
+                else if (op == OP_LoadGlobal1DF16 || op == OP_StoreGlobal1DF16 || op == OP_LoadGlobal2DTF16 || op == OP_StoreGlobal2DTF16) p->wide_f16 = true;
+                else p->wide_bf16 = true;
+                if (writes_tensor(op)) continue;
+                for (size_t k = 0; k < loaded_before; k++) p->wide_rereads = p->wide_rereads || loaded[k] == x.operand;
+                loaded.push_back(x.operand);
             }
             memcpy(p->wide_alias, ws.alias_slots, sizeof(p->wide_alias));
             memcpy(p->wide_vector_alias, ws.vector_alias, sizeof(p->wide_vector_alias));
@@ -1743,6 +1797,7 @@ int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *t
     if (!code || (!(ti && base_ptrs) && n_tensors > 0) || n_tensors < 0 || n_tensors > GINT_MAX_TENSORS) return GINT_ERR_INVALID_ARGUMENT;
     gint_ctx ctx;   // (the default options; no device)
     ctx.max_smem_optin = 227 * 1024;
+    ctx.num_sms = 148;
     for (const auto &im : g_images)
         if (im.K > 0) {
             ctx.direct.push_back(Variant{im.P, im.K, nullptr, 0, false, 0, im.rf, im.vec, im.wide});

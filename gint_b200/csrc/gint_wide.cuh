@@ -34,8 +34,9 @@
 
 namespace gint {
 
-/* wide form: an element-wise instruction or a tile access in a loop body (no out-of-line math: its 4 U calls per handler would
- * make every live pool register a saved one) */
+/* wide form: an element-wise instruction or a tile access in a loop body. Of the math that the tile kernels run out of line only
+ * division, square root and reciprocal, which take four values per call (div4 and the like below): 4 U calls per handler would make
+ * every live pool register a saved one. */
 template <int OP> __host__ __device__ constexpr bool wide_ok()
 {
     if constexpr (OP >= GINT_N_OPCODES) return false;

@@ -26,6 +26,8 @@ int wide_element_bytes(int op)
                      op == OP_LoadGlobal2DWF32 || op == OP_StoreGlobal2DWF32;
     return f32 ? 4 : 2;
 }
+/* instructions that a streaming kernel runs out of line, four values at a time (and WOP_Silu) */
+bool wide_out_of_line(int op) { return op == OP_FDiv || op == OP_FRDiv || op == OP_FSqrt || op == OP_FRcp; }
 bool wide_is_load(int op) { return GINT_WIDE_TILE_OP(op) && !writes_tensor(op); }
 
 /* instruction `b` is instruction `a` one tile (times `tiles`) further on */
@@ -339,8 +341,7 @@ bool wide_transform(const std::vector<Insn> &in, const gint_tensor_info &ti, int
      * sums: 250 us there, 340 us here). */
     if (!out->flat_tiles)
         for (const Insn &x : p) {
-            const int op = x.op - GINT_WIDE_FIRST;
-            if (x.op == WOP_Silu || op == OP_FDiv || op == OP_FRDiv || op == OP_FSqrt || op == OP_FRcp) return false;
+            if (x.op == WOP_Silu || wide_out_of_line(x.op - GINT_WIDE_FIRST)) return false;
         }
     out->vector = n_outside == 0 && wide_vector(out, ti, n_tensors);
     return true;

@@ -68,20 +68,20 @@ def test_a_gathered_row_is_aligned_for_every_index():
     """A gathered launch multiplies the row index with the batch stride also where the batch has one row, so 4-element accesses need
     a stride of whole groups of 4 elements there too (an odd row of an odd stride starts at any byte)."""
     for rows in (1, 2):
-        for n, aligned in ((1024, True), (1029, False), (1026, False), (1028, True)):
-            slots = [slot(n, elm=2, batch=(rows, n)), slot(n, elm=2, batch=(rows, 1032))]
-            r = route(scaled_rows(*HALF, n, 8), slots, count=rows, gather_mask=1)
+        for n, aligned in ((2048, True), (2053, False), (2050, False), (2052, True)):
+            slots = [slot(n, elm=2, batch=(rows, n)), slot(n, elm=2, batch=(rows, 2056))]
+            r = route(scaled_rows(*HALF, n, 16), slots, count=rows, gather_mask=1)
             assert r == (WIDE_VECTOR if aligned else WIDE), (rows, n, r)
     # without the gather a batch of one row never uses its stride
-    assert route(scaled_rows(*HALF, 1029, 8), [slot(1029, elm=2, batch=(1, 1029)), slot(1029, elm=2, batch=(1, 1032))], count=1) == WIDE_VECTOR
+    assert route(scaled_rows(*HALF, 2053, 16), [slot(2053, elm=2, batch=(1, 2053)), slot(2053, elm=2, batch=(1, 2056))], count=1) == WIDE_VECTOR
 
 
 def test_a_gathered_f32_row_is_aligned_for_every_index():
     """The 16-byte accesses of the tile kernels rest on the same rule."""
     for rows in (1, 2):
-        for stride, aligned in ((1024, True), (1029, False), (1026, False)):
-            slots = [slot(1024, batch=(rows, stride)), slot(1024, batch=(rows, 1024))]
-            r = route(scaled_rows(*SINGLE, 1024, 8), slots, count=rows, gather_mask=1)
+        for stride, aligned in ((2048, True), (2053, False), (2050, False)):
+            slots = [slot(2048, batch=(rows, stride)), slot(2048, batch=(rows, 2048))]
+            r = route(scaled_rows(*SINGLE, 2048, 16), slots, count=rows, gather_mask=1)
             assert (r == EARLY) == aligned and r != WIDE_VECTOR, (rows, stride, r)
 
 
@@ -110,17 +110,17 @@ def counted(tiles):
     return [(O.LoadImm, 0)] + [i for k in range(tiles) for i in (at(HALF[0], 128 * k, 0), at(HALF[1], 128 * k, 1), (O.LoadImm, 0x3F800000), (O.FAdd, 0))]
 
 
-@pytest.mark.parametrize("second", [4, 8])
+@pytest.mark.parametrize("second", [8, 16])
 def test_equal_running_values_of_two_loops_are_not_one_value(second):
     """A value that is the same in all four width positions may multiply data in the vector layout. Two loops that add the same terms
     to the same start give the same value only if they run equally often, so a shuffle of both is not such a value."""
-    prog = counted(4) + counted(second) + [(O.FShuf2, 0)]      # two positions of each
-    for k in range(8):
+    prog = counted(8) + counted(second) + [(O.FShuf2, 0)]      # two positions of each
+    for k in range(16):
         prog += [(O.Dup, 0), at(HALF[0], 128 * k, 0), (O.FMul, 0), at(HALF[1], 128 * k, 1)]
     prog += [(O.Pop, 0), (O.Halt, 0)]
-    rows = [slot(1024, elm=2, batch=(64, 1024))] * 2
+    rows = [slot(2048, elm=2, batch=(64, 2048))] * 2
     assert route(prog, rows) == WIDE
-    one = counted(4) + [i for k in range(8) for i in ((O.Dup, 0), at(HALF[0], 128 * k, 0), (O.FMul, 0), at(HALF[1], 128 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
+    one = counted(8) + [i for k in range(16) for i in ((O.Dup, 0), at(HALF[0], 128 * k, 0), (O.FMul, 0), at(HALF[1], 128 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
     assert route(one, rows) == WIDE_VECTOR
 
 
@@ -131,9 +131,9 @@ def test_what_one_loop_stores_the_same_lanes_load_in_the_next(shift, bases, want
     accesses 32 elements apart meet in the same lane, in the vector layout only those 128 apart: by one slot (`shift`) or by two
     slots over one buffer (`bases`: bytes between them)."""
     n_slot, off = (1, shift) if shift is not None else (3, 0)
-    prog = [i for k in range(8) for i in (at(HALF[0], 128 * k, 0), at(HALF[1], 128 * k, 1))]
+    prog = [i for k in range(16) for i in (at(HALF[0], 128 * k, 0), at(HALF[1], 128 * k, 1))]
     prog += [i for k in range(4) for i in (at(HALF[0], 128 * k + off, n_slot), (O.FNeg, 0), at(HALF[1], 128 * k, 2))] + [(O.Halt, 0)]
-    rows = [slot(1024, elm=2, batch=(64, 1024))] * 4
+    rows = [slot(2048, elm=2, batch=(64, 2048))] * 4
     addr = [t << 36 for t in range(1, 5)]
     if bases is not None:
         addr[3] = addr[1] + bases
@@ -145,10 +145,10 @@ def test_what_one_loop_stores_the_same_lanes_load_in_the_next(shift, bases, want
 def test_only_sums_of_two_byte_2dt_tiles_change_their_order(load, elm, want):
     """The vector layout adds the elements of 2DT tiles in another order. That is taken for 2-byte elements alone, whose values carry far
     fewer bits than the sum; f32 and u8 sums keep the program's order, as every other sum does."""
-    prog = [(O.LoadImm, 0)] + [i for k in range(4) for i in ((load, (32 * k << 4)), (O.Dup, 0), (O.FMul, 0), (O.FAdd, 0))]
+    prog = [(O.LoadImm, 0)] + [i for k in range(12) for i in ((load, (32 * k << 4)), (O.Dup, 0), (O.FMul, 0), (O.FAdd, 0))]
     prog += [(O.WarpAllReduceSum, 0)]
-    prog += [i for k in range(4) for i in ((O.Dup, 0), (load, (32 * k << 4)), (O.FMul, 0), at(O.StoreGlobal2DTBF16, 32 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
-    rows = [slot(128, elm=elm, batch=(64, 512), shape2=4, stride2=128), slot(128, elm=2, batch=(64, 512), shape2=4, stride2=128)]
+    prog += [i for k in range(12) for i in ((O.Dup, 0), (load, (32 * k << 4)), (O.FMul, 0), at(O.StoreGlobal2DTBF16, 32 * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
+    rows = [slot(384, elm=elm, batch=(64, 1536), shape2=4, stride2=384), slot(384, elm=2, batch=(64, 1536), shape2=4, stride2=384)]
     assert route(prog, rows) == want
 
 
@@ -158,3 +158,54 @@ def test_a_program_too_long_for_the_tile_kernels_has_no_other_route(tiles, want)
     depend on addresses, so such a program has no stream with loops either."""
     rows = [slot(128 * tiles, elm=2, batch=(64, 128 * tiles))] * 2
     assert route(scaled_rows(*HALF, 128 * tiles, tiles), rows) == want
+
+
+def normalised_rows(load, store, tiles, step=128):
+    """out = x * sum(x): every row loaded twice."""
+    p = [(O.LoadImm, 0)] + [i for k in range(tiles) for i in (at(load, step * k, 0), (O.FAdd, 0))] + [(O.WarpAllReduceSum, 0)]
+    if step == 128:      # ... and over the four width values
+        p += [(O.Dup, 0), (O.FPermW, 0x01000302), (O.FAdd, 0), (O.Dup, 0), (O.FPermW, 0x02030001), (O.FAdd, 0)]
+    return p + [i for k in range(tiles) for i in ((O.Dup, 0), at(load, step * k, 0), (O.FMul, 0), at(store, step * k, 1))] + [(O.Pop, 0), (O.Halt, 0)]
+
+
+@pytest.mark.parametrize("tiles,rows,want", [(2, 1184, WIDE), (2, 1185, 0), (3, 9472, WIDE), (3, 9473, 0), (4, 59200, WIDE), (4, 59201, 0), (5, 200000, WIDE)])
+def test_short_f32_rows_stream_only_in_small_launches(tiles, rows, want):
+    """Both sides of the lines: unaligned f32 rows that are loaded twice."""
+    n = 128 * tiles - 3
+    r = route(normalised_rows(*SINGLE, tiles), [slot(n, batch=(rows, n))] * 2, count=rows)
+    assert r & (WIDE | WIDE_VECTOR) == want, r
+
+
+@pytest.mark.parametrize("form,tiles,n,rows,want", [("once", 15, 1917, 100, 0), ("once", 16, 2045, 1184, WIDE), ("once", 16, 2045, 1185, 0), ("twice", 16, 2048, 100, 0)])
+def test_f32_rows_loaded_once_stream_only_where_long_and_few(form, tiles, n, rows, want):
+    prog = scaled_rows(*SINGLE, n, tiles) if form == "once" else normalised_rows(*SINGLE, tiles)      # (the last: aligned rows of whole tiles)
+    assert route(prog, [slot(n, batch=(rows, n))] * 2, count=rows) & (WIDE | WIDE_VECTOR) == want
+
+
+@pytest.mark.parametrize("tiles,aligned,rows,want", [(4, True, 9, WIDE_VECTOR), (5, True, 9, 0), (8, True, 90000, WIDE_VECTOR), (10, True, 1184, WIDE_VECTOR), (10, True, 1185, 0),
+                                                     (11, True, 90000, WIDE_VECTOR), (10, False, 9, 0), (11, False, 1184, WIDE), (11, False, 1185, 0), (16, False, 90000, WIDE)])
+def test_half_precision_rows(tiles, aligned, rows, want):
+    n = 128 * tiles - (0 if aligned else 1)
+    assert route(normalised_rows(*HALF, tiles), [slot(n, elm=2, batch=(rows, n))] * 2, count=rows) & (WIDE | WIDE_VECTOR) == want
+
+
+@pytest.mark.parametrize("load,store,elm,tiles,aligned,want", [
+    (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 3, True, 0), (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 4, True, WIDE_VECTOR),
+    (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 4, False, 0), (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 5, False, WIDE),
+    (O.LoadGlobal2DTF16, O.StoreGlobal2DTF16, 2, 9, False, 0), (O.LoadGlobal2DTF16, O.StoreGlobal2DTF16, 2, 10, False, WIDE),
+    (O.LoadGlobal2DTF32, O.StoreGlobal2DTF32, 4, 5, True, 0), (O.LoadGlobal2DTF32, O.StoreGlobal2DTF32, 4, 6, True, WIDE)])
+def test_2dt_rows(load, store, elm, tiles, aligned, want):
+    n = 32 * tiles - (0 if aligned else 1)
+    slots = [slot(n, elm=elm, batch=(64, 4 * n), shape2=4, stride2=n)] * 2
+    assert route(normalised_rows(load, store, tiles, 32), slots) & (WIDE | WIDE_VECTOR) == want
+
+
+@pytest.mark.parametrize("load,store,elm,math,whole,n,want", [
+    (*SINGLE, 4, False, False, 1 << 22, 0), (*SINGLE, 4, False, False, (1 << 22) + 128, FLAT), (*SINGLE, 4, True, False, 1 << 25, 0),
+    (*SINGLE, 4, False, True, 1 << 23, 0), (*SINGLE, 4, False, True, (1 << 23) + 128, FLAT), (*HALF, 2, True, True, 1 << 21, 0), (*HALF, 2, True, True, (1 << 21) + 128, FLAT),
+    (HALF[0], SINGLE[1], 2, True, True, 1 << 22, 0), (HALF[0], SINGLE[1], 2, True, True, (1 << 22) + 128, FLAT)])
+def test_flat_programs(load, store, elm, math, whole, n, want):
+    prog = [at(load, 0, 0), (O.FSqrt, 0) if math else (O.FNeg, 0), at(store, 0, 1), (O.Halt, 0)]
+    length = n if whole else n - 1
+    slots = [slot(length, elm=elm, grid1=n // 128, step1=128), slot(length, elm=4 if store == SINGLE[1] else elm, grid1=n // 128, step1=128)]
+    assert route(prog, slots, count=n // 128) & FLAT == want
