@@ -1230,11 +1230,24 @@ __device__ __forceinline__ void state_declare()
 
 extern __shared__ __align__(16) unsigned char g_smem[];
 
+/* The streaming kernels in the natural layout keep the offset form: with the address in a register the 8-tile one spills less and is
+ * slower all the same (RMSNorm 10007 x 2029 54.6 -> 55.5 us, 112 x 1558 10.3 -> 12.2). */
+#if defined(GINT_WIDE) && !defined(GINT_WIDE_V)
+#define GINT_TILES_BY_OFFSET 1
+#endif
+__device__ __forceinline__ uint32_t tiles_word(const TileInfo *tiles)
+{
+#ifdef GINT_TILES_BY_OFFSET
+    return (uint32_t)(reinterpret_cast<const unsigned char *>(tiles) - g_smem);
+#else
+    return (uint32_t)__cvta_generic_to_shared(tiles);
+#endif
+}
 __device__ __forceinline__ void context_set(const Ctx &cx)
 {
     asm volatile("mov.b32 %%gl4, %0;" ::"r"(cx.lane * 4));
     asm volatile("mov.b32 %%gx0, %0; mov.b32 %%gx1, %1; mov.b32 %%gx2, %2; mov.b32 %%gx3, %3; mov.b32 %%gx4, %4; mov.b32 %%gx5, %5;"
-                 ::"r"((uint32_t)__cvta_generic_to_shared(cx.tiles)), "r"(cx.lane), "r"(cx.hidden), "r"(cx.ring_mask), "r"(cx.rows), "r"(cx.rows_stride));
+                 ::"r"(tiles_word(cx.tiles)), "r"(cx.lane), "r"(cx.hidden), "r"(cx.ring_mask), "r"(cx.rows), "r"(cx.rows_stride));
 }
 __device__ __forceinline__ Ctx handler_context()
 {
@@ -1244,8 +1257,12 @@ __device__ __forceinline__ Ctx handler_context()
     cx.lane4 = lane4;
     asm volatile("mov.b32 %0, %%gx0; mov.b32 %1, %%gx1; mov.b32 %2, %%gx2; mov.b32 %3, %%gx3; mov.b32 %4, %%gx4; mov.b32 %5, %%gx5;"
                  : "=r"(tiles), "=r"(cx.lane), "=r"(cx.hidden), "=r"(cx.ring_mask), "=r"(cx.rows), "=r"(cx.rows_stride));
+#ifdef GINT_TILES_BY_OFFSET
+    cx.tiles = reinterpret_cast<TileInfo *>(g_smem + tiles);
+#else
     cx.tiles = reinterpret_cast<TileInfo *>(__cvta_shared_to_generic(tiles));
     __builtin_assume(__isShared(cx.tiles));   // its accesses are shared-memory instructions on that address
+#endif
     return cx;
 }
 
