@@ -1256,7 +1256,7 @@ constexpr uint64_t kFlatMinTiles = 16384;   // 2^21 elements
  * and square root 0.94 at 2.5 M, 1.1 to 1.4 from 4 M on; bodies that need a fourth slot 0.85 to 1.0.
  *
  * f32 rows that are not fast. RMSNorm, which loads its row twice: 2 tiles 1.15 at 1000 rows, 0.99 at 2400, 0.60 at 200 000; 3 tiles 1.36 at
- * 1000, 1.04 at 10 000, 0.87 at 60 000; 4 tiles 1.25 at 10 000, 1.07 at 60 000, 0.96 at 200 000; 5 and more 1.06 to 2.8. Rows loaded once
+ * 1000, 1.04 at 10 000, 0.87 at 60 000; 4 tiles 1.25 at 10 000, 1.07 at 60 000, 0.96 at 200 000; 5 and more 1.0 to 2.6. Rows loaded once
  * (sums, scaling): 3 to 9 tiles 0.7 to 1.05, 16 and 32 tiles 1.0 to 1.5 up to 1000 rows, 0.84 to 1.07 above. Fast rows: RMSNorm
  * 16384 x 4096 114 us there, 121 here; sums of 65536 x 1024 50 against 75.
  *
@@ -1264,7 +1264,7 @@ constexpr uint64_t kFlatMinTiles = 16384;   // 2^21 elements
  * 10 tiles 1.25 to 1.4 up to 1000 rows, 0.94 at 20 000; 11 tiles 1.02 to 1.6, 15 and more 1.2 to 3.2. Natural layout: 2 to 9 tiles 0.5 to 1.2,
  * 11 and 13 tiles 1.07 to 1.4 up to 1000 rows where the row is loaded twice, 0.8 to 1.05 above, 16 and more 1.1 to 2.6.
  *
- * 2DT rows. Vector layout, 4 tiles and more: 1.07 to 2.9. Natural layout: 2 and 3 tiles 0.47 to 1.02; bf16 5 tiles 1.01 to 1.09, more 1.08 to 2.1;
+ * 2DT rows. Vector layout, 4 tiles and more: 1.07 to 2.9. Natural layout: 2 and 3 tiles 0.47 to 1.02; bf16 5 tiles 0.91 to 1.09, more 1.08 to 2.1;
  * f32 5 tiles 0.94 to 0.98, 6 and more 1.06 to 3.0; f16 5 and 6 tiles 0.88 to 0.95, 9 tiles 0.93 to 0.98, 10 and more 1.03 to 1.8 (u8: as f16).
  */
 bool wide_pays(const gint_ctx *ctx, const Program *p, bool vector, bool fast, uint32_t count)
@@ -1280,7 +1280,7 @@ bool wide_pays(const gint_ctx *ctx, const Program *p, bool vector, bool fast, ui
     }
     if (p->wide_2dt) {
         if (vector) return tiles >= 4;
-        return tiles >= (p->wide_f16 || p->wide_u8 ? 10 : f32_only ? 6 : 5);
+        return tiles >= (p->wide_f16 || p->wide_u8 ? 10 : 6);
     }
     if (f32_only) {
         if (fast) return false;

@@ -20,10 +20,9 @@
  * One warp runs one logical program. Programs that are nothing but one loop over 1-D tiles, whose logical programs follow one
  * another in memory, run "flat": the whole launch is one loop, cut among all warps.
  *
- * Measured (one B200, us per pass, tile kernels -> here): a + b over 40 000 003 elements 91 -> 79 (148 -> 54 warp instructions per
- * tile; 6.1 TB/s); a * sigmoid(a) * b in f16 over 24 000 500 elements 85 -> 59; RMSNorm of 10007 unaligned rows of 2029 values 77 -> 55 (262 -> 113);
- * RMSNorm of bf16 heads (8, 4096, 16, 128) 187 -> 151
- * (246 -> 164). U = 8 with 3 slots (128 registers, 16 warps per SM) beats U = 8 with 2 slots (96
+ * Measured (one B200, us per launch on the device, tile kernels -> here): a + b over 40 000 003 elements 84 -> 76 (53 warp instructions
+ * per tile; 6.2 TB/s per pass); a * sigmoid(a) * b in f16 over as many 133 -> 93 (162); RMSNorm of 10 000 unaligned rows of 2029 values
+ * 72 -> 56 (113); RMSNorm of 50 000 bf16 rows of 128 23.4 -> 18.9 (166), of 512 82 -> 46. U = 8 with 3 slots (128 registers, 16 warps per SM) beats U = 8 with 2 slots (96
  * registers, 20 warps; f16 57 against 67: calls spill) and U = 4 with 4 slots for long loops (79 against 83; 59 against 64); short
  * loops leave U = 8 half empty (heads of 128: 150 at U = 4, 210 at U = 8). What bounds the flat programs is memory (a + b) and the
  * exponential and division (f16); the row programs wait for memory round trips and for the instruction cache.

@@ -191,7 +191,7 @@ def test_half_precision_rows(tiles, aligned, rows, want):
 
 @pytest.mark.parametrize("load,store,elm,tiles,aligned,want", [
     (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 3, True, 0), (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 4, True, WIDE_VECTOR),
-    (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 4, False, 0), (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 5, False, WIDE),
+    (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 5, False, 0), (O.LoadGlobal2DTBF16, O.StoreGlobal2DTBF16, 2, 6, False, WIDE),
     (O.LoadGlobal2DTF16, O.StoreGlobal2DTF16, 2, 9, False, 0), (O.LoadGlobal2DTF16, O.StoreGlobal2DTF16, 2, 10, False, WIDE),
     (O.LoadGlobal2DTF32, O.StoreGlobal2DTF32, 4, 5, True, 0), (O.LoadGlobal2DTF32, O.StoreGlobal2DTF32, 4, 6, True, WIDE)])
 def test_2dt_rows(load, store, elm, tiles, aligned, want):

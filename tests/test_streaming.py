@@ -363,7 +363,7 @@ def test_streaming_2dt_rows(rows, dim, dtype):
         if dtype in ("f16", "bf16") and dim % 128 == 0:
             assert r == STREAMING_VECTOR
         else:
-            assert (r == STREAMING) == (tiles >= {"f32": 6, "bf16": 5}.get(dtype, 10)) and r != STREAMING_VECTOR
+            assert (r == STREAMING) == (tiles >= {"f32": 6, "bf16": 6}.get(dtype, 10)) and r != STREAMING_VECTOR
         rows_2dt(x, y, w, grid_dim=-(-rows // 4), **kw)
         return [y]
     if dtype in ("f32", "u8") or -(-dim // 32) % 4 != 0:
