@@ -9,7 +9,7 @@ Pipeline, per interpreter kernel in ``gint_b200/csrc/kernels/*.cu``:
 
 then ``gint_capi.cu`` (host code) is compiled and everything is linked into ``gint_b200/libgint_b200.so`` with the CUDA
 runtime linked statically. nvcc cross-compiles without a GPU, so this also runs on a CPU-only machine. A unit is rebuilt
-when it or any header is newer than its output.
+when its source, a header that it includes (listed in a .d file by its last build) or this file is newer than its output.
 """
 from __future__ import annotations
 
@@ -54,10 +54,15 @@ def _run(cmd: list[str], what: str) -> str:
     return r.stderr + r.stdout
 
 
-def _newest_header() -> float:
-    hdrs = glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh")) + [HOT_HEADER] + \
-        glob.glob(os.path.join(PKG_DIR, "..", "include", "*.h")) + [__file__]
-    return max(os.path.getmtime(h) for h in hdrs)
+def _outdated(obj: str) -> bool:
+    """Is a file that `obj` was made from (its .d file) newer than it, or not known?"""
+    dep = obj[:-2] + ".d"
+    if not os.path.exists(obj) or not os.path.exists(dep):
+        return True
+    with open(dep) as f:
+        files = f.read().split(":", 1)[1].replace("\\\n", " ").split()
+    made = os.path.getmtime(obj)
+    return any(not os.path.exists(h) or os.path.getmtime(h) > made for h in files + [__file__])
 
 
 def _write_hot_header(ordered: bool) -> None:
@@ -78,7 +83,7 @@ def _build_kernel(src: str, extra: list[str]) -> tuple[str, str]:
     sym = stem.replace("gint_", "gint_cubin_").replace("_p", "_").replace("_k", "_")   # gint_cubin_direct_4_1
     cubin, obj = (os.path.join(OBJ_DIR, stem + ext) for ext in (".cubin", ".o"))
     t0 = time.time()
-    log = _run([_nvcc(), "-arch=sm_100a", "-cubin", "-Xptxas", "-v", "-I", OBJ_DIR] + COMMON + extra + [src, "-o", cubin], f"nvcc {stem}")
+    log = _run([_nvcc(), "-arch=sm_100a", "-cubin", "-Xptxas", "-v", "-I", OBJ_DIR, "-MD", "-MF", obj[:-2] + ".d"] + COMMON + extra + [src, "-o", cubin], f"nvcc {stem}")
     log += f"build time: {time.time() - t0:.0f} s\n"
     asm = os.path.join(OBJ_DIR, stem + ".S")
     with open(asm, "w") as f:
@@ -97,23 +102,22 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False, e
     if not os.path.exists(stamp) or open(stamp).read() != flags_now:
         force = True
     _write_hot_header(hot_order)
-    hdr_time = _newest_header()
     kernels = sorted(glob.glob(os.path.join(KERNELS, "*.cu")))
     todo, objs = [], []
     for src in kernels:
         obj = os.path.join(OBJ_DIR, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
-        if force or not os.path.exists(obj) or os.path.getmtime(obj) < max(os.path.getmtime(src), hdr_time):
+        if force or _outdated(obj):
             todo.append(src)
     logs = []
     capi_src = os.path.join(CSRC, "gint_capi.cu")
     capi_obj = os.path.join(OBJ_DIR, "gint_capi.o")
     objs.append(capi_obj)
-    capi_todo = force or not os.path.exists(capi_obj) or os.path.getmtime(capi_obj) < max(os.path.getmtime(capi_src), hdr_time)
+    capi_todo = force or _outdated(capi_obj)
     with concurrent.futures.ThreadPoolExecutor(max_workers=jobs or os.cpu_count() or 4) as ex:
         futs = [ex.submit(_build_kernel, s, extra) for s in todo]
         if capi_todo:
-            futs.append(ex.submit(lambda: ("gint_capi", _run([_nvcc()] + ARCH + COMMON + ["-Xcompiler", "-fPIC", "-c", capi_src, "-o", capi_obj],
+            futs.append(ex.submit(lambda: ("gint_capi", _run([_nvcc()] + ARCH + COMMON + ["-Xcompiler", "-fPIC", "-MD", "-MF", capi_obj[:-2] + ".d", "-c", capi_src, "-o", capi_obj],
                                                               "nvcc gint_capi"))))
         for f in concurrent.futures.as_completed(futs):
             logs.append(f.result())
