@@ -878,6 +878,7 @@ uint64_t tensor_extent_bytes(const gint_tensor_info &ti, int t)
 }  // namespace
 
 #include "gint_wide_host.h"
+#include "gint_forms_host.h"
 
 namespace {
 
@@ -897,7 +898,7 @@ struct KernelImage {
     const unsigned char *begin;
     const unsigned char *end;
     const char *name;
-    int P, K;          // K == 0: indirect kernel; K == -1: checked kernel
+    int P, K;          // K == 0: indirect kernel; K == -1: checked kernel; K == -2: form kernel P
     cudaLibrary_t lib;
     cudaKernel_t kernel;
     bool loaded;
@@ -927,6 +928,9 @@ KernelImage g_images[] = {
 #undef GINT_X_IMG
 #define GINT_X_IMG(P) {gint_cubin_checked_##P, gint_cubin_checked_##P##_end, "gint_geval_checked_" #P, P, -1, nullptr, nullptr, false, false},
     GINT_CHECKED_VARIANTS(GINT_X_IMG)
+#undef GINT_X_IMG
+#define GINT_X_IMG(name, form) {gint_cubin_##name, gint_cubin_##name##_end, "gint_form_" #name, form, -2, nullptr, nullptr, false, false},
+    GINT_FORM_KERNELS(GINT_X_IMG)
 #undef GINT_X_IMG
 };
 std::mutex g_images_mu;
@@ -1016,6 +1020,7 @@ struct Program {
     bool wide_f32 = false, wide_f16 = false, wide_bf16 = false, wide_u8 = false, wide_2dt = false, wide_math = false, wide_rereads = false;
     uint32_t wide_rows = 0;     // slots of which every logical program has its own part
     uint2 wide_inline[gint::kInlineCodeSlots];
+    Form form;                  // the form the program has, if any (gint_forms_host.h)
     PlanMemo memo[6] = {};      // last launch plan of the plain stream [0], the early-issue stream [1], the RF stream [2], the vector-layout stream [3], the streaming kernels in the natural [4] and the vector layout [5]
     std::mutex memo_mu;
 };
@@ -1065,6 +1070,8 @@ struct gint_ctx {
     std::vector<Variant> direct;
     Variant indirect{12, 1, nullptr, 0, false, 0};
     Variant checked{12, 1, nullptr, 0, false, 0};
+    const void *form_fn[GINT_N_FORM_KERNELS] = {};
+    std::atomic<bool> form_launched{false};
     gint_device_status *status_dev = nullptr;   // status word of the checked launches (allocated on first use)
     std::string last_error;
     int opt_tiles_per_warp = 0;
@@ -1075,6 +1082,7 @@ struct gint_ctx {
     int opt_lower = 1;          // DupBroadcastW -> Bcast_k (lower_lane_moves); applies to programs created afterwards
     int opt_rf = 1;             // launches use a program's RF stream (virtual registers in shared memory) when it has one
     int opt_rf_create = 1;      // programs created from now on get an RF stream when they qualify
+    int opt_forms = 1;          // launches of programs that have a form run on its kernel
     int opt_wide = 1;           // launches use a program's stream with loops (streaming kernels) when it has one
     int opt_vec = 0;            // vector-layout stream and kernels for the programs that qualify (creation and launch). Off unless asked
                                 // for: measured on the conductor graph, the fused program alone gains 2-3 % (175 -> 169 us) but the whole
@@ -1383,6 +1391,43 @@ Route choose_route(const gint_ctx *ctx, const Program *p, const uint64_t *base_p
     return r;
 }
 
+/* Does a launch run on the kernel of the program's form, and with which arguments? Not where the caller has asked for a particular
+ * configuration of the interpreter, and not where the stored tensor overlaps one that is read: the form reads logical programs ahead. */
+int choose_form(const gint_ctx *ctx, const Program *p, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather,
+                gint::RowsArgs *a, RowsPlan *plan)
+{
+    const Form &f = p->form;
+    if (f.kind == FORM_NONE || !ctx->opt_forms || !ctx->opt_wide || !ctx->opt_early_issue || !ctx->opt_rf || ctx->opt_vec || ctx->opt_prefetch || ctx->opt_tiles_per_warp) return FORM_NONE;
+    if ((uint64_t)first + count >= (1ull << 31)) return FORM_NONE;
+    if (!plan_rows(f.rows, count, ctx->num_sms, ctx->max_smem_optin, plan)) return FORM_NONE;
+    *a = f.rows;
+    uint64_t lo[gint::ROWS_N_SLOTS], hi[gint::ROWS_N_SLOTS];
+    for (int s = 0; s < gint::ROWS_N_SLOTS; s++) {
+        if (f.tensor[s] < 0) continue;
+        a->slot[s].base = lo[s] = base_ptrs[f.tensor[s]];
+        hi[s] = lo[s] + f.extent[s];
+        if ((lo[s] & f.base_align) != 0) return FORM_NONE;
+        if (!gather || !((gather->mask >> f.tensor[s]) & 1u)) continue;
+        if (s == f.store) return FORM_NONE;
+        hi[s] = lo[s] + gather->extent_bytes;
+        if (!f.gathers[s]) continue;
+        /* (an index into a single row moves it as well, but not by a digit) */
+        if (f.gather_digit[s] < 0 || (a->grid.gather_mask && a->grid.gather_dim != f.gather_digit[s])) return FORM_NONE;
+        a->grid.gather_dim = f.gather_digit[s];
+        a->grid.gather_mask |= 1u << s;
+        a->grid.gather_index = gather->index;
+        a->grid.gather_rows = gather->rows;
+    }
+    for (int s = 0; s < gint::ROWS_N_SLOTS; s++)
+        if (f.tensor[s] >= 0 && s != f.store && lo[s] < hi[f.store] && lo[f.store] < hi[s]) return FORM_NONE;
+    a->first = first;
+    a->count = count;
+    a->depth = plan->depth;
+    a->grid.simple = a->grid.n_dims == 1 && first + count <= a->grid.size[0];
+    if (ctx->opt_max_blocks > 0 && (uint32_t)ctx->opt_max_blocks < plan->grid) plan->grid = (uint32_t)ctx->opt_max_blocks;
+    return f.kind;
+}
+
 int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int n_tensors, uint32_t first, uint32_t count,
                   void *stream, const GatherArgs *gather = nullptr)
 {
@@ -1393,6 +1438,17 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
     if (count == 0) return GINT_OK;
     if ((uint64_t)first + (uint64_t)count > 0xFFFFFFFFull) return fail(ctx, GINT_ERR_TOO_LARGE, "logical program range overflows 32 bits");
     DeviceGuard guard(ctx->device);
+    if (p->form.kind != FORM_NONE && ctx->form_fn[0] && ctx->form_fn[1]) {
+        gint::RowsArgs a;
+        RowsPlan plan;
+        if (choose_form(ctx, p, base_ptrs, first, count, gather, &a, &plan)) {
+            void *args[1] = {&a};
+            cudaError_t e = cudaLaunchKernel(ctx->form_fn[plan.team == 4], dim3(plan.grid), dim3(plan.teams * plan.team * 32u), args, plan.smem, (cudaStream_t)stream);
+            if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaLaunchKernel", e);
+            ctx->form_launched = true;
+            return GINT_OK;
+        }
+    }
     const Route route = choose_route(ctx, p, base_ptrs, first, count, gather);
     if (route.wide) {
         const bool vector = route.wide == 2;
@@ -1520,7 +1576,9 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
         normalise(code, n_words, n_tensors, &prog);
         WideStream ws;
         bool fits = false;
-        if (wide_transform(prog, p->ti, n_tensors, &ws))
+        const bool loops = wide_transform(prog, p->ti, n_tensors, &ws);
+        if (loops && ctx->opt_fuse && ctx->opt_lower) match_rows(ws.prog, p->ti, &p->form);
+        if (loops && !ws.slow_rows)
             for (auto &v : ctx->direct) fits = fits || (v.wide == 1 && v.ok && v.P >= ws.max_depth);
         if (fits) {
             std::vector<Insn> numbered = ws.prog;
@@ -1814,6 +1872,31 @@ int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *t
     return r.wide ? (r.wide << 4) | (flat ? 1 << 6 : 0) : (r.early ? 1 : 0) | (r.rf ? 2 : 0) | (r.vec ? 4 : 0);
 }
 
+int gint_debug_form(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs, uint32_t first,
+                    uint32_t count, uint32_t gather_mask, uint64_t gather_extent_bytes, uint32_t logical, int64_t row, uint32_t *out_offsets)
+{
+    if (!code || (!(ti && base_ptrs) && n_tensors > 0) || n_tensors < 0 || n_tensors > GINT_MAX_TENSORS) return GINT_ERR_INVALID_ARGUMENT;
+    gint_ctx ctx;   // (the default options; no device)
+    ctx.max_smem_optin = 227 * 1024;
+    ctx.num_sms = 148;
+    Program *p = nullptr;
+    ProgramStreams streams;
+    const int rc = build_program(&ctx, code, n_words, ti, n_tensors, &p, &streams);
+    if (rc != GINT_OK) return rc;
+    const GatherArgs ga{gather_mask, nullptr, gather_extent_bytes, 1u};
+    gint::RowsArgs a;
+    RowsPlan plan;
+    const int kind = choose_form(&ctx, p, base_ptrs, first, count, gather_mask ? &ga : nullptr, &a, &plan);
+    if (kind && out_offsets) {
+        uint32_t off[gint::ROWS_N_SLOTS];
+        gint::form_offsets(a.grid, a.slot, logical, row, off);
+        for (int s = 0; s < gint::ROWS_N_SLOTS; s++)
+            if (p->form.tensor[s] >= 0) out_offsets[p->form.tensor[s]] = off[s];
+    }
+    delete p;
+    return kind ? kind | (int)(plan.team << 8) : 0;
+}
+
 int gint_create(int device, gint_ctx **out)
 {
     if (!out) return GINT_ERR_INVALID_ARGUMENT;
@@ -1837,7 +1920,12 @@ int gint_create(int device, gint_ctx **out)
     for (auto &im : g_images) {
         if (!im.loaded) continue;
         if (im.K == 0) ctx->indirect.fn = (const void *)im.kernel;
-        else if (im.K < 0) ctx->checked.fn = (const void *)im.kernel;
+        else if (im.K == -1) ctx->checked.fn = (const void *)im.kernel;
+        else if (im.K == -2) {
+            const void *fn = (const void *)im.kernel;
+            if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin) == cudaSuccess) ctx->form_fn[im.P] = fn;
+            else cudaGetLastError();
+        }
         else ctx->direct.push_back(Variant{im.P, im.K, (const void *)im.kernel, 0, false, 0, im.rf, im.vec, im.wide});
     }
     int usable = 0;
@@ -2031,6 +2119,9 @@ int gint_program_launch_info(gint_ctx *ctx, uint64_t handle, uint32_t grid_dim, 
     out->registers_in_smem = g.v->rf ? p->st.max_reg_idx + 1 : 0;
     out->vector_layout = g.v->vec || g.v->wide == 2 ? 1 : 0;
     out->streaming = g.v->wide ? 1 : 0;
+    gint::RowsArgs a;
+    RowsPlan plan;
+    out->form = ctx->form_fn[0] && ctx->form_fn[1] ? choose_form(ctx, p, base_ptrs, 0u, count, nullptr, &a, &plan) : 0;
     return GINT_OK;
 }
 
@@ -2119,11 +2210,24 @@ int gint_device_status_read(gint_ctx *ctx, gint_device_status *out, int clear)
 {
     if (!ctx || !out) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "null argument");
     memset(out, 0, sizeof(*out));
-    if (!ctx->status_dev) return GINT_OK;     // no checked launch so far
+    if (!ctx->status_dev && !ctx->form_launched) return GINT_OK;     // nothing that reports anything so far
     DeviceGuard guard(ctx->device);
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemcpy(out, ctx->status_dev, sizeof(*out), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && clear) e = cudaMemset(ctx->status_dev, 0, sizeof(*out));
+    if (ctx->status_dev) {
+        if (e == cudaSuccess) e = cudaMemcpy(out, ctx->status_dev, sizeof(*out), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && clear) e = cudaMemset(ctx->status_dev, 0, sizeof(*out));
+    }
+    for (auto &im : g_images) {   // form kernels count the teams that gave up waiting for a copy
+        void *flag = nullptr;
+        size_t bytes = 0;
+        uint32_t n = 0;
+        if (im.K != -2 || !im.loaded || !ctx->form_launched) continue;
+        if (e == cudaSuccess) e = cudaLibraryGetGlobal(&flag, &bytes, im.lib, "gint_form_gave_up");
+        if (e == cudaSuccess) e = cudaMemcpy(&n, flag, sizeof(n), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && n && clear) e = cudaMemset(flag, 0, sizeof(n));
+        if (n && out->code == GINT_DEVICE_OK) { out->code = GINT_DEVICE_GAVE_UP; out->slot = -1; }
+        out->count += n;
+    }
     if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "reading the device status", e);
     return GINT_OK;
 }
@@ -2428,7 +2532,7 @@ int gint_debug_transform(const int32_t *code, int n_words, const gint_tensor_inf
     if (rc != GINT_OK) return rc;
     if (early_issue & 8) {   // the stream with loops for the streaming kernels, if the program qualifies; a flat one starts with LoopBegin 0
         WideStream ws;
-        if (!ti || !wide_transform(prog, *ti, n_tensors, &ws)) return 0;
+        if (!ti || !wide_transform(prog, *ti, n_tensors, &ws) || ws.slow_rows) return 0;
         if ((int)ws.prog.size() > max_insns) return GINT_ERR_INVALID_ARGUMENT;
         for (size_t i = 0; i < ws.prog.size(); i++) { out_ops[i] = ws.prog[i].op; out_operands[i] = ws.prog[i].operand; }
         return (int)ws.prog.size();
@@ -2521,6 +2625,10 @@ int gint_set_option(gint_ctx *ctx, const char *name, int value)
     }
     if (strcmp(name, "register_file") == 0) {   // virtual registers in shared memory: programs created and launches made from now on
         ctx->opt_rf = ctx->opt_rf_create = value != 0;
+        return GINT_OK;
+    }
+    if (strcmp(name, "forms") == 0) {   // launches made from now on
+        ctx->opt_forms = value != 0;
         return GINT_OK;
     }
     if (strcmp(name, "streaming") == 0) {   // launches made from now on

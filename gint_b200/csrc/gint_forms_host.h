@@ -1,0 +1,257 @@
+/*
+ * gint_forms_host.h -- host side of the form kernels: recognises the program shapes that have a kernel of their own and lays out
+ * their launches. Included by gint_capi.cu only, after gint_wide_host.h.
+ */
+#pragma once
+
+#include "gint_form_types.h"
+
+namespace {
+
+enum { FORM_NONE = 0, FORM_ROWS = 1 };
+
+struct Form {
+    int kind = FORM_NONE;
+    int tensor[gint::ROWS_N_SLOTS] = {-1, -1, -1, -1};   // tensor slot of every operand of the form; -1: none
+    int store = 0;                                       // which of them is stored to
+    uint64_t extent[gint::ROWS_N_SLOTS] = {};            // bytes from the base pointer that the operand's accesses reach
+    int gather_digit[gint::ROWS_N_SLOTS] = {};           // digit that is the slot's innermost batch dimension; -1: it has one entry
+    bool gathers[gint::ROWS_N_SLOTS] = {};               // ... whose stride is not 0: an index chooses among its rows
+    uint32_t base_align = 3;                             // alignment of the base pointers (minus 1)
+    gint::RowsArgs rows;                                 // all but pointers, range and shared memory
+};
+
+struct FormDim { uint32_t size, stride; bool batch0; };
+
+/* The digits of a slot's place (decode_tiles in gint_interp.cuh), those of one value left out. Fails where the block grid cuts
+ * dimension 1, or an element index could leave 31 bits. */
+bool form_dims(const gint_tensor_info &ti, int t, int n, std::vector<FormDim> *dims, uint64_t *reach)
+{
+    dims->clear();
+    if (ti.block_grid_dims[t][0] != 1) return false;
+    const int64_t step2 = (int64_t)ti.block_grid_steps[t][1] * ti.block_shape_stride_2[t][1];
+    if (step2 < 0 || step2 >= (1ll << 31)) return false;
+    if (ti.block_grid_dims[t][1] != 1) dims->push_back(FormDim{(uint32_t)ti.block_grid_dims[t][1], (uint32_t)step2, false});
+    for (int j = 0; j < 4; j++) {
+        if (ti.batch_strides[t][j] < 0) return false;
+        if (ti.batch_shape[t][j] != 1) dims->push_back(FormDim{(uint32_t)ti.batch_shape[t][j], (uint32_t)ti.batch_strides[t][j], j == 0});
+    }
+    uint64_t last = (uint64_t)n;
+    for (const FormDim &d : *dims) {
+        if (d.size < 1 || d.size >= (1u << 31)) return false;
+        if (d.stride != 0 && (uint64_t)(d.size - 1) > (1ull << 31) / d.stride) return false;
+        last += (uint64_t)(d.size - 1) * d.stride;
+    }
+    *reach = last;
+    return last < (1ull << 31) - 8192;
+}
+
+void form_magic(uint32_t size, uint32_t *magic, uint32_t *shift)
+{
+    uint32_t l = 0;
+    while ((1ull << l) < size) l++;
+    *magic = (uint32_t)(((1ull << (31 + l)) + size - 1) / size);   // size in [2, 2^31): below 2^32; exact for numbers below 2^31
+    *shift = l;
+}
+
+/* The slots' common digits. A slot whose strides are all 0 is the same for every logical program whatever its digits are. */
+bool form_grid(const gint_tensor_info &ti, const int *tensor, int n_slots, const int *n, int elem_bytes, gint::FormGrid *grid, gint::FormSlot *slots, Form *f)
+{
+    std::vector<FormDim> common, dims;
+    bool have = false;
+    memset(grid, 0, sizeof(*grid));
+    grid->gather_dim = -1;
+    for (int s = 0; s < n_slots; s++) {
+        slots[s] = gint::FormSlot{};
+        if (tensor[s] < 0) continue;
+        uint64_t reach = 0;
+        if (ti.elm_size[tensor[s]] != elem_bytes || n[s] < 1 || !form_dims(ti, tensor[s], n[s], &dims, &reach)) return false;
+        slots[s].n = n[s];
+        f->extent[s] = reach * (uint64_t)elem_bytes;
+        bool moves = false;
+        for (const FormDim &d : dims) moves = moves || d.stride != 0;
+        f->gather_digit[s] = -1;
+        f->gathers[s] = ti.batch_strides[tensor[s]][0] != 0;
+        for (size_t j = 0; j < dims.size(); j++) if (dims[j].batch0) f->gather_digit[s] = (int)j;
+        slots[s].stationary = !moves;
+        if (!moves) continue;
+        if (have && dims.size() != common.size()) return false;
+        for (size_t j = 0; have && j < dims.size(); j++) if (dims[j].size != common[j].size) return false;
+        common = dims;
+        have = true;
+        for (size_t j = 0; j < dims.size(); j++) slots[s].stride[j] = dims[j].stride;
+    }
+    grid->n_dims = (uint32_t)common.size();
+    for (size_t j = 0; j < common.size(); j++) {
+        grid->size[j] = common[j].size;
+        form_magic(common[j].size, &grid->magic[j], &grid->shift[j]);
+    }
+    return true;
+}
+
+/* what stands between the loops, as steps on the one value of the stack */
+bool rows_steps(const std::vector<Insn> &p, size_t from, size_t to, gint::RowsArgs *a)
+{
+    a->n_steps = 0;
+    for (size_t i = from; i < to; i++) {
+        if (p[i].op == WOP_Remap) continue;   // (the form works in the natural layout)
+        if (a->n_steps == gint::kRowsSteps) return false;
+        uint32_t step = (uint32_t)p[i].op, operand = p[i].operand;
+        if (p[i].op == OP_Dup && i + 2 < to && p[i + 1].op == OP_FPermW && p[i + 2].op == OP_FAdd) {
+            step = gint::kRowsFold;
+            operand = p[i + 1].operand;
+            i += 2;
+        } else if (p[i].op != OP_WarpAllReduceSum && p[i].op != OP_FAddImm && p[i].op != OP_FMulImm && p[i].op != OP_FMAImm && p[i].op != OP_FNeg &&
+                   p[i].op != OP_FRSqrt && p[i].op != OP_FSqrt && p[i].op != OP_FRcp) return false;
+        a->step[a->n_steps] = step;
+        a->operand[a->n_steps++] = operand;
+    }
+    a->mean = a->n_steps == 6 && a->step[0] == OP_WarpAllReduceSum && a->step[1] == gint::kRowsFold && a->operand[1] == 0x01000302u &&
+              a->step[2] == gint::kRowsFold && a->operand[2] == 0x02030001u && a->step[3] == OP_FMulImm && a->step[4] == OP_FAddImm && a->step[5] == OP_FRSqrt;
+    return true;
+}
+
+/*
+ * Row programs of f32 tiles: a running sum over the tiles of x (terms x, x * x, or fma(x, x)), steps on it, then either its store as
+ * a tile or a second loop over the same tiles that stores
+ *     s * x  [* w]  [silu]  [+ r]
+ * Every operand's tiles start at element 0 of its row and are contiguous.
+ */
+bool match_rows(const std::vector<Insn> &p, const gint_tensor_info &ti, Form *f)
+{
+    gint::RowsArgs &a = f->rows;
+    memset(&a, 0, sizeof(a));
+    const int kLoad = GINT_W(LoadGlobal1DF32), kStore = GINT_W(StoreGlobal1DF32);
+    for (int &t : f->tensor) t = -1;
+    size_t i = 0;
+    auto is = [&](int op) { return i < p.size() && p[i].op == op; };
+    auto slot = [&](int s) {   // the operand of p[i]: element 0 of a slot
+        const int t = (int)(p[i].operand & 15u);
+        if ((p[i].operand >> 4) != 0 || t >= GINT_MAX_TENSORS || ti.block_shape_stride_1[t][1] != 1) return false;
+        f->tensor[s] = t;
+        i++;
+        return true;
+    };
+    if (is(OP_LoadGlobal1DF32)) {   // two tiles are no loop: load, [square], load, [square], add
+        const bool square = p.size() > 3 && p[1].op == OP_Dup;
+        const size_t len = square ? 3 : 1;
+        if (p.size() < 2 * len + 2 || !slot(gint::ROWS_X) || p[len].op != OP_LoadGlobal1DF32 || p[len].operand != p[0].operand + (128u << 4) || p[2 * len].op != OP_FAdd) return false;
+        if (square && (p[2].op != OP_FMul || p[4].op != OP_Dup || p[5].op != OP_FMul)) return false;
+        a.init = -0.0f;
+        a.tiles = 2;
+        a.reduce = square ? gint::ROWS_SUM_SQUARES : gint::ROWS_SUM;
+        i = 2 * len + 1;
+    } else {
+        if (!is(OP_LoadImm)) return false;
+        memcpy(&a.init, &p[i++].operand, 4);
+        if (!is(WOP_LoopBegin) || p[i].operand == 0) return false;
+        a.tiles = p[i++].operand;
+        if (!is(kLoad) || !slot(gint::ROWS_X)) return false;
+        if (is(WOP_AccAdd)) a.reduce = gint::ROWS_SUM;
+        else if (is(WOP_AccFMASquare)) a.reduce = gint::ROWS_FMA_SQUARES;
+        else if (is(WOP_Square)) {
+            a.reduce = gint::ROWS_SUM_SQUARES;
+            i++;
+            if (!is(WOP_AccAdd)) return false;
+        } else return false;
+        i++;
+        if (!is(WOP_LoopEnd)) return false;
+        i++;
+    }
+    const size_t from = i;
+    while (i < p.size() && p[i].op != WOP_LoopBegin && p[i].op != OP_StoreGlobal1DF32) i++;
+    if (!rows_steps(p, from, i, &a)) return false;
+    if (is(OP_StoreGlobal1DF32)) {
+        const int t = (int)(p[i].operand & 15u);
+        if (t >= GINT_MAX_TENSORS || (ti.block_shape_stride_1[t][1] != 1 && ti.block_shape_stride_1[t][0] != 1)) return false;
+        f->tensor[gint::ROWS_Z] = t;
+        a.store_at = (int)(p[i++].operand >> 4);
+    } else {
+        if (!is(WOP_LoopBegin) || p[i].operand != a.tiles) return false;
+        i++;
+        const int x = f->tensor[gint::ROWS_X];
+        if (!is(kLoad) || !slot(gint::ROWS_X) || f->tensor[gint::ROWS_X] != x) return false;
+        if (!is(WOP_MulKeep)) return false;
+        i++;
+        a.map = gint::ROWS_MAP;
+        if (is(kLoad) && i + 1 < p.size() && p[i + 1].op == GINT_W(FMul)) {
+            if (!slot(gint::ROWS_W)) return false;
+            i++;
+            a.map |= gint::ROWS_MAP_W;
+        }
+        if (is(WOP_Silu)) {
+            memcpy(&a.silu, &p[i++].operand, 4);
+            a.map |= gint::ROWS_MAP_SILU;
+        }
+        if (is(kLoad) && i + 1 < p.size() && p[i + 1].op == GINT_W(FAdd)) {
+            if (!slot(gint::ROWS_R)) return false;
+            i++;
+            a.map |= gint::ROWS_MAP_R;
+        }
+        if (!is(kStore) || !slot(gint::ROWS_Z)) return false;
+        if (!is(WOP_LoopEnd)) return false;
+        i++;
+        if (is(OP_Pop)) i++;
+    }
+    if (!is(OP_Halt)) return false;
+    int n[gint::ROWS_N_SLOTS] = {};
+    for (int s = 0; s < gint::ROWS_N_SLOTS; s++) {
+        if (f->tensor[s] < 0) continue;
+        n[s] = ti.block_shape_stride_1[f->tensor[s]][0];
+        if (s != gint::ROWS_Z && f->tensor[s] == f->tensor[gint::ROWS_Z]) return false;
+    }
+    f->store = gint::ROWS_Z;
+    if (!form_grid(ti, f->tensor, gint::ROWS_N_SLOTS, n, 4, &a.grid, a.slot, f)) return false;
+    a.full_tiles = a.tiles;
+    uint32_t stage = 0;
+    for (int s = 0; s < gint::ROWS_N_SLOTS; s++) {
+        if (f->tensor[s] < 0) continue;
+        if (s == gint::ROWS_Z && !a.map) break;
+        if ((uint32_t)n[s] / 128u < a.full_tiles) a.full_tiles = (uint32_t)n[s] / 128u;
+        if (s == gint::ROWS_Z) break;
+        uint32_t &area = a.slot[s].stationary ? a.stationary_bytes : stage;
+        const uint64_t elements = (uint64_t)n[s] < 128ull * a.tiles ? (uint64_t)n[s] : 128ull * a.tiles;
+        if (elements > 65536u) return false;
+        a.slot[s].area = area;
+        area += (((uint32_t)elements * 4u + 15u) & ~15u) + 16u;   // a row may start anywhere in its first 16 bytes
+    }
+    a.stage_bytes = stage + 16u;                                  // ... and the stage's note of where its rows start
+    f->kind = FORM_ROWS;
+    return true;
+}
+
+/*
+ * Team size, teams per block and stages per team. An SM's shared memory holds as many rows as fit, at least two per team (one
+ * computed, the others on their way), and there are no more teams than rows. Measured (one B200, us, cold buffers; one warp per row /
+ * four / the interpreter):
+ *   many warps of one row each are the fastest where 12 of them have their two stages: RMSNorm 100 000 x 700 109 / 174 / 190,
+ *   60 000 x 1025 89 / 126 / 181; silu(rmsnorm) + residual 65 536 x 1024 137 / 158 / 195. Longer rows leave too few warps, and
+ *   four share a row: RMSNorm 16384 x 4096 101 / 97 / 119, silu 12 000 x 4095 176 / 110 / 220, 38 000 x 1301 150 / 142 / 216;
+ *   so do they where there are at most two rows per SM: silu 100 x 1024 17 / 13 / 26. More than 24 warps or 8 teams gain nothing.
+ * Left to the interpreter: sums of short rows in large launches (100 000 x 512 65 here, 56 there; 60 000 x 768 49 and 50;
+ * 5000 x 300 12.3 and 13.4), whose rows are read once and all of whose work is the reduction; SiLU with one team per SM (8000 x 8192 213
+ * here, 187 there); rows of which two and the stationary ones do not fit (RMSNorm of 20 000 values).
+ */
+struct RowsPlan { uint32_t team, teams, depth, grid, smem; };
+bool plan_rows(const gint::RowsArgs &a, uint32_t count, int sms, int max_smem, RowsPlan *plan)
+{
+    const uint32_t exchange = 1024u, barriers = 32u;   // per team
+    if (!a.map && a.tiles < 6 && count > 32u * (uint32_t)sms) return false;
+    if ((uint64_t)a.stationary_bytes + 16u + 2ull * a.stage_bytes + exchange + barriers > (uint64_t)max_smem) return false;
+    const uint32_t room = (uint32_t)max_smem - a.stationary_bytes - 16u;
+    uint32_t t = (count + (uint32_t)sms - 1) / (uint32_t)sms;
+    plan->team = a.tiles >= 4 && (t <= 2 || room / (2u * (a.stage_bytes + 16u)) < 12u) ? 4 : 1;
+    const uint32_t extra = (plan->team > 1 ? exchange : 0u) + barriers, most = plan->team > 1 ? 8 : 24;
+    if (t > most) t = most;
+    while (t > 1 && t * (2 * a.stage_bytes + extra) > room) t--;
+    if ((a.map & gint::ROWS_MAP_SILU) && t == 1 && count > 2u * (uint32_t)sms) return false;
+    const uint32_t d = (room - t * extra) / (t * a.stage_bytes);
+    plan->teams = t;
+    plan->depth = d > 4 ? 4 : d;
+    plan->smem = a.stationary_bytes + 16u + t * (plan->depth * a.stage_bytes + extra);
+    const uint32_t blocks = (count + t - 1) / t;
+    plan->grid = blocks < (uint32_t)sms ? blocks : (uint32_t)sms;
+    return true;
+}
+
+}  // namespace

@@ -18,6 +18,9 @@ extern "C" {
 #define GINT_WIDEV_VARIANTS(X) X(3, 8) X(4, 4)  /* ... in the vector layout */
 #define GINT_INDIRECT_VARIANTS(X) X(12)
 #define GINT_CHECKED_VARIANTS(X) X(12)
+/* kernels of program forms (gint_forms_host.h): X(source and kernel name, index) */
+#define GINT_FORM_KERNELS(X) X(rows_f32, 0) X(rows4_f32, 1)
+#define GINT_N_FORM_KERNELS 2
 
 #define GINT_X_DECL(P, K)                                        \
     extern const unsigned char gint_cubin_direct_##P##_##K[];     \
@@ -53,6 +56,12 @@ GINT_INDIRECT_VARIANTS(GINT_X_DECL)
     extern const unsigned char gint_cubin_checked_##P[];   \
     extern const unsigned char gint_cubin_checked_##P##_end[];
 GINT_CHECKED_VARIANTS(GINT_X_DECL)
+#undef GINT_X_DECL
+
+#define GINT_X_DECL(name, form)                          \
+    extern const unsigned char gint_cubin_##name[];       \
+    extern const unsigned char gint_cubin_##name##_end[];
+GINT_FORM_KERNELS(GINT_X_DECL)
 #undef GINT_X_DECL
 
 #ifdef __cplusplus

@@ -14,6 +14,7 @@ struct WideStream {
     uint32_t flat_tiles = 0;                       // tiles per logical program if the program is one flat loop, else 0
     uint32_t flat_grid = 0;                        // logical programs the flat form covers
     uint32_t access_bytes[GINT_MAX_TENSORS] = {};  // widest element with which the program accesses a slot
+    bool slow_rows = false;                        // a row program that the streaming kernels run slower than the tile kernels
     uint8_t vector_alias[GINT_MAX_TENSORS] = {};   // ... of accesses in different loops, which the vector layout makes with other lanes
     bool vector = false;                           // the kernels in the vector layout may run it (base pointers aligned to 4 elements)
 };
@@ -341,7 +342,7 @@ bool wide_transform(const std::vector<Insn> &in, const gint_tensor_info &ti, int
      * sums: 250 us there, 340 us here). */
     if (!out->flat_tiles)
         for (const Insn &x : p) {
-            if (x.op == WOP_Silu || wide_out_of_line(x.op - GINT_WIDE_FIRST)) return false;
+            if (x.op == WOP_Silu || wide_out_of_line(x.op - GINT_WIDE_FIRST)) out->slow_rows = true;
         }
     out->vector = n_outside == 0 && wide_vector(out, ti, n_tensors);
     return true;

@@ -43,8 +43,8 @@ class BytecodeStatsC(ctypes.Structure):
 
 class LaunchInfoC(ctypes.Structure):
     _fields_ = [(n, c_int32) for n in ("pool_size", "tiles_per_warp", "warps_per_block", "grid_blocks", "smem_bytes",
-                                       "regs_per_thread", "blocks_per_sm", "num_sms", "early_loads", "registers_in_smem", "vector_layout", "streaming")] + \
-               [("reserved", c_int32 * 4)]
+                                       "regs_per_thread", "blocks_per_sm", "num_sms", "early_loads", "registers_in_smem", "vector_layout", "streaming", "form")] + \
+               [("reserved", c_int32 * 3)]
 
 
 GINT_OK = 0
@@ -66,7 +66,7 @@ class DeviceStatusC(ctypes.Structure):
                 ("lane", c_uint32), ("count", c_uint32)]
 
 
-DEVICE_CODES = {0: "ok", 1: "load out of range", 2: "store out of range", 3: "instruction budget exhausted", 4: "bad dispatch"}
+DEVICE_CODES = {0: "ok", 1: "load out of range", 2: "store out of range", 3: "instruction budget exhausted", 4: "bad dispatch", 5: "a wait gave up"}
 
 
 class PlanStepC(ctypes.Structure):
@@ -84,6 +84,8 @@ SIGNATURES = {
     "gint_debug_transform": (c_int, [POINTER(c_int32), c_int, POINTER(HTensorInfo), c_int, c_int, c_int, POINTER(c_int32), POINTER(c_uint32), c_int]),
     "gint_debug_predecode_batch": (c_int, [POINTER(c_int32), c_int, c_int, POINTER(c_uint32), c_int]),
     "gint_debug_route": (c_int, [POINTER(c_int32), c_int, POINTER(HTensorInfo), c_int, POINTER(c_uint64), c_uint32, c_uint32, c_uint32, c_uint64]),
+    "gint_debug_form": (c_int, [POINTER(c_int32), c_int, POINTER(HTensorInfo), c_int, POINTER(c_uint64), c_uint32, c_uint32, c_uint32, c_uint64,
+                                c_uint32, c_int64, POINTER(c_uint32)]),
     "gint_debug_fused_table": (c_int, [POINTER(c_int32), c_int]),
     "gint_create": (c_int, [c_int, POINTER(c_void_p)]),
     "gint_destroy": (None, [c_void_p]),

@@ -80,7 +80,9 @@ typedef struct gint_launch_info {
     int32_t registers_in_smem; /* virtual registers kept in shared memory (the pool then holds the operand stack alone); 0: in the pool */
     int32_t vector_layout;    /* 1: full 1-D tiles live in the pool with lane l holding elements 4l..4l+3 (16-byte accesses) */
     int32_t streaming;        /* 1: a streaming kernel (tile loops found again) */
-    int32_t reserved[4];
+    int32_t form;             /* not 0: the launch runs on the kernel of the program's form (1: rows); the fields above then describe the
+                               * interpreter kernel that runs it where the form does not apply */
+    int32_t reserved[3];
 } gint_launch_info;
 
 /* What a checked launch (gint_execute_checked) found; all zero = nothing. The FIRST event is described, `count` counts all. */
@@ -89,7 +91,8 @@ typedef enum gint_device_code {
     GINT_DEVICE_LOAD_OUT_OF_RANGE = 1,    /* a tile load or gather outside the tensor's declared byte range: skipped, value 0 */
     GINT_DEVICE_STORE_OUT_OF_RANGE = 2,   /* a tile store or scatter outside it: skipped */
     GINT_DEVICE_INSTRUCTION_BUDGET = 3,   /* more instructions executed than the program holds (a dispatch error): stopped */
-    GINT_DEVICE_BAD_DISPATCH = 4          /* no handler for an (opcode, stack depth) pair; `address` holds the key: stopped */
+    GINT_DEVICE_BAD_DISPATCH = 4,         /* no handler for an (opcode, stack depth) pair; `address` holds the key: stopped */
+    GINT_DEVICE_GAVE_UP = 5               /* (any launch) a form kernel waited in vain for a copy of its own and stopped; nothing else is filled in */
 } gint_device_code;
 
 typedef struct gint_device_status {
@@ -132,6 +135,12 @@ int gint_debug_predecode_batch(const int32_t *code, int n_words, int n_tensors, 
  * registers in shared memory, bit 2 the vector-layout stream, 0 the stream as written. Negative: the status of a refused program. */
 int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs,
                      uint32_t first, uint32_t count, uint32_t gather_mask, uint64_t gather_extent_bytes);
+
+/* Does a launch run on the kernel of the program's form (default options; needs no device)? 0: no; else bits 0-7 the form (1: rows),
+ * bits 8-15 the warps per logical program. out_offsets (or NULL) receives, by tensor slot, the element offset at which logical
+ * program `logical` starts; `row` stands for the entry of the row index in a gathered launch. Negative: the status of a refused program. */
+int gint_debug_form(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs, uint32_t first,
+                    uint32_t count, uint32_t gather_mask, uint64_t gather_extent_bytes, uint32_t logical, int64_t row, uint32_t *out_offsets);
 
 /* The instruction list the kernels actually run for a program, after the optional early-issue and fusion passes (for
  * tests; no GPU needed): out_ops[i] is a format opcode, an internal opcode (>= 106) or -1 for an instruction absorbed into

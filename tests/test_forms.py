@@ -1,0 +1,308 @@
+"""Form kernels: which programs and launches run on them (CPU, gint_debug_form) and that they give the interpreter's bits (GPU)."""
+import ctypes
+import random
+
+import numpy as np
+import pytest
+import torch
+
+import cases as C  # tests/cases.py
+from conftest import bits_equal, mismatch_report
+from gint_b200 import bytecode, get_executor
+from gint_b200 import opcodes as O
+from gint_b200.host import capi, frontend as F
+from gint_b200.host.utils import fill_tensor_info
+from test_streaming import _perf_cases
+
+ROWS = 1
+
+
+def form(pd, bases, first=0, count=1, gather_mask=0, extent=1 << 30, logical=0, row=0, infos=None):
+    """(form, warps per logical program, element offsets of `logical` by tensor slot)"""
+    code = np.ascontiguousarray(np.asarray(pd.program, dtype=np.int32).reshape(-1))
+    ti = capi.HTensorInfo()
+    fill_tensor_info(ti, pd.input_infos)
+    n = len(pd.input_infos)
+    if infos:
+        infos(ti)
+    off = (ctypes.c_uint32 * 8)()
+    r = capi.load_library().gint_debug_form(code.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), code.size, ctypes.byref(ti), n, (ctypes.c_uint64 * 8)(*bases),
+                                            first, count, gather_mask, extent, logical, row, off)
+    assert r >= 0, r
+    return r & 255, r >> 8, list(off[:n]), ti
+
+
+@bytecode
+def rows_program(x, w, r, z, REGW, WARP, n=1024, tiles=None, reduce="squares", steps="mean", scale=True, silu=False, c=1.0, add=False, first="load"):
+    """The shapes that a row program can have: z = [silu](s * x [* w]) [+ r] with s from a sum over x; without `scale` z = s."""
+    rows = x.shape[0]
+    xb, wb, rb = [F.make_block_1d(t, n, 1, 1, n, [t.strides[0] if t.ndim == 2 else 0], [rows]) for t in (x, w, r)]
+    zb = F.make_block_1d(z, n if scale else 1, 1, 1, n if scale else 1, [z.strides[0]], [rows])
+    offs = range(0, 128 * (tiles or -(-n // 128)), 128)
+    if reduce == "fma" or first == "zero":
+        F.fpush(0.0)
+    for off in offs:
+        F.fldg_1d(off, xb)
+        if reduce == "squares":
+            F.dup()
+            F.fmul()
+        if reduce == "fma":
+            F.dup()
+            F.fma()
+        elif off or first == "zero":
+            F.fadd()
+    if steps != "none":
+        F.warp_allreduce_fsum()
+        F.dup()
+        F.fperm_w(2, 3, 0, 1)
+        F.fadd()
+        F.dup()
+        F.fperm_w(1, 0, 3, 2)
+        F.fadd()
+    if steps == "mean":
+        F.fmulimm(1.0 / n)
+        F.faddimm(1e-6)
+        F.frsqrt()
+    elif steps == "others":
+        F.dup()
+        F.fperm_w(0, 0, 3, 1)
+        F.fadd()
+        F.fmaimm(0.25, 1.5)
+        F.fneg()
+        F.fmulimm(-0.5)
+        F.fsqrt()
+        F.frcp()
+    if not scale:
+        F.fstg_1d(0, zb)
+        F.halt()
+        return
+    for off in offs:
+        F.dup()
+        F.fldg_1d(off, xb)
+        F.fmul()
+        if w is not r:
+            F.fldg_1d(off, wb)
+            F.fmul()
+        if silu:
+            F.dup()
+            F.fneg()
+            F.fexp()
+            F.faddimm(c)
+            F.frdiv()
+        if add:
+            F.fldg_1d(off, rb)
+            F.fadd()
+        F.fstg_1d(off, zb)
+    F.pop()
+    F.halt()
+
+
+FAR = [(t + 1) << 36 for t in range(8)]
+
+
+def program(rows=64, n=1024, w_rows=False, **kw):
+    t = C.to_interfaces([torch.empty(rows, n), torch.empty(rows, n) if w_rows else torch.empty(n), torch.empty(rows, n), torch.empty(rows, n)])
+    return rows_program.get_program(*t, n=n, **kw)
+
+
+@pytest.mark.parametrize("kw", [{}, {"silu": True}, {"add": True}, {"silu": True, "add": True}, {"reduce": "sum"}, {"reduce": "fma"}, {"first": "zero"}, {"steps": "others"},
+                                {"steps": "none"}, {"scale": False}, {"n": 129}, {"n": 256}, {"n": 257}, {"w_rows": True}, {"tiles": 9}])
+def test_row_programs_have_the_form(kw):
+    assert form(program(**kw), FAR, count=64)[0] == ROWS
+
+
+def test_what_a_launch_on_the_form_needs():
+    pd = program()
+    assert form(pd, FAR, count=64)[0] == ROWS
+    assert form(pd, [FAR[0] + 4, FAR[1] + 12, FAR[2], FAR[3] + 8], count=64)[0] == ROWS          # any element may be the first
+    assert form(pd, [FAR[0] + 2] + FAR[1:], count=64)[0] == 0                                     # ... but no part of one
+    end = 4 * 64 * 1024
+    for bases, want in ((FAR[:3] + [FAR[0]], 0), (FAR[:3] + [FAR[0] + end - 4], 0), (FAR[:3] + [FAR[0] + end], ROWS), (FAR[:3] + [FAR[1] + 4092], 0)):
+        assert form(pd, bases, count=64)[0] == want                                               # what is stored is read by no other logical program
+    assert form(pd, FAR, first=(1 << 31) - 60, count=64)[0] == 0                                  # logical programs are counted in 31 bits
+    assert form(program(n=20000), FAR, count=64)[0] == 0                                          # two rows and the weights in shared memory
+    assert form(program(rows=4736, n=640, scale=False), FAR, count=4736)[0] == ROWS               # short rows: only few sums
+    assert form(program(rows=4737, n=640, scale=False), FAR, count=4737)[0] == 0
+    assert form(program(rows=4737, n=641, scale=False), FAR, count=4737)[0] == ROWS
+    assert form(program(n=8192, silu=True, add=True), FAR, count=296)[0] == ROWS                  # one team per SM
+    assert form(program(n=8192, silu=True, add=True), FAR, count=297)[0] == 0
+
+
+@pytest.mark.parametrize("n,rows,warps", [(384, 10, 1), (385, 296, 4), (385, 297, 1), (2200, 5000, 1), (2400, 5000, 4)])
+def test_warps_per_row(n, rows, warps):
+    assert form(program(rows=rows, n=n), FAR, count=rows)[:2] == (ROWS, warps)
+
+
+def test_gathered_rows_of_a_form():
+    """An index replaces the digit of the innermost batch dimension. Where that has one row, the index still moves the row."""
+    pd = program()
+    assert form(pd, FAR, count=64, gather_mask=1)[0] == ROWS
+    assert form(pd, FAR, count=64, gather_mask=8)[0] == 0                                         # not what is stored
+    assert form(program(rows=1), FAR, count=1, gather_mask=1)[0] == 0
+    assert form(program(rows=1), FAR, count=1)[0] == ROWS
+    assert form(pd, FAR, count=64, gather_mask=2)[0] == ROWS                                      # (weights: the same row for every index)
+
+
+def decode(ti, t, r, gathered, row):
+    """decode_tiles (gint_interp.cuh) for a slot whose block grid does not cut dimension 1"""
+    off, step2 = 0, ti.block_grid_steps[t][1] * ti.block_shape_stride_2[t][1]
+    if ti.block_grid_dims[t][1] != 1:
+        off, r = off + r % ti.block_grid_dims[t][1] * step2, r // ti.block_grid_dims[t][1]
+    for j in range(4):
+        size, stride = ti.batch_shape[t][j], ti.batch_strides[t][j]
+        b = r % size
+        off += (row if gathered and j == 0 else b) * stride
+        r //= size
+    return off & 0xFFFFFFFF
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_offsets_are_those_of_the_descriptor_decode(seed):
+    """Digits of any size and order, slots that do not move, leftover digits, a gathered digit."""
+    pd = program()
+    rng = random.Random(seed)
+    gather = seed % 3 == 0
+    sizes = [rng.choice([1, 1, 2, 3, 7, 64, 1000, 4099]) for _ in range(5)]      # grid dimension 2, four batch dimensions
+    if gather:
+        sizes[1] = rng.randint(2, 50)
+    moving = [t for t in (0, 1, 3) if t != 1 or rng.random() < 0.5]
+    strides = {t: [rng.randint(1, 40) if t in moving else 0 for _ in range(5)] for t in (0, 1, 3)}
+    plain = rng.random() < 0.5                                                    # a slot that does not move may have any digits
+
+    def infos(ti):
+        for t in (0, 1, 3):                                                       # (slot 2 is not accessed by this program)
+            one = plain and t not in moving
+            ti.block_grid_dims[t][1] = 1 if one else sizes[0]
+            ti.block_grid_steps[t][1], ti.block_shape_stride_2[t][1] = strides[t][0], 1
+            for j in range(4):
+                ti.batch_shape[t][j], ti.batch_strides[t][j] = (1 if one else sizes[j + 1]), strides[t][j + 1]
+    total = min(int(np.prod(sizes, dtype=np.float64)) * 2, (1 << 31) - 2)
+    for logical in [0, total // 2] + [rng.randrange(total) for _ in range(20)]:
+        kind, _, off, ti = form(pd, FAR, first=logical, count=1, gather_mask=1 if gather else 0, logical=logical, row=13, infos=infos)
+        reach = max(sum((s - 1) * d for s, d in zip(sizes, strides[t])) + 1024 for t in moving)
+        assert (kind == ROWS) == (reach < (1 << 31) - 8192 and 4 * reach < 1 << 36), (sizes, strides)
+        for t in (0, 1, 3) if kind else ():
+            assert off[t] == decode(ti, t, logical, gather and t == 0, 13), (t, logical, sizes)
+
+
+# ---------------------------------------------------------------------------------------------- on the GPU
+
+def both(launch):
+    ex, got = get_executor(), []
+    for on in (1, 0):
+        ex.set_option("forms", on)
+        try:
+            got.append([t.cpu() for t in launch()])
+        finally:
+            ex.set_option("forms", 1)
+    return got
+
+
+def same_bits(launch):
+    for a, b in zip(*both(launch)):
+        assert bits_equal(a, b), mismatch_report(a, b)
+
+
+def runs_on_form(program_, tensors, rows, **kw):
+    return get_executor().launch_info(program_, C.to_interfaces(tensors), rows, **kw)["form"] == ROWS
+
+
+SHAPES = [(1, 129), (3, 255), (700, 256), (5, 257), (40, 384), (7, 513), (300, 1000), (33, 1024), (2000, 1025), (9, 2029), (400, 2304), (20, 4095), (150, 4096), (5, 6001), (3, 9000)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [{}, {"silu": True, "add": True}, {"silu": True, "c": 0.5}, {"add": True, "reduce": "fma"}, {"reduce": "sum", "steps": "others"}, {"scale": False},
+                                {"scale": False, "reduce": "sum", "first": "zero"}, {"steps": "none"}], ids=str)
+def test_rows_give_the_bits_of_the_interpreter(kw):
+    """Row lengths around whole tiles and groups of tiles, one and four warps per row, rows and base pointers at any element."""
+    for k, (rows, n) in enumerate(SHAPES):
+        g = torch.Generator(device="cuda").manual_seed(k)
+        pad = [k % 4, (k // 2) % 4, (k + 1) % 4, (k + 2) % 3]
+        x, w, r, z = [torch.randn(rows * n + 8, device="cuda", generator=g)[p:p + rows * n].view(rows, n) for p in pad]
+        w = w[0]
+
+        def launch():
+            out = torch.full((rows * n + 8,), 9.0, device="cuda")
+            o = out[pad[3] + 1:pad[3] + 1 + rows * n].view(rows, n)
+            rows_program(x, w, r, o, grid_dim=rows, n=n, **kw)
+            return [out]
+        assert runs_on_form(rows_program, [x, w, r, z], rows, n=n, **kw) or (n < 600 and not kw.get("scale", True)), (rows, n)   # (few tiles are no loop)
+        same_bits(launch)
+
+
+@pytest.mark.gpu
+def test_rows_with_extreme_values():
+    """SiLU's quotient where its plain steps do not hold: zeros of both signs, subnormal and huge values, infinities, NaN, every size of exp(-x)."""
+    rows, n = 64, 1030
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(rows, n, device="cuda", generator=g) * torch.logspace(-40, 38, rows, device="cuda")[:, None]
+    x[:, 5], x[:, 6], x[::3, 7], x[::5, 8], x[::7, 9] = 0.0, -0.0, float("inf"), float("-inf"), float("nan")
+    w = torch.randn(n, device="cuda", generator=g) * torch.logspace(-30, 3, n, device="cuda")
+    for kw in ({"steps": "none", "reduce": "sum", "silu": True}, {"silu": True, "add": True}, {"reduce": "fma"}):
+        def launch():
+            z = torch.empty(rows, n, device="cuda")
+            rows_program(x, w, x, z, grid_dim=rows, n=n, **kw)
+            return [z]
+        same_bits(launch)
+
+
+@pytest.mark.gpu
+def test_silu_of_any_bits():
+    """A million random bit patterns and a million ordinary values: 8 * w through SiLU (x = 1 everywhere, eight tiles, no steps)."""
+    rows, n = 1024, 1024
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.ones(rows, n, device="cuda")
+    for w in (torch.randint(-2 ** 31, 2 ** 31, (rows, n), device="cuda", generator=g).to(torch.int32).view(torch.float32), torch.randn(rows, n, device="cuda", generator=g)):
+        def launch():
+            z = torch.empty(rows, n, device="cuda")
+            rows_program(x, w, x, z, grid_dim=rows, n=n, steps="none", reduce="sum", silu=True)
+            return [z]
+        same_bits(launch)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,n", [(40, 1025), (400, 384), (30, 4096)])
+def test_gathered_and_partial_launches_of_rows(rows, n):
+    m, ex = _perf_cases(), get_executor()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    table, x, w = torch.randn(rows + 5, n, device="cuda", generator=g)[:rows], torch.randn(rows, n, device="cuda", generator=g), torch.randn(n, device="cuda", generator=g)
+    idx = torch.randint(-rows, rows, (rows,), device="cuda", generator=g)
+    idx[0], idx[1], idx[2] = rows + 100, -rows - 7, -1        # clamped, clamped, from the end
+    st = torch.cuda.current_stream().cuda_stream
+
+    def gathered():
+        z = torch.full((rows, n), 9.0, device="cuda")
+        ex.execute_gathered(m.rmsnorm_silu_residual, C.to_interfaces([z, x, w, table]), rows, (3,), idx, cuda_stream=st)
+        return [z]
+    same_bits(gathered)
+
+    def part():
+        z = torch.full((rows, n), 9.0, device="cuda")
+        ex.execute_range(m.rmsnorm, C.to_interfaces([x, w, z]), 3, rows - 7, cuda_stream=st)
+        y = x.clone()
+        m.rmsnorm(y, w, y, grid_dim=rows)                      # in place: the interpreter
+        return [z, y]
+    same_bits(part)
+
+
+@pytest.mark.gpu
+def test_rows_in_a_graph_and_on_few_blocks():
+    m, ex = _perf_cases(), get_executor()
+    x, w, z = torch.randn(500, 777, device="cuda"), torch.randn(777, device="cuda"), torch.zeros(500, 777, device="cuda")
+    m.rmsnorm(x, w, z, grid_dim=500)
+    want = z.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        m.rmsnorm(x, w, z, grid_dim=500, cuda_stream=torch.cuda.current_stream().cuda_stream)
+    z.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bits_equal(z.cpu(), want.cpu())
+    ex.set_option("max_blocks", 3)
+    try:
+        z.zero_()
+        m.rmsnorm(x, w, z, grid_dim=500)
+        assert bits_equal(z.cpu(), want.cpu())
+    finally:
+        ex.set_option("max_blocks", 0)
+    assert ex.device_status()["code"] == 0
