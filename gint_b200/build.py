@@ -27,6 +27,8 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 KERNELS = os.path.join(CSRC, "kernels")
 OBJ_DIR = os.path.join(CSRC, "build")
 HOT_HEADER = os.path.join(OBJ_DIR, "gint_hot_handlers.h")
+LANE_HEADER = os.path.join(OBJ_DIR, "gint_lane_programs.h")
+LANE_PROGRAMS = ("bmm4x4", "inv4x4")
 LIB_PATH = os.path.join(PKG_DIR, "libgint_b200.so")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -77,6 +79,24 @@ def _write_hot_header(ordered: bool) -> None:
             f.write(text)
 
 
+def _write_lane_header() -> None:
+    """The small-matrix programs that get a kernel of their own (gint_lanes.cuh), as constant tables: the recorded streams, which do not
+    depend on the batch size."""
+    import json
+    with open(os.path.join(PKG_DIR, "data", "programs.json")) as f:
+        records = json.load(f)
+    text = "/* written by gint_b200/build.py from data/programs.json */\n#pragma once\nnamespace gint {\n"
+    for name in LANE_PROGRAMS:
+        code = [v for pair in records[name + "_b1"]["bytecode"] for v in (pair if isinstance(pair, list) else [pair])]
+        pairs = list(zip(code[::2], code[1::2]))
+        text += f"struct LaneCode_{name} {{\n    static constexpr int n = {len(pairs)};\n    static constexpr int code[{len(pairs)}][2] = {{" + \
+            ", ".join(f"{{{op}, {arg}}}" for op, arg in pairs) + "};\n};\n"
+    text += "}  // namespace gint\n#define GINT_LANE_PROGRAMS(X) " + " ".join(f"X({name})" for name in LANE_PROGRAMS) + "\n"
+    if not os.path.exists(LANE_HEADER) or open(LANE_HEADER).read() != text:
+        with open(LANE_HEADER, "w") as f:
+            f.write(text)
+
+
 def _build_kernel(src: str, extra: list[str]) -> tuple[str, str]:
     """CUDA C++ -> cubin -> object with the cubin as a byte array."""
     stem = os.path.basename(src)[:-3]                       # gint_direct_p4_k1
@@ -102,6 +122,7 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False, e
     if not os.path.exists(stamp) or open(stamp).read() != flags_now:
         force = True
     _write_hot_header(hot_order)
+    _write_lane_header()
     kernels = sorted(glob.glob(os.path.join(KERNELS, "*.cu")))
     todo, objs = [], []
     for src in kernels:
@@ -117,7 +138,7 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False, e
     with concurrent.futures.ThreadPoolExecutor(max_workers=jobs or os.cpu_count() or 4) as ex:
         futs = [ex.submit(_build_kernel, s, extra) for s in todo]
         if capi_todo:
-            futs.append(ex.submit(lambda: ("gint_capi", _run([_nvcc()] + ARCH + COMMON + ["-Xcompiler", "-fPIC", "-MD", "-MF", capi_obj[:-2] + ".d", "-c", capi_src, "-o", capi_obj],
+            futs.append(ex.submit(lambda: ("gint_capi", _run([_nvcc()] + ARCH + COMMON + ["-I", OBJ_DIR, "-Xcompiler", "-fPIC", "-MD", "-MF", capi_obj[:-2] + ".d", "-c", capi_src, "-o", capi_obj],
                                                               "nvcc gint_capi"))))
         for f in concurrent.futures.as_completed(futs):
             logs.append(f.result())

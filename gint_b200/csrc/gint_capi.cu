@@ -1391,20 +1391,18 @@ Route choose_route(const gint_ctx *ctx, const Program *p, const uint64_t *base_p
     return r;
 }
 
-/* Does a launch run on the kernel of the program's form, and with which arguments? Not where the caller has asked for a particular
- * configuration of the interpreter, and not where the stored tensor overlaps one that is read: the form reads logical programs ahead. */
-int choose_form(const gint_ctx *ctx, const Program *p, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather,
-                gint::RowsArgs *a, RowsPlan *plan)
+/* Does a launch run on the kernel of the program's form, and how? Not where the caller has asked for a particular configuration of the
+ * interpreter, and not where a stored tensor overlaps one that is read: the forms read logical programs ahead. */
+int choose_rows(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
 {
-    const Form &f = p->form;
-    if (f.kind == FORM_NONE || !ctx->opt_forms || !ctx->opt_wide || !ctx->opt_early_issue || !ctx->opt_rf || ctx->opt_vec || ctx->opt_prefetch || ctx->opt_tiles_per_warp) return FORM_NONE;
-    if ((uint64_t)first + count >= (1ull << 31)) return FORM_NONE;
-    if (!plan_rows(f.rows, count, ctx->num_sms, ctx->max_smem_optin, plan)) return FORM_NONE;
-    *a = f.rows;
+    RowsPlan plan;
+    if (!plan_rows(f.rows, count, ctx->num_sms, ctx->max_smem_optin, &plan)) return FORM_NONE;
+    gint::RowsArgs &a = l->rows;
+    a = f.rows;
     uint64_t lo[gint::ROWS_N_SLOTS], hi[gint::ROWS_N_SLOTS];
     for (int s = 0; s < gint::ROWS_N_SLOTS; s++) {
         if (f.tensor[s] < 0) continue;
-        a->slot[s].base = lo[s] = base_ptrs[f.tensor[s]];
+        a.slot[s].base = lo[s] = base_ptrs[f.tensor[s]];
         hi[s] = lo[s] + f.extent[s];
         if ((lo[s] & f.base_align) != 0) return FORM_NONE;
         if (!gather || !((gather->mask >> f.tensor[s]) & 1u)) continue;
@@ -1412,20 +1410,54 @@ int choose_form(const gint_ctx *ctx, const Program *p, const uint64_t *base_ptrs
         hi[s] = lo[s] + gather->extent_bytes;
         if (!f.gathers[s]) continue;
         /* (an index into a single row moves it as well, but not by a digit) */
-        if (f.gather_digit[s] < 0 || (a->grid.gather_mask && a->grid.gather_dim != f.gather_digit[s])) return FORM_NONE;
-        a->grid.gather_dim = f.gather_digit[s];
-        a->grid.gather_mask |= 1u << s;
-        a->grid.gather_index = gather->index;
-        a->grid.gather_rows = gather->rows;
+        if (f.gather_digit[s] < 0 || (a.grid.gather_mask && a.grid.gather_dim != f.gather_digit[s])) return FORM_NONE;
+        a.grid.gather_dim = f.gather_digit[s];
+        a.grid.gather_mask |= 1u << s;
+        a.grid.gather_index = gather->index;
+        a.grid.gather_rows = gather->rows;
     }
     for (int s = 0; s < gint::ROWS_N_SLOTS; s++)
         if (f.tensor[s] >= 0 && s != f.store && lo[s] < hi[f.store] && lo[f.store] < hi[s]) return FORM_NONE;
-    a->first = first;
-    a->count = count;
-    a->depth = plan->depth;
-    a->grid.simple = a->grid.n_dims == 1 && first + count <= a->grid.size[0];
-    if (ctx->opt_max_blocks > 0 && (uint32_t)ctx->opt_max_blocks < plan->grid) plan->grid = (uint32_t)ctx->opt_max_blocks;
-    return f.kind;
+    a.first = first;
+    a.count = count;
+    a.depth = plan.depth;
+    a.grid.simple = a.grid.n_dims == 1 && first + count <= a.grid.size[0];
+    l->kernel = plan.team == 4 ? 1 : 0;
+    l->grid = plan.grid;
+    l->threads = plan.teams * plan.team * 32u;
+    l->smem = plan.smem;
+    l->warps_per_program = plan.team;
+    return FORM_ROWS;
+}
+
+int choose_lanes(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
+{
+    const uint32_t used = f.lane_loads | f.lane_stores;
+    if ((gather && (gather->mask & used)) || first + count > f.lane_tiles) return FORM_NONE;
+    l->lanes = f.lanes;
+    for (int t = 0; t < GINT_MAX_TENSORS; t++) {
+        if (!((used >> t) & 1u)) continue;
+        if ((base_ptrs[t] & 15u) != 0) return FORM_NONE;
+        l->lanes.base[t] = base_ptrs[t];
+        for (int u = 0; u < t; u++)
+            if (((used >> u) & 1u) && (((f.lane_stores >> t) | (f.lane_stores >> u)) & 1u) && base_ptrs[t] < base_ptrs[u] + f.lane_reach[u] && base_ptrs[u] < base_ptrs[t] + f.lane_reach[t])
+                return FORM_NONE;
+    }
+    l->lanes.first = first;
+    l->lanes.count = count;
+    if (!plan_lanes(f, count, ctx->num_sms, ctx->max_smem_optin, l)) return FORM_NONE;
+    l->kernel = kLaneKernelFirst + f.lane_program;
+    return FORM_LANES;
+}
+
+int choose_form(const gint_ctx *ctx, const Program *p, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
+{
+    const Form &f = p->form;
+    if (f.kind == FORM_NONE || !ctx->opt_forms || !ctx->opt_wide || !ctx->opt_early_issue || !ctx->opt_rf || ctx->opt_vec || ctx->opt_prefetch || ctx->opt_tiles_per_warp) return FORM_NONE;
+    if ((uint64_t)first + count >= (1ull << 31)) return FORM_NONE;
+    const int kind = f.kind == FORM_ROWS ? choose_rows(ctx, f, base_ptrs, first, count, gather, l) : choose_lanes(ctx, f, base_ptrs, first, count, gather, l);
+    if (ctx->opt_max_blocks > 0 && (uint32_t)ctx->opt_max_blocks < l->grid) l->grid = (uint32_t)ctx->opt_max_blocks;
+    return kind;
 }
 
 int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int n_tensors, uint32_t first, uint32_t count,
@@ -1438,12 +1470,12 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
     if (count == 0) return GINT_OK;
     if ((uint64_t)first + (uint64_t)count > 0xFFFFFFFFull) return fail(ctx, GINT_ERR_TOO_LARGE, "logical program range overflows 32 bits");
     DeviceGuard guard(ctx->device);
-    if (p->form.kind != FORM_NONE && ctx->form_fn[0] && ctx->form_fn[1]) {
-        gint::RowsArgs a;
-        RowsPlan plan;
-        if (choose_form(ctx, p, base_ptrs, first, count, gather, &a, &plan)) {
-            void *args[1] = {&a};
-            cudaError_t e = cudaLaunchKernel(ctx->form_fn[plan.team == 4], dim3(plan.grid), dim3(plan.teams * plan.team * 32u), args, plan.smem, (cudaStream_t)stream);
+    if (p->form.kind != FORM_NONE) {
+        FormLaunch l;
+        const int kind = choose_form(ctx, p, base_ptrs, first, count, gather, &l);
+        if (kind && ctx->form_fn[l.kernel]) {
+            void *args[1] = {kind == FORM_ROWS ? (void *)&l.rows : (void *)&l.lanes};
+            cudaError_t e = cudaLaunchKernel(ctx->form_fn[l.kernel], dim3(l.grid), dim3(l.threads), args, l.smem, (cudaStream_t)stream);
             if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaLaunchKernel", e);
             ctx->form_launched = true;
             return GINT_OK;
@@ -1578,6 +1610,7 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
         bool fits = false;
         const bool loops = wide_transform(prog, p->ti, n_tensors, &ws);
         if (loops && ctx->opt_fuse && ctx->opt_lower) match_rows(ws.prog, p->ti, &p->form);
+        if (p->form.kind == FORM_NONE && ctx->opt_fuse && ctx->opt_lower) match_lanes(prog, p->ti, n_tensors, p->st.pool_size, &p->form);
         if (loops && !ws.slow_rows)
             for (auto &v : ctx->direct) fits = fits || (v.wide == 1 && v.ok && v.P >= ws.max_depth);
         if (fits) {
@@ -1884,17 +1917,16 @@ int gint_debug_form(const int32_t *code, int n_words, const gint_tensor_info *ti
     const int rc = build_program(&ctx, code, n_words, ti, n_tensors, &p, &streams);
     if (rc != GINT_OK) return rc;
     const GatherArgs ga{gather_mask, nullptr, gather_extent_bytes, 1u};
-    gint::RowsArgs a;
-    RowsPlan plan;
-    const int kind = choose_form(&ctx, p, base_ptrs, first, count, gather_mask ? &ga : nullptr, &a, &plan);
-    if (kind && out_offsets) {
+    FormLaunch l;
+    const int kind = choose_form(&ctx, p, base_ptrs, first, count, gather_mask ? &ga : nullptr, &l);
+    if (kind == FORM_ROWS && out_offsets) {
         uint32_t off[gint::ROWS_N_SLOTS];
-        gint::form_offsets(a.grid, a.slot, logical, row, off);
+        gint::form_offsets(l.rows.grid, l.rows.slot, logical, row, off);
         for (int s = 0; s < gint::ROWS_N_SLOTS; s++)
             if (p->form.tensor[s] >= 0) out_offsets[p->form.tensor[s]] = off[s];
     }
     delete p;
-    return kind ? kind | (int)(plan.team << 8) : 0;
+    return kind ? kind | (int)(l.warps_per_program << 8) : 0;
 }
 
 int gint_create(int device, gint_ctx **out)
@@ -2119,9 +2151,9 @@ int gint_program_launch_info(gint_ctx *ctx, uint64_t handle, uint32_t grid_dim, 
     out->registers_in_smem = g.v->rf ? p->st.max_reg_idx + 1 : 0;
     out->vector_layout = g.v->vec || g.v->wide == 2 ? 1 : 0;
     out->streaming = g.v->wide ? 1 : 0;
-    gint::RowsArgs a;
-    RowsPlan plan;
-    out->form = ctx->form_fn[0] && ctx->form_fn[1] ? choose_form(ctx, p, base_ptrs, 0u, count, nullptr, &a, &plan) : 0;
+    FormLaunch l;
+    out->form = choose_form(ctx, p, base_ptrs, 0u, count, nullptr, &l);
+    if (out->form && !ctx->form_fn[l.kernel]) out->form = 0;
     return GINT_OK;
 }
 
@@ -2217,11 +2249,11 @@ int gint_device_status_read(gint_ctx *ctx, gint_device_status *out, int clear)
         if (e == cudaSuccess) e = cudaMemcpy(out, ctx->status_dev, sizeof(*out), cudaMemcpyDeviceToHost);
         if (e == cudaSuccess && clear) e = cudaMemset(ctx->status_dev, 0, sizeof(*out));
     }
-    for (auto &im : g_images) {   // form kernels count the teams that gave up waiting for a copy
+    for (auto &im : g_images) {   // the row kernels count the teams that gave up waiting for a copy
         void *flag = nullptr;
         size_t bytes = 0;
         uint32_t n = 0;
-        if (im.K != -2 || !im.loaded || !ctx->form_launched) continue;
+        if (im.K != -2 || im.P >= kLaneKernelFirst || !im.loaded || !ctx->form_launched) continue;
         if (e == cudaSuccess) e = cudaLibraryGetGlobal(&flag, &bytes, im.lib, "gint_form_gave_up");
         if (e == cudaSuccess) e = cudaMemcpy(&n, flag, sizeof(n), cudaMemcpyDeviceToHost);
         if (e == cudaSuccess && n && clear) e = cudaMemset(flag, 0, sizeof(n));

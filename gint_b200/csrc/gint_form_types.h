@@ -76,4 +76,14 @@ struct RowsArgs {
     uint32_t depth, stage_bytes, stationary_bytes;
 };
 
+/* Lane programs (gint_lanes.cuh): tile t of slot s covers rows 32 t .. 32 t + 31 of rows[s], each `stride` elements apart. */
+struct LaneArgs {
+    u64 base[8];
+    uint32_t stride[8];
+    int rows[8];
+    uint32_t first, count;           // tiles
+    uint32_t depth;
+};
+constexpr uint32_t kLaneTileBytes = 2048;   // 32 rows of 16 floats
+
 }  // namespace gint

@@ -5,10 +5,11 @@
 #pragma once
 
 #include "gint_form_types.h"
+#include "gint_lane_programs.h"
 
 namespace {
 
-enum { FORM_NONE = 0, FORM_ROWS = 1 };
+enum { FORM_NONE = 0, FORM_ROWS = 1, FORM_LANES = 2 };
 
 struct Form {
     int kind = FORM_NONE;
@@ -19,6 +20,18 @@ struct Form {
     bool gathers[gint::ROWS_N_SLOTS] = {};               // ... whose stride is not 0: an index chooses among its rows
     uint32_t base_align = 3;                             // alignment of the base pointers (minus 1)
     gint::RowsArgs rows;                                 // all but pointers, range and shared memory
+    /* lane programs: which one, its slots, the tiles of the block grid */
+    int lane_program = 0;
+    uint32_t lane_loads = 0, lane_stores = 0, lane_tiles = 0;
+    uint64_t lane_reach[GINT_MAX_TENSORS] = {};
+    gint::LaneArgs lanes;
+};
+/* a launch on a form kernel */
+struct FormLaunch {
+    int kernel = 0;              // of GINT_FORM_KERNELS
+    uint32_t grid = 0, threads = 0, smem = 0, warps_per_program = 0;
+    gint::RowsArgs rows;
+    gint::LaneArgs lanes;
 };
 
 struct FormDim { uint32_t size, stride; bool batch0; };
@@ -251,6 +264,68 @@ bool plan_rows(const gint::RowsArgs &a, uint32_t count, int sms, int max_smem, R
     plan->smem = a.stationary_bytes + 16u + t * (plan->depth * a.stage_bytes + extra);
     const uint32_t blocks = (count + t - 1) / t;
     plan->grid = blocks < (uint32_t)sms ? blocks : (uint32_t)sms;
+    return true;
+}
+
+
+/*
+ * Lane programs (gint_lanes.cuh): exactly the instructions of a program that was compiled ahead of time, over rows of 16 floats whose accesses
+ * are never masked along the row, and a block grid that steps by whole tiles of 32 rows.
+ */
+struct LaneCode { const int (*code)[2]; int n; };
+#define GINT_X_LANE(name) {gint::LaneCode_##name::code, gint::LaneCode_##name::n},
+const LaneCode kLanePrograms[] = {GINT_LANE_PROGRAMS(GINT_X_LANE)};
+#undef GINT_X_LANE
+constexpr int kLaneKernelFirst = 2;   // of GINT_FORM_KERNELS
+
+bool match_lanes(const std::vector<Insn> &p, const gint_tensor_info &ti, int n_tensors, int pool_size, Form *f)
+{
+    int found = -1;
+    for (size_t k = 0; k < sizeof(kLanePrograms) / sizeof(kLanePrograms[0]); k++) {
+        const LaneCode &c = kLanePrograms[k];
+        bool same = (size_t)c.n == p.size();
+        for (size_t i = 0; same && i < p.size(); i++) same = p[i].op == c.code[i][0] && (!GINT_OP_USES_OPERAND(p[i].op) || p[i].operand == (uint32_t)c.code[i][1]);
+        if (same) found = (int)k;
+    }
+    if (found < 0 || !rf_equivalent(p, pool_size)) return false;   // (the compiled program keeps its registers apart from the stack)
+    f->lane_loads = f->lane_stores = f->lane_tiles = 0;
+    for (const Insn &x : p)
+        if (is_tensor_op(x.op)) (writes_tensor(x.op) ? f->lane_stores : f->lane_loads) |= 1u << (x.operand & 15u);
+    if (f->lane_loads & f->lane_stores) return false;
+    memset(&f->lanes, 0, sizeof(f->lanes));
+    for (int t = 0; t < n_tensors; t++) {
+        if (!(((f->lane_loads | f->lane_stores) >> t) & 1u)) continue;
+        const int64_t rows = ti.block_shape_stride_1[t][0], stride = ti.block_shape_stride_1[t][1], tiles = ti.block_grid_dims[t][0];
+        if (ti.elm_size[t] != 4 || ti.block_shape_stride_2[t][0] < 16 || ti.block_shape_stride_2[t][1] != 1 || rows < 1 || tiles < 1) return false;
+        if (stride < 16 || stride % 4 != 0 || (tiles > 1 && ti.block_grid_steps[t][0] != 32) || ti.block_grid_dims[t][1] != 1) return false;
+        for (int j = 0; j < 4; j++) if (ti.batch_shape[t][j] != 1) return false;
+        if (f->lane_tiles && f->lane_tiles != (uint32_t)tiles) return false;
+        if ((rows + 32) * stride >= (1ll << 31) || tiles * 32 >= (1ll << 31)) return false;
+        f->lane_tiles = (uint32_t)tiles;
+        f->lane_reach[t] = 4ull * (uint64_t)((rows - 1) * stride + 16);
+        f->lanes.stride[t] = (uint32_t)stride;
+        f->lanes.rows[t] = (int)rows;
+    }
+    f->lane_program = found;
+    f->kind = FORM_LANES;
+    return true;
+}
+
+/* 16 warps per SM with two to four stages each; fewer where there are fewer tiles. */
+bool plan_lanes(const Form &f, uint32_t count, int sms, int max_smem, FormLaunch *l)
+{
+    const uint32_t n_in = (uint32_t)__builtin_popcount(f.lane_loads), n_out = (uint32_t)__builtin_popcount(f.lane_stores);
+    uint32_t w = (count + (uint32_t)sms - 1) / (uint32_t)sms;
+    if (w > 16) w = 16;
+    const uint32_t tiles = (uint32_t)max_smem / w / gint::kLaneTileBytes;
+    if (tiles < 2 * n_in + n_out) return false;
+    const uint32_t d = (tiles - n_out) / n_in;
+    l->lanes.depth = d > 4 ? 4 : d;
+    l->smem = w * (l->lanes.depth * n_in + n_out) * gint::kLaneTileBytes;
+    l->threads = w * 32u;
+    const uint32_t blocks = (count + w - 1) / w;
+    l->grid = blocks < (uint32_t)sms ? blocks : (uint32_t)sms;
+    l->warps_per_program = 1;
     return true;
 }
 

@@ -14,7 +14,7 @@ from gint_b200.host import capi, frontend as F
 from gint_b200.host.utils import fill_tensor_info
 from test_streaming import _perf_cases
 
-ROWS = 1
+ROWS, LANES = 1, 2
 
 
 def form(pd, bases, first=0, count=1, gather_mask=0, extent=1 << 30, logical=0, row=0, infos=None):
@@ -185,6 +185,56 @@ def test_offsets_are_those_of_the_descriptor_decode(seed):
             assert off[t] == decode(ti, t, logical, gather and t == 0, 13), (t, logical, sizes)
 
 
+def matrix_program(kind, batch=1000, stride=16):
+    m = _perf_cases()
+    t = C.to_interfaces([torch.empty(batch, 16)] * (3 if kind == "bmm4x4" else 2))
+    pd = getattr(m, kind).get_program(*t)
+    for info in pd.input_infos:
+        info.block_shape_stride_1[1] = stride
+    return pd
+
+
+@pytest.mark.parametrize("kind,n_slots", [("bmm4x4", 3), ("inv4x4", 2)])
+def test_what_a_launch_of_a_lane_program_needs(kind, n_slots):
+    pd, out = matrix_program(kind), n_slots - 1
+    tiles, size = 32, 64 * 1000
+    assert form(pd, FAR, count=tiles)[:2] == (LANES, 1)
+    assert form(pd, FAR, first=30, count=2)[0] == LANES and form(pd, FAR, first=30, count=3)[0] == 0      # tiles behind the grid wrap
+    assert form(matrix_program(kind, stride=20), FAR, count=tiles)[0] == LANES
+    assert form(matrix_program(kind, stride=18), FAR, count=tiles)[0] == 0 and form(matrix_program(kind, stride=12), FAR, count=tiles)[0] == 0
+    assert form(pd, FAR, count=tiles, gather_mask=1)[0] == 0
+    for t in range(n_slots):
+        assert form(pd, [b + (8 if k == t else 0) for k, b in enumerate(FAR)], count=tiles)[0] == 0       # 16-byte rows
+        assert form(pd, [b + (16 if k == t else 0) for k, b in enumerate(FAR)], count=tiles)[0] == LANES
+    for at, want in ((0, 0), (size - 16, 0), (size, LANES), (-size, LANES), (16 - size, 0)):
+        assert form(pd, [FAR[0] + at if k == out else b for k, b in enumerate(FAR)], count=tiles)[0] == want
+    if kind == "bmm4x4":
+        assert form(pd, [FAR[0], FAR[0], FAR[2]], count=tiles)[0] == LANES                                # a @ a
+    for info, change in ((0, ("block_shape_stride_2", [15, 1])), (1, ("block_shape_stride_2", [16, 2])), (0, ("block_grid_steps", [31, 0])), (out, ("elm_size", 2)),
+                         (1, ("block_grid_dims", [31, 1]))):
+        pd = matrix_program(kind)
+        infos = [type(i)(**vars(i)) for i in pd.input_infos]
+        setattr(infos[info], *change)
+        pd.input_infos[:] = infos
+        assert form(pd, FAR, count=tiles)[0] == 0, (info, change)
+
+
+@pytest.mark.parametrize("kind", ["bmm4x4", "inv4x4"])
+def test_a_lane_program_is_one_to_the_last_operand(kind):
+    pd = matrix_program(kind)
+    code = np.asarray(pd.program, dtype=np.int32).reshape(-1, 2)
+    ops = {O.LoadGlobal2DWF32, O.StoreGlobal2DWF32, O.DupBroadcastW, O.FPermW, O.FShuf2, O.LoadImm4F}
+    for i in range(len(code) - 1):
+        changed = code.copy()
+        if code[i, 0] in ops:
+            changed[i, 1] ^= 1 if code[i, 0] in (O.DupBroadcastW, O.FPermW, O.FShuf2, O.LoadImm4F) else 64
+        elif code[i, 0] in (O.FAdd, O.FMul, O.FSub, O.FRSub):
+            changed[i, 0] = O.FDiv
+        else:
+            continue
+        assert form(type(pd)(changed, pd.input_infos), FAR, count=32)[0] == 0, i
+
+
 # ---------------------------------------------------------------------------------------------- on the GPU
 
 def both(launch):
@@ -306,3 +356,28 @@ def test_rows_in_a_graph_and_on_few_blocks():
     finally:
         ex.set_option("max_blocks", 0)
     assert ex.device_status()["code"] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["bmm4x4", "inv4x4"])
+@pytest.mark.parametrize("batch", [1, 31, 33, 64, 1000, 4747, 80001])
+def test_lane_programs_give_the_bits_of_the_interpreter(kind, batch):
+    """Last tiles of any size, fewer tiles than warps and many rounds of them, ranges, singular and extreme matrices; guard bands."""
+    m, ex = _perf_cases(), get_executor()
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    a, b = torch.randn(batch, 16, device="cuda", generator=g), torch.randn(batch, 16, device="cuda", generator=g)
+    a[::5] = 0.0
+    a[3::7] *= 1e20
+    b[1::9, 3] = float("inf")
+    program_, tiles = getattr(m, kind), -(-batch // 32)
+    for first, count in ((0, tiles), (tiles // 3, tiles - tiles // 3), (0, (tiles + 1) // 2)):
+        def launch():
+            buffer = torch.full((batch + 64, 16), 9.0, device="cuda")
+            c = buffer[32:32 + batch]
+            tensors = [a, b, c] if kind == "bmm4x4" else [a, c]
+            ex.execute_range(program_, C.to_interfaces(tensors), first, count, cuda_stream=torch.cuda.current_stream().cuda_stream)
+            return [buffer]
+        same_bits(launch)
+    c = torch.empty_like(a)
+    tensors = [a, b, c] if kind == "bmm4x4" else [a, c]
+    assert ex.launch_info(program_, C.to_interfaces(tensors), tiles)["form"] == LANES
