@@ -7,6 +7,7 @@
  * (executor_impl.py:66-72), descriptors travel as kernel parameters, so a launch is a single cudaLaunchKernel
  * with no allocation and no copy and every captured launch in a CUDA graph is self-contained.
  */
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -1450,12 +1451,38 @@ int choose_lanes(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, 
     return FORM_LANES;
 }
 
+int choose_heads(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
+{
+    gint::HeadsArgs &a = l->heads;
+    a = f.heads;
+    l->kernel = f.head_kernel;
+    for (int s = 0; s < 3; s++) {
+        const uint64_t lo = base_ptrs[f.tensor[s]], out = base_ptrs[f.tensor[f.store]];
+        if ((lo & 1u) != 0 || (gather && ((gather->mask >> f.tensor[s]) & 1u))) return FORM_NONE;
+        if (s != f.store && lo < out + f.extent[f.store] && out < lo + f.extent[s]) return FORM_NONE;
+        a.slot[s].base = lo;
+        if (l->kernel == kHeadsKernelFirst + 3 && (lo & 7u) != 0) l->kernel = kHeadsKernelFirst + 2;
+    }
+    uint64_t all = 1;
+    for (uint32_t j = 0; j < a.grid.n_dims && all < (1ull << 31); j++) all *= a.grid.size[j];
+    if (first == 0 && count == all) sort_digits(&a);
+    a.first = first;
+    a.count = count;
+    l->threads = count <= 8u * (uint32_t)ctx->num_sms ? 32u : 256u;
+    const uint32_t per_block = l->threads / 32u, blocks = (count + per_block - 1) / per_block, resident = 4u * (uint32_t)ctx->num_sms;
+    l->grid = per_block == 1 || blocks < resident ? blocks : resident;
+    l->smem = 0;
+    l->warps_per_program = 1;
+    return FORM_HEADS;
+}
+
 int choose_form(const gint_ctx *ctx, const Program *p, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
 {
     const Form &f = p->form;
     if (f.kind == FORM_NONE || !ctx->opt_forms || !ctx->opt_wide || !ctx->opt_early_issue || !ctx->opt_rf || ctx->opt_vec || ctx->opt_prefetch || ctx->opt_tiles_per_warp) return FORM_NONE;
     if ((uint64_t)first + count >= (1ull << 31)) return FORM_NONE;
-    const int kind = f.kind == FORM_ROWS ? choose_rows(ctx, f, base_ptrs, first, count, gather, l) : choose_lanes(ctx, f, base_ptrs, first, count, gather, l);
+    const int kind = f.kind == FORM_ROWS ? choose_rows(ctx, f, base_ptrs, first, count, gather, l)
+                     : f.kind == FORM_LANES ? choose_lanes(ctx, f, base_ptrs, first, count, gather, l) : choose_heads(ctx, f, base_ptrs, first, count, gather, l);
     if (ctx->opt_max_blocks > 0 && (uint32_t)ctx->opt_max_blocks < l->grid) l->grid = (uint32_t)ctx->opt_max_blocks;
     return kind;
 }
@@ -1474,7 +1501,7 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
         FormLaunch l;
         const int kind = choose_form(ctx, p, base_ptrs, first, count, gather, &l);
         if (kind && ctx->form_fn[l.kernel]) {
-            void *args[1] = {kind == FORM_ROWS ? (void *)&l.rows : (void *)&l.lanes};
+            void *args[1] = {kind == FORM_ROWS ? (void *)&l.rows : kind == FORM_LANES ? (void *)&l.lanes : (void *)&l.heads};
             cudaError_t e = cudaLaunchKernel(ctx->form_fn[l.kernel], dim3(l.grid), dim3(l.threads), args, l.smem, (cudaStream_t)stream);
             if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaLaunchKernel", e);
             ctx->form_launched = true;
@@ -1610,6 +1637,7 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
         bool fits = false;
         const bool loops = wide_transform(prog, p->ti, n_tensors, &ws);
         if (loops && ctx->opt_fuse && ctx->opt_lower) match_rows(ws.prog, p->ti, &p->form);
+        if (loops && p->form.kind == FORM_NONE && ctx->opt_fuse && ctx->opt_lower) match_heads(ws.prog, p->ti, &p->form);
         if (p->form.kind == FORM_NONE && ctx->opt_fuse && ctx->opt_lower) match_lanes(prog, p->ti, n_tensors, p->st.pool_size, &p->form);
         if (loops && !ws.slow_rows)
             for (auto &v : ctx->direct) fits = fits || (v.wide == 1 && v.ok && v.P >= ws.max_depth);
@@ -1919,9 +1947,11 @@ int gint_debug_form(const int32_t *code, int n_words, const gint_tensor_info *ti
     const GatherArgs ga{gather_mask, nullptr, gather_extent_bytes, 1u};
     FormLaunch l;
     const int kind = choose_form(&ctx, p, base_ptrs, first, count, gather_mask ? &ga : nullptr, &l);
-    if (kind == FORM_ROWS && out_offsets) {
+    if ((kind == FORM_ROWS || kind == FORM_HEADS) && out_offsets) {
+        static_assert((int)gint::ROWS_N_SLOTS == (int)gint::HEADS_N_SLOTS, "slots of a form");
         uint32_t off[gint::ROWS_N_SLOTS];
-        gint::form_offsets(l.rows.grid, l.rows.slot, logical, row, off);
+        if (kind == FORM_ROWS) gint::form_offsets(l.rows.grid, l.rows.slot, logical, row, off);
+        else gint::form_offsets(l.heads.grid, l.heads.slot, logical, row, off);
         for (int s = 0; s < gint::ROWS_N_SLOTS; s++)
             if (p->form.tensor[s] >= 0) out_offsets[p->form.tensor[s]] = off[s];
     }

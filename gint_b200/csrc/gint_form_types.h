@@ -76,6 +76,18 @@ struct RowsArgs {
     uint32_t depth, stage_bytes, stationary_bytes;
 };
 
+/* Head programs (gint_heads.cuh): four short rows of bfloat16 elements per logical program, one per width value. */
+enum { HEADS_X = 0, HEADS_W, HEADS_Y, HEADS_ROW, HEADS_N_SLOTS };   // HEADS_ROW: not a tensor; its offset is the first row along dimension 2
+struct HeadsArgs {
+    FormGrid grid;
+    FormSlot slot[HEADS_N_SLOTS];
+    uint32_t row_stride[HEADS_Y + 1];   // elements between the four rows (W: 0)
+    int rows;                        // along dimension 2, in every slot
+    uint32_t first, count;
+    float init, factor, addend;
+    uint32_t fused;                  // the factor and the addend in one fma
+};
+
 /* Lane programs (gint_lanes.cuh): tile t of slot s covers rows 32 t .. 32 t + 31 of rows[s], each `stride` elements apart. */
 struct LaneArgs {
     u64 base[8];

@@ -4,12 +4,14 @@
  */
 #pragma once
 
+#include <utility>
+
 #include "gint_form_types.h"
 #include "gint_lane_programs.h"
 
 namespace {
 
-enum { FORM_NONE = 0, FORM_ROWS = 1, FORM_LANES = 2 };
+enum { FORM_NONE = 0, FORM_ROWS = 1, FORM_LANES = 2, FORM_HEADS = 3 };
 
 struct Form {
     int kind = FORM_NONE;
@@ -25,6 +27,8 @@ struct Form {
     uint32_t lane_loads = 0, lane_stores = 0, lane_tiles = 0;
     uint64_t lane_reach[GINT_MAX_TENSORS] = {};
     gint::LaneArgs lanes;
+    int head_kernel = 0;
+    gint::HeadsArgs heads;
 };
 /* a launch on a form kernel */
 struct FormLaunch {
@@ -32,6 +36,7 @@ struct FormLaunch {
     uint32_t grid = 0, threads = 0, smem = 0, warps_per_program = 0;
     gint::RowsArgs rows;
     gint::LaneArgs lanes;
+    gint::HeadsArgs heads;
 };
 
 struct FormDim { uint32_t size, stride; bool batch0; };
@@ -327,6 +332,94 @@ bool plan_lanes(const Form &f, uint32_t count, int sms, int max_smem, FormLaunch
     l->grid = blocks < (uint32_t)sms ? blocks : (uint32_t)sms;
     l->warps_per_program = 1;
     return true;
+}
+
+
+/*
+ * Normalisation of short bfloat16 rows, four per logical program (2DT tiles): a sum of squares by fma over two to four tiles of x, times a
+ * factor plus an addend, 1 / sqrt, and y = (that * x) * w, w being one row for all.
+ */
+constexpr int kHeadsKernelFirst = 4;   // of GINT_FORM_KERNELS: rows of two tiles
+
+bool match_heads(const std::vector<Insn> &p, const gint_tensor_info &ti, Form *f)
+{
+    gint::HeadsArgs &a = f->heads;
+    memset(&a, 0, sizeof(a));
+    for (int &t : f->tensor) t = -1;
+    const int kLoad = GINT_W(LoadGlobal2DTBF16), kStore = GINT_W(StoreGlobal2DTBF16);
+    size_t i = 0;
+    auto take = [&](int op, uint32_t *operand) {
+        if (i >= p.size() || p[i].op != op) return false;
+        if (operand) *operand = p[i].operand;
+        i++;
+        return true;
+    };
+    uint32_t init, tiles, tiles2, x, x2, w, y, factor, addend;
+    if (!take(OP_LoadImm, &init) || !take(WOP_LoopBegin, &tiles) || !take(kLoad, &x) || !take(WOP_AccFMASquare, nullptr) || !take(WOP_LoopEnd, nullptr)) return false;
+    if (!take(OP_WarpAllReduceSum, nullptr)) return false;
+    if (take(OP_FMAImm, &factor)) {
+        a.fused = 1;
+        a.factor = __half2float(__ushort_as_half((unsigned short)(factor & 0xFFFFu)));
+        a.addend = __half2float(__ushort_as_half((unsigned short)(factor >> 16)));
+    } else {
+        if (!take(OP_FMulImm, &factor) || !take(OP_FAddImm, &addend)) return false;
+        memcpy(&a.factor, &factor, 4);
+        memcpy(&a.addend, &addend, 4);
+    }
+    if (!take(OP_FRSqrt, nullptr) || !take(WOP_LoopBegin, &tiles2) || !take(kLoad, &x2) || !take(WOP_MulKeep, nullptr) || !take(kLoad, &w) || !take(GINT_W(FMul), nullptr)) return false;
+    if (!take(kStore, &y) || !take(WOP_LoopEnd, nullptr)) return false;
+    take(OP_Pop, nullptr);
+    if (!take(OP_Halt, nullptr)) return false;
+    memcpy(&a.init, &init, 4);
+    if (tiles < 2 || tiles > 4 || tiles2 != tiles || x2 != x || x >= GINT_MAX_TENSORS || w >= GINT_MAX_TENSORS || y >= GINT_MAX_TENSORS || y == x || y == w) return false;   // (offsets 0)
+    const int tensor[3] = {(int)x, (int)w, (int)y}, n1 = ti.block_shape_stride_1[x][0];
+    int n[3] = {n1, n1, n1};
+    if (n1 <= 32 * ((int)tiles - 1)) return false;
+    for (int t : tensor) {
+        if (ti.block_shape_stride_1[t][0] != n1 || ti.block_shape_stride_1[t][1] != 1 || ti.block_shape_stride_2[t][1] < 0) return false;
+        if (ti.block_shape_stride_2[t][0] != ti.block_shape_stride_2[x][0] || ti.block_grid_dims[t][1] != ti.block_grid_dims[x][1] || ti.block_grid_steps[t][1] != ti.block_grid_steps[x][1]) return false;
+    }
+    if (ti.block_shape_stride_2[w][1] != 0 || ti.block_shape_stride_2[x][0] < 1 || ti.block_grid_steps[x][1] < 0) return false;
+    if ((int64_t)ti.block_grid_dims[x][1] * ti.block_grid_steps[x][1] >= (1ll << 31)) return false;
+    if (!form_grid(ti, tensor, 3, n, 2, &a.grid, a.slot, f) || !a.slot[gint::HEADS_W].stationary) return false;
+    for (int s = 0; s < 3; s++) {
+        const int64_t stride2 = ti.block_shape_stride_2[tensor[s]][1];
+        f->tensor[s] = tensor[s];
+        /* four rows from the first one on, as far as there are rows */
+        const int64_t begin = (int64_t)(ti.block_grid_dims[x][1] - 1) * ti.block_grid_steps[x][1], end = ti.block_shape_stride_2[x][0] - 1;
+        f->extent[s] += (uint64_t)(2 * stride2 * (begin + 3 < end ? begin + 3 : end)) - (uint64_t)(2 * stride2 * begin);
+        if (f->extent[s] / 2 >= (1ull << 31) - 8192) return false;
+        a.row_stride[s] = (uint32_t)stride2;
+    }
+    if (ti.block_grid_dims[x][1] != 1) {
+        if (a.grid.n_dims == 0 || a.grid.size[0] != (uint32_t)ti.block_grid_dims[x][1]) return false;   // (the slots that move share the digits)
+        a.slot[gint::HEADS_ROW].stride[0] = (uint32_t)ti.block_grid_steps[x][1];
+    }
+    a.rows = ti.block_shape_stride_2[x][0];
+    f->store = gint::HEADS_Y;
+    /* four elements per lane and access: rows of 128, every offset of a row a multiple of 4 elements */
+    bool fours = n1 == 128 && tiles == 4;
+    for (int s = 0; s < 3; s++) {
+        fours = fours && a.row_stride[s] % 4 == 0;
+        for (uint32_t stride : a.slot[s].stride) fours = fours && stride % 4 == 0;
+    }
+    f->head_kernel = kHeadsKernelFirst + (fours ? 3 : (int)tiles - 2);
+    f->kind = FORM_HEADS;
+    return true;
+}
+
+/* The digits in the order of the strides of x, so that logical programs that follow one another lie next to one another. For launches of
+ * the whole grid, which is the same set of logical programs in any order. */
+void sort_digits(gint::HeadsArgs *a)
+{
+    gint::FormGrid &g = a->grid;
+    for (uint32_t i = 1; i < g.n_dims; i++)
+        for (uint32_t j = i; j > 0 && a->slot[gint::HEADS_X].stride[j] < a->slot[gint::HEADS_X].stride[j - 1]; j--) {
+            std::swap(g.size[j], g.size[j - 1]);
+            std::swap(g.magic[j], g.magic[j - 1]);
+            std::swap(g.shift[j], g.shift[j - 1]);
+            for (gint::FormSlot &s : a->slot) std::swap(s.stride[j], s.stride[j - 1]);
+        }
 }
 
 }  // namespace

@@ -1,0 +1,3 @@
+// Normalisation of bfloat16 rows of 4 tiles of 32 elements (gint_heads.cuh).
+#include "../gint_heads.cuh"
+GINT_DEFINE_HEADS_KERNEL(4)

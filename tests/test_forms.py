@@ -14,7 +14,7 @@ from gint_b200.host import capi, frontend as F
 from gint_b200.host.utils import fill_tensor_info
 from test_streaming import _perf_cases
 
-ROWS, LANES = 1, 2
+ROWS, LANES, HEADS = 1, 2, 3
 
 
 def form(pd, bases, first=0, count=1, gather_mask=0, extent=1 << 30, logical=0, row=0, infos=None):
@@ -235,6 +235,73 @@ def test_a_lane_program_is_one_to_the_last_operand(kind):
         assert form(type(pd)(changed, pd.input_infos), FAR, count=32)[0] == 0, i
 
 
+@bytecode
+def heads_program(x, y, w, REGW, WARP, fused=True, load="fldg_2dt_bf16", reduce="fma"):
+    """rmsnorm over the last dimension of (batch, heads, tokens, dim) views, four tokens per logical program."""
+    B, NH, T, H = x.shape
+    xb, yb = [F.make_block_2d(t, [H, T], [t.strides[-1], t.strides[-2]], [1, -(-T // REGW)], [0, REGW], [t.strides[0], t.strides[1]], [B, NH]) for t in (x, y)]
+    wb = F.make_block_2d(w, [H, T], [w.strides[-1], 0], [1, -(-T // REGW)], [0, REGW], [0, 0], [B, NH])
+    F.fpush(0.0)
+    for c in range(0, H, WARP):
+        getattr(F, load)(c, xb)
+        F.dup()
+        if reduce == "fma":
+            F.fma()
+        else:
+            F.fmul()
+            F.fadd()
+    F.warp_allreduce_fsum()
+    if fused:
+        F.fmaimm(1 / H, 1e-5)
+    else:
+        F.fmulimm(1 / H)
+        F.faddimm(1e-5)
+    F.frsqrt()
+    for c in range(0, H, WARP):
+        F.dup()
+        getattr(F, load)(c, xb)
+        F.fmul()
+        getattr(F, load)(c, wb)
+        F.fmul()
+        getattr(F, load.replace("fldg", "fstg"))(c, yb)
+    F.halt()
+
+
+def head_views(batch, tokens, heads, dim, device="cpu", dtype=torch.bfloat16):
+    return [torch.empty(batch, tokens, heads, dim, dtype=dtype, device=device).transpose(1, 2) for _ in range(2)] + [torch.empty(dim, dtype=dtype, device=device)]
+
+
+def head_program(*shape, **kw):
+    return heads_program.get_program(*C.to_interfaces(head_views(*shape, dtype=kw.pop("dtype", torch.bfloat16))), **kw)
+
+
+@pytest.mark.parametrize("dim,kw,want", [(64, {}, HEADS), (33, {}, HEADS), (80, {"fused": False}, HEADS), (128, {}, HEADS), (32, {}, 0), (129, {}, 0), (128, {"reduce": "square"}, 0),
+                                         (128, {"load": "fldg_2dt_f16", "dtype": torch.float16}, 0)])
+def test_head_programs_have_the_form(dim, kw, want):
+    assert form(head_program(2, 37, 3, dim, **kw), FAR, count=60)[0] == want
+
+
+def test_what_a_launch_of_heads_needs():
+    pd, size = head_program(2, 37, 3, 64), 2 * 2 * 37 * 3 * 64
+    assert form(pd, [FAR[0] + 2, FAR[1] + 6, FAR[2] + 2], count=60)[0] == HEADS
+    assert form(pd, [FAR[0] + 1] + FAR[1:], count=60)[0] == 0
+    assert form(pd, FAR, count=60, gather_mask=1)[0] == 0
+    for at, want in ((0, 0), (size - 2, 0), (size, HEADS)):                       # (the last four rows of a head end with its tokens)
+        assert form(pd, [FAR[0], FAR[0] + at, FAR[2]], count=60)[0] == want
+
+
+@pytest.mark.parametrize("shape", [(2, 37, 3, 64), (1, 8, 5, 128), (3, 4, 1, 96), (1, 1, 1, 80)])
+def test_a_whole_launch_of_heads_takes_every_logical_program_once(shape):
+    """The offsets of a launch of the whole grid are those of its logical programs, in the order of the addresses; a part keeps their numbers."""
+    pd = head_program(*shape)
+    total = shape[0] * shape[2] * -(-shape[1] // 4)
+    offsets = [form(pd, FAR, count=total, logical=r)[2] for r in range(total)]
+    want = [[decode(form(pd, FAR, count=total)[3], t, r, False, 0) for t in range(3)] for r in range(total)]
+    assert sorted(offsets) == sorted(want) and [o[0] for o in offsets] == sorted(w[0] for w in want)
+    for r in range(0, total - 1, 3):
+        assert form(pd, FAR, first=r, count=1, logical=r)[2] == want[r]
+
+
 # ---------------------------------------------------------------------------------------------- on the GPU
 
 def both(launch):
@@ -381,3 +448,41 @@ def test_lane_programs_give_the_bits_of_the_interpreter(kind, batch):
     c = torch.empty_like(a)
     tensors = [a, b, c] if kind == "bmm4x4" else [a, c]
     assert ex.launch_info(program_, C.to_interfaces(tensors), tiles)["form"] == LANES
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,tokens,heads,dim", [(1, 1, 1, 128), (2, 37, 3, 64), (1, 6, 2, 33), (2, 12, 3, 80), (1, 31, 2, 96), (3, 50, 7, 127), (2, 333, 5, 128), (4, 1000, 6, 64), (8, 1001, 5, 128)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_heads(batch, tokens, heads, dim, shift):
+    """Single elements (rows of two to four tiles, base pointers at any element): the bits of the interpreter's tile kernels. Rows of 128 at 8-byte
+    boundaries add their squares in another order, as the streaming kernels do: one bfloat16 rounding of the 64-bit value, to which sum, rsqrt and
+    products in f32 add less than 2^-18."""
+    ex = get_executor()
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    count = batch * tokens * heads * dim
+    flat = (torch.randn(count + 8, device="cuda", generator=g) * 1.5 + 0.5).bfloat16()
+    x = flat[shift:shift + count].view(batch, tokens, heads, dim).transpose(1, 2)
+    w = torch.rand(dim + 8, device="cuda", generator=g).bfloat16()[shift:shift + dim]
+    total = batch * heads * -(-tokens // 4)
+    fours = dim == 128 and shift == 0
+    for first, n in ((0, total), (total // 3, total - total // 3)):
+        got = []
+        for on in (1, 0):
+            ex.set_option("streaming", on)
+            try:
+                buffer = torch.full((count + 128,), 9.0, device="cuda").bfloat16()
+                y = buffer[64 + shift:64 + shift + count].view(batch, tokens, heads, dim).transpose(1, 2)
+                assert (ex.launch_info(heads_program, C.to_interfaces([x, y, w]), total)["form"] == HEADS) == bool(on)
+                ex.execute_range(heads_program, C.to_interfaces([x, y, w]), first, n, cuda_stream=torch.cuda.current_stream().cuda_stream)
+                got.append(buffer.cpu())
+            finally:
+                ex.set_option("streaming", 1)
+        if not fours:
+            assert bits_equal(*got), mismatch_report(*got)
+        else:
+            xd = x.double()
+            want = torch.full((count + 128,), 9.0, dtype=torch.float64, device="cuda")
+            inside = (got[1] != 9.0).cuda()
+            full = (xd * torch.rsqrt(xd.pow(2).sum(-1, keepdim=True) * 2.0 ** -7 + float(torch.tensor(1e-5).half())) * w.double()).transpose(1, 2).reshape(-1)
+            want[64:64 + count] = torch.where(inside[64:64 + count], full, want[64:64 + count])
+            torch.testing.assert_close(got[0].double(), want.cpu(), rtol=2.0 ** -8 + 2.0 ** -18, atol=0.0)
