@@ -1476,13 +1476,44 @@ int choose_heads(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, 
     return FORM_HEADS;
 }
 
+int choose_flat(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
+{
+    if (gather || first + count > f.flat_grid) return FORM_NONE;
+    const uint64_t out = base_ptrs[f.tensor[2]], bytes = (uint64_t)f.flat_n * f.flat_element_bytes;
+    for (int s = 0; s < 3; s++) {
+        if (f.tensor[s] < 0) continue;
+        const uint64_t at = base_ptrs[f.tensor[s]];
+        if ((at & 15u) != 0) return FORM_NONE;
+        if (at != out && at < out + bytes && out < at + bytes) return FORM_NONE;   // (in place: a thread stores what it alone has loaded)
+    }
+    const uint64_t begin = (uint64_t)first * f.flat_step, end = (uint64_t)(first + count) * f.flat_step < f.flat_n ? (uint64_t)(first + count) * f.flat_step : f.flat_n;
+    if (begin >= end) return FORM_NONE;
+    gint::FlatArgs &a = l->flat;
+    a = f.flat;
+    a.x = (const void *)base_ptrs[f.tensor[0]];
+    a.y = f.tensor[1] < 0 ? nullptr : (const void *)base_ptrs[f.tensor[1]];
+    a.z = (void *)out;
+    const uint32_t group = 16u / f.flat_element_bytes;
+    a.begin = (uint32_t)(begin / group);
+    a.end = (uint32_t)(end / group);
+    a.rest = (uint32_t)(end % group);
+    const uint32_t blocks = (a.end - a.begin + 255u) / 256u, resident = 4u * (uint32_t)ctx->num_sms;
+    l->kernel = f.flat_kernel;
+    l->threads = 256u;
+    l->grid = blocks < 1 ? 1 : blocks < resident ? blocks : resident;
+    l->smem = 0;
+    l->warps_per_program = 1;
+    return FORM_FLAT;
+}
+
 int choose_form(const gint_ctx *ctx, const Program *p, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
 {
     const Form &f = p->form;
     if (f.kind == FORM_NONE || !ctx->opt_forms || !ctx->opt_wide || !ctx->opt_early_issue || !ctx->opt_rf || ctx->opt_vec || ctx->opt_prefetch || ctx->opt_tiles_per_warp) return FORM_NONE;
     if ((uint64_t)first + count >= (1ull << 31)) return FORM_NONE;
     const int kind = f.kind == FORM_ROWS ? choose_rows(ctx, f, base_ptrs, first, count, gather, l)
-                     : f.kind == FORM_LANES ? choose_lanes(ctx, f, base_ptrs, first, count, gather, l) : choose_heads(ctx, f, base_ptrs, first, count, gather, l);
+                     : f.kind == FORM_LANES ? choose_lanes(ctx, f, base_ptrs, first, count, gather, l) : f.kind == FORM_HEADS ? choose_heads(ctx, f, base_ptrs, first, count, gather, l)
+                     : choose_flat(ctx, f, base_ptrs, first, count, gather, l);
     if (ctx->opt_max_blocks > 0 && (uint32_t)ctx->opt_max_blocks < l->grid) l->grid = (uint32_t)ctx->opt_max_blocks;
     return kind;
 }
@@ -1501,7 +1532,7 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
         FormLaunch l;
         const int kind = choose_form(ctx, p, base_ptrs, first, count, gather, &l);
         if (kind && ctx->form_fn[l.kernel]) {
-            void *args[1] = {kind == FORM_ROWS ? (void *)&l.rows : kind == FORM_LANES ? (void *)&l.lanes : (void *)&l.heads};
+            void *args[1] = {kind == FORM_ROWS ? (void *)&l.rows : kind == FORM_LANES ? (void *)&l.lanes : kind == FORM_HEADS ? (void *)&l.heads : (void *)&l.flat};
             cudaError_t e = cudaLaunchKernel(ctx->form_fn[l.kernel], dim3(l.grid), dim3(l.threads), args, l.smem, (cudaStream_t)stream);
             if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaLaunchKernel", e);
             ctx->form_launched = true;
@@ -1638,6 +1669,7 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
         const bool loops = wide_transform(prog, p->ti, n_tensors, &ws);
         if (loops && ctx->opt_fuse && ctx->opt_lower) match_rows(ws.prog, p->ti, &p->form);
         if (loops && p->form.kind == FORM_NONE && ctx->opt_fuse && ctx->opt_lower) match_heads(ws.prog, p->ti, &p->form);
+        if (loops && p->form.kind == FORM_NONE && ctx->opt_fuse && ctx->opt_lower) match_flat(ws, p->ti, &p->form);
         if (p->form.kind == FORM_NONE && ctx->opt_fuse && ctx->opt_lower) match_lanes(prog, p->ti, n_tensors, p->st.pool_size, &p->form);
         if (loops && !ws.slow_rows)
             for (auto &v : ctx->direct) fits = fits || (v.wide == 1 && v.ok && v.P >= ws.max_depth);

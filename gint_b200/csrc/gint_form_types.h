@@ -88,6 +88,16 @@ struct HeadsArgs {
     uint32_t fused;                  // the factor and the addend in one fma
 };
 
+/* z = [silu](x) [+ y | * y] (gint_flat.cuh): groups [begin, end) of 16 bytes, then `rest` single elements. */
+enum { FLAT_SILU = 1, FLAT_ADD = 2, FLAT_MUL = 4 };
+struct FlatArgs {
+    const void *x, *y;
+    void *z;
+    uint32_t begin, end, rest;
+    uint32_t map;                    // a set of FLAT_...; at most one of FLAT_ADD and FLAT_MUL
+    float silu;
+};
+
 /* Lane programs (gint_lanes.cuh): tile t of slot s covers rows 32 t .. 32 t + 31 of rows[s], each `stride` elements apart. */
 struct LaneArgs {
     u64 base[8];

@@ -11,7 +11,7 @@
 
 namespace {
 
-enum { FORM_NONE = 0, FORM_ROWS = 1, FORM_LANES = 2, FORM_HEADS = 3 };
+enum { FORM_NONE = 0, FORM_ROWS = 1, FORM_LANES = 2, FORM_HEADS = 3, FORM_FLAT = 4 };
 
 struct Form {
     int kind = FORM_NONE;
@@ -29,6 +29,10 @@ struct Form {
     gint::LaneArgs lanes;
     int head_kernel = 0;
     gint::HeadsArgs heads;
+    /* flat: tensor[] holds x, y (-1: none), z */
+    int flat_kernel = 0;
+    uint32_t flat_n = 0, flat_step = 0, flat_grid = 0, flat_element_bytes = 0;
+    gint::FlatArgs flat;
 };
 /* a launch on a form kernel */
 struct FormLaunch {
@@ -37,6 +41,7 @@ struct FormLaunch {
     gint::RowsArgs rows;
     gint::LaneArgs lanes;
     gint::HeadsArgs heads;
+    gint::FlatArgs flat;
 };
 
 struct FormDim { uint32_t size, stride; bool batch0; };
@@ -420,6 +425,55 @@ void sort_digits(gint::HeadsArgs *a)
             std::swap(g.shift[j], g.shift[j - 1]);
             for (gint::FormSlot &s : a->slot) std::swap(s.stride[j], s.stride[j - 1]);
         }
+}
+
+
+/* [silu](x) [+ y | * y] as one flat loop (WideStream::flat_tiles) over slots of one length and type, from element 0 on. */
+constexpr int kFlatKernelFirst = 8;   // of GINT_FORM_KERNELS: f32, f16, bf16
+
+bool match_flat(const WideStream &ws, const gint_tensor_info &ti, Form *f)
+{
+    const std::vector<Insn> &p = ws.prog;
+    const int loads[3] = {GINT_W(LoadGlobal1DF32), GINT_W(LoadGlobal1DF16), GINT_W(LoadGlobal1DBF16)};
+    const int stores[3] = {GINT_W(StoreGlobal1DF32), GINT_W(StoreGlobal1DF16), GINT_W(StoreGlobal1DBF16)};
+    memset(&f->flat, 0, sizeof(f->flat));
+    for (int &t : f->tensor) t = -1;
+    size_t i = 1;
+    int type = 0;
+    auto is = [&](int op) { return i < p.size() && p[i].op == op; };
+    if (!ws.flat_tiles || p[0].op != WOP_LoopBegin) return false;
+    while (type < 3 && !is(loads[type])) type++;
+    if (type == 3) return false;
+    f->tensor[0] = (int)p[i++].operand;
+    if (is(WOP_Silu)) {
+        memcpy(&f->flat.silu, &p[i++].operand, 4);
+        f->flat.map |= gint::FLAT_SILU;
+    }
+    if (is(loads[type])) {
+        f->tensor[1] = (int)p[i++].operand;
+        if (!is(GINT_W(FAdd)) && !is(GINT_W(FMul))) return false;
+        f->flat.map |= is(GINT_W(FAdd)) ? gint::FLAT_ADD : gint::FLAT_MUL;
+        i++;
+    }
+    if (!f->flat.map || !is(stores[type])) return false;
+    f->tensor[2] = (int)p[i++].operand;
+    if (!is(WOP_LoopEnd) || i + 2 != p.size()) return false;
+    f->flat_n = 0;
+    for (int s = 0; s < 3; s++) {
+        const int t = f->tensor[s];
+        if (t < 0) continue;
+        if (t >= GINT_MAX_TENSORS || ti.block_shape_stride_1[t][0] < 1 || ti.block_shape_stride_1[t][1] != 1 || ti.elm_size[t] != (type ? 2 : 4)) return false;   // (an offset makes it larger)
+        if (f->flat_n && f->flat_n != (uint32_t)ti.block_shape_stride_1[t][0]) return false;
+        f->flat_n = (uint32_t)ti.block_shape_stride_1[t][0];
+    }
+    if (f->tensor[2] == f->tensor[0] || f->tensor[2] == f->tensor[1]) return false;
+    f->flat_step = ws.flat_tiles * 128u;
+    f->flat_grid = ws.flat_grid;
+    f->flat_kernel = kFlatKernelFirst + type;
+    f->flat_element_bytes = type ? 2u : 4u;
+    f->store = 2;
+    f->kind = FORM_FLAT;
+    return true;
 }
 
 }  // namespace

@@ -19,8 +19,9 @@ extern "C" {
 #define GINT_INDIRECT_VARIANTS(X) X(12)
 #define GINT_CHECKED_VARIANTS(X) X(12)
 /* kernels of program forms (gint_forms_host.h): X(source and kernel name, index) */
-#define GINT_FORM_KERNELS(X) X(rows_f32, 0) X(rows4_f32, 1) X(lanes_bmm4x4, 2) X(lanes_inv4x4, 3) X(heads_bf16_2, 4) X(heads_bf16_3, 5) X(heads_bf16_4, 6) X(heads_bf16_fours, 7)
-#define GINT_N_FORM_KERNELS 8
+#define GINT_FORM_KERNELS(X) X(rows_f32, 0) X(rows4_f32, 1) X(lanes_bmm4x4, 2) X(lanes_inv4x4, 3) X(heads_bf16_2, 4) X(heads_bf16_3, 5) X(heads_bf16_4, 6) X(heads_bf16_fours, 7) \
+    X(flat_f32, 8) X(flat_f16, 9) X(flat_bf16, 10)
+#define GINT_N_FORM_KERNELS 11
 
 #define GINT_X_DECL(P, K)                                        \
     extern const unsigned char gint_cubin_direct_##P##_##K[];     \

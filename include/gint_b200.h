@@ -80,7 +80,7 @@ typedef struct gint_launch_info {
     int32_t registers_in_smem; /* virtual registers kept in shared memory (the pool then holds the operand stack alone); 0: in the pool */
     int32_t vector_layout;    /* 1: full 1-D tiles live in the pool with lane l holding elements 4l..4l+3 (16-byte accesses) */
     int32_t streaming;        /* 1: a streaming kernel (tile loops found again) */
-    int32_t form;             /* not 0: the launch runs on the kernel of the program's form (1: rows, 2: lane program, 3: heads); the fields above then describe the
+    int32_t form;             /* not 0: the launch runs on the kernel of the program's form (1: rows, 2: lane program, 3: heads, 4: flat); the fields above then describe the
                                * interpreter kernel that runs it where the form does not apply */
     int32_t reserved[3];
 } gint_launch_info;
@@ -136,7 +136,7 @@ int gint_debug_predecode_batch(const int32_t *code, int n_words, int n_tensors, 
 int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs,
                      uint32_t first, uint32_t count, uint32_t gather_mask, uint64_t gather_extent_bytes);
 
-/* Does a launch run on the kernel of the program's form (default options; needs no device)? 0: no; else bits 0-7 the form (1: rows, 2: lane program, 3: heads),
+/* Does a launch run on the kernel of the program's form (default options; needs no device)? 0: no; else bits 0-7 the form (1: rows, 2: lane program, 3: heads, 4: flat),
  * bits 8-15 the warps per logical program. out_offsets (or NULL) receives, by tensor slot, the element offset at which logical
  * program `logical` of a program over rows starts (a launch of the whole grid of heads numbers them as they lie in memory); `row` stands for the entry of the row index in a gathered launch. Negative: the status of a refused program. */
 int gint_debug_form(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs, uint32_t first,

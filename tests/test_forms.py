@@ -14,7 +14,7 @@ from gint_b200.host import capi, frontend as F
 from gint_b200.host.utils import fill_tensor_info
 from test_streaming import _perf_cases
 
-ROWS, LANES, HEADS = 1, 2, 3
+ROWS, LANES, HEADS, FLAT = 1, 2, 3, 4
 
 
 def form(pd, bases, first=0, count=1, gather_mask=0, extent=1 << 30, logical=0, row=0, infos=None):
@@ -302,6 +302,51 @@ def test_a_whole_launch_of_heads_takes_every_logical_program_once(shape):
         assert form(pd, FAR, first=r, count=1, logical=r)[2] == want[r]
 
 
+@bytecode
+def flat_program(x, y, z, REGW, WARP, op="silu_fmul", dtype="f32", tiles=1, start=0):
+    n, = x.shape
+    suffix, block = "" if dtype == "f32" else "_" + dtype, 128 * tiles
+    xb, yb, zb = [F.make_block_1d(t, t.shape[0], t.strides[0], -(-n // block), block) for t in (x, y, z)]
+    for off in range(start, start + block, 128):
+        getattr(F, "fldg_1d" + suffix)(off, xb)
+        if op.startswith("silu"):
+            F.dup()
+            F.fneg()
+            F.fexp()
+            F.faddimm(1.0)
+            F.frdiv()
+        if op != "silu":
+            getattr(F, "fldg_1d" + suffix)(off, yb)
+            getattr(F, op.replace("silu_", ""))()
+        getattr(F, "fstg_1d" + suffix)(off, zb)
+    F.halt()
+
+
+TYPES = {"f32": torch.float32, "f16": torch.float16, "bf16": torch.bfloat16}
+
+
+def flat(n=5000, ny=None, stride=1, **kw):
+    t = [torch.empty(k * stride, dtype=TYPES[kw.get("dtype", "f32")])[::stride] for k in (n, ny or n, n)]
+    return flat_program.get_program(*C.to_interfaces(t), **kw)
+
+
+@pytest.mark.parametrize("kw,want", [({}, FLAT), ({"op": "fadd"}, FLAT), ({"op": "fmul", "dtype": "f16"}, FLAT), ({"op": "silu", "dtype": "bf16"}, FLAT), ({"op": "silu_fadd", "tiles": 4}, FLAT),
+                                     ({"op": "fsub"}, 0), ({"start": 128}, 0), ({"ny": 4999}, 0), ({"stride": 2}, 0), ({"n": 1}, FLAT)])
+def test_flat_programs_have_the_form(kw, want):
+    assert form(flat(**kw), FAR, count=1)[0] == want
+
+
+def test_what_a_flat_launch_needs():
+    pd, size = flat(), 4 * 5000
+    for t in range(3):
+        assert form(pd, [b + (4 if k == t else 0) for k, b in enumerate(FAR)], count=40)[0] == 0          # 16-byte groups
+        assert form(pd, [b + (16 if k == t else 0) for k, b in enumerate(FAR)], count=40)[0] == FLAT
+    assert form(pd, FAR, first=39, count=1)[0] == FLAT and form(pd, FAR, first=39, count=2)[0] == 0
+    assert form(pd, FAR, count=40, gather_mask=1)[0] == 0
+    for at, want in ((0, FLAT), (16, 0), (size - 16, 0), (size, FLAT)):                                   # in place, but not shifted
+        assert form(pd, [FAR[0], FAR[1], FAR[0] + at], count=40)[0] == want
+
+
 # ---------------------------------------------------------------------------------------------- on the GPU
 
 def both(launch):
@@ -486,3 +531,28 @@ def test_heads(batch, tokens, heads, dim, shift):
             full = (xd * torch.rsqrt(xd.pow(2).sum(-1, keepdim=True) * 2.0 ** -7 + float(torch.tensor(1e-5).half())) * w.double()).transpose(1, 2).reshape(-1)
             want[64:64 + count] = torch.where(inside[64:64 + count], full, want[64:64 + count])
             torch.testing.assert_close(got[0].double(), want.cpu(), rtol=2.0 ** -8 + 2.0 ** -18, atol=0.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("op", ["fadd", "fmul", "silu", "silu_fmul", "silu_fadd"])
+def test_flat_launches_give_the_bits_of_the_interpreter(op, dtype):
+    """Lengths around groups, warps' shares and blocks, a group per thread and several, ranges, in place; zeros, infinities and NaN."""
+    ex, dt = get_executor(), TYPES[dtype]
+    for n, tiles in ((1, 1), (3, 4), (8, 1), (127, 1), (1025, 4), (4096, 1), (40003, 4), (1 << 20, 1), (1212416, 1), (1212421, 4), (5000007, 4)):
+        g = torch.Generator(device="cuda").manual_seed(n)
+        x, y = [(torch.randn(n, device="cuda", generator=g) * 3).to(dt) for _ in range(2)]
+        for k, v in enumerate((0.0, -0.0, float("inf"), float("-inf"), float("nan"), 1e-7, -95.0)):
+            x[k + 11:k + 12] = v
+        total = -(-n // (128 * tiles))
+        kw = {"op": op, "dtype": dtype, "tiles": tiles}
+        assert ex.launch_info(flat_program, C.to_interfaces([x, y, torch.empty_like(x)]), total, **kw)["form"] == FLAT
+        for first, count in {(0, total), (total // 3, total - total // 3), (0, -(-total // 2))}:
+            def launch():
+                buffer = torch.full((n + 128,), 9.0, device="cuda").to(dt)
+                z, inplace = buffer[64:64 + n], x.clone()
+                st = torch.cuda.current_stream().cuda_stream
+                ex.execute_range(flat_program, C.to_interfaces([x, y, z]), first, count, cuda_stream=st, **kw)
+                ex.execute_range(flat_program, C.to_interfaces([inplace, y, inplace]), first, count, cuda_stream=st, **kw)
+                return [buffer, inplace]
+            same_bits(launch)
