@@ -1554,6 +1554,21 @@ static __device__ __noinline__ void stage_for_warp(uint2 *code_s, const uint2 *c
     __syncwarp();
 }
 
+/* ... and a candidate of a batch from the caller's words: the checks are done (check_candidate in gint_capi.cu), the entries are made here. */
+static __device__ __noinline__ uint32_t stage_raw_for_warp(uint2 *code_s, const int2 *raw, uint32_t n, gint_tensor_info *ti_s, const gint_tensor_info *ti_g,
+                                                           uint32_t out_slot, u64 out, int lane)
+{
+    const uint32_t entries = stream_entries(n);
+    for (uint32_t i = lane; i < entries; i += 32) code_s[i] = stream_entry(raw, n, i);
+    const int *src = reinterpret_cast<const int *>(ti_g);
+    int *dst = reinterpret_cast<int *>(ti_s);
+    for (uint32_t i = lane; i < sizeof(gint_tensor_info) / 4; i += 32) dst[i] = __ldg(src + i);
+    __syncwarp();
+    if (lane == 0) ti_s->base_ptr[out_slot] = (int64_t)out;
+    __syncwarp();
+    return entries;
+}
+
 /* Direct mode: every logical program runs the same bytecode. Persistent blocks of kWarpsPerBlock warps;
  * shared memory = [program | descriptor block | kWarpsPerBlock x K TileInfo | kWarpsPerBlock x load staging]. */
 template <int P, int K, bool THREADED = true>
@@ -1664,16 +1679,20 @@ __device__ __forceinline__ void geval_indirect_body(const IndirectArgs &a)
     cx.ring_mask = 0;
     context_set(cx);
     for (uint32_t g = blockIdx.x * kWarpsPerBlock + warp; g < a.grid_dim; g += gridDim.x * kWarpsPerBlock) {
-        const IndirectEntry e = a.table[g];
-        __syncwarp();  // every lane is done with the previous program's code and descriptors
-        if (e.n_slots == 0) continue;   // warp-uniform: the entry belongs to the whole warp
-        stage_for_warp(code_s, e.code, e.n_slots, ti_s, e.ti, lane);
-        if (e.patch_slot) {
-            if (lane == 0) ti_s->base_ptr[e.patch_slot - 1u] = (int64_t)e.patch_ptr;
+        uint32_t n_slots;
+        if (a.raw) {
+            const uint32_t n = a.raw_count[g];
+            __syncwarp();  // every lane is done with the previous program's code and descriptors
+            if (n == 0) continue;   // warp-uniform
+            n_slots = stage_raw_for_warp(code_s, a.raw + (size_t)g * a.raw_stride, n, ti_s, a.raw_ti, a.out_slot, a.out_base + (u64)g * a.out_stride, lane);
+        } else {
+            const IndirectEntry e = a.table[g];
             __syncwarp();
+            n_slots = e.n_slots;
+            stage_for_warp(code_s, e.code, n_slots, ti_s, e.ti, lane);
         }
         decode_tiles<1>(ti_s, (int)a.n_tensors, g, a.grid_dim, cx.tiles, lane);
-        interpret<P, 1, false>(code_s, e.n_slots);
+        interpret<P, 1, false>(code_s, n_slots);
     }
 }
 

@@ -81,9 +81,8 @@ struct LaunchArgs {
 struct IndirectEntry {
     const uint2 *code;              // pre-decoded program of this logical program
     const gint_tensor_info *ti;     // its descriptor block in device memory
-    uint32_t n_slots;               // entries in `code`; 0: nothing to run (an invalid candidate of a batch)
-    uint32_t patch_slot;            // 1 + tensor slot whose base pointer is replaced by patch_ptr for this logical program; 0: none
-    u64 patch_ptr;                  // (batches of candidate programs share one descriptor block and differ in one pointer)
+    uint32_t n_slots;               // entries in `code`
+    uint32_t reserved;
 };
 
 
@@ -93,6 +92,37 @@ struct IndirectArgs {
     uint32_t grid_dim;
     uint32_t code_smem_bytes; // shared-memory bytes reserved per warp for its program
     uint32_t reserved;        // always 0; doubles as the zero the assembler cannot see (fma_barrier in gint_interp.cuh)
+    /* batches of candidate programs (raw != nullptr, no table): the caller's words, which a warp makes into its stream itself */
+    const int2 *raw;          // {opcode, operand}, raw_stride of them per candidate
+    const uint32_t *raw_count; // instructions including the Halt; 0: an invalid candidate
+    const gint_tensor_info *raw_ti; // the one descriptor block
+    uint32_t raw_stride;
+    uint32_t out_slot;        // tensor slot whose base pointer moves on by out_stride bytes per candidate
+    u64 out_base, out_stride;
 };
+
+/* The operand word of an instruction as the kernels want it: lane selectors clamped to 0 .. 3 (what the reference's compare tree computes
+ * for any operand, gint/kernel/interpreter/instructions/move.py:58-66). */
+__host__ __device__ inline uint32_t stream_operand(int op, uint32_t operand)
+{
+    if (op == OP_DupBroadcastW) return (int)operand < 0 ? 0u : (int)operand > 3 ? 3u : operand;
+    if (op != OP_FPermW && op != OP_FShuf2) return operand;
+    uint32_t r = 0;
+    for (int w = 0; w < 4; w++) {
+        const uint32_t b = (operand >> (8 * w)) & 0xFFu;
+        r |= (b > 3u ? 3u : b) << (8 * w);
+    }
+    return r;
+}
+/* Entry i of the stream of a program of n instructions (n - 1 of them and a Halt): the previous instruction's operand, this one's opcode; two
+ * entries behind the Halt, and one more where their number is odd. */
+__host__ __device__ inline uint32_t stream_entries(uint32_t n) { return (n + 3u) & ~1u; }
+__host__ __device__ inline uint2 stream_entry(const int2 *raw, uint32_t n, uint32_t i)
+{
+    uint2 e;
+    e.x = i > 0 && i < n ? stream_operand(raw[i - 1].x, (uint32_t)raw[i - 1].y) : 0u;
+    e.y = i + 1 < n ? (uint32_t)raw[i].x : (uint32_t)OP_Halt;
+    return e;
+}
 
 }  // namespace gint
