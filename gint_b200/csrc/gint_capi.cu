@@ -955,7 +955,7 @@ KernelImage g_images[] = {
 #define GINT_X_IMG(P) {gint_cubin_checked_##P, gint_cubin_checked_##P##_end, "gint_geval_checked_" #P, P, -1, nullptr, nullptr, false, false},
     GINT_CHECKED_VARIANTS(GINT_X_IMG)
 #undef GINT_X_IMG
-#define GINT_X_IMG(name, form) {gint_cubin_##name, gint_cubin_##name##_end, "gint_form_" #name, form, -2, nullptr, nullptr, false, false},
+#define GINT_X_IMG(file, name, index) {gint_cubin_##file, gint_cubin_##file##_end, "gint_form_" #name, index, -2, nullptr, nullptr, false, false},
     GINT_FORM_KERNELS(GINT_X_IMG)
 #undef GINT_X_IMG
 };
@@ -1448,7 +1448,7 @@ int choose_rows(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, u
     a.count = count;
     a.depth = plan.depth;
     a.grid.simple = a.grid.n_dims == 1 && first + count <= a.grid.size[0];
-    l->kernel = plan.team == 4 ? 1 : 0;
+    l->kernel = rows_kernel(a) + (plan.team == 4);
     l->grid = plan.grid;
     l->threads = plan.teams * plan.team * 32u;
     l->smem = plan.smem;

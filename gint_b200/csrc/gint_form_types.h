@@ -60,6 +60,16 @@ template <int N> __host__ __device__ inline void form_offsets(const FormGrid &g,
 enum { ROWS_SUM = 0, ROWS_SUM_SQUARES, ROWS_FMA_SQUARES };
 enum { ROWS_X = 0, ROWS_W, ROWS_R, ROWS_Z, ROWS_N_SLOTS };
 enum { ROWS_MAP = 1, ROWS_MAP_W = 2, ROWS_MAP_SILU = 4, ROWS_MAP_R = 8 };
+enum { STEPS_ANY = 0, STEPS_TOTAL, STEPS_TOTAL_THEN, STEPS_MEAN };   // the sum over lanes and width values: alone; and steps on single values; and FMulImm, FAddImm, FRSqrt
+/* shapes that have kernels of their own: X(name, reduction, map, steps); the last kernels run any */
+#define GINT_ROWS_SHAPES(X)                                                                                        \
+    X(norm, ROWS_SUM_SQUARES, ROWS_MAP | ROWS_MAP_W, STEPS_MEAN)                                                   \
+    X(norm_silu_add, ROWS_SUM_SQUARES, ROWS_MAP | ROWS_MAP_W | ROWS_MAP_SILU | ROWS_MAP_R, STEPS_MEAN)             \
+    X(sum, ROWS_SUM, 0, STEPS_TOTAL)                                                                               \
+    X(any, -1, -1, STEPS_ANY)
+#define GINT_X_SHAPE(name, r, m, s) struct Rows_##name { static constexpr int reduce = r, map = m, steps = s; };
+GINT_ROWS_SHAPES(GINT_X_SHAPE)
+#undef GINT_X_SHAPE
 constexpr int kRowsSteps = 12;
 constexpr uint32_t kRowsFold = 0x80;   // step: Dup, FPermW (operand), FAdd
 
@@ -71,7 +81,8 @@ struct RowsArgs {
     uint32_t reduce, map;            // ROWS_SUM ...; 0 or a set of ROWS_MAP...
     float init, silu;
     int store_at;                    // without a map: the running value is stored as a tile at this element
-    uint32_t n_steps, mean;          // mean: the steps are the sum over lanes and width values, FMulImm, FAddImm, FRSqrt
+    uint32_t n_steps;
+    uint32_t steps;                  // STEPS_...
     uint32_t step[kRowsSteps], operand[kRowsSteps];
     uint32_t depth, stage_bytes, stationary_bytes;
 };

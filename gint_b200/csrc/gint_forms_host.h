@@ -129,8 +129,11 @@ bool rows_steps(const std::vector<Insn> &p, size_t from, size_t to, gint::RowsAr
         a->step[a->n_steps] = step;
         a->operand[a->n_steps++] = operand;
     }
-    a->mean = a->n_steps == 6 && a->step[0] == OP_WarpAllReduceSum && a->step[1] == gint::kRowsFold && a->operand[1] == 0x01000302u &&
-              a->step[2] == gint::kRowsFold && a->operand[2] == 0x02030001u && a->step[3] == OP_FMulImm && a->step[4] == OP_FAddImm && a->step[5] == OP_FRSqrt;
+    bool total = a->n_steps >= 3 && a->step[0] == OP_WarpAllReduceSum && a->step[1] == gint::kRowsFold && a->operand[1] == 0x01000302u &&
+                 a->step[2] == gint::kRowsFold && a->operand[2] == 0x02030001u;
+    for (uint32_t k = 3; k < a->n_steps; k++) total = total && a->step[k] != OP_WarpAllReduceSum && a->step[k] != gint::kRowsFold;
+    const bool mean = total && a->n_steps == 6 && a->step[3] == OP_FMulImm && a->step[4] == OP_FAddImm && a->step[5] == OP_FRSqrt;
+    a->steps = !total ? gint::STEPS_ANY : mean ? gint::STEPS_MEAN : a->n_steps == 3 ? gint::STEPS_TOTAL : gint::STEPS_TOTAL_THEN;
     return true;
 }
 
@@ -243,28 +246,40 @@ bool match_rows(const std::vector<Insn> &p, const gint_tensor_info &ti, Form *f)
     return true;
 }
 
+/* of GINT_FORM_KERNELS: two per shape, the first of them with one warp per logical program */
+int rows_kernel(const gint::RowsArgs &a)
+{
+    int k = 0;
+#define GINT_X_SHAPE(name, r, m, s)                                                                                                              \
+    if ((gint::Rows_##name::map < 0) || (a.reduce == (uint32_t)gint::Rows_##name::reduce && a.map == (uint32_t)gint::Rows_##name::map && a.steps == (uint32_t)gint::Rows_##name::steps)) return k; \
+    k += 2;
+    using namespace gint;
+    GINT_ROWS_SHAPES(GINT_X_SHAPE)
+#undef GINT_X_SHAPE
+    return k - 2;
+}
+
 /*
  * Team size, teams per block and stages per team. An SM's shared memory holds as many rows as fit, at least two per team (one
  * computed, the others on their way), and there are no more teams than rows. Measured (one B200, us, cold buffers; one warp per row /
  * four / the interpreter):
- *   many warps of one row each are the fastest where 12 of them have their two stages: RMSNorm 100 000 x 700 109 / 174 / 190,
- *   60 000 x 1025 89 / 126 / 181; silu(rmsnorm) + residual 65 536 x 1024 137 / 158 / 195. Longer rows leave too few warps, and
- *   four share a row: RMSNorm 16384 x 4096 101 / 97 / 119, silu 12 000 x 4095 176 / 110 / 220, 38 000 x 1301 150 / 142 / 216;
- *   so do they where there are at most two rows per SM: silu 100 x 1024 17 / 13 / 26. More than 24 warps or 8 teams gain nothing.
- * Left to the interpreter: sums of short rows in large launches (100 000 x 512 65 here, 56 there; 60 000 x 768 49 and 50;
- * 5000 x 300 12.3 and 13.4), whose rows are read once and all of whose work is the reduction; SiLU with one team per SM (8000 x 8192 213
- * here, 187 there); rows of which two and the stationary ones do not fit (RMSNorm of 20 000 values).
+ *   many warps of one row each are the fastest where 12 of them have their two stages: RMSNorm 100 000 x 700 104 / 174 / 188,
+ *   60 000 x 1025 92 / 126 / 182; silu(rmsnorm) + residual 65 536 x 1024 139 / 158 / 180. Longer rows leave too few warps, and
+ *   four share a row: RMSNorm 16384 x 4096 101 / 96 / 119, silu 12 000 x 4095 176 / 106 / 221, 38 000 x 1301 150 / 139 / 219;
+ *   so do they where there are at most two rows per SM: silu 100 x 1024 17 / 13 / 26. Rows of two or three tiles gain up to 32 warps
+ *   (600 000 x 129: 335 with 16, 236 with 24, 225); more than 8 teams of four gain nothing.
+ * Left to the interpreter: SiLU with one team per SM (8000 x 8192 213 here, 187 there); rows of which two and the stationary ones
+ * do not fit (RMSNorm of 20 000 values).
  */
 struct RowsPlan { uint32_t team, teams, depth, grid, smem; };
 bool plan_rows(const gint::RowsArgs &a, uint32_t count, int sms, int max_smem, RowsPlan *plan)
 {
     const uint32_t exchange = 1024u, barriers = 32u;   // per team
-    if (!a.map && a.tiles < 6 && count > 32u * (uint32_t)sms) return false;
     if ((uint64_t)a.stationary_bytes + 16u + 2ull * a.stage_bytes + exchange + barriers > (uint64_t)max_smem) return false;
     const uint32_t room = (uint32_t)max_smem - a.stationary_bytes - 16u;
     uint32_t t = (count + (uint32_t)sms - 1) / (uint32_t)sms;
     plan->team = a.tiles >= 4 && (t <= 2 || room / (2u * (a.stage_bytes + 16u)) < 12u) ? 4 : 1;
-    const uint32_t extra = (plan->team > 1 ? exchange : 0u) + barriers, most = plan->team > 1 ? 8 : 24;
+    const uint32_t extra = (plan->team > 1 ? exchange : 0u) + barriers, most = plan->team > 1 ? 8 : 32;
     if (t > most) t = most;
     while (t > 1 && t * (2 * a.stage_bytes + extra) > room) t--;
     if ((a.map & gint::ROWS_MAP_SILU) && t == 1 && count > 2u * (uint32_t)sms) return false;
@@ -286,7 +301,7 @@ struct LaneCode { const int (*code)[2]; int n; };
 #define GINT_X_LANE(name) {gint::LaneCode_##name::code, gint::LaneCode_##name::n},
 const LaneCode kLanePrograms[] = {GINT_LANE_PROGRAMS(GINT_X_LANE)};
 #undef GINT_X_LANE
-constexpr int kLaneKernelFirst = 2;   // of GINT_FORM_KERNELS
+constexpr int kLaneKernelFirst = 8;   // of GINT_FORM_KERNELS
 
 bool match_lanes(const std::vector<Insn> &p, const gint_tensor_info &ti, int n_tensors, int pool_size, Form *f)
 {
@@ -344,7 +359,7 @@ bool plan_lanes(const Form &f, uint32_t count, int sms, int max_smem, FormLaunch
  * Normalisation of short bfloat16 rows, four per logical program (2DT tiles): a sum of squares by fma over two to four tiles of x, times a
  * factor plus an addend, 1 / sqrt, and y = (that * x) * w, w being one row for all.
  */
-constexpr int kHeadsKernelFirst = 4;   // of GINT_FORM_KERNELS: rows of two tiles
+constexpr int kHeadsKernelFirst = 10;   // of GINT_FORM_KERNELS: rows of two tiles
 
 bool match_heads(const std::vector<Insn> &p, const gint_tensor_info &ti, Form *f)
 {
@@ -429,7 +444,7 @@ void sort_digits(gint::HeadsArgs *a)
 
 
 /* [silu](x) [+ y | * y] as one flat loop (WideStream::flat_tiles) over slots of one length and type, from element 0 on. */
-constexpr int kFlatKernelFirst = 8;   // of GINT_FORM_KERNELS: f32, f16, bf16
+constexpr int kFlatKernelFirst = 14;   // of GINT_FORM_KERNELS: f32, f16, bf16
 
 bool match_flat(const WideStream &ws, const gint_tensor_info &ti, Form *f)
 {

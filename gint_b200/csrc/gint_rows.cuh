@@ -15,12 +15,13 @@
  *   - A team is one warp where enough of them have room for their stages, else four warps that take a width value each and share
  *     the row's stages (plan_rows in gint_forms_host.h has both sides).
  *
- * Measured (one B200, us per pass among others, interpreter -> here): RMSNorm 16384 x 4096 122 -> 97 (5.6 TB/s), 10007 x 2029 55 -> 33,
- * 100 000 x 700 190 -> 109, 600 000 x 129 556 -> 275, 148 x 4096 19 -> 9; silu(rmsnorm) + residual of gathered rows 65536 x 1024
- * 195 -> 137 (5.9 TB/s), 12 000 x 4095 220 -> 110; sums of 65536 rows of 1024 67 -> 61, of 12 000 rows of 4095 62 -> 46. Long rows are
- * bound by memory, rows of a few tiles by issue (about 280 warp instructions per row of two tiles, most of them the reduction and
- * the masked ends). What mattered, on the way there: a row's fixed cost (copies by every thread with cp.async 42 -> 37 on the
- * 2029s, steps in a loop over a switch 50 -> 38), the quotient of SiLU (gint_silu.cuh; 155 -> 137), the number of rows on their way.
+ * Measured (one B200, us per pass among others, interpreter -> here): RMSNorm 16384 x 4096 122 -> 96 (5.6 TB/s), 10007 x 2029 55 -> 33,
+ * 100 000 x 700 188 -> 104, 600 000 x 129 558 -> 225, 148 x 4096 19 -> 9; silu(rmsnorm) + residual of gathered rows 65536 x 1024
+ * 180 -> 139 (5.9 TB/s), 12 000 x 4095 221 -> 106; sums of 65536 rows of 1024 66 -> 59, of 12 000 rows of 4095 62 -> 45, of 150 000 rows of 300
+ * 80 -> 53. Long rows are bound by memory, rows of a few tiles by issue. What mattered, on the way there: a row's fixed cost (copies by
+ * every thread with cp.async 42 -> 37 on the 2029s, steps in a loop over a switch 50 -> 38), the quotient of SiLU (gint_silu.cuh;
+ * 155 -> 137), the number of rows on their way, and how much code lies between one row and the next: the usual shapes have kernels of their
+ * own (GINT_ROWS_SHAPES), the one kernel for all of them was slower on short rows (600 000 x 129 285 with it, 236; sums of 300 93, 53).
  */
 #pragma once
 
@@ -113,53 +114,14 @@ template <int TEAM> struct Team {
     }
 };
 
-/* what stands between the loops: instructions on the one value of the stack, as the interpreter executes them */
-template <int TEAM> __device__ __forceinline__ void rows_steps(const RowsArgs &a, Team<TEAM> &team, float (&s)[4 / TEAM])
+/* steps from `from` on that work on every value by itself, up to one that does not: what stands between the loops are instructions on
+ * the one value of the stack, as the interpreter executes them. Returns the first step not done. */
+template <int N> __device__ __forceinline__ uint32_t rows_each(const RowsArgs &a, uint32_t from, float (&s)[N])
 {
-    constexpr int N = 4 / TEAM;
-    if (a.mean) {   // the usual steps: total of the row, times a factor, plus epsilon, 1 / sqrt
-#pragma unroll
-        for (int m = 16; m >= 1; m >>= 1)
-#pragma unroll
-            for (int w = 0; w < N; w++) s[w] = __fadd_rn(s[w], __shfl_xor_sync(0xffffffffu, s[w], m));
-        float v[4];
-        if constexpr (TEAM == 1) {
-#pragma unroll
-            for (int w = 0; w < 4; w++) v[w] = s[w];
-        } else {
-            team.exchange_all(s, v);
-        }
-        /* every lane has the same four values, and the two foldings give every one of them the same total */
-        const float total = __fadd_rn(__fadd_rn(v[0], v[2]), __fadd_rn(v[1], v[3]));
-        const float f = rsqrtf(__fadd_rn(__fmul_rn(total, __uint_as_float(a.operand[3])), __uint_as_float(a.operand[4])));
-#pragma unroll
-        for (int w = 0; w < N; w++) s[w] = f;
-        return;
-    }
-    for (uint32_t k = 0; k < a.n_steps; k++) {
+    for (uint32_t k = from; k < a.n_steps; k++) {
         const uint32_t operand = a.operand[k];
         const float imm = __uint_as_float(operand);
         switch (a.step[k]) {
-        case kRowsFold:
-        {
-            float v[4];
-            if constexpr (TEAM == 1) {
-#pragma unroll
-                for (int w = 0; w < 4; w++) v[w] = s[w];
-            } else {
-                team.exchange_all(s, v);
-            }
-            const uint32_t sel = operand >> (8 * N * (team.thread >> 5));
-#pragma unroll
-            for (int w = 0; w < N; w++) s[w] = __fadd_rn(s[w], rows_pick(v, (sel >> (8 * w)) & 3u));
-        }
-            break;
-        case OP_WarpAllReduceSum:
-#pragma unroll
-            for (int m = 16; m >= 1; m >>= 1)
-#pragma unroll
-                for (int w = 0; w < N; w++) s[w] = __fadd_rn(s[w], __shfl_xor_sync(0xffffffffu, s[w], m));
-            break;
         case OP_FAddImm:
 #pragma unroll
             for (int w = 0; w < N; w++) s[w] = __fadd_rn(s[w], imm);
@@ -190,6 +152,53 @@ template <int TEAM> __device__ __forceinline__ void rows_steps(const RowsArgs &a
 #pragma unroll
             for (int w = 0; w < N; w++) s[w] = __frcp_rn(s[w]);
             break;
+        default: return k;
+        }
+    }
+    return a.n_steps;
+}
+template <int TEAM, int STEPS> __device__ __forceinline__ void rows_steps(const RowsArgs &a, Team<TEAM> &team, float (&s)[4 / TEAM])
+{
+    constexpr int N = 4 / TEAM;
+    if (STEPS != STEPS_ANY || a.steps != STEPS_ANY) {   // the usual beginning: the sum over lanes and width values, which is one value for all
+        float v[4];
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1)
+#pragma unroll
+            for (int w = 0; w < N; w++) s[w] = __fadd_rn(s[w], __shfl_xor_sync(0xffffffffu, s[w], m));
+        if constexpr (TEAM == 1) {   // (reducing the four together takes 8 shuffles instead of 20, but three more in a row: 100 000 x 512 97 -> 104 us)
+#pragma unroll
+            for (int w = 0; w < 4; w++) v[w] = s[w];
+        } else {
+            team.exchange_all(s, v);
+        }
+        /* every lane has the same four values, and the two foldings give every one of them the same total */
+        const float t = __fadd_rn(__fadd_rn(v[0], v[2]), __fadd_rn(v[1], v[3]));
+        float one[1] = {t};
+        if (STEPS == STEPS_MEAN || (STEPS == STEPS_ANY && a.steps == STEPS_MEAN)) one[0] = rsqrtf(__fadd_rn(__fmul_rn(t, __uint_as_float(a.operand[3])), __uint_as_float(a.operand[4])));
+        else if (STEPS == STEPS_ANY) rows_each<1>(a, 3u, one);
+#pragma unroll
+        for (int w = 0; w < N; w++) s[w] = one[0];
+        return;
+    }
+    for (uint32_t k = rows_each<N>(a, 0u, s); k < a.n_steps; k = rows_each<N>(a, k + 1u, s)) {
+        const uint32_t operand = a.operand[k];
+        if (a.step[k] == kRowsFold) {   // Dup, FPermW, FAdd
+            float v[4];
+            if constexpr (TEAM == 1) {
+#pragma unroll
+                for (int w = 0; w < 4; w++) v[w] = s[w];
+            } else {
+                team.exchange_all(s, v);
+            }
+            const uint32_t sel = operand >> (8 * N * (team.thread >> 5));
+#pragma unroll
+            for (int w = 0; w < N; w++) s[w] = __fadd_rn(s[w], rows_pick(v, (sel >> (8 * w)) & 3u));
+        } else {                        // WarpAllReduceSum
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1)
+#pragma unroll
+                for (int w = 0; w < N; w++) s[w] = __fadd_rn(s[w], __shfl_xor_sync(0xffffffffu, s[w], m));
         }
     }
 }
@@ -272,7 +281,8 @@ __device__ __forceinline__ void rows_map(const RowsArgs &a, const float *x, cons
 
 /* Shared memory: [stationary rows | per team: `depth` stages | teams of more than one warp: exchange areas | barriers: one of the
  * stationary rows, per team one per stage]. */
-template <int TEAM> __device__ __forceinline__ void rows_body(const RowsArgs &a)
+/* SHAPE: RowsAny, or a program's shape at compile time -- less code between one row and the next (plan in gint_forms_host.h) */
+template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const RowsArgs &a)
 {
     constexpr int N = 4 / TEAM;
     const uint32_t teams = blockDim.x / (TEAM * 32);
@@ -346,17 +356,19 @@ template <int TEAM> __device__ __forceinline__ void rows_body(const RowsArgs &a)
 #pragma unroll
         for (int i = 0; i < N; i++) s[i] = a.init;
         const int left = a.slot[ROWS_X].n - at;
-        if (a.reduce == ROWS_SUM) rows_reduce<ROWS_SUM, N>(a, in[ROWS_X], left, s);
+        if constexpr (SHAPE::reduce >= 0) rows_reduce<SHAPE::reduce, N>(a, in[ROWS_X], left, s);
+        else if (a.reduce == ROWS_SUM) rows_reduce<ROWS_SUM, N>(a, in[ROWS_X], left, s);
         else if (a.reduce == ROWS_SUM_SQUARES) rows_reduce<ROWS_SUM_SQUARES, N>(a, in[ROWS_X], left, s);
         else rows_reduce<ROWS_FMA_SQUARES, N>(a, in[ROWS_X], left, s);
-        rows_steps<TEAM>(a, team, s);
-        switch (a.map) {
+        rows_steps<TEAM, SHAPE::steps>(a, team, s);
+        if constexpr (SHAPE::map > 0) rows_map<SHAPE::map, N>(a, in[ROWS_X], in[ROWS_W], in[ROWS_R], z, at, s);
+        else switch (SHAPE::map == 0 ? 0u : a.map) {
         case 0:
 #pragma unroll
             for (int i = 0; i < N; i++)
                 if (a.store_at + i * 32 < a.slot[ROWS_Z].n - at) z[a.store_at + i * 32] = s[i];
             break;
-#define GINT_ROWS_MAP(m) case ROWS_MAP | (m): rows_map<ROWS_MAP | (m), N>(a, in[ROWS_X], in[ROWS_W], in[ROWS_R], z, at, s); break;
+#define GINT_ROWS_MAP(m) case ROWS_MAP | (m): if constexpr (SHAPE::map < 0) rows_map<ROWS_MAP | (m), N>(a, in[ROWS_X], in[ROWS_W], in[ROWS_R], z, at, s); break;
         GINT_ROWS_MAP(0)
         GINT_ROWS_MAP(ROWS_MAP_W)
         GINT_ROWS_MAP(ROWS_MAP_R)
@@ -380,3 +392,8 @@ template <int TEAM> __device__ __forceinline__ void rows_body(const RowsArgs &a)
 }
 
 }  // namespace gint
+
+/* one warp per logical program (24 of them per block hold 80 registers each), and four */
+#define GINT_DEFINE_ROWS_KERNELS(shape)                                                                                                          \
+    extern "C" __global__ void __launch_bounds__(1024) gint_form_rows1_##shape(const __grid_constant__ gint::RowsArgs a) { gint::rows_body<1, gint::Rows_##shape>(a); } \
+    extern "C" __global__ void __launch_bounds__(1024) gint_form_rows4_##shape(const __grid_constant__ gint::RowsArgs a) { gint::rows_body<4, gint::Rows_##shape>(a); }

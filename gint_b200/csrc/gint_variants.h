@@ -18,10 +18,14 @@ extern "C" {
 #define GINT_WIDEV_VARIANTS(X) X(3, 8) X(4, 4)  /* ... in the vector layout */
 #define GINT_INDIRECT_VARIANTS(X) X(12)
 #define GINT_CHECKED_VARIANTS(X) X(12)
-/* kernels of program forms (gint_forms_host.h): X(source and kernel name, index) */
-#define GINT_FORM_KERNELS(X) X(rows_f32, 0) X(rows4_f32, 1) X(lanes_bmm4x4, 2) X(lanes_inv4x4, 3) X(heads_bf16_2, 4) X(heads_bf16_3, 5) X(heads_bf16_4, 6) X(heads_bf16_fours, 7) \
-    X(flat_f32, 8) X(flat_f16, 9) X(flat_bf16, 10)
-#define GINT_N_FORM_KERNELS 11
+/* kernels of program forms (gint_forms_host.h), and the files that they are in: X(file, kernel name, index) */
+#define GINT_FORM_KERNELS(X)                                                                                                    \
+    X(rows_norm, rows1_norm, 0) X(rows_norm, rows4_norm, 1) X(rows_norm_silu_add, rows1_norm_silu_add, 2)                        \
+    X(rows_norm_silu_add, rows4_norm_silu_add, 3) X(rows_sum, rows1_sum, 4) X(rows_sum, rows4_sum, 5) X(rows_any, rows1_any, 6)   \
+    X(rows_any, rows4_any, 7) X(lanes_bmm4x4, lanes_bmm4x4, 8) X(lanes_inv4x4, lanes_inv4x4, 9) X(heads_bf16, heads_bf16_2, 10)    \
+    X(heads_bf16, heads_bf16_3, 11) X(heads_bf16, heads_bf16_4, 12) X(heads_bf16, heads_bf16_fours, 13) X(flat_f32, flat_f32, 14) \
+    X(flat_f16, flat_f16, 15) X(flat_bf16, flat_bf16, 16)
+#define GINT_N_FORM_KERNELS 17
 
 #define GINT_X_DECL(P, K)                                        \
     extern const unsigned char gint_cubin_direct_##P##_##K[];     \
@@ -59,9 +63,9 @@ GINT_INDIRECT_VARIANTS(GINT_X_DECL)
 GINT_CHECKED_VARIANTS(GINT_X_DECL)
 #undef GINT_X_DECL
 
-#define GINT_X_DECL(name, form)                          \
-    extern const unsigned char gint_cubin_##name[];       \
-    extern const unsigned char gint_cubin_##name##_end[];
+#define GINT_X_DECL(file, name, index)                   \
+    extern const unsigned char gint_cubin_##file[];       \
+    extern const unsigned char gint_cubin_##file##_end[];
 GINT_FORM_KERNELS(GINT_X_DECL)
 #undef GINT_X_DECL
 

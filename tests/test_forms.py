@@ -121,9 +121,7 @@ def test_what_a_launch_on_the_form_needs():
         assert form(pd, bases, count=64)[0] == want                                               # what is stored is read by no other logical program
     assert form(pd, FAR, first=(1 << 31) - 60, count=64)[0] == 0                                  # logical programs are counted in 31 bits
     assert form(program(n=20000), FAR, count=64)[0] == 0                                          # two rows and the weights in shared memory
-    assert form(program(rows=4736, n=640, scale=False), FAR, count=4736)[0] == ROWS               # short rows: only few sums
-    assert form(program(rows=4737, n=640, scale=False), FAR, count=4737)[0] == 0
-    assert form(program(rows=4737, n=641, scale=False), FAR, count=4737)[0] == ROWS
+    assert form(program(rows=100000, n=300, scale=False), FAR, count=100000)[0] == ROWS           # sums, however short and many
     assert form(program(n=8192, silu=True, add=True), FAR, count=296)[0] == ROWS                  # one team per SM
     assert form(program(n=8192, silu=True, add=True), FAR, count=297)[0] == 0
 
@@ -369,11 +367,12 @@ def runs_on_form(program_, tensors, rows, **kw):
     return get_executor().launch_info(program_, C.to_interfaces(tensors), rows, **kw)["form"] == ROWS
 
 
+KEPT = []
 SHAPES = [(1, 129), (3, 255), (700, 256), (5, 257), (40, 384), (7, 513), (300, 1000), (33, 1024), (2000, 1025), (9, 2029), (400, 2304), (20, 4095), (150, 4096), (5, 6001), (3, 9000)]
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kw", [{}, {"silu": True, "add": True}, {"silu": True, "c": 0.5}, {"add": True, "reduce": "fma"}, {"reduce": "sum", "steps": "others"}, {"scale": False},
+@pytest.mark.parametrize("kw", [{}, {"silu": True, "add": True}, {"silu": True, "c": 0.5}, {"add": True, "reduce": "fma"}, {"reduce": "sum", "steps": "others"}, {"scale": False}, {"reduce": "sum", "steps": "total", "scale": False},
                                 {"scale": False, "reduce": "sum", "first": "zero"}, {"steps": "none"}], ids=str)
 def test_rows_give_the_bits_of_the_interpreter(kw):
     """Row lengths around whole tiles and groups of tiles, one and four warps per row, rows and base pointers at any element."""
@@ -454,6 +453,7 @@ def test_rows_in_a_graph_and_on_few_blocks():
     m.rmsnorm(x, w, z, grid_dim=500)
     want = z.clone()
     graph = torch.cuda.CUDAGraph()
+    KEPT.append(graph)      # (torch allocates its capture state with the first graph alive and frees it with the last: other tests count allocations)
     with torch.cuda.graph(graph):
         m.rmsnorm(x, w, z, grid_dim=500, cuda_stream=torch.cuda.current_stream().cuda_stream)
     z.zero_()
