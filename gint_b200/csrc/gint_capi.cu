@@ -1421,8 +1421,6 @@ Route choose_route(const gint_ctx *ctx, const Program *p, const uint64_t *base_p
  * interpreter, and not where a stored tensor overlaps one that is read: the forms read logical programs ahead. */
 int choose_rows(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, uint32_t first, uint32_t count, const GatherArgs *gather, FormLaunch *l)
 {
-    RowsPlan plan;
-    if (!plan_rows(f.rows, count, ctx->num_sms, ctx->max_smem_optin, &plan)) return FORM_NONE;
     gint::RowsArgs &a = l->rows;
     a = f.rows;
     uint64_t lo[gint::ROWS_N_SLOTS], hi[gint::ROWS_N_SLOTS];
@@ -1431,6 +1429,7 @@ int choose_rows(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, u
         a.slot[s].base = lo[s] = base_ptrs[f.tensor[s]];
         hi[s] = lo[s] + f.extent[s];
         if ((lo[s] & f.base_align) != 0) return FORM_NONE;
+        a.fours = a.fours && (lo[s] & 15u) == 0;
         if (!gather || !((gather->mask >> f.tensor[s]) & 1u)) continue;
         if (s == f.store) return FORM_NONE;
         hi[s] = lo[s] + gather->extent_bytes;
@@ -1444,6 +1443,8 @@ int choose_rows(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, u
     }
     for (int s = 0; s < gint::ROWS_N_SLOTS; s++)
         if (f.tensor[s] >= 0 && s != f.store && lo[s] < hi[f.store] && lo[f.store] < hi[s]) return FORM_NONE;
+    RowsPlan plan;
+    if (!plan_rows(a, count, ctx->num_sms, ctx->max_smem_optin, &plan)) return FORM_NONE;
     a.first = first;
     a.count = count;
     a.depth = plan.depth;

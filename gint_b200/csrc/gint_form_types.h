@@ -70,6 +70,12 @@ enum { STEPS_ANY = 0, STEPS_TOTAL, STEPS_TOTAL_THEN, STEPS_MEAN };   // the sum 
 #define GINT_X_SHAPE(name, r, m, s) struct Rows_##name { static constexpr int reduce = r, map = m, steps = s; };
 GINT_ROWS_SHAPES(GINT_X_SHAPE)
 #undef GINT_X_SHAPE
+struct RowsShape { bool fours; };
+constexpr RowsShape kRowsShapes[] = {
+#define GINT_X_SHAPE(name, r, m, s) {(m) > 0 && (s) == STEPS_MEAN},   // has a pass of four elements at a time
+    GINT_ROWS_SHAPES(GINT_X_SHAPE)
+#undef GINT_X_SHAPE
+};
 constexpr int kRowsSteps = 12;
 constexpr uint32_t kRowsFold = 0x80;   // step: Dup, FPermW (operand), FAdd
 
@@ -85,6 +91,7 @@ struct RowsArgs {
     uint32_t steps;                  // STEPS_...
     uint32_t step[kRowsSteps], operand[kRowsSteps];
     uint32_t depth, stage_bytes, stationary_bytes;
+    uint32_t fours;                  // every row of every operand starts at a 16-byte boundary; one length, a multiple of four
 };
 
 /* Head programs (gint_heads.cuh): four short rows of bfloat16 elements per logical program, one per width value. */

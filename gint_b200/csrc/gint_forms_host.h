@@ -241,6 +241,12 @@ bool match_rows(const std::vector<Insn> &p, const gint_tensor_info &ti, Form *f)
         a.slot[s].area = area;
         area += (((uint32_t)elements * 4u + 15u) & ~15u) + 16u;   // a row may start anywhere in its first 16 bytes
     }
+    a.fours = a.map != 0 && n[gint::ROWS_Z] % 4 == 0;
+    for (int s = 0; s < gint::ROWS_N_SLOTS; s++) {
+        if (f->tensor[s] < 0) continue;
+        a.fours = a.fours && n[s] == n[gint::ROWS_Z];
+        for (uint32_t stride : a.slot[s].stride) a.fours = a.fours && stride % 4 == 0;
+    }
     a.stage_bytes = stage + 16u;                                  // ... and the stage's note of where its rows start
     f->kind = FORM_ROWS;
     return true;
@@ -260,14 +266,23 @@ int rows_kernel(const gint::RowsArgs &a)
 }
 
 /*
- * Team size, teams per block and stages per team. An SM's shared memory holds as many rows as fit, at least two per team (one
- * computed, the others on their way), and there are no more teams than rows. Measured (one B200, us, cold buffers; one warp per row /
- * four / the interpreter):
- *   many warps of one row each are the fastest where 12 of them have their two stages: RMSNorm 100 000 x 700 104 / 174 / 188,
- *   60 000 x 1025 92 / 126 / 182; silu(rmsnorm) + residual 65 536 x 1024 139 / 158 / 180. Longer rows leave too few warps, and
- *   four share a row: RMSNorm 16384 x 4096 101 / 96 / 119, silu 12 000 x 4095 176 / 106 / 221, 38 000 x 1301 150 / 139 / 219;
- *   so do they where there are at most two rows per SM: silu 100 x 1024 17 / 13 / 26. Rows of two or three tiles gain up to 32 warps
- *   (600 000 x 129: 335 with 16, 236 with 24, 225); more than 8 teams of four gain nothing.
+ * Team size, teams per block and stages per team; every team has two to four stages (one computed, the others on their way), and there are no
+ * more teams than rows. Measured (one B200, us per launch back to back, cold buffers, floor = bytes at 6557 GB/s):
+ *
+ * A pass that only scales is bound by memory, and memory serves it best with about 100 KB of rows per SM staged, two or three per team: more
+ * rows at once are more pages read and written in turn. RMSNorm 16384 x 4096 86 with 98 KB, 91 with 197 KB (floor 82), 30 000 x 2048 78 and
+ * 88 (75), 20 000 x 3072 78 and 85 (75), 13 000 x 6000 102 and 107 (95), 40 000 x 1536 78 and 93 (75), 60 000 x 1025 80 and 94 (75); one warp
+ * per row of aligned rows 90 KB (100 000 x 768 101 with 74 KB, 110 with 98 KB, 100 000 x 700 94 with 90 KB, 102 with 112 KB).
+ * Four warps per row from 1400 elements on (40 000 x 1535 one warp 91, four 80; 60 000 x 1025 80 and 104), four elements at a time from
+ * 1000 on (60 000 x 1024 80 and 77; 80 000 x 900 94 and 103).
+ *
+ * SiLU is bound by issue: as many warps as have two stages, a multiple of four of them (one per scheduler and round: 65536 x 1024 118 with
+ * 12, 129 with 13), one per row where that makes eight of them, or twelve if they go one element at a time (30 000 x 1536 88 with 8, four
+ * per row 98; 38 000 x 1301 150 with 8, four per row 136; 12 000 x 4096 four per row 85, one 140).
+ *
+ * Sums: all the warps that have two stages. Rows of two or three tiles gain up to 32 warps (RMSNorm 600 000 x 129 335 with 16, 236 with 24,
+ * 225) and up to four stages (300 000 x 256 104 with two, 98). At most two rows per SM: four warps per row (silu 100 x 1024 13, one warp 17).
+ *
  * Left to the interpreter: SiLU with one team per SM (8000 x 8192 213 here, 187 there); rows of which two and the stationary ones
  * do not fit (RMSNorm of 20 000 values).
  */
@@ -276,22 +291,34 @@ bool plan_rows(const gint::RowsArgs &a, uint32_t count, int sms, int max_smem, R
 {
     const uint32_t exchange = 1024u, barriers = 32u;   // per team
     if ((uint64_t)a.stationary_bytes + 16u + 2ull * a.stage_bytes + exchange + barriers > (uint64_t)max_smem) return false;
-    const uint32_t room = (uint32_t)max_smem - a.stationary_bytes - 16u;
-    uint32_t t = (count + (uint32_t)sms - 1) / (uint32_t)sms;
-    plan->team = a.tiles >= 4 && (t <= 2 || room / (2u * (a.stage_bytes + 16u)) < 12u) ? 4 : 1;
-    const uint32_t extra = (plan->team > 1 ? exchange : 0u) + barriers, most = plan->team > 1 ? 8 : 32;
-    if (t > most) t = most;
+    const uint32_t room = (uint32_t)max_smem - a.stationary_bytes - 16u, need = (count + (uint32_t)sms - 1) / (uint32_t)sms;
+    const uint32_t one = room / (2u * a.stage_bytes + barriers);   // teams of one warp that have two stages
+    const bool silu = (a.map & gint::ROWS_MAP_SILU) != 0, scales = a.map && !silu;
+    const bool fours = a.fours && gint::kRowsShapes[rows_kernel(a) / 2].fours;
+    uint32_t row_bytes = 0;   // of a stage
+    for (int s = 0; s < gint::ROWS_Z; s++)
+        if (a.slot[s].n && !a.slot[s].stationary) row_bytes += 4u * ((uint32_t)a.slot[s].n < 128u * a.tiles ? (uint32_t)a.slot[s].n : 128u * a.tiles);
+    bool four;
+    if (a.tiles < 4) four = false;
+    else if (need <= 2) four = true;
+    else if (scales) four = a.slot[gint::ROWS_X].n >= (fours ? 1000 : 1400);
+    else four = one < (silu && fours ? 8u : 12u);
+    plan->team = four ? 4 : 1;
+    const uint32_t extra = (four ? exchange : 0u) + barriers, best = four || !fours ? 100u * 1024u : 90u * 1024u;
+    uint32_t t = need < (four ? 8u : 32u) ? need : four ? 8u : 32u;
+    if (scales && t > 1 && t * 2u * row_bytes > best) t = best / (2u * row_bytes) ? best / (2u * row_bytes) : 1u;
     while (t > 1 && t * (2 * a.stage_bytes + extra) > room) t--;
-    if ((a.map & gint::ROWS_MAP_SILU) && t == 1 && count > 2u * (uint32_t)sms) return false;
-    const uint32_t d = (room - t * extra) / (t * a.stage_bytes);
+    if (!four && a.map && t > 4) t &= ~3u;
+    if (silu && t == 1 && need > 2u) return false;
+    uint32_t d = (room - t * extra) / (t * a.stage_bytes);
+    if (scales && a.tiles > 3 && d > best / (t * row_bytes + 1u)) d = best / (t * row_bytes + 1u);
     plan->teams = t;
-    plan->depth = d > 4 ? 4 : d;
+    plan->depth = d > 4 ? 4 : d < 2 ? 2 : d;
     plan->smem = a.stationary_bytes + 16u + t * (plan->depth * a.stage_bytes + extra);
     const uint32_t blocks = (count + t - 1) / t;
     plan->grid = blocks < (uint32_t)sms ? blocks : (uint32_t)sms;
     return true;
 }
-
 
 /*
  * Lane programs (gint_lanes.cuh): exactly the instructions of a program that was compiled ahead of time, over rows of 16 floats whose accesses

@@ -279,6 +279,48 @@ __device__ __forceinline__ void rows_map(const RowsArgs &a, const float *x, cons
     }
 }
 
+/* The second pass four elements at a time, where s is one value and every row starts at a 16-byte boundary and has a multiple of four elements
+ * (the same number in every operand): tiles go to the team's warps in turn, U of them together. */
+template <int MAP, int TEAM>
+__device__ __forceinline__ void rows_map_fours(const RowsArgs &a, const float *x, const float *wt, const float *r, float *z, int thread, float s)
+{
+    constexpr int U = 2, STEP = TEAM * 128;
+    const int n = min(a.slot[ROWS_Z].n, (int)a.tiles * 128);
+    for (int e = 4 * thread; e < n; e += U * STEP) {
+        float o[4 * U];
+        float4 v[U], g[U], h[U];
+        const bool both = e + STEP < n;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (u > 0 && !both) {
+                v[u] = g[u] = h[u] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+                continue;
+            }
+            v[u] = *reinterpret_cast<const float4 *>(x + e + u * STEP);
+            if constexpr ((MAP & ROWS_MAP_W) != 0) g[u] = *reinterpret_cast<const float4 *>(wt + e + u * STEP);
+            if constexpr ((MAP & ROWS_MAP_R) != 0) h[u] = *reinterpret_cast<const float4 *>(r + e + u * STEP);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            o[4 * u] = __fmul_rn(s, v[u].x); o[4 * u + 1] = __fmul_rn(s, v[u].y); o[4 * u + 2] = __fmul_rn(s, v[u].z); o[4 * u + 3] = __fmul_rn(s, v[u].w);
+            if constexpr ((MAP & ROWS_MAP_W) != 0) {
+                o[4 * u] = __fmul_rn(g[u].x, o[4 * u]); o[4 * u + 1] = __fmul_rn(g[u].y, o[4 * u + 1]);
+                o[4 * u + 2] = __fmul_rn(g[u].z, o[4 * u + 2]); o[4 * u + 3] = __fmul_rn(g[u].w, o[4 * u + 3]);
+            }
+        }
+        if constexpr ((MAP & ROWS_MAP_SILU) != 0) silu(o, a.silu);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (u > 0 && !both) continue;
+            if constexpr ((MAP & ROWS_MAP_R) != 0) {
+                o[4 * u] = __fadd_rn(h[u].x, o[4 * u]); o[4 * u + 1] = __fadd_rn(h[u].y, o[4 * u + 1]);
+                o[4 * u + 2] = __fadd_rn(h[u].z, o[4 * u + 2]); o[4 * u + 3] = __fadd_rn(h[u].w, o[4 * u + 3]);
+            }
+            *reinterpret_cast<float4 *>(z + e + u * STEP) = make_float4(o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
+        }
+    }
+}
+
 /* Shared memory: [stationary rows | per team: `depth` stages | teams of more than one warp: exchange areas | barriers: one of the
  * stationary rows, per team one per stage]. */
 /* SHAPE: RowsAny, or a program's shape at compile time -- less code between one row and the next (plan in gint_forms_host.h) */
@@ -361,7 +403,10 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
         else if (a.reduce == ROWS_SUM_SQUARES) rows_reduce<ROWS_SUM_SQUARES, N>(a, in[ROWS_X], left, s);
         else rows_reduce<ROWS_FMA_SQUARES, N>(a, in[ROWS_X], left, s);
         rows_steps<TEAM, SHAPE::steps>(a, team, s);
-        if constexpr (SHAPE::map > 0) rows_map<SHAPE::map, N>(a, in[ROWS_X], in[ROWS_W], in[ROWS_R], z, at, s);
+        if constexpr (SHAPE::map > 0 && SHAPE::steps == STEPS_MEAN) {
+            if (a.fours) rows_map_fours<SHAPE::map, TEAM>(a, in[ROWS_X] - at, in[ROWS_W] - at, in[ROWS_R] - at, z - at, team.thread, s[0]);
+            else rows_map<SHAPE::map, N>(a, in[ROWS_X], in[ROWS_W], in[ROWS_R], z, at, s);
+        } else if constexpr (SHAPE::map > 0) rows_map<SHAPE::map, N>(a, in[ROWS_X], in[ROWS_W], in[ROWS_R], z, at, s);
         else switch (SHAPE::map == 0 ? 0u : a.map) {
         case 0:
 #pragma unroll

@@ -126,9 +126,11 @@ def test_what_a_launch_on_the_form_needs():
     assert form(program(n=8192, silu=True, add=True), FAR, count=297)[0] == 0
 
 
-@pytest.mark.parametrize("n,rows,warps", [(384, 10, 1), (385, 296, 4), (385, 297, 1), (2200, 5000, 1), (2400, 5000, 4)])
-def test_warps_per_row(n, rows, warps):
-    assert form(program(rows=rows, n=n), FAR, count=rows)[:2] == (ROWS, warps)
+@pytest.mark.parametrize("n,rows,kw,warps", [(384, 10, {}, 1), (385, 296, {}, 4), (385, 297, {}, 1), (996, 5000, {}, 1), (1000, 5000, {}, 4), (1001, 5000, {}, 1), (1399, 5000, {}, 1), (1401, 5000, {}, 4),
+                                             (1000, 5000, {"steps": "others"}, 1), (1536, 5000, {"silu": True, "add": True}, 1), (1537, 5000, {"silu": True, "add": True}, 4),
+                                             (1792, 5000, {"silu": True, "add": True}, 4), (2200, 5000, {"scale": False}, 1), (2600, 5000, {"scale": False}, 4)])
+def test_warps_per_row(n, rows, kw, warps):
+    assert form(program(rows=rows, n=n, **kw), FAR, count=rows)[:2] == (ROWS, warps)
 
 
 def test_gathered_rows_of_a_form():
@@ -369,6 +371,7 @@ def runs_on_form(program_, tensors, rows, **kw):
 
 KEPT = []
 SHAPES = [(1, 129), (3, 255), (700, 256), (5, 257), (40, 384), (7, 513), (300, 1000), (33, 1024), (2000, 1025), (9, 2029), (400, 2304), (20, 4095), (150, 4096), (5, 6001), (3, 9000)]
+ALIGNED = [(1, 132), (700, 256), (40, 384), (300, 1000), (2000, 1024), (9, 2028), (400, 2304), (150, 4096), (5000, 644), (3, 9000)]   # four elements at a time
 
 
 @pytest.mark.gpu
@@ -376,9 +379,9 @@ SHAPES = [(1, 129), (3, 255), (700, 256), (5, 257), (40, 384), (7, 513), (300, 1
                                 {"scale": False, "reduce": "sum", "first": "zero"}, {"steps": "none"}], ids=str)
 def test_rows_give_the_bits_of_the_interpreter(kw):
     """Row lengths around whole tiles and groups of tiles, one and four warps per row, rows and base pointers at any element."""
-    for k, (rows, n) in enumerate(SHAPES):
+    for k, (rows, n) in enumerate(SHAPES + ALIGNED):
         g = torch.Generator(device="cuda").manual_seed(k)
-        pad = [k % 4, (k // 2) % 4, (k + 1) % 4, (k + 2) % 3]
+        pad = [k % 4, (k // 2) % 4, (k + 1) % 4, (k + 2) % 3] if k < len(SHAPES) else [4, 0, 8, 3]
         x, w, r, z = [torch.randn(rows * n + 8, device="cuda", generator=g)[p:p + rows * n].view(rows, n) for p in pad]
         w = w[0]
 
