@@ -1846,7 +1846,10 @@ int build_program(gint_ctx *ctx, const int32_t *code, int n_words, const gint_te
     p->rf_slots = (uint32_t)rfs.size();
     p->vec_slots = (uint32_t)vecs.size();
     uint32_t code_smem;
-    if ((int)direct_smem(stream_view(p, !early.empty()), 1, &code_smem) > ctx->max_smem_optin) wides.clear();   // the tile kernels refuse it
+    if ((int)direct_smem(stream_view(p, !early.empty()), 1, &code_smem) > ctx->max_smem_optin) {   // the tile kernels refuse it: no other route
+        wides.clear();
+        p->form.kind = FORM_NONE;
+    }
     p->wide_slots = (uint32_t)wides.size();
     *out = p;
     return GINT_OK;

@@ -363,16 +363,21 @@ bool match_lanes(const std::vector<Insn> &p, const gint_tensor_info &ti, int n_t
     return true;
 }
 
-/* 16 warps per SM with two to four stages each; fewer where there are fewer tiles. */
+/* Launches that L2 holds: 16 warps per SM with up to four stages. Larger ones: 12 with as many as make 84 KB of tiles, two at least -- as with rows
+ * (plan_rows), more tiles at once are slower. Measured (one B200, us, back to back): product of 4 194 304 matrices 122 with 12 x 2 stages, 128 with 16 x 2,
+ * 131 with 16 x 3 (floor 123); inverse 88 with 12 x 3, 94 with 12 x 4, 98 with 16 x 3, 100 with 16 x 4 (floor 82); of 300 000 the product 13.3
+ * and 12.4. Fewer tiles than warps: fewer warps. */
 bool plan_lanes(const Form &f, uint32_t count, int sms, int max_smem, FormLaunch *l)
 {
     const uint32_t n_in = (uint32_t)__builtin_popcount(f.lane_loads), n_out = (uint32_t)__builtin_popcount(f.lane_stores);
+    const bool large = (uint64_t)count * (n_in + n_out) * gint::kLaneTileBytes > (100ull << 20);
     uint32_t w = (count + (uint32_t)sms - 1) / (uint32_t)sms;
-    if (w > 16) w = 16;
+    if (w > (large ? 12u : 16u)) w = large ? 12u : 16u;
     const uint32_t tiles = (uint32_t)max_smem / w / gint::kLaneTileBytes;
     if (tiles < 2 * n_in + n_out) return false;
-    const uint32_t d = (tiles - n_out) / n_in;
-    l->lanes.depth = d > 4 ? 4 : d;
+    uint32_t d = (tiles - n_out) / n_in;
+    if (large && d > 84u * 1024u / (w * n_in * gint::kLaneTileBytes)) d = 84u * 1024u / (w * n_in * gint::kLaneTileBytes);
+    l->lanes.depth = d > 4 ? 4 : d < 2 ? 2 : d;
     l->smem = w * (l->lanes.depth * n_in + n_out) * gint::kLaneTileBytes;
     l->threads = w * 32u;
     const uint32_t blocks = (count + w - 1) / w;

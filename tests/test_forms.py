@@ -133,6 +133,12 @@ def test_warps_per_row(n, rows, kw, warps):
     assert form(program(rows=rows, n=n, **kw), FAR, count=rows)[:2] == (ROWS, warps)
 
 
+def test_a_program_too_long_for_the_tile_kernels_has_no_form():
+    """What is refused must not depend on the route: the tile kernels keep the whole program in shared memory."""
+    assert form(flat(n=128 * 5000, tiles=5000, op="fadd"), FAR, count=1)[0] == FLAT
+    assert form(flat(n=128 * 12000, tiles=12000, op="fadd"), FAR, count=1)[0] == 0
+
+
 def test_gathered_rows_of_a_form():
     """An index replaces the digit of the innermost batch dimension. Where that has one row, the index still moves the row."""
     pd = program()
