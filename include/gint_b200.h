@@ -302,7 +302,9 @@ int gint_execute_indirect_static(gint_ctx *ctx, const uint64_t *handles, int n_p
  * per lane run on the kernels that access them with one 16-byte access per lane; default 0: no measurable gain on the
  * benchmark programs), "streaming" (1 = launches use the streaming kernels for programs whose tile loops were found again,
  * default; results are the same bits, but for sums of f16 and bf16 2DT tiles whose rows and base pointers are aligned to 4
- * elements: their terms are added in another order). */
+ * elements: their terms are added in another order), "forms" (1 = launches of programs that have a form run on its kernel,
+ * default; the same bits, but for the sums just named, of rows of 128 bf16 elements; any other option away from its default, max_blocks apart,
+ * turns the forms off as well). */
 int gint_set_option(gint_ctx *ctx, const char *name, int value);
 
 #ifdef __cplusplus
