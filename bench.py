@@ -38,9 +38,9 @@ NOMINAL_HBM_GBS = 8000.0
 L2_BYTES = 126 * 1024 * 1024
 # DRAM bytes per leading unit (row / matrix) of one launch, from the ncu captures summarised under profiles/ (small cases of
 # the same kernels; traffic grows in proportion to the units): dram__bytes_read.sum per unit as captured, plus the unit's
-# output bytes for the write side -- in the captures part of the output is still dirty in L2 when the kernel ends (89 MB
+# output bytes for the write side -- in the captures part of the output is still dirty in L2 when the kernel ends (85 MB
 # of 134 MB written for RMSNorm), so dram__bytes_write.sum itself understates what a launch eventually writes.
-NCU_DRAM_BYTES_PER_UNIT = {"rmsnorm": 142910976 / 8192 + 16384, "bmm4x4": 134820864 / 1048576 + 64, "inv4x4": 67267584 / 1048576 + 64}
+NCU_DRAM_BYTES_PER_UNIT = {"rmsnorm": 134277120 / 8192 + 16384, "bmm4x4": 134231552 / 1048576 + 64, "inv4x4": 67125248 / 1048576 + 64}
 
 
 def measured_peak():
@@ -337,7 +337,7 @@ def run_program_bench(name: str, world: int, rank: int, steps: int, warmup: int,
         "launches_per_step": wl.launches_per_run(),
         "l2": "inputs larger than L2" if n_sets == 1 else f"rotating {n_sets} buffer sets (> 2x L2)",
         "passes_per_timed_step": passes,
-        "geometry": {k: info[k] for k in ("pool_size", "tiles_per_warp", "grid_blocks", "regs_per_thread", "blocks_per_sm", "smem_bytes")},
+        "geometry": {k: info[k] for k in ("form", "pool_size", "tiles_per_warp", "grid_blocks", "regs_per_thread", "blocks_per_sm", "smem_bytes")},
         "frac_of_measured_peak": total_bytes / (per_step_ms * 1e-3) / 1e9 / (peak_gbs * world),
         "frac_of_8TBs": total_bytes / (per_step_ms * 1e-3) / 1e9 / (NOMINAL_HBM_GBS * world),
     }, wls
