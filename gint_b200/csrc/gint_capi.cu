@@ -2021,6 +2021,32 @@ int gint_debug_form(const int32_t *code, int n_words, const gint_tensor_info *ti
     return kind ? kind | (int)(l.warps_per_program << 8) : 0;
 }
 
+int gint_debug_rows(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs, uint32_t count, uint32_t *out)
+{
+    if (!code || !ti || !base_ptrs || !out || n_tensors < 1 || n_tensors > GINT_MAX_TENSORS) return GINT_ERR_INVALID_ARGUMENT;
+    gint_ctx ctx;
+    ctx.max_smem_optin = 227 * 1024;
+    ctx.num_sms = 148;
+    Program *p = nullptr;
+    ProgramStreams streams;
+    const int rc = build_program(&ctx, code, n_words, ti, n_tensors, &p, &streams);
+    if (rc != GINT_OK) return rc;
+    FormLaunch l;
+    const int kind = choose_form(&ctx, p, base_ptrs, 0u, count, nullptr, &l);
+    if (kind == FORM_ROWS) {
+        const gint::RowsArgs &a = l.rows;
+        const uint32_t team = l.warps_per_program, launch[8] = {team, l.threads / (32u * team), a.depth, a.tiles, a.full_tiles, a.stage_bytes, a.stationary_bytes, l.smem};
+        memcpy(out, launch, sizeof(launch));
+        for (int s = 0; s < gint::ROWS_Z; s++) {
+            out[8 + 3 * s] = (uint32_t)a.slot[s].n;
+            out[9 + 3 * s] = a.slot[s].area;
+            out[10 + 3 * s] = a.slot[s].stationary;
+        }
+    }
+    delete p;
+    return kind == FORM_ROWS ? 1 : 0;
+}
+
 int gint_create(int device, gint_ctx **out)
 {
     if (!out) return GINT_ERR_INVALID_ARGUMENT;

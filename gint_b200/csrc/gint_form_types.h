@@ -29,7 +29,7 @@ struct FormGrid {
 struct FormSlot {
     u64 base;
     uint32_t stride[kFormDims];      // elements
-    int n;                           // elements of a row (dimension 1 of the block); 0: the form has no such operand
+    int n;                           // elements of a row (dimension 1 of the block; of row programs no more than their tiles cover); 0: the form has no such operand
     uint32_t area;                   // shared memory: byte offset in the stage, or in the stationary area
     uint32_t stationary;             // the same row for every logical program: staged once
 };

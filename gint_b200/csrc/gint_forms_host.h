@@ -233,13 +233,13 @@ bool match_rows(const std::vector<Insn> &p, const gint_tensor_info &ti, Form *f)
     for (int s = 0; s < gint::ROWS_N_SLOTS; s++) {
         if (f->tensor[s] < 0) continue;
         if (s == gint::ROWS_Z && !a.map) break;
+        if ((uint64_t)n[s] > 128ull * a.tiles) a.slot[s].n = (int)(128u * a.tiles);   // the elements that the program has to do with: what is staged, and what the kernels' masks go by
         if ((uint32_t)n[s] / 128u < a.full_tiles) a.full_tiles = (uint32_t)n[s] / 128u;
         if (s == gint::ROWS_Z) break;
         uint32_t &area = a.slot[s].stationary ? a.stationary_bytes : stage;
-        const uint64_t elements = (uint64_t)n[s] < 128ull * a.tiles ? (uint64_t)n[s] : 128ull * a.tiles;
-        if (elements > 65536u) return false;
+        if (a.slot[s].n > 65536) return false;
         a.slot[s].area = area;
-        area += (((uint32_t)elements * 4u + 15u) & ~15u) + 16u;   // a row may start anywhere in its first 16 bytes
+        area += (((uint32_t)a.slot[s].n * 4u + 15u) & ~15u) + 16u;   // a row may start anywhere in its first 16 bytes
     }
     a.fours = a.map != 0 && n[gint::ROWS_Z] % 4 == 0;
     for (int s = 0; s < gint::ROWS_N_SLOTS; s++) {
@@ -297,7 +297,7 @@ bool plan_rows(const gint::RowsArgs &a, uint32_t count, int sms, int max_smem, R
     const bool fours = a.fours && gint::kRowsShapes[rows_kernel(a) / 2].fours;
     uint32_t row_bytes = 0;   // of a stage
     for (int s = 0; s < gint::ROWS_Z; s++)
-        if (a.slot[s].n && !a.slot[s].stationary) row_bytes += 4u * ((uint32_t)a.slot[s].n < 128u * a.tiles ? (uint32_t)a.slot[s].n : 128u * a.tiles);
+        if (!a.slot[s].stationary) row_bytes += 4u * (uint32_t)a.slot[s].n;
     bool four;
     if (a.tiles < 4) four = false;
     else if (need <= 2) four = true;

@@ -274,7 +274,7 @@ __device__ __forceinline__ void rows_map(const RowsArgs &a, const float *x, cons
     for (; k + U <= full; k += U) map_tiles<MAP, N, U, false>(x + k * 128, wt + k * 128, r + k * 128, z + k * 128, left, a.silu, s);
     for (; k < tiles; k += U) {
 #pragma unroll
-        for (int t = 0; t < ROWS_N_SLOTS; t++) left[t] = min(a.slot[t].n, tiles * 128) - at - k * 128;
+        for (int t = 0; t < ROWS_N_SLOTS; t++) left[t] = a.slot[t].n - at - k * 128;
         map_tiles<MAP, N, U, true>(x + k * 128, wt + k * 128, r + k * 128, z + k * 128, left, a.silu, s);
     }
 }
@@ -285,7 +285,7 @@ template <int MAP, int TEAM>
 __device__ __forceinline__ void rows_map_fours(const RowsArgs &a, const float *x, const float *wt, const float *r, float *z, int thread, float s)
 {
     constexpr int U = 2, STEP = TEAM * 128;
-    const int n = min(a.slot[ROWS_Z].n, (int)a.tiles * 128);
+    const int n = a.slot[ROWS_Z].n;
     for (int e = 4 * thread; e < n; e += U * STEP) {
         float o[4 * U];
         float4 v[U], g[U], h[U];
@@ -346,11 +346,11 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
         uint32_t bytes = 0;
 #pragma unroll
         for (int t = 0; t < ROWS_Z; t++)
-            if (a.slot[t].n && a.slot[t].stationary) bytes += row_bytes(a.slot[t].base, min(a.slot[t].n, (int)a.tiles * 128));
+            if (a.slot[t].n && a.slot[t].stationary) bytes += row_bytes(a.slot[t].base, a.slot[t].n);
         bar_expect(bars, bytes);
 #pragma unroll
         for (int t = 0; t < ROWS_Z; t++)
-            if (a.slot[t].n && a.slot[t].stationary) copy_row(smem + a.slot[t].area, a.slot[t].base, row_bytes(a.slot[t].base, min(a.slot[t].n, (int)a.tiles * 128)), bars);
+            if (a.slot[t].n && a.slot[t].stationary) copy_row(smem + a.slot[t].area, a.slot[t].base, row_bytes(a.slot[t].base, a.slot[t].n), bars);
     }
     const uint32_t step = gridDim.x * teams;
     uint32_t now = blockIdx.x + gridDim.x * (uint32_t)team.id;   // logical programs, relative to first: the one computed,
@@ -369,7 +369,7 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
             *reinterpret_cast<uint4 *>(g_form_smem + own + (stage + 1u) * a.stage_bytes - 16u) = make_uint4(off[ROWS_X], off[ROWS_W], off[ROWS_R], off[ROWS_Z]);
 #pragma unroll
             for (int t = 0; t < ROWS_Z; t++) {
-                bytes[t] = a.slot[t].n && !a.slot[t].stationary ? row_bytes(a.slot[t].base + 4ull * off[t], min(a.slot[t].n, (int)a.tiles * 128)) : 0u;
+                bytes[t] = a.slot[t].n && !a.slot[t].stationary ? row_bytes(a.slot[t].base + 4ull * off[t], a.slot[t].n) : 0u;
                 sum += bytes[t];
             }
             bar_expect(bar, sum);

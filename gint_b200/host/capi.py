@@ -86,6 +86,7 @@ SIGNATURES = {
     "gint_debug_route": (c_int, [POINTER(c_int32), c_int, POINTER(HTensorInfo), c_int, POINTER(c_uint64), c_uint32, c_uint32, c_uint32, c_uint64]),
     "gint_debug_form": (c_int, [POINTER(c_int32), c_int, POINTER(HTensorInfo), c_int, POINTER(c_uint64), c_uint32, c_uint32, c_uint32, c_uint64,
                                 c_uint32, c_int64, POINTER(c_uint32)]),
+    "gint_debug_rows": (c_int, [POINTER(c_int32), c_int, POINTER(HTensorInfo), c_int, POINTER(c_uint64), c_uint32, POINTER(c_uint32)]),
     "gint_debug_fused_table": (c_int, [POINTER(c_int32), c_int]),
     "gint_create": (c_int, [c_int, POINTER(c_void_p)]),
     "gint_destroy": (None, [c_void_p]),

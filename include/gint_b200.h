@@ -142,6 +142,12 @@ int gint_debug_route(const int32_t *code, int n_words, const gint_tensor_info *t
 int gint_debug_form(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs, uint32_t first,
                     uint32_t count, uint32_t gather_mask, uint64_t gather_extent_bytes, uint32_t logical, int64_t row, uint32_t *out_offsets);
 
+/* How a launch of `count` logical programs lies in shared memory where it runs on the row form (default options; needs no device). 1, and in out[0..16]: warps
+ * per logical program, teams of so many warps per block, stages per team, tiles of a row, tiles that are whole in every operand, bytes of a stage, bytes of
+ * the rows that are staged once per block, bytes in all; then for x, w and r each the elements of a row that are read (0: no such operand), the
+ * row's byte offset in its area and whether it is staged once. 0: no row form. Negative: the status of a refused program. */
+int gint_debug_rows(const int32_t *code, int n_words, const gint_tensor_info *ti, int n_tensors, const uint64_t *base_ptrs, uint32_t count, uint32_t *out);
+
 /* The instruction list the kernels actually run for a program, after the optional early-issue and fusion passes (for
  * tests; no GPU needed): out_ops[i] is a format opcode, an internal opcode (>= 106) or -1 for an instruction absorbed into
  * the fused handler before it. With early_issue != 0 the descriptors in `ti` also decide which 1-D accesses become their

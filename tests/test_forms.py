@@ -133,6 +133,59 @@ def test_warps_per_row(n, rows, kw, warps):
     assert form(program(rows=rows, n=n, **kw), FAR, count=rows)[:2] == (ROWS, warps)
 
 
+def row_layout(pd, bases, count):
+    """gint_debug_rows: the launch's numbers and, by operand, (elements read, byte offset of the row, staged once), or None"""
+    code = np.ascontiguousarray(np.asarray(pd.program, dtype=np.int32).reshape(-1))
+    ti = capi.HTensorInfo()
+    fill_tensor_info(ti, pd.input_infos)
+    out = (ctypes.c_uint32 * 17)()
+    r = capi.load_library().gint_debug_rows(code.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), code.size, ctypes.byref(ti), len(pd.input_infos), (ctypes.c_uint64 * 8)(*bases), count, out)
+    assert r >= 0, r
+    names = ("team", "teams", "depth", "tiles", "full", "stage", "stationary", "smem")
+    return (dict(zip(names, out[:8])), [tuple(out[8 + 3 * s:11 + 3 * s]) for s in range(3)]) if r else None
+
+
+def last_element_read(tiles, full, left, team, reduce):
+    """The largest element of a staged row that the threads of a team read (rows_reduce, rows_map in gint_rows.cuh), where the row has `left` elements."""
+    values = 4 // team
+    U = {1: 8 if reduce else 4, 4: 2}[values]
+    last = -1
+    for at in {lane + 32 * values * warp for warp in range(team) for lane in (0, 31)}:
+        k = 0
+        while k < tiles:
+            masked = k + U > full
+            for u in range(U):
+                for i in range(values):
+                    e = at + 128 * (k + u) + 32 * i
+                    if not masked or e < left:
+                        last = max(last, e)
+            k += U
+    return last
+
+
+@pytest.mark.parametrize("n,tiles,rows", [(12000, 65, 5000), (6001, 41, 5000), (20000, 137, 5000), (1500, 5, 5000), (1500, 5, 100), (700, 3, 9), (1024, 9, 64), (1029, None, 64), (4096, None, 700),
+                                          (129, None, 9000), (9000, None, 3)])
+@pytest.mark.parametrize("kw", [{}, {"scale": False}, {"silu": True, "add": True}, {"w_rows": True, "add": True}])
+def test_staged_rows_hold_what_is_read(n, tiles, rows, kw):
+    """Rows of which the program sums a part, the whole, or more than there is: no thread reads behind what was staged, and the stages lie in the block's memory."""
+    layout = row_layout(program(rows=rows, n=n, tiles=tiles, **kw), FAR, rows)
+    if layout is None:
+        assert n > 4096 or (n < 256 and not kw.get("scale", True))      # (two tiles that are only summed are no loop)
+        return
+    a, operands = layout
+    staged = min(n, 128 * a["tiles"])
+    areas = {0: [], 1: []}
+    for s, (left, area, once) in enumerate(operands):
+        if left:
+            for reduce in ((True, False) if s == 0 else (False,)):
+                assert last_element_read(a["tiles"], a["full"], left, a["team"], reduce) < staged
+            areas[once].append((area, area + (4 * staged + 12 + 15 & ~15)))      # (a row may start at any of the four elements of its first 16 bytes)
+    for once, end in ((0, a["stage"] - 16), (1, a["stationary"])):
+        for (_, e), (b, _) in zip(sorted(areas[once]), sorted(areas[once])[1:] + [(end, None)]):
+            assert e <= b
+    assert a["stationary"] + a["teams"] * (a["depth"] * (a["stage"] + 8) + (1024 if a["team"] > 1 else 0)) + 8 <= a["smem"] <= 227 * 1024
+
+
 def test_a_program_too_long_for_the_tile_kernels_has_no_form():
     """What is refused must not depend on the route: the tile kernels keep the whole program in shared memory."""
     assert form(flat(n=128 * 5000, tiles=5000, op="fadd"), FAR, count=1)[0] == FLAT
@@ -398,6 +451,23 @@ def test_rows_give_the_bits_of_the_interpreter(kw):
             return [out]
         assert runs_on_form(rows_program, [x, w, r, z], rows, n=n, **kw) or (n < 600 and not kw.get("scale", True)), (rows, n)   # (few tiles are no loop)
         same_bits(launch)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,n,tiles", [(9, 700, 3), (100, 1500, 5), (2000, 1500, 5), (2000, 1536, 7), (2000, 6001, 41), (400, 12000, 65), (1000, 8192, 33), (64, 1024, 9)])
+@pytest.mark.parametrize("kw", [{}, {"scale": False}, {"silu": True, "add": True}, {"reduce": "fma", "add": True}], ids=str)
+def test_rows_of_which_a_part_is_summed(rows, n, tiles, kw):
+    """Programs over a part of their rows, whose number of tiles is no multiple of a group; what lies behind is left alone."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, r = torch.randn(rows, n, device="cuda", generator=g), torch.randn(rows, n, device="cuda", generator=g)
+    x[:, 128 * tiles:] = float("nan")
+
+    def launch():
+        out = torch.full((rows, n), 9.0, device="cuda")
+        rows_program(x, r[0], r, out, grid_dim=rows, n=n, tiles=tiles, **kw)
+        return [out]
+    assert runs_on_form(rows_program, [x, r[0], r, x], rows, n=n, tiles=tiles, **kw) == (n < 12000 or not kw.get("silu"))      # (one team per SM)
+    same_bits(launch)
 
 
 @pytest.mark.gpu
