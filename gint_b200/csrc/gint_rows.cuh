@@ -91,10 +91,13 @@ template <int TEAM> struct Team {
         if constexpr (TEAM == 1) __syncwarp();
         else asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(TEAM * 32) : "memory");
     }
-    /* sync, and whether `ok` holds for all of the team */
+    /* sync, and whether `ok` holds for all of the team (a vote alone orders no memory accesses) */
     __device__ __forceinline__ bool all(bool ok) const
     {
-        if constexpr (TEAM == 1) return __all_sync(0xffffffffu, ok);
+        if constexpr (TEAM == 1) {
+            __syncwarp();
+            return __all_sync(0xffffffffu, ok);
+        }
         uint32_t r;
         asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbar.red.and.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
                      : "=r"(r) : "r"(id + 1), "n"(TEAM * 32), "r"((uint32_t)ok) : "memory");
