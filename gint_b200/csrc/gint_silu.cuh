@@ -53,7 +53,7 @@ template <int N> __device__ __forceinline__ void silu(float (&x)[N], float c)
         for (int i = 0; i < N; i++) x[i] = q[i];
     } else {
 #pragma unroll
-        for (int i = 0; i < N; i++) x[i] = __fdiv_rn(x[i], -minus_d[i]);
+        for (int i = 0; i < N; i++) x[i] = __fdiv_rn(x[i], __fadd_rn(-minus_d[i], 0.0f));   // (exp(-x) + c is never -0, as -minus_d is where it is zero)
     }
 }
 

@@ -362,7 +362,7 @@ def test_a_whole_launch_of_heads_takes_every_logical_program_once(shape):
 
 
 @bytecode
-def flat_program(x, y, z, REGW, WARP, op="silu_fmul", dtype="f32", tiles=1, start=0):
+def flat_program(x, y, z, REGW, WARP, op="silu_fmul", dtype="f32", tiles=1, start=0, c=1.0):
     n, = x.shape
     suffix, block = "" if dtype == "f32" else "_" + dtype, 128 * tiles
     xb, yb, zb = [F.make_block_1d(t, t.shape[0], t.strides[0], -(-n // block), block) for t in (x, y, z)]
@@ -372,7 +372,7 @@ def flat_program(x, y, z, REGW, WARP, op="silu_fmul", dtype="f32", tiles=1, star
             F.dup()
             F.fneg()
             F.fexp()
-            F.faddimm(1.0)
+            F.faddimm(c)
             F.frdiv()
         if op != "silu":
             getattr(F, "fldg_1d" + suffix)(off, yb)
@@ -498,6 +498,25 @@ def test_silu_of_any_bits():
             rows_program(x, w, x, z, grid_dim=rows, n=n, steps="none", reduce="sum", silu=True)
             return [z]
         same_bits(launch)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c", [-1.0, -0.0])
+def test_silu_where_the_divisor_is_zero(c):
+    """x / (exp(-x) + c): a sum that cancels, or that both terms leave at zero, is +0, and the sign of the quotient is that of x."""
+    n = 1024
+    v = torch.tensor([1e-10, -1e-10, 1e-30, -1e-42, 0.0, -0.0, 3e-8, -3e-8, 150.0, 1e30, float("inf"), -150.0, float("-inf"), float("nan"), 1.0, -1.0], device="cuda")
+    v = torch.cat([v, v.roll(3), v.repeat_interleave(4)]).repeat(11)[:n].contiguous()
+    x = torch.ones(4, n, device="cuda")
+
+    def launch():
+        z, y = torch.empty(4, n, device="cuda"), torch.empty(n, device="cuda")
+        rows_program(x, v / 8, x, z, grid_dim=4, n=n, steps="none", reduce="sum", silu=True, c=c)
+        flat_program(v, v, y, grid_dim=n // 128, op="silu", c=c)
+        return [z, y]
+    assert runs_on_form(rows_program, [x, v, x, x], 4, n=n, steps="none", reduce="sum", silu=True, c=c)
+    assert get_executor().launch_info(flat_program, C.to_interfaces([v, v, v.clone()]), n // 128, op="silu", c=c)["form"] == FLAT
+    same_bits(launch)
 
 
 @pytest.mark.gpu
