@@ -1109,6 +1109,7 @@ struct gint_ctx {
     int opt_rf = 1;             // launches use a program's RF stream (virtual registers in shared memory) when it has one
     int opt_rf_create = 1;      // programs created from now on get an RF stream when they qualify
     int opt_forms = 1;          // launches of programs that have a form run on its kernel
+    uint32_t opt_row_wait_ms = (uint32_t)(gint::kRowsWaitNs / 1000000ull);   // row kernels: how long a wait for a copy may take
     int opt_wide = 1;           // launches use a program's stream with loops (streaming kernels) when it has one
     int opt_vec = 0;            // vector-layout stream and kernels for the programs that qualify (creation and launch). Off unless asked
                                 // for: measured on the conductor graph, the fused program alone gains 2-3 % (175 -> 169 us) but the whole
@@ -1448,6 +1449,7 @@ int choose_rows(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, u
     a.first = first;
     a.count = count;
     a.depth = plan.depth;
+    a.wait_ns = ctx->opt_row_wait_ms * 1000000ull;
     a.grid.simple = a.grid.n_dims == 1 && first + count <= a.grid.size[0];
     l->kernel = rows_kernel(a) + (plan.team == 4);
     l->grid = plan.grid;
@@ -2779,6 +2781,11 @@ int gint_set_option(gint_ctx *ctx, const char *name, int value)
     }
     if (strcmp(name, "forms") == 0) {   // launches made from now on
         ctx->opt_forms = value != 0;
+        return GINT_OK;
+    }
+    if (strcmp(name, "row_wait_ms") == 0) {   // launches made from now on
+        if (value < 0 || value > 60000) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "row_wait_ms must be 0 to 60000");
+        ctx->opt_row_wait_ms = (uint32_t)value;
         return GINT_OK;
     }
     if (strcmp(name, "streaming") == 0) {   // launches made from now on

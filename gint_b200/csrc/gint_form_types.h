@@ -79,6 +79,8 @@ constexpr RowsShape kRowsShapes[] = {
 constexpr int kRowsSteps = 12;
 constexpr uint32_t kRowsFold = 0x80;   // step: Dup, FPermW (operand), FAdd
 
+constexpr u64 kRowsWaitNs = 4000000000ull;   // how long a wait for a copy may take where the caller has not said otherwise
+
 struct RowsArgs {
     FormGrid grid;
     FormSlot slot[ROWS_N_SLOTS];
@@ -91,6 +93,7 @@ struct RowsArgs {
     uint32_t steps;                  // STEPS_...
     uint32_t step[kRowsSteps], operand[kRowsSteps];
     uint32_t depth, stage_bytes, stationary_bytes;
+    u64 wait_ns;                     // a wait for a copy that takes longer gives up; 0: there is none
     uint32_t fours;                  // every row of every operand starts at a 16-byte boundary; one length, a multiple of four
 };
 

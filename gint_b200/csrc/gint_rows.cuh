@@ -53,21 +53,28 @@ __device__ __forceinline__ long long form_clamp(const FormGrid &g, long long row
     return row < 0 ? 0 : row >= (long long)g.gather_rows ? (long long)g.gather_rows - 1 : row;
 }
 
-/* Barriers of the bulk copies. A wait gives up after some seconds (no copy takes that long), which the caller hands on. */
+/* Barriers of the bulk copies. A wait gives up after `limit` ns (RowsArgs::wait_ns; a copy takes a microsecond or two, more only where its page has to be
+ * brought in first). */
 extern "C" __device__ unsigned int gint_form_gave_up;   // teams whose wait gave up (gint_device_status_read)
 __device__ __forceinline__ void bar_init(uint32_t bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity)
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, u64 limit)
 {
-    for (int k = 0; k < 100000; k++) {
-        uint32_t done;
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done || limit == 0) return done;
+    u64 begin, now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(begin));
+    do {
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         if (done) return true;
-    }
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    } while (now - begin < limit);
     return false;
 }
 /* the 16-byte groups that n floats from p on touch */
@@ -384,11 +391,11 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
         ask += step;
     };
     for (uint32_t d = 0; d + 1 < a.depth; d++) issue(d);
-    bool ok = bar_wait(bars, 0u);
+    bool ok = bar_wait(bars, 0u, a.wait_ns);
     uint32_t stage = 0, parity = 0;
     const int at = (team.thread & 31) + 32 * N * (team.thread >> 5);   // the thread's first element of a tile: lane + 32 * width value
     for (; now < a.count; now += step) {
-        ok = bar_wait(own_bars + 8u * stage, parity) && ok;
+        ok = bar_wait(own_bars + 8u * stage, parity, a.wait_ns) && ok;
         if (!team.all(ok)) break;   // (also: every thread is done with the stage before this one)
         const uint4 note = *reinterpret_cast<const uint4 *>(g_form_smem + own + (stage + 1u) * a.stage_bytes - 16u);
         issue(stage == 0 ? a.depth - 1u : stage - 1u);
@@ -432,11 +439,11 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
         }
         if (++stage == a.depth) { stage = 0; parity ^= 1u; }
     }
-    if (now < a.count && team.thread == 0) {   // gave up: the copies that are on their way end before the block does
+    if (now < a.count && team.thread == 0) {   // gave up: the copies that are on their way get the usual time to end before the block does
         atomicAdd(&gint_form_gave_up, 1u);
-        bar_wait(bars, 0u);
+        bar_wait(bars, 0u, kRowsWaitNs);
         for (; now < ask && now < a.count; now += step) {
-            bar_wait(own_bars + 8u * stage, parity);
+            bar_wait(own_bars + 8u * stage, parity, kRowsWaitNs);
             if (++stage == a.depth) { stage = 0; parity ^= 1u; }
         }
     }

@@ -569,6 +569,30 @@ def test_rows_in_a_graph_and_on_few_blocks():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows,n", [(20000, 4096), (300000, 256)])
+def test_a_wait_that_runs_out_is_reported(rows, n):
+    """Four warps per row and one, more rows than L2 holds: with no time to wait, teams give up. The launch ends, the rows that they leave are not
+    written, and the status says so."""
+    ex = get_executor()
+    x, w = torch.randn(rows, n, device="cuda"), torch.randn(n, device="cuda")
+    z, want = torch.full((rows, n), 9.0, device="cuda"), torch.empty(rows, n, device="cuda")
+    rows_program(x, w, x, want, grid_dim=rows, n=n)
+    assert ex.device_status()["code"] == 0
+    ex.set_option("row_wait_ms", 0)
+    try:
+        rows_program(x, w, x, z, grid_dim=rows, n=n)
+    finally:
+        ex.set_option("row_wait_ms", 4000)
+    torch.cuda.synchronize()
+    assert ex.device_status()["what"] == "a wait gave up"
+    left = (z == 9.0).all(1)
+    assert left.any() and bits_equal(z[~left].cpu(), want[~left].cpu())
+    assert ex.device_status()["code"] == 0
+    rows_program(x, w, x, z, grid_dim=rows, n=n)
+    assert bits_equal(z.cpu(), want.cpu()) and ex.device_status()["code"] == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["bmm4x4", "inv4x4"])
 @pytest.mark.parametrize("batch", [1, 31, 33, 64, 1000, 4747, 80001])
 def test_lane_programs_give_the_bits_of_the_interpreter(kind, batch):
