@@ -1098,6 +1098,7 @@ struct gint_ctx {
     Variant checked{12, 1, nullptr, 0, false, 0};
     const void *form_fn[GINT_N_FORM_KERNELS] = {};
     std::atomic<bool> form_launched{false};
+    volatile uint32_t *gave_up = nullptr;       // the device's word for row kernels that gave up (gave_up_word)
     gint_device_status *status_dev = nullptr;   // status word of the checked launches (allocated on first use)
     std::string last_error;
     int opt_tiles_per_warp = 0;
@@ -1134,6 +1135,14 @@ int fail(gint_ctx *ctx, int status, const char *what, cudaError_t e = cudaSucces
         ctx->last_error = buf;
     }
     return status;
+}
+
+/* Results of an earlier launch that were not completed (a row kernel gave up) are not worked on: every launch fails until
+ * gint_device_status_read has handed that on. */
+int refuse_incomplete(gint_ctx *ctx)
+{
+    if (!ctx->gave_up || !*ctx->gave_up) return GINT_OK;
+    return fail(ctx, GINT_ERR_INCOMPLETE, "an earlier launch waited too long for copies of its own and left rows of its result unwritten (gint_device_status_read clears this)");
 }
 
 struct DeviceGuard {
@@ -1450,6 +1459,7 @@ int choose_rows(const gint_ctx *ctx, const Form &f, const uint64_t *base_ptrs, u
     a.count = count;
     a.depth = plan.depth;
     a.wait_ns = ctx->opt_row_wait_ms * 1000000ull;
+    a.gave_up = ctx->gave_up;
     a.grid.simple = a.grid.n_dims == 1 && first + count <= a.grid.size[0];
     l->kernel = rows_kernel(a) + (plan.team == 4);
     l->grid = plan.grid;
@@ -1554,6 +1564,7 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
     if (!p) return fail(ctx, GINT_ERR_BAD_HANDLE, "unknown program handle");
     if (n_tensors != p->n_tensors) return fail(ctx, GINT_ERR_ARG_COUNT, "number of arguments does not match the program");
     if (count == 0) return GINT_OK;
+    if (int rc = refuse_incomplete(ctx)) return rc;
     if ((uint64_t)first + (uint64_t)count > 0xFFFFFFFFull) return fail(ctx, GINT_ERR_TOO_LARGE, "logical program range overflows 32 bits");
     DeviceGuard guard(ctx->device);
     if (p->form.kind != FORM_NONE) {
@@ -1936,6 +1947,7 @@ const char *gint_status_string(int status)
     case GINT_ERR_NO_DEVICE: return "no usable device or kernel image";
     case GINT_ERR_TOO_LARGE: return "program or batch too large";
     case GINT_ERR_OUT_OF_MEMORY: return "out of memory";
+    case GINT_ERR_INCOMPLETE: return "an earlier launch was not completed";
     }
     return "unknown status";
 }
@@ -2049,6 +2061,27 @@ int gint_debug_rows(const int32_t *code, int n_words, const gint_tensor_info *ti
     return kind == FORM_ROWS ? 1 : 0;
 }
 
+namespace {
+/* A device's word of host memory in which its row kernels report that they gave up: one per process, never freed, as a captured graph may hold its
+ * address for longer than any context lives. */
+volatile uint32_t *gave_up_word(int device)
+{
+    static std::mutex mu;
+    static std::vector<uint32_t *> words;
+    std::lock_guard<std::mutex> lk(mu);
+    if ((size_t)device >= words.size()) words.resize((size_t)device + 1, nullptr);
+    if (!words[(size_t)device]) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (a context may be made while a stream is captured)
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) memset(words[(size_t)device] = (uint32_t *)p, 0, 64);
+        else cudaGetLastError();
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    return words[(size_t)device];
+}
+}  // namespace
+
 int gint_create(int device, gint_ctx **out)
 {
     if (!out) return GINT_ERR_INVALID_ARGUMENT;
@@ -2069,8 +2102,10 @@ int gint_create(int device, gint_ctx **out)
         delete ctx;
         return GINT_ERR_NO_DEVICE;
     }
+    ctx->gave_up = gave_up_word(device);
     for (auto &im : g_images) {
         if (!im.loaded) continue;
+        if (im.K == -2 && im.P < kLaneKernelFirst && !ctx->gave_up) continue;   // row kernels, which could not report
         if (im.K == 0) ctx->indirect.fn = (const void *)im.kernel;
         else if (im.K == -1) ctx->checked.fn = (const void *)im.kernel;
         else if (im.K == -2) {
@@ -2313,6 +2348,7 @@ int gint_execute_checked(gint_ctx *ctx, uint64_t handle, const uint64_t *base_pt
     {
         int rc = refuse_capture(ctx, stream, "gint_execute_checked");
         if (rc != GINT_OK) return rc;
+        if ((rc = refuse_incomplete(ctx)) != GINT_OK) return rc;
     }
     {
         std::lock_guard<std::mutex> lk(ctx->mu);
@@ -2362,23 +2398,17 @@ int gint_device_status_read(gint_ctx *ctx, gint_device_status *out, int clear)
 {
     if (!ctx || !out) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "null argument");
     memset(out, 0, sizeof(*out));
-    if (!ctx->status_dev && !ctx->form_launched) return GINT_OK;     // nothing that reports anything so far
+    if (!ctx->status_dev && !ctx->form_launched && !(ctx->gave_up && *ctx->gave_up)) return GINT_OK;     // nothing that reports anything so far
     DeviceGuard guard(ctx->device);
     cudaError_t e = cudaDeviceSynchronize();
     if (ctx->status_dev) {
         if (e == cudaSuccess) e = cudaMemcpy(out, ctx->status_dev, sizeof(*out), cudaMemcpyDeviceToHost);
         if (e == cudaSuccess && clear) e = cudaMemset(ctx->status_dev, 0, sizeof(*out));
     }
-    for (auto &im : g_images) {   // the row kernels count the teams that gave up waiting for a copy
-        void *flag = nullptr;
-        size_t bytes = 0;
-        uint32_t n = 0;
-        if (im.K != -2 || im.P >= kLaneKernelFirst || !im.loaded || !ctx->form_launched) continue;
-        if (e == cudaSuccess) e = cudaLibraryGetGlobal(&flag, &bytes, im.lib, "gint_form_gave_up");
-        if (e == cudaSuccess) e = cudaMemcpy(&n, flag, sizeof(n), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess && n && clear) e = cudaMemset(flag, 0, sizeof(n));
-        if (n && out->code == GINT_DEVICE_OK) { out->code = GINT_DEVICE_GAVE_UP; out->slot = -1; }
-        out->count += n;
+    if (ctx->gave_up && *ctx->gave_up) {
+        if (out->code == GINT_DEVICE_OK) { out->code = GINT_DEVICE_GAVE_UP; out->slot = -1; }
+        out->count++;
+        if (clear) *ctx->gave_up = 0u;
     }
     if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "reading the device status", e);
     return GINT_OK;
@@ -2429,6 +2459,7 @@ int gint_execute_indirect(gint_ctx *ctx, const uint64_t *handles, int n_programs
     {
         int rc = refuse_capture(ctx, stream, "gint_execute_indirect");
         if (rc != GINT_OK) return rc;
+        if ((rc = refuse_incomplete(ctx)) != GINT_OK) return rc;
     }
     /* One indirect launch of a context at a time builds its tables: the scratch (host image and device copy) is shared by
      * every call, and its layout depends on n_programs. */
@@ -2519,6 +2550,7 @@ int gint_execute_batch(gint_ctx *ctx, const int32_t *codes, int n_programs, int 
     {
         int rc = refuse_capture(ctx, stream, "gint_execute_batch");
         if (rc != GINT_OK) return rc;
+        if ((rc = refuse_incomplete(ctx)) != GINT_OK) return rc;
     }
     std::lock_guard<std::mutex> ind_lock(ctx->ind_mu);
     /* scratch layout: [one gint_tensor_info, padded to 640 | n_programs instruction counts | the candidates' words as they are] */
@@ -2625,6 +2657,7 @@ int gint_execute_indirect_static(gint_ctx *ctx, const uint64_t *handles, int n_p
     cudaStream_t stream = (cudaStream_t)cuda_stream;
     int rc = refuse_capture(ctx, stream, "gint_execute_indirect_static");
     if (rc != GINT_OK) return rc;
+    if ((rc = refuse_incomplete(ctx)) != GINT_OK) return rc;
     /* Held from set-up to the kernel launch: the host image is shared, and the uploads and the launch of one call must not be
      * interleaved with another thread's. */
     std::lock_guard<std::mutex> lk(g_static_mu);

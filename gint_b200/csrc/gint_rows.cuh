@@ -55,7 +55,6 @@ __device__ __forceinline__ long long form_clamp(const FormGrid &g, long long row
 
 /* Barriers of the bulk copies. A wait gives up after `limit` ns (RowsArgs::wait_ns; a copy takes a microsecond or two, more only where its page has to be
  * brought in first). */
-extern "C" __device__ unsigned int gint_form_gave_up;   // teams whose wait gave up (gint_device_status_read)
 __device__ __forceinline__ void bar_init(uint32_t bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes)
 {
@@ -440,7 +439,8 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
         if (++stage == a.depth) { stage = 0; parity ^= 1u; }
     }
     if (now < a.count && team.thread == 0) {   // gave up: the copies that are on their way get the usual time to end before the block does
-        atomicAdd(&gint_form_gave_up, 1u);
+        *a.gave_up = 1u;
+        __threadfence_system();
         bar_wait(bars, 0u, kRowsWaitNs);
         for (; now < ask && now < a.count; now += step) {
             bar_wait(own_bars + 8u * stage, parity, kRowsWaitNs);

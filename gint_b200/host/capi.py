@@ -59,6 +59,7 @@ GINT_ERR_CUDA = -8
 GINT_ERR_NO_DEVICE = -9
 GINT_ERR_TOO_LARGE = -10
 GINT_ERR_OUT_OF_MEMORY = -11
+GINT_ERR_INCOMPLETE = -12
 
 class DeviceStatusC(ctypes.Structure):
     """gint_device_status"""

@@ -50,7 +50,8 @@ typedef enum gint_status {
     GINT_ERR_CUDA = -8,              /* a CUDA runtime call failed; see gint_last_error() */
     GINT_ERR_NO_DEVICE = -9,         /* no usable sm_100 device / kernel image */
     GINT_ERR_TOO_LARGE = -10,        /* program or batch exceeds a documented limit */
-    GINT_ERR_OUT_OF_MEMORY = -11
+    GINT_ERR_OUT_OF_MEMORY = -11,
+    GINT_ERR_INCOMPLETE = -12        /* an earlier launch on the device gave up (GINT_DEVICE_GAVE_UP): every launch returns this until gint_device_status_read clears it */
 } gint_status;
 
 /* Result of the static walk over a straight-line program (gint/host/analyzer.py:137-158, BytecodeStats). */
@@ -92,7 +93,8 @@ typedef enum gint_device_code {
     GINT_DEVICE_STORE_OUT_OF_RANGE = 2,   /* a tile store or scatter outside it: skipped */
     GINT_DEVICE_INSTRUCTION_BUDGET = 3,   /* more instructions executed than the program holds (a dispatch error): stopped */
     GINT_DEVICE_BAD_DISPATCH = 4,         /* no handler for an (opcode, stack depth) pair; `address` holds the key: stopped */
-    GINT_DEVICE_GAVE_UP = 5               /* (any launch) a form kernel waited in vain for a copy of its own and stopped; nothing else is filled in */
+    GINT_DEVICE_GAVE_UP = 5               /* (any launch on the device) row kernels waited too long for copies of their own (option row_wait_ms) and left rows
+                                           * unwritten; nothing else is filled in */
 } gint_device_code;
 
 typedef struct gint_device_status {

@@ -572,7 +572,7 @@ def test_rows_in_a_graph_and_on_few_blocks():
 @pytest.mark.parametrize("rows,n", [(20000, 4096), (300000, 256)])
 def test_a_wait_that_runs_out_is_reported(rows, n):
     """Four warps per row and one, more rows than L2 holds: with no time to wait, teams give up. The launch ends, the rows that they leave are not
-    written, and the status says so."""
+    written, and every launch after it fails until the status is read, which says why."""
     ex = get_executor()
     x, w = torch.randn(rows, n, device="cuda"), torch.randn(n, device="cuda")
     z, want = torch.full((rows, n), 9.0, device="cuda"), torch.empty(rows, n, device="cuda")
@@ -584,7 +584,15 @@ def test_a_wait_that_runs_out_is_reported(rows, n):
     finally:
         ex.set_option("row_wait_ms", 4000)
     torch.cuda.synchronize()
-    assert ex.device_status()["what"] == "a wait gave up"
+    before, plan = ex.launches, ex.build_plan([(rows_program, [x, w, x, want], rows)])
+    add, tile = C.vec_add_128, [torch.zeros(128, device="cuda") for _ in range(3)]
+    for call in (lambda: rows_program(x, w, x, want, grid_dim=rows, n=n), lambda: add(*tile, grid_dim=1), lambda: plan.run(torch.cuda.current_stream().cuda_stream),
+                 lambda: ex.execute_indirect([add], [tile], [0]), lambda: ex.execute_indirect([add], [tile], [0], static_tables=True),
+                 lambda: ex.execute_checked(add, C.to_interfaces(tile), 1)):
+        with pytest.raises(capi.GintError) as e:
+            call()
+        assert e.value.status == capi.GINT_ERR_INCOMPLETE
+    assert ex.launches == before and ex.device_status(clear=False)["what"] == "a wait gave up" and ex.device_status()["count"] == 1
     left = (z == 9.0).all(1)
     assert left.any() and bits_equal(z[~left].cpu(), want[~left].cpu())
     assert ex.device_status()["code"] == 0
