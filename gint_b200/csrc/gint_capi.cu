@@ -1097,7 +1097,6 @@ struct gint_ctx {
     Variant indirect{12, 1, nullptr, 0, false, 0};
     Variant checked{12, 1, nullptr, 0, false, 0};
     const void *form_fn[GINT_N_FORM_KERNELS] = {};
-    std::atomic<bool> form_launched{false};
     volatile uint32_t *gave_up = nullptr;       // the device's word for row kernels that gave up (gave_up_word)
     gint_device_status *status_dev = nullptr;   // status word of the checked launches (allocated on first use)
     std::string last_error;
@@ -1574,7 +1573,6 @@ int launch_direct(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, int
             void *args[1] = {kind == FORM_ROWS ? (void *)&l.rows : kind == FORM_LANES ? (void *)&l.lanes : kind == FORM_HEADS ? (void *)&l.heads : (void *)&l.flat};
             cudaError_t e = cudaLaunchKernel(ctx->form_fn[l.kernel], dim3(l.grid), dim3(l.threads), args, l.smem, (cudaStream_t)stream);
             if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaLaunchKernel", e);
-            ctx->form_launched = true;
             return GINT_OK;
         }
     }
@@ -2398,19 +2396,18 @@ int gint_device_status_read(gint_ctx *ctx, gint_device_status *out, int clear)
 {
     if (!ctx || !out) return fail(ctx, GINT_ERR_INVALID_ARGUMENT, "null argument");
     memset(out, 0, sizeof(*out));
-    if (!ctx->status_dev && !ctx->form_launched && !(ctx->gave_up && *ctx->gave_up)) return GINT_OK;     // nothing that reports anything so far
-    DeviceGuard guard(ctx->device);
-    cudaError_t e = cudaDeviceSynchronize();
-    if (ctx->status_dev) {
+    if (ctx->status_dev) {   // checked launches were made
+        DeviceGuard guard(ctx->device);
+        cudaError_t e = cudaDeviceSynchronize();
         if (e == cudaSuccess) e = cudaMemcpy(out, ctx->status_dev, sizeof(*out), cudaMemcpyDeviceToHost);
         if (e == cudaSuccess && clear) e = cudaMemset(ctx->status_dev, 0, sizeof(*out));
+        if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "reading the device status", e);
     }
     if (ctx->gave_up && *ctx->gave_up) {
         if (out->code == GINT_DEVICE_OK) { out->code = GINT_DEVICE_GAVE_UP; out->slot = -1; }
         out->count++;
         if (clear) *ctx->gave_up = 0u;
     }
-    if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "reading the device status", e);
     return GINT_OK;
 }
 

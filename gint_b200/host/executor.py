@@ -315,8 +315,8 @@ class B200Executor(BaseExecutor):
         self.launches += 1
 
     def device_status(self, clear: bool = True, device: Optional[int] = None) -> dict:
-        """What the checked launches on ``device`` found so far (waits for the device): ``code`` 0 means nothing; otherwise
-        the first event's kind, tensor slot, logical program, instruction index, address and lane, and the event count."""
+        """What the checked launches on ``device`` found so far (waits for the device, if there were any), and whether a launch that has
+        ended so far gave up: ``code`` 0 means nothing; otherwise the first event's kind, tensor slot, logical program, instruction index, address and lane, and the event count."""
         _, ctx = self._ctx(device)
         st = capi.DeviceStatusC()
         rc = self._lib.gint_device_status_read(ctx, ctypes.byref(st), 1 if clear else 0)

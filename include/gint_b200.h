@@ -215,7 +215,8 @@ int gint_execute_range(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs
 int gint_execute_checked(gint_ctx *ctx, uint64_t handle, const uint64_t *base_ptrs, const uint64_t *lo, const uint64_t *hi,
                          int n_tensors, uint32_t grid_dim, void *cuda_stream);
 
-/* Wait for the device, copy the status word of the checked launches so far into *out and, if `clear` is not 0, reset it. */
+/* Wait for the device, copy the status word of the checked launches so far into *out and, if `clear` is not 0, reset it. Where no checked launch has been
+ * made there is nothing to wait for: *out says what the launches that have ended so far reported (GINT_DEVICE_GAVE_UP), also during a capture. */
 int gint_device_status_read(gint_ctx *ctx, gint_device_status *out, int clear);
 
 /* gint_execute with gathered rows: for every descriptor slot in `gather_mask`, the index along the tensor's INNERMOST batch

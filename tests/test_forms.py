@@ -601,6 +601,31 @@ def test_a_wait_that_runs_out_is_reported(rows, n):
 
 
 @pytest.mark.gpu
+def test_reading_the_status_waits_for_checked_launches_only():
+    """A context that has made no checked launch reads its status without waiting, also while a stream is captured."""
+    lib, ctx, status = capi.load_library(), ctypes.c_void_p(), capi.DeviceStatusC()
+    assert lib.gint_create(torch.cuda.current_device(), ctypes.byref(ctx)) == 0
+    try:
+        pd = program(rows=64)
+        code = np.ascontiguousarray(np.asarray(pd.program, dtype=np.int32).reshape(-1))
+        ti, handle = capi.HTensorInfo(), ctypes.c_uint64()
+        fill_tensor_info(ti, pd.input_infos)
+        assert lib.gint_program_create(ctx, code.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), code.size, ctypes.byref(ti), 4, ctypes.byref(handle)) == 0
+        t = [torch.ones(64, 1024, device="cuda") for _ in range(4)]
+        graph, bases = torch.cuda.CUDAGraph(), (ctypes.c_uint64 * 8)(*[x.data_ptr() for x in t])
+        KEPT.append(graph)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            assert lib.gint_execute(ctx, handle, bases, 4, 64, torch.cuda.current_stream().cuda_stream) == 0
+            assert lib.gint_device_status_read(ctx, ctypes.byref(status), 1) == 0 and status.code == 0
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.allclose(t[3], torch.ones_like(t[3]))
+    finally:
+        lib.gint_destroy(ctx)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["bmm4x4", "inv4x4"])
 @pytest.mark.parametrize("batch", [1, 31, 33, 64, 1000, 4747, 80001])
 def test_lane_programs_give_the_bits_of_the_interpreter(kind, batch):
