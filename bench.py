@@ -337,7 +337,8 @@ def run_program_bench(name: str, world: int, rank: int, steps: int, warmup: int,
         "launches_per_step": wl.launches_per_run(),
         "l2": "inputs larger than L2" if n_sets == 1 else f"rotating {n_sets} buffer sets (> 2x L2)",
         "passes_per_timed_step": passes,
-        "geometry": {k: info[k] for k in ("form", "pool_size", "tiles_per_warp", "grid_blocks", "regs_per_thread", "blocks_per_sm", "smem_bytes")},
+        "geometry": {k: info[k] for k in (("form", "form_grid_blocks", "form_threads", "form_smem_bytes") if info["form"] else
+                                          ("form", "pool_size", "tiles_per_warp", "grid_blocks", "regs_per_thread", "blocks_per_sm", "smem_bytes"))},
         "frac_of_measured_peak": total_bytes / (per_step_ms * 1e-3) / 1e9 / (peak_gbs * world),
         "frac_of_8TBs": total_bytes / (per_step_ms * 1e-3) / 1e9 / (NOMINAL_HBM_GBS * world),
     }, wls

@@ -2307,6 +2307,11 @@ int gint_program_launch_info(gint_ctx *ctx, uint64_t handle, uint32_t grid_dim, 
     FormLaunch l;
     out->form = choose_form(ctx, p, base_ptrs, 0u, count, nullptr, &l);
     if (out->form && !ctx->form_fn[l.kernel]) out->form = 0;
+    if (out->form) {
+        out->form_grid_blocks = (int32_t)l.grid;
+        out->form_threads = (int32_t)l.threads;
+        out->form_smem_bytes = (int32_t)l.smem;
+    }
     return GINT_OK;
 }
 

@@ -512,7 +512,7 @@ class B200Executor(BaseExecutor):
         info = capi.LaunchInfoC()
         rc = self._lib.gint_program_launch_info(ctx, line.handle, grid_dim, ctypes.byref(info))
         self._check(ctx, rc, "gint_program_launch_info")
-        return {name: getattr(info, name) for name, _ in capi.LaunchInfoC._fields_ if name != "reserved"}
+        return {name: getattr(info, name) for name, _ in capi.LaunchInfoC._fields_}
 
     def set_option(self, name: str, value: int, device: Optional[int] = None) -> None:
         _, ctx = self._ctx(device)

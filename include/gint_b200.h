@@ -82,8 +82,10 @@ typedef struct gint_launch_info {
     int32_t vector_layout;    /* 1: full 1-D tiles live in the pool with lane l holding elements 4l..4l+3 (16-byte accesses) */
     int32_t streaming;        /* 1: a streaming kernel (tile loops found again) */
     int32_t form;             /* not 0: the launch runs on the kernel of the program's form (1: rows, 2: lane program, 3: heads, 4: flat); the fields above then describe the
-                               * interpreter kernel that runs it where the form does not apply */
-    int32_t reserved[3];
+                               * interpreter kernel that runs it where the form does not apply, and the next three the launch itself */
+    int32_t form_grid_blocks;
+    int32_t form_threads;     /* per block */
+    int32_t form_smem_bytes;  /* per block */
 } gint_launch_info;
 
 /* What a checked launch (gint_execute_checked) found; all zero = nothing. The FIRST event is described, `count` counts all. */

@@ -428,6 +428,28 @@ def runs_on_form(program_, tensors, rows, **kw):
     return get_executor().launch_info(program_, C.to_interfaces(tensors), rows, **kw)["form"] == ROWS
 
 
+@pytest.mark.gpu
+def test_launch_info_describes_the_launch_of_a_form():
+    """Blocks, threads and shared memory of the launch itself, and none of them without the form."""
+    ex, m = get_executor(), _perf_cases()
+    x, w, out = torch.zeros(16384, 4096, device="cuda"), torch.zeros(4096, device="cuda"), torch.zeros(16384, 4096, device="cuda")
+    t = C.to_interfaces([x, w, out])
+    a, _ = row_layout(m.rmsnorm.get_program(*t), FAR, 16384)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    info = ex.launch_info(m.rmsnorm, t, 16384)
+    assert (info["form"], info["form_grid_blocks"], info["form_threads"], info["form_smem_bytes"]) == (ROWS, sms, 32 * a["team"] * a["teams"], a["smem"])
+    ex.set_option("forms", 0)
+    try:
+        info = ex.launch_info(m.rmsnorm, t, 16384)
+    finally:
+        ex.set_option("forms", 1)
+    assert (info["form"], info["form_grid_blocks"], info["form_threads"], info["form_smem_bytes"]) == (0, 0, 0, 0)
+    n = 40003
+    x, y, z = [torch.zeros(n, device="cuda") for _ in range(3)]
+    info = ex.launch_info(flat_program, C.to_interfaces([x, y, z]), -(-n // 128), op="fadd")
+    assert (info["form"], info["form_grid_blocks"], info["form_threads"], info["form_smem_bytes"]) == (FLAT, -(-(n // 4) // 256), 256, 0)
+
+
 KEPT = []
 SHAPES = [(1, 129), (3, 255), (700, 256), (5, 257), (40, 384), (7, 513), (300, 1000), (33, 1024), (2000, 1025), (9, 2029), (400, 2304), (20, 4095), (150, 4096), (5, 6001), (3, 9000)]
 ALIGNED = [(1, 132), (700, 256), (40, 384), (300, 1000), (2000, 1024), (9, 2028), (400, 2304), (150, 4096), (5000, 644), (3, 9000)]   # four elements at a time
