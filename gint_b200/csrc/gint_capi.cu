@@ -968,7 +968,11 @@ int load_images()
     int usable = 0;
     for (auto &im : g_images) {
         if (!im.loaded) {
-            cudaError_t e = cudaLibraryLoadData(&im.lib, im.begin, nullptr, nullptr, 0, nullptr, nullptr, 0);
+            const KernelImage *same = &g_images[0];   // an entry before it that is in the same file
+            while (same != &im && !(same->loaded && same->begin == im.begin)) same++;
+            cudaError_t e = cudaSuccess;
+            if (same != &im) im.lib = same->lib;
+            else e = cudaLibraryLoadData(&im.lib, im.begin, nullptr, nullptr, 0, nullptr, nullptr, 0);
             if (e == cudaSuccess) e = cudaLibraryGetKernel(&im.kernel, im.lib, im.name);
             if (e != cudaSuccess) {
                 g_images_error = std::string(im.name) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
