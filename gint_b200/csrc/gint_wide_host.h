@@ -344,7 +344,7 @@ bool wide_transform(const std::vector<Insn> &in, const gint_tensor_info &ti, int
         for (const Insn &x : p) {
             if (x.op == WOP_Silu || wide_out_of_line(x.op - GINT_WIDE_FIRST)) out->slow_rows = true;
         }
-    out->vector = n_outside == 0 && wide_vector(out, ti, n_tensors);
+    out->vector = !out->slow_rows && n_outside == 0 && wide_vector(out, ti, n_tensors);   // (the streaming kernels do not run slow rows, and forms ask for no layout)
     return true;
 }
 
