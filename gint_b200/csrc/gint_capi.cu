@@ -2508,7 +2508,6 @@ int gint_execute_indirect(gint_ctx *ctx, const uint64_t *handles, int n_programs
         h_tab[i].code = progs[(size_t)indices[i]]->code_dev;
         h_tab[i].ti = d_ti + indices[i];
         h_tab[i].n_slots = progs[(size_t)indices[i]]->n_slots;
-        h_tab[i].reserved = 0;
     }
     cudaError_t e = cudaMemcpyAsync(ctx->ind_dev, ctx->ind_host, need, cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return fail(ctx, GINT_ERR_CUDA, "cudaMemcpyAsync(indirect tables)", e);
@@ -2682,7 +2681,6 @@ int gint_execute_indirect_static(gint_ctx *ctx, const uint64_t *handles, int n_p
             h->table[i].code = progs[indices[i]]->code_dev;
             h->table[i].ti = d->ti + indices[i];
             h->table[i].n_slots = progs[indices[i]]->n_slots;
-            h->table[i].reserved = 0;
         }
         /* Two copies of exactly the used parts. The source is ordinary (pageable) host memory: the runtime stages it and
          * returns once the host image may be reused by the next call. */

@@ -63,11 +63,11 @@ template <class P, int I, int SP> __device__ __forceinline__ void lane_run(LaneS
     constexpr uint32_t sel[4] = {arg & 3u, (arg >> 8) & 3u, (arg >> 16) & 3u, (arg >> 24) & 3u};
     if constexpr (op == OP_Halt) return;
     else {
-        constexpr bool push = op == OP_LoadGlobal2DWF32 || op == OP_LoadImm4F || op == OP_LoadImm || op == OP_Dup || op == OP_DupBroadcastW || (op >= OP_FLoadReg0 && op <= OP_FLoadReg7);
-        constexpr bool pop = op == OP_StoreGlobal2DWF32 || op == OP_Pop || op == OP_FAdd || op == OP_FMul || op == OP_FSub || op == OP_FRSub || op == OP_FDiv || op == OP_FRDiv ||
+        constexpr bool push = op == OP_LoadGlobal2DWF32 || op == OP_LoadImm4F || op == OP_Dup || op == OP_DupBroadcastW || (op >= OP_FLoadReg0 && op <= OP_FLoadReg7);
+        constexpr bool pop = op == OP_StoreGlobal2DWF32 || op == OP_Pop || op == OP_FAdd || op == OP_FMul || op == OP_FSub || op == OP_FRSub || op == OP_FDiv ||
                              op == OP_FShuf2 || (op >= OP_FStoreReg0 && op <= OP_FStoreReg7);
         constexpr int next = SP + (push ? 1 : 0) - (pop ? 1 : 0) + (op == OP_Dup2 ? 2 : 0);
-        static_assert(push || pop || op == OP_Dup2 || op == OP_Swap || op == OP_FPermW || op == OP_FNeg || op == OP_Nop, "not a lane program");
+        static_assert(push || pop || op == OP_Dup2 || op == OP_Swap || op == OP_FPermW, "not a lane program");
         float t[4] = {}, b[4] = {};
         if constexpr (SP >= 1) {
 #pragma unroll
@@ -82,7 +82,6 @@ template <class P, int I, int SP> __device__ __forceinline__ void lane_run(LaneS
             if constexpr (op == OP_LoadGlobal2DWF32) s.stack[SP][w] = s.in[L::index(L::loads, (int)(arg & 15u))][arg >> 6][w];
             else if constexpr (op == OP_StoreGlobal2DWF32) s.out[L::index(L::stores, (int)(arg & 15u))][arg >> 6][w] = t[w];
             else if constexpr (op == OP_LoadImm4F) s.stack[SP][w] = (float)(signed char)(arg >> (8 * w));
-            else if constexpr (op == OP_LoadImm) s.stack[SP][w] = __uint_as_float(arg);
             else if constexpr (op == OP_Dup) s.stack[SP][w] = t[w];
             else if constexpr (op == OP_Dup2) { s.stack[SP][w] = b[w]; s.stack[SP + 1][w] = t[w]; }
             else if constexpr (op == OP_Swap) { s.stack[T][w] = b[w]; s.stack[S][w] = t[w]; }
@@ -96,8 +95,6 @@ template <class P, int I, int SP> __device__ __forceinline__ void lane_run(LaneS
             else if constexpr (op == OP_FSub) s.stack[S][w] = __fsub_rn(t[w], b[w]);
             else if constexpr (op == OP_FRSub) s.stack[S][w] = __fsub_rn(b[w], t[w]);
             else if constexpr (op == OP_FDiv) s.stack[S][w] = __fdiv_rn(t[w], b[w]);
-            else if constexpr (op == OP_FRDiv) s.stack[S][w] = __fdiv_rn(b[w], t[w]);
-            else if constexpr (op == OP_FNeg) s.stack[T][w] = __uint_as_float(__float_as_uint(t[w]) ^ 0x80000000u);
         }
         lane_run<P, I + 1, next>(s);
     }

@@ -82,9 +82,7 @@ struct IndirectEntry {
     const uint2 *code;              // pre-decoded program of this logical program
     const gint_tensor_info *ti;     // its descriptor block in device memory
     uint32_t n_slots;               // entries in `code`
-    uint32_t reserved;
 };
-
 
 struct IndirectArgs {
     const IndirectEntry *table;
