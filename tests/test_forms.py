@@ -471,7 +471,7 @@ def test_rows_give_the_bits_of_the_interpreter(kw):
             o = out[pad[3] + 1:pad[3] + 1 + rows * n].view(rows, n)
             rows_program(x, w, r, o, grid_dim=rows, n=n, **kw)
             return [out]
-        assert runs_on_form(rows_program, [x, w, r, z], rows, n=n, **kw) or (n < 600 and not kw.get("scale", True)), (rows, n)   # (few tiles are no loop)
+        assert runs_on_form(rows_program, [x, w, r, z], rows, n=n, **kw) == (n > 256 or kw.get("scale", True)), (rows, n)   # (two tiles that are only summed are no loop)
         same_bits(launch)
 
 
@@ -493,14 +493,15 @@ def test_rows_of_which_a_part_is_summed(rows, n, tiles, kw):
 
 
 @pytest.mark.gpu
-def test_rows_with_extreme_values():
-    """SiLU's quotient where its plain steps do not hold: zeros of both signs, subnormal and huge values, infinities, NaN, every size of exp(-x)."""
-    rows, n = 64, 1030
+@pytest.mark.parametrize("n", [1028, 1030])
+def test_rows_with_extreme_values(n):
+    """Single elements and (1028) four at a time. SiLU's quotient where its plain steps do not hold: zeros of both signs, subnormal and huge values, infinities, NaN, every size of exp(-x)."""
+    rows = 64
     g = torch.Generator(device="cuda").manual_seed(1)
     x = torch.randn(rows, n, device="cuda", generator=g) * torch.logspace(-40, 38, rows, device="cuda")[:, None]
     x[:, 5], x[:, 6], x[::3, 7], x[::5, 8], x[::7, 9] = 0.0, -0.0, float("inf"), float("-inf"), float("nan")
     w = torch.randn(n, device="cuda", generator=g) * torch.logspace(-30, 3, n, device="cuda")
-    for kw in ({"steps": "none", "reduce": "sum", "silu": True}, {"silu": True, "add": True}, {"reduce": "fma"}):
+    for kw in ({"steps": "none", "reduce": "sum", "silu": True}, {"silu": True, "add": True}, {"reduce": "fma"}, {}):
         def launch():
             z = torch.empty(rows, n, device="cuda")
             rows_program(x, w, x, z, grid_dim=rows, n=n, **kw)
@@ -520,6 +521,22 @@ def test_silu_of_any_bits():
             rows_program(x, w, x, z, grid_dim=rows, n=n, steps="none", reduce="sum", silu=True)
             return [z]
         same_bits(launch)
+
+
+@pytest.mark.gpu
+def test_silu_of_all_bits():
+    """Every 32-bit value through SiLU, in the order of the bits, so that most groups take the plain steps together."""
+    ex, n = get_executor(), 1 << 26
+    st, z = torch.cuda.current_stream().cuda_stream, torch.empty(2, n, device="cuda")
+    for k in range(64):
+        x = torch.arange(k * n - (1 << 31), (k + 1) * n - (1 << 31), dtype=torch.int64, device="cuda").to(torch.int32).view(torch.float32)
+        for on in (1, 0):
+            ex.set_option("forms", on)
+            try:
+                flat_program(x, x, z[on], grid_dim=n // 128, op="silu", cuda_stream=st)
+            finally:
+                ex.set_option("forms", 1)
+        assert torch.equal(z[0].view(torch.int32), z[1].view(torch.int32)), k
 
 
 @pytest.mark.gpu
@@ -676,9 +693,9 @@ def test_lane_programs_give_the_bits_of_the_interpreter(kind, batch):
 @pytest.mark.parametrize("batch,tokens,heads,dim", [(1, 1, 1, 128), (2, 37, 3, 64), (1, 6, 2, 33), (2, 12, 3, 80), (1, 31, 2, 96), (3, 50, 7, 127), (2, 333, 5, 128), (4, 1000, 6, 64), (8, 1001, 5, 128)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_heads(batch, tokens, heads, dim, shift):
-    """Single elements (rows of two to four tiles, base pointers at any element): the bits of the interpreter's tile kernels. Rows of 128 at 8-byte
-    boundaries add their squares in another order, as the streaming kernels do: one bfloat16 rounding of the 64-bit value, to which sum, rsqrt and
-    products in f32 add less than 2^-18."""
+    """The bits of the interpreter: of its tile kernels, or, for rows of 128 at 8-byte boundaries, of its streaming kernel in the vector layout, which
+    adds the squares in the same order. Those are also held against the tile kernels' order: one bfloat16 rounding of the 64-bit value, to which sum,
+    rsqrt and products in f32 add less than 2^-18. Among the values: rows of zeros, huge and tiny ones, infinities and NaN."""
     ex = get_executor()
     g = torch.Generator(device="cuda").manual_seed(dim)
     count = batch * tokens * heads * dim
@@ -687,27 +704,38 @@ def test_heads(batch, tokens, heads, dim, shift):
     w = torch.rand(dim + 8, device="cuda", generator=g).bfloat16()[shift:shift + dim]
     total = batch * heads * -(-tokens // 4)
     fours = dim == 128 and shift == 0
-    for first, n in ((0, total), (total // 3, total - total // 3)):
-        got = []
-        for on in (1, 0):
-            ex.set_option("streaming", on)
-            try:
-                buffer = torch.full((count + 128,), 9.0, device="cuda").bfloat16()
-                y = buffer[64 + shift:64 + shift + count].view(batch, tokens, heads, dim).transpose(1, 2)
-                assert (ex.launch_info(heads_program, C.to_interfaces([x, y, w]), total)["form"] == HEADS) == bool(on)
-                ex.execute_range(heads_program, C.to_interfaces([x, y, w]), first, n, cuda_stream=torch.cuda.current_stream().cuda_stream)
-                got.append(buffer.cpu())
-            finally:
-                ex.set_option("streaming", 1)
-        if not fours:
-            assert bits_equal(*got), mismatch_report(*got)
-        else:
-            xd = x.double()
-            want = torch.full((count + 128,), 9.0, dtype=torch.float64, device="cuda")
-            inside = (got[1] != 9.0).cuda()
-            full = (xd * torch.rsqrt(xd.pow(2).sum(-1, keepdim=True) * 2.0 ** -7 + float(torch.tensor(1e-5).half())) * w.double()).transpose(1, 2).reshape(-1)
-            want[64:64 + count] = torch.where(inside[64:64 + count], full, want[64:64 + count])
-            torch.testing.assert_close(got[0].double(), want.cpu(), rtol=2.0 ** -8 + 2.0 ** -18, atol=0.0)
+
+    def run(first, n, **options):
+        for name, on in options.items():
+            ex.set_option(name, on)
+        try:
+            buffer = torch.full((count + 128,), 9.0, device="cuda").bfloat16()
+            y = buffer[64 + shift:64 + shift + count].view(batch, tokens, heads, dim).transpose(1, 2)
+            assert (ex.launch_info(heads_program, C.to_interfaces([x, y, w]), total)["form"] == HEADS) == (not options)
+            ex.execute_range(heads_program, C.to_interfaces([x, y, w]), first, n, cuda_stream=torch.cuda.current_stream().cuda_stream)
+            return buffer.cpu()
+        finally:
+            for name in options:
+                ex.set_option(name, 1)
+    for extreme in (False, True):
+        if extreme:
+            rows = x.reshape(-1, dim).clone()
+            for k, v in enumerate((0.0, 1e30, 1e-30, -1e-40, 3e38)):
+                rows[k::11] *= v
+            for k, v in enumerate((float("inf"), float("-inf"), float("nan"), -0.0)):
+                rows[5 + k::13, dim - 1 - k] = v
+            flat[shift:shift + count] = rows.view(batch, heads, tokens, dim).transpose(1, 2).reshape(-1)
+        for first, n in ((0, total), (total // 3, total - total // 3)):
+            got, other = run(first, n), run(first, n, forms=0) if fours else run(first, n, streaming=0)
+            assert bits_equal(got, other), mismatch_report(got, other)
+            if fours and not extreme:
+                tile = run(first, n, streaming=0)
+                xd = x.double()
+                want = torch.full((count + 128,), 9.0, dtype=torch.float64, device="cuda")
+                inside = (tile != 9.0).cuda()
+                full = (xd * torch.rsqrt(xd.pow(2).sum(-1, keepdim=True) * 2.0 ** -7 + float(torch.tensor(1e-5).half())) * w.double()).transpose(1, 2).reshape(-1)
+                want[64:64 + count] = torch.where(inside[64:64 + count], full, want[64:64 + count])
+                torch.testing.assert_close(got.double(), want.cpu(), rtol=2.0 ** -8 + 2.0 ** -18, atol=0.0)
 
 
 @pytest.mark.gpu

@@ -144,6 +144,17 @@ def test_what_is_no_loop_has_no_stream(kw):
 
 # ---------------------------------------------------------------------------------------------- on the GPU
 
+@pytest.fixture(autouse=True)
+def interpreter(request):
+    """Many of these programs have a form, whose kernel would run them (tests/test_forms.py): off here."""
+    if "gpu" not in request.keywords:
+        yield
+        return
+    get_executor().set_option("forms", 0)
+    yield
+    get_executor().set_option("forms", 1)
+
+
 def route_of(program, tensors, first, count, gathered=(), **kw):
     """The kernels that a launch of `program` on these tensors runs on (gint_debug_route)."""
     args = C.to_interfaces(tensors)
@@ -405,7 +416,7 @@ def test_launch_info_reports_the_streaming_kernel():
     m, ex = _perf_cases(), get_executor()
     x, w, out = torch.zeros(100, 2029, device="cuda"), torch.zeros(2029, device="cuda"), torch.zeros(100, 2029, device="cuda")
     info = ex.launch_info(m.rmsnorm, [x, w, out], 100)
-    assert (info["streaming"], info["pool_size"], info["tiles_per_warp"], info["warps_per_block"]) == (1, 3, 8, 1), info
+    assert (info["form"], info["streaming"], info["pool_size"], info["tiles_per_warp"], info["warps_per_block"]) == (0, 1, 3, 8, 1), info
     ex.set_option("streaming", 0)
     try:
         info = ex.launch_info(m.rmsnorm, [x, w, out], 100)
