@@ -93,7 +93,7 @@ struct RowsArgs {
     uint32_t steps;                  // STEPS_...
     uint32_t step[kRowsSteps], operand[kRowsSteps];
     uint32_t depth, stage_bytes, stationary_bytes;
-    u64 wait_ns;                     // a wait for a copy that takes longer gives up; 0: there is none
+    u64 wait_ns;                     // a wait for a copy that takes longer gives up; 0: every team gives up before its first row
     volatile uint32_t *gave_up;      // host memory: set by a team that gives up
     uint32_t fours;                  // every row of every operand starts at a 16-byte boundary; one length, a multiple of four
 };

@@ -62,19 +62,18 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes)
 }
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, u64 limit)
 {
-    uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done || limit == 0) return done;
-    u64 begin, now;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(begin));
-    do {
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
+    u64 begin = 0, now;
+    for (;;) {
+        for (int k = 0; k < 64; k++) {
+            uint32_t done;
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+            if (done) return true;
+        }
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-    } while (now - begin < limit);
-    return false;
+        if (begin == 0) begin = now;
+        else if (now - begin >= limit) return false;
+    }
 }
 /* the 16-byte groups that n floats from p on touch */
 __device__ __forceinline__ uint32_t row_bytes(u64 p, int n) { return ((uint32_t)(p & 15u) + 4u * (uint32_t)n + 15u) & ~15u; }
@@ -390,7 +389,7 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
         ask += step;
     };
     for (uint32_t d = 0; d + 1 < a.depth; d++) issue(d);
-    bool ok = bar_wait(bars, 0u, a.wait_ns);
+    bool ok = bar_wait(bars, 0u, a.wait_ns) && a.wait_ns != 0;
     uint32_t stage = 0, parity = 0;
     const int at = (team.thread & 31) + 32 * N * (team.thread >> 5);   // the thread's first element of a tile: lane + 32 * width value
     for (; now < a.count; now += step) {
@@ -451,7 +450,9 @@ template <int TEAM, class SHAPE> __device__ __forceinline__ void rows_body(const
 
 }  // namespace gint
 
-/* one warp per logical program (24 of them per block hold 80 registers each), and four */
+/* One block per SM, of up to 32 teams of one warp or eight of four (plan_rows): at most 64 registers. Without the 1 the compiler takes the bound for two blocks
+ * and 32 registers in some of them, and a small change elsewhere moves a kernel from one side to the other (RMSNorm 60 000 x 1024 140 us at
+ * 32 registers, 78 at 48 to 52). */
 #define GINT_DEFINE_ROWS_KERNELS(shape)                                                                                                          \
-    extern "C" __global__ void __launch_bounds__(1024) gint_form_rows1_##shape(const __grid_constant__ gint::RowsArgs a) { gint::rows_body<1, gint::Rows_##shape>(a); } \
-    extern "C" __global__ void __launch_bounds__(1024) gint_form_rows4_##shape(const __grid_constant__ gint::RowsArgs a) { gint::rows_body<4, gint::Rows_##shape>(a); }
+    extern "C" __global__ void __launch_bounds__(1024, 1) gint_form_rows1_##shape(const __grid_constant__ gint::RowsArgs a) { gint::rows_body<1, gint::Rows_##shape>(a); } \
+    extern "C" __global__ void __launch_bounds__(1024, 1) gint_form_rows4_##shape(const __grid_constant__ gint::RowsArgs a) { gint::rows_body<4, gint::Rows_##shape>(a); }

@@ -314,10 +314,11 @@ int gint_execute_indirect_static(gint_ctx *ctx, const uint64_t *handles, int n_p
  * benchmark programs), "streaming" (1 = launches use the streaming kernels for programs whose tile loops were found again,
  * default; results are the same bits, but for sums of f16 and bf16 2DT tiles whose rows and base pointers are aligned to 4
  * elements: their terms are added in another order), "forms" (1 = launches of programs that have a form run on its kernel,
- * default; the same bits, but for the sums just named, of rows of 128 bf16 elements; any other option away from its default, max_blocks and
+ * default; the same bits, but for the sums just named, of rows of 128 bf16 elements; rows are copied in whole groups of 16 bytes, so up to 12 bytes beside a row's first
+ * and last element are read and not used; any other option away from its default, max_blocks and
  * row_wait_ms apart, turns the forms off as well), "row_wait_ms" (0 to 60000, default 4000: the row kernels bring rows into shared memory
  * with asynchronous copies, which take microseconds, more only where a page of managed memory has to be moved first; one that takes longer
- * than this is given up, see GINT_DEVICE_GAVE_UP). */
+ * than this is given up, see GINT_DEVICE_GAVE_UP; 0: at once, for tests of that). */
 int gint_set_option(gint_ctx *ctx, const char *name, int value);
 
 #ifdef __cplusplus

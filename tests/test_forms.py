@@ -608,9 +608,9 @@ def test_rows_in_a_graph_and_on_few_blocks():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("rows,n", [(20000, 4096), (300000, 256)])
+@pytest.mark.parametrize("rows,n", [(700, 4096), (20000, 4096), (5000, 256), (300000, 256)])
 def test_a_wait_that_runs_out_is_reported(rows, n):
-    """Four warps per row and one, more rows than L2 holds: with no time to wait, teams give up. The launch ends, the rows that they leave are not
+    """Four warps per row and one: with no time to wait, teams give up while their first rows are on the way. The launch ends, no row is
     written, and every launch after it fails until the status is read, which says why."""
     ex = get_executor()
     x, w = torch.randn(rows, n, device="cuda"), torch.randn(n, device="cuda")
@@ -632,8 +632,7 @@ def test_a_wait_that_runs_out_is_reported(rows, n):
             call()
         assert e.value.status == capi.GINT_ERR_INCOMPLETE
     assert ex.launches == before and ex.device_status(clear=False)["what"] == "a wait gave up" and ex.device_status()["count"] == 1
-    left = (z == 9.0).all(1)
-    assert left.any() and bits_equal(z[~left].cpu(), want[~left].cpu())
+    assert (z == 9.0).all()
     assert ex.device_status()["code"] == 0
     rows_program(x, w, x, z, grid_dim=rows, n=n)
     assert bits_equal(z.cpu(), want.cpu()) and ex.device_status()["code"] == 0
