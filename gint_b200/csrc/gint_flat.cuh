@@ -5,7 +5,7 @@
  * with a branch per element; short launches on the tile kernels pay a block's set-up and six dependent dispatches for one tile. Here the
  * quotient is that of gint_silu.cuh and everything else is one loop over 16-byte accesses; a warp's groups of one step lie together.
  *
- * Measured (one B200, us per launch back to back, interpreter -> here): silu(x) * y of 24 000 500 f16 values 59.6 -> 27.5 (5.2 TB/s; 90
+ * Measured (one B200, us per launch back to back, interpreter -> here): silu(x) * y of 24 000 500 f16 values 59.1 -> 28.8 (5.0 TB/s; 90
  * warp instructions per 128 values, issue slots 0.58 busy), f32 57.6 -> 47.3 (6.1 TB/s); x + y in f32 of 10^6 7.7 -> 4.2, 10^7 25.0 -> 21.2,
  * 40 000 003 76.8 -> 75.6, 8 * 10^7 149.0 -> 146.5 (6.55 TB/s, the rate of a copy); f16 of 24 000 500 34.6 -> 25.8. Eight groups per
  * thread and operand in f32: four keep more warps and pages open and were slower (8 * 10^7 154); SiLU of 2-byte elements is bound by issue

@@ -2,8 +2,8 @@
  * gint_form_types.h -- launch arguments of the form kernels, shared by the kernels (gint_rows.cuh) and the host side
  * (gint_forms_host.h).
  *
- * A form is a shape of programs that has a kernel of its own: the host recognises it in the stream with loops (gint_wide_host.h)
- * and a launch hands the kernel what is particular to the program -- slots, sizes, immediates -- as arguments.
+ * A form is a shape of programs that has a kernel of its own: the host recognises it in the stream with loops (gint_wide_host.h; lane
+ * programs in the program as written, instruction for instruction) and a launch hands the kernel what is particular to the program -- slots, sizes, immediates -- as arguments.
  */
 #pragma once
 

@@ -267,7 +267,8 @@ int rows_kernel(const gint::RowsArgs &a)
 
 /*
  * Team size, teams per block and stages per team; every team has two to four stages (one computed, the others on their way), and there are no
- * more teams than rows. Measured (one B200, us per launch back to back, cold buffers, floor = bytes at 6557 GB/s):
+ * more teams than rows. Measured (one B200, us per launch back to back, cold buffers, floor = bytes at 6557 GB/s; both sides of a line at the step that drew it, those of
+ * SiLU with a residual of which L2 held a part):
  *
  * A pass that only scales is bound by memory, and memory serves it best with about 100 KB of rows per SM staged, two or three per team: more
  * rows at once are more pages read and written in turn. RMSNorm 16384 x 4096 86 with 98 KB, 91 with 197 KB (floor 82), 30 000 x 2048 78 and
@@ -282,6 +283,10 @@ int rows_kernel(const gint::RowsArgs &a)
  *
  * Sums: all the warps that have two stages. Rows of two or three tiles gain up to 32 warps (RMSNorm 600 000 x 129 335 with 16, 236 with 24,
  * 225) and up to four stages (300 000 x 256 104 with two, 98). At most two rows per SM: four warps per row (silu 100 x 1024 13, one warp 17).
+ *
+ * What is chosen measures now: RMSNorm 16384 x 4096 86, 30 000 x 2048 78, 20 000 x 3072 78, 13 000 x 6000 101, 40 000 x 1536 79, 40 000 x 1535 80, 60 000 x 1024
+ * 80, 80 000 x 900 93, 100 000 x 768 100, 300 000 x 256 97, 600 000 x 129 215; silu + residual 65536 x 1024 139 (floor 123), 12 000 x 4096 98 (90), 30 000 x 1536
+ * 92 (85), 38 000 x 1301 132, 150 000 x 300 117 (83), 100 x 1024 6.5.
  *
  * Left to the interpreter: SiLU with one team per SM (8000 x 8192 213 here, 187 there); rows of which two and the stationary ones
  * do not fit (RMSNorm of 20 000 values).

@@ -13,9 +13,9 @@
  *     go on with (10 shuffles instead of 20, one square root instead of four). The terms of every sum meet in the same order.
  *   - Rows of 128 at 8-byte boundaries have a kernel of their own, four elements per access (heads_body_fours).
  *
- * Measured (one B200, us, cold buffers, interpreter -> here): heads (8, 4096, 16, 128) 149 -> 51 (5.8 TB/s; 63 by the kernel of single
- * elements), (8, 8192, 12, 64) 164 -> 55, (2, 4096, 24, 96) 63 -> 25, (3, 777, 12, 80) 19 -> 10. Now about 240 warp instructions per logical
- * program, issue slots 0.7 busy. Two logical programs on their way: 51 with four elements per access; no gain for single
+ * Measured (one B200, us, cold buffers, interpreter -> here): heads (8, 4096, 16, 128) 145 -> 48.7 (5.5 TB/s; 63 by the kernel of single
+ * elements), (8, 8192, 12, 64) 164 -> 55, (2, 4096, 24, 96) 63 -> 25, (3, 777, 12, 80) 19 -> 10. Now 249 warp instructions per logical
+ * program, issue slots 0.72 busy. Two logical programs on their way: 51 with four elements per access; no gain for single
  * elements (55 and 57).
  */
 #pragma once

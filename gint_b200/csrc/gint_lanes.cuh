@@ -13,7 +13,7 @@
  * asynchronous copies, 16 bytes of a row at a position that keeps the lanes' 16-byte reads free of bank conflicts; results leave the same way
  * through a tile of shared memory, so that global memory sees whole lines only.
  *
- * Measured (one B200, us, interpreter -> here; bound by memory now): inverse of 4 194 304 matrices 299 -> 88 (6.1 TB/s),
+ * Measured (one B200, us, interpreter -> here; bound by memory now): inverse of 4 194 304 matrices 299 -> 89 (6.0 TB/s),
  * 1 048 576 89 -> 25, 33 24 -> 6; product of 4 194 304 174 -> 122 (6.6 TB/s, the rate of a copy), 1 048 576 54 -> 35, 33 21 -> 6.5.
  */
 #pragma once

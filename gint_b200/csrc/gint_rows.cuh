@@ -15,10 +15,10 @@
  *   - A team is one warp where enough of them have room for their stages, else four warps that take a width value each and share
  *     the row's stages (plan_rows in gint_forms_host.h has both sides).
  *
- * Measured (one B200, us per pass among others, interpreter -> here): RMSNorm 16384 x 4096 122 -> 96 (5.6 TB/s), 10007 x 2029 55 -> 33,
- * 100 000 x 700 188 -> 104, 600 000 x 129 558 -> 225, 148 x 4096 19 -> 9; silu(rmsnorm) + residual of gathered rows 65536 x 1024
- * 180 -> 139 (5.9 TB/s), 12 000 x 4095 221 -> 106; sums of 65536 rows of 1024 66 -> 59, of 12 000 rows of 4095 62 -> 45, of 150 000 rows of 300
- * 80 -> 53. Long rows are bound by memory, rows of a few tiles by issue. What mattered, on the way there: a row's fixed cost (copies by
+ * Measured (one B200, us per launch back to back, interpreter -> here): RMSNorm 16384 x 4096 113 -> 86 (6.3 TB/s), 10007 x 2029 53 -> 31,
+ * 100 000 x 700 188 -> 97, 600 000 x 129 552 -> 215, 148 x 4096 15 -> 6.4; silu(rmsnorm) + residual of gathered rows 65536 x 1024
+ * 171 -> 139 (5.8 TB/s), 12 000 x 4095 215 -> 99; sums of 65536 rows of 1024 52 -> 43.5, of 12 000 rows of 4095 49 -> 33, of 150 000 rows of 300
+ * 71 -> 49. Long rows are bound by memory, rows of a few tiles by issue. What mattered, each at its step on the way there: a row's fixed cost (copies by
  * every thread with cp.async 42 -> 37 on the 2029s, steps in a loop over a switch 50 -> 38), the quotient of SiLU (gint_silu.cuh;
  * 155 -> 137), the number of rows on their way, and how much code lies between one row and the next: the usual shapes have kernels of their
  * own (GINT_ROWS_SHAPES), the one kernel for all of them was slower on short rows (600 000 x 129 285 with it, 236; sums of 300 93, 53).
@@ -189,7 +189,7 @@ template <int TEAM, int STEPS> __device__ __forceinline__ void rows_steps(const 
         for (int w = 0; w < N; w++) s[w] = one[0];
         return;
     }
-    for (uint32_t k = rows_each<N>(a, 0u, s); k < a.n_steps; k = rows_each<N>(a, k + 1u, s)) {
+    if constexpr (STEPS == STEPS_ANY) for (uint32_t k = rows_each<N>(a, 0u, s); k < a.n_steps; k = rows_each<N>(a, k + 1u, s)) {
         const uint32_t operand = a.operand[k];
         if (a.step[k] == kRowsFold) {   // Dup, FPermW, FAdd
             float v[4];
